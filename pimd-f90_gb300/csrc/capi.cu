@@ -338,7 +338,8 @@ static int create(Engine &E, const pimd_params *p, int nrep, const int *brep) {
         (rc = dalloc(E, &kp.txdip, P * 4 * S * 3)) || (rc = dalloc(E, &kp.grdq, P * N * 27)) ||
         (rc = dalloc(E, &kp.Tdd, P * E.cap * kp.ndd * 6)) || (rc = dalloc(E, &kp.Tself, P * N * 18)) ||
         (rc = dalloc(E, &kp.pairs, P * E.cap)) || (rc = dalloc(E, &kp.npair, P)) ||
-        (rc = dalloc(E, &kp.tab, P * kp.ntab * S)) || (rc = dalloc(E, &kp.Spart, P * maxgroups * kp.nk * 3)) ||
+        (rc = dalloc(E, &kp.tab, P * kp.ntab * S)) ||
+        (E.precision == PIMD_MIXED && (rc = dalloc(E, &kp.Spart, P * maxgroups * kp.nk * 3))) ||
         (rc = dalloc(E, &kp.Sq, P * kp.nk)) || (rc = dalloc(E, &kp.Sm, P * kp.nk)) || (rc = dalloc(E, &kp.Sdip, P * kp.nk * 3)) ||
         (rc = dalloc(E, &kp.acc, P * NACC)) || (rc = dalloc(E, &kp.err, 1)) || (rc = dalloc(E, &kp.allconv, 1)) ||
         (rc = dalloc(E, &kp.dstep, 2)) || (rc = dalloc(E, &kp.fin_counter, 1)) ||
@@ -392,6 +393,7 @@ static int create(Engine &E, const pimd_params *p, int nrep, const int *brep) {
     }
     pot_init_constants(E);
     ewald_init(E);
+    if (E.precision != PIMD_MIXED && dg_init(E)) return fail(E, PIMD_ERR_NOMEM, "cudaMalloc");
     if (E.precision == PIMD_MIXED && (rc = cuda_check(E, mixed_init(E), "mixed tables"))) return rc;
     neighbors_init(E);
     if (kp.model == 3) adjoint_init(E);
@@ -632,6 +634,7 @@ int run_forces(Engine &E, int t, int check_every, double *Upott, double *virialt
     PHASE("after_qq", launch_after_qq(E));
     kp.fx_mode = 0;
     if (E.tape_on) tape_record(E, 0);
+    if (!mixed) PHASE("dd_x", launch_dg_dipoles(E));
     kp.dd_async = (mixed && dd_async_ok(E)) ? 1 : 0;
     if (E.capturing) {
         int rc = capture_dipole_loop(E, mixed);

@@ -156,6 +156,23 @@ struct KP {
     unsigned long long cond;      // CUDA-graph conditional handle of the dipole loop (0: host loop)
 };
 
+// Digit operands of the FP64 engine's reciprocal sums (ewald_dg.cu). Runs are taken in slots, the
+// longest kz extent first.
+struct DgArgs {
+    int jn, nslot, nslotp;      // |kz| rows (lmax + 1), runs, the same rounded up to whole blocks
+    int nx8, nv8, nvd8;         // 8-column tiles of X, of V and of the force pass's V
+    int ksf, nst;               // field k-steps (8 harmonics each), 16-site tiles of a bead
+    int xsteps;                 // 16-site steps the X buffer holds
+    const int4 *slot;           // (kx, ky, kzlo, nkz) of each slot
+    const int *slotk;           // first k-vector of each slot
+    const double2 *slotkv;      // (k_x, k_y) of each slot
+    void *Xd, *Zd, *Qd;         // digits in the order of the product's fragments
+    uint4 *V, *Vd;
+    int *vexp, *vdexp;          // scale exponents of V: [P][nslotp][2], [P][nslotp][3]
+    int *zexp, *xbad;           // [P] scale of Z; a table or weight that is not finite
+    double2 *exyc;              // [P][nslot][dipole sites] e^{i(kx x + ky y)} in FP64 (may be null)
+};
+
 // refresh kp.ptf from the FP64 constants (after they are set or changed)
 inline void kp_float_tables(KP &kp) {
     for (int i = 0; i < 5; i++)
@@ -254,6 +271,9 @@ struct Engine {
     int tf_wglob_d = 0;               // the same for the dipole-force mode's weights
     const int2 *d_tfkpm = nullptr;    // per (run slot, j): k-vectors of kz = +j, -j
     alignas(64) unsigned char tc_map[128];  // CUtensorMap of the FP32 tables tabf
+    DgArgs dg;                 // FP64 engine: digit operands of the reciprocal sums
+    bool dg_xall = false;      // the X buffer holds the dipole sites of every bead
+    bool dg_xdip = false;      // ... and does so for this force call's positions
     size_t cap = 0;
     std::vector<KRun> h_runs;
     std::vector<KChunk> h_chunks;
@@ -456,6 +476,12 @@ int launch_adj_dforce_tc(Engine &E);
 int launch_adj_qforce_tc(Engine &E);
 bool field_pdl_ok(const Engine &E);
 int launch_field_qd_tc(Engine &E, int s0, int s1);  // ewald_std_qd force pass on the tensor cores
+// digit-product reciprocal sums of the FP64 engine (ewald_dg.cu)
+int dg_init(Engine &E);                  // 0, or 1 when a buffer could not be allocated
+void launch_dg_tables(Engine &E);        // after the ssincos tables
+void launch_dg_dipoles(Engine &E);       // X of the dipole sites, before the dipole iterations
+void launch_dg_sfac(Engine &E, int op, int s0, int nsites, int skipconv);
+int launch_dg_field(Engine &E, int mode, int s0, int s1, int part);
 // launchers (spc.cu): q-SPC/Fw and SPC/F
 void launch_sites_spc(Engine &E);
 void launch_pair_spc(Engine &E);

@@ -12,10 +12,10 @@
 // factor changes: U0 = sum_kz e^{i kz z} W_k, U1 = sum_kz e^{i kz z} W_k kz, then
 // E += Im(e^{i(kx x+ky y)} U0) (kx, ky) + Im(e^{i(kx x+ky y)} U1) z-hat, phi += Re(...).
 //
-// Precision: the template type R is the arithmetic of the phases and per-tile / per-chunk
-// sums (double in the FP64 engine, float in the mixed engine). The e^{i n 2pi x/L} tables
-// always come from the FP64 recurrence (k.r reduced in FP64) and are stored as R; tile
-// partials and chunk partials are added in FP64.
+// The FP64 engine forms both as exact digit products on the tensor cores instead (ewald_dg.cu), and
+// shares the tables, the finishing passes and the reciprocal virial. Here the phases and the sums
+// of a tile or chunk are in FP32 (the mixed engine, where its tensor-core passes of ewald_tc.cu do
+// not apply); tile and chunk partials are added in FP64.
 #include <algorithm>
 
 #include "dipole_check.cuh"
@@ -118,19 +118,10 @@ __global__ void __launch_bounds__(128) k_ewald_tables_m(KP kp) {
     }
 }
 
-// k-vector components in the arithmetic type of the phase sums: FP64 from kinfo, FP32 from
-// the precomputed FP32 tables (no double-to-float conversion inside the mixed kernels)
+// k-vector components of the phase sums from the precomputed FP32 tables (no double-to-float
+// conversion inside the kernels)
 template <typename R>
 struct KV;
-template <>
-struct KV<double> {
-    PIMD_D static void run_xy(const KP &kp, int r, double &x, double &y) {
-        const double4_32a v = kp.kinfo[kp.runs[r].kbeg];
-        x = v.x;
-        y = v.y;
-    }
-    PIMD_D static double z(const KP &kp, int k) { return kp.kinfo[k].z; }
-};
 template <>
 struct KV<float> {
     PIMD_D static void run_xy(const KP &kp, int r, float &x, float &y) {
@@ -976,7 +967,7 @@ static void run_spass(Engine &E, int s0, int nsites, int skipconv) {
         else
             run_spass_t<OP, float>(E, s0, nsites, skipconv);
     } else {
-        run_spass_t<OP, double>(E, s0, nsites, skipconv);
+        launch_dg_sfac(E, OP, s0, nsites, skipconv);
     }
 }
 
@@ -1069,10 +1060,14 @@ static void run_field(Engine &E, int s0, int s1) {
         else
             launch_field_nt<MODE, 64, float>(E, s0, s1);
     } else {
-        if ((size_t)LZ * 128 * 16 <= 64 * 1024)
-            launch_field_nt<MODE, 128, double>(E, s0, s1);
-        else
-            launch_field_nt<MODE, 64, double>(E, s0, s1);
+        const int ns = launch_dg_field(E, MODE, s0, s1, 0);
+        k_field_finish<MODE, 128><<<dim3((s1 - s0 + 127) / 128, E.kp.P), 128, 0, E.stream>>>(E.kp, s0, s1, ns);
+        ++E.nlaunch;
+        if (MODE == F_QD) {  // the dipole half of the force pass, at the dipole sites
+            const int d0 = E.kp.fd, d1 = E.kp.ld, nd = launch_dg_field(E, MODE, d0, d1, 1);
+            k_field_finish<MODE, 128><<<dim3((d1 - d0 + 127) / 128, E.kp.P), 128, 0, E.stream>>>(E.kp, d0, d1, nd);
+            ++E.nlaunch;
+        }
     }
 }
 
@@ -1130,7 +1125,6 @@ static int sfac_tiles(Engine &E) {
 void ewald_init(Engine &E) {
     if (sfac_tiles(E) != 0) E.sf_tiled = false;  // allocation failed: untiled kernel
     tc_init(E);
-    ewald_attrs<double>();
     ewald_attrs<float>();
     // k_field_f stages [1 or 2][64 runs][LZM] complex weights: 50 KB for LZM = 49 in QD mode
 #define PIMD_FF_ATTR(MODE, LZM) cudaFuncSetAttribute(k_field_f<MODE, LZM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
@@ -1151,6 +1145,7 @@ void launch_ewald_tables(Engine &E) {
     else
         k_ewald_tables<double><<<g, 128, 0, E.stream>>>(E.kp);
     ++E.nlaunch;
+    if (E.precision != PIMD_PREC_MIXED) launch_dg_tables(E);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1182,7 +1177,7 @@ void adj_structure_factor(Engine &E, const double *dipbuf, const float4 *dipf32,
     } else if (E.precision == PIMD_PREC_MIXED) {
         run_spass_t<OP_MU, float>(E, E.kp.fd, E.kp.ld - E.kp.fd, 1);
     } else {
-        run_spass_t<OP_MU, double>(E, E.kp.fd, E.kp.ld - E.kp.fd, 1);
+        launch_dg_sfac(E, OP_MU, E.kp.fd, E.kp.ld - E.kp.fd, 1);
     }
     E.kp = keep;
 }
@@ -1258,10 +1253,9 @@ void adj_dipole_field(Engine &E, double2 *Sm_u, double *bacc, double *Dr) {
         else
             adj_field_t<64, float>(E, Dr);
     } else {
-        if ((size_t)LZ * 128 * 16 <= 64 * 1024)
-            adj_field_t<128, double>(E, Dr);
-        else
-            adj_field_t<64, double>(E, Dr);
+        const int s0 = E.kp.fd, s1 = E.kp.ld, ns = launch_dg_field(E, F_D, s0, s1, 0);
+        k_adj_fsum<<<dim3((s1 - s0 + 127) / 128, E.kp.P), 128, 0, E.stream>>>(E.kp, s0, s1, ns, Dr);
+        ++E.nlaunch;
     }
     E.kp = keep;
 }
