@@ -568,7 +568,7 @@ int run_forces(Engine &E, int t, int check_every, double *Upott, double *virialt
     if (kp.model >= 4) {  // pot_spc.f90: no induced dipoles
         PHASE("sites", launch_sites_spc(E));
         PHASE("neighbors", launch_neighbors(E));
-        PHASE("pair_qq", launch_pair_spc(E));
+        PHASE("pair_qq", launch_pair_qq(E));
         PHASE("ewald_tables", launch_ewald_tables(E));
         PHASE("ewald_pw", launch_ewald_pw(E));
         PHASE("finish", launch_finish_spc(E));

@@ -53,6 +53,13 @@ struct PairTablesF {
     float box[3], boxi[3];
 };
 
+// Q(2/3, x): the x at which the number of terms of the reference's series and continued fraction
+// changes, and 1 / (2/3 + n) (pairs.cu)
+constexpr int GQ_TERMS = 13;
+struct GqBounds {
+    double ser[GQ_TERMS + 1], fra[GQ_TERMS + 1], inv[GQ_TERMS + 1];
+};
+
 // k-space run: a maximal block of consecutive k-vectors with equal (kx, ky); kz runs over
 // [kzlo, kzlo + nkz). kbeg is the index of the first k-vector of the run.
 struct KRun {
@@ -82,6 +89,9 @@ struct KP {
     EwC ew;
     EwCf ewf;  // FP32 copy for the mixed engine
     PairTables pt;
+    GqBounds gq;     // FP64 pair kernels: Q(2/3, x)'s numbers of terms, 1 / Gamma(2/3)
+    double gq_norm;
+    int box49[3];    // high words of 0.49 box edges: |r| below needs no minimum image
     // buffers
     const double *RRt, *RRc;
     double *dRRt, *dipI, *dipE, *chg;
@@ -438,7 +448,8 @@ bool nbr_from_inputs(const Engine &E);
 // launchers (pot.cu)
 void pot_init_constants(Engine &E);
 void launch_sites(Engine &E);
-void launch_pair_qq(Engine &E);
+void launch_pair_qq(Engine &E);       // pairs.cu
+void pair_math_init(Engine &E);
 void launch_after_qq(Engine &E);
 void launch_dd_real(Engine &E);
 void launch_dd_update(Engine &E);
@@ -484,7 +495,6 @@ void launch_dg_sfac(Engine &E, int op, int s0, int nsites, int skipconv);
 int launch_dg_field(Engine &E, int mode, int s0, int s1, int part);
 // launchers (spc.cu): q-SPC/Fw and SPC/F
 void launch_sites_spc(Engine &E);
-void launch_pair_spc(Engine &E);
 void launch_finish_spc(Engine &E);
 
 }  // namespace pimd

@@ -32,7 +32,7 @@ struct TT {
 };
 
 void pot_init_constants(Engine &E) {
-    (void)E;
+    pair_math_init(E);
     nasa_upload_constants();
 }
 
@@ -266,150 +266,6 @@ __global__ void __launch_bounds__(SITES_NT) k_sites(KP kp) {
         }
     }
     block_reduce_add<14, SITES_NT>(av, kp.acc + (size_t)b * NACC);
-}
-
-// ---------------------------------------------------------------------------------------
-// ---------------------------------------------------------------------------------------
-// pot_ttm.f90:159-228: O-O van der Waals and the charge-charge real-space sum (screened
-// Coulomb with Thole smearing below 5 A) over all site pairs of each neighbour pair. Also
-// caches the dipole-dipole tensors of the induced-dipole iterations (pot_ttm.f90:311-342).
-template <int MODEL>
-__global__ void __launch_bounds__(128) k_pair_qq(KP kp) {
-    using T = TT<MODEL>;
-    const int b = blockIdx.y, N = kp.N;
-    const int np = kp.npair[b];
-    const double4_32a *pos = kp.pos + (size_t)b * kp.S;
-    double av[14];
-#pragma unroll
-    for (int i = 0; i < 14; i++) av[i] = 0.0;
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < np; p += gridDim.x * blockDim.x) {
-        const int2 ij = kp.pairs[(size_t)b * kp.cap + p];
-        const int i = ij.x, j = ij.y;
-        double4_32a si[5], sj[5], ci[5], cj[5];
-#pragma unroll
-        for (int k = 1; k <= 4; k++) {
-            si[k] = pos[(k - 1) * N + i];
-            sj[k] = pos[(k - 1) * N + j];
-            ci[k] = posc_of(kp, b)[(k - 1) * N + i];
-            cj[k] = posc_of(kp, b)[(k - 1) * N + j];
-        }
-        double Rij[3];
-        Rij[0] = min_image_rn(__dsub_rn(si[1].x, sj[1].x), kp.box[0], kp.boxi[0]);
-        Rij[1] = min_image_rn(__dsub_rn(si[1].y, sj[1].y), kp.box[1], kp.boxi[1]);
-        Rij[2] = min_image_rn(__dsub_rn(si[1].z, sj[1].z), kp.box[2], kp.boxi[2]);
-        const double dRsq = dot3_rn(Rij[0], Rij[1], Rij[2]);
-        {  // van der Waals (pot_ttm.f90:168-190)
-            const double dRij = sqrt(dRsq);
-            const double R2i = 1.0 / dRsq, R4i = R2i * R2i, R6i = R2i * R2i * R2i, R8i = R6i * R2i;
-            const double tv = kp.vdwD * exp(-kp.vdwE * dRij);
-            av[ACC_UVDW] += R6i * ((kp.vdwA * R6i + kp.vdwB * R4i) + kp.vdwC) + tv;
-            const double xr = dRij - kp.rc1;
-            const double sc = R8i * 6.0 * kp.vdwC + tv * kp.vdwE / dRij + kp.shiftA * (xr * xr) + kp.shiftB * (xr * xr * xr);
-            double d[3], Rc[3];
-            const double xyz_i[3] = {ci[1].x, ci[1].y, ci[1].z}, xyz_j[3] = {cj[1].x, cj[1].y, cj[1].z};
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                d[c] = -(sc * Rij[c]);
-                Rc[c] = min_image_rn(__dsub_rn(xyz_i[c], xyz_j[c]), kp.box[c], kp.boxi[c]);
-            }
-            double *dRi = kp.dR + 3 * ((size_t)b * kp.S + i), *dRj = kp.dR + 3 * ((size_t)b * kp.S + j);
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                atomicAdd(dRi + c, d[c]);
-                atomicAdd(dRj + c, -d[c]);
-            }
-            av[ACC_VIRIALC] += Rc[0] * d[0] + Rc[1] * d[1] + Rc[2] * d[2];
-#pragma unroll
-            for (int col = 0; col < 3; col++)
-#pragma unroll
-                for (int c = 0; c < 3; c++) av[ACC_VIRT + c + 3 * col] += d[col] * Rij[c];
-        }
-        const double Rij0[3] = {__dadd_rn(__dsub_rn(Rij[0], si[1].x), sj[1].x),
-                                __dadd_rn(__dsub_rn(Rij[1], si[1].y), sj[1].y),
-                                __dadd_rn(__dsub_rn(Rij[2], si[1].z), sj[1].z)};
-        double Fi[5][4], Fj[5][4];
-#pragma unroll
-        for (int k = 0; k < 5; k++)
-#pragma unroll
-            for (int c = 0; c < 4; c++) Fi[k][c] = Fj[k][c] = 0.0;
-        unsigned err = 0;
-#pragma unroll
-        for (int isp = 1; isp <= 4; isp++) {
-#pragma unroll
-            for (int jsp = 1; jsp <= 4; jsp++) {
-                if (!T::qq_active(isp, jsp)) continue;
-                const double Rs[3] = {
-                    min_image_rn(__dsub_rn(__dadd_rn(si[isp].x, Rij0[0]), sj[jsp].x), kp.box[0], kp.boxi[0]),
-                    min_image_rn(__dsub_rn(__dadd_rn(si[isp].y, Rij0[1]), sj[jsp].y), kp.box[1], kp.boxi[1]),
-                    min_image_rn(__dsub_rn(__dadd_rn(si[isp].z, Rij0[2]), sj[jsp].z), kp.box[2], kp.boxi[2])};
-                const double d2 = dot3_rn(Rs[0], Rs[1], Rs[2]);
-                double ts0, ts1;
-                smear01<double>(d2, kp.pt.apol_qq[isp][jsp], kp.pt.ra_qq[isp][jsp], kp.ew, &ts0, &ts1, &err);
-                const double qi = si[isp].w, qj = sj[jsp].w;
-#pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    Fi[isp][c] += ts1 * qj * Rs[c];
-                    Fj[jsp][c] -= ts1 * qi * Rs[c];
-                }
-                Fi[isp][3] += ts0 * qj;
-                Fj[jsp][3] += ts0 * qi;
-                if (T::chg(isp) && T::chg(jsp)) {
-                    double d[3];
-#pragma unroll
-                    for (int c = 0; c < 3; c++) d[c] = -ts1 * qi * qj * Rs[c];
-                    const double Rc[3] = {ci[isp].x - cj[jsp].x + Rij0[0], ci[isp].y - cj[jsp].y + Rij0[1],
-                                          ci[isp].z - cj[jsp].z + Rij0[2]};
-                    av[ACC_VIRIALC] += Rc[0] * d[0] + Rc[1] * d[1] + Rc[2] * d[2];
-#pragma unroll
-                    for (int col = 0; col < 3; col++)
-#pragma unroll
-                        for (int c = 0; c < 3; c++) av[ACC_VIRT + c + 3 * col] += d[col] * Rs[c];
-                }
-            }
-        }
-        // dipole tensors with the wrapped Rij0 of the iteration loop (pot_ttm.f90:318-319)
-        const double Rw[3] = {min_image_rn(Rij0[0], kp.box[0], kp.boxi[0]), min_image_rn(Rij0[1], kp.box[1], kp.boxi[1]),
-                              min_image_rn(Rij0[2], kp.box[2], kp.boxi[2])};
-        double *Tp = kp.Tdd + ((size_t)b * kp.cap + p) * kp.ndd * 6;
-        int t = 0;
-#pragma unroll
-        for (int isp = T::FDI; isp <= T::LDI; isp++)
-#pragma unroll
-            for (int jsp = T::FDI; jsp <= T::LDI; jsp++, t++) {
-                const double Rs[3] = {
-                    min_image_rn(__dsub_rn(__dadd_rn(si[isp].x, Rw[0]), sj[jsp].x), kp.box[0], kp.boxi[0]),
-                    min_image_rn(__dsub_rn(__dadd_rn(si[isp].y, Rw[1]), sj[jsp].y), kp.box[1], kp.boxi[1]),
-                    min_image_rn(__dsub_rn(__dadd_rn(si[isp].z, Rw[2]), sj[jsp].z), kp.box[2], kp.boxi[2])};
-                double t1, t2;
-                smear2<double>(dot3_rn(Rs[0], Rs[1], Rs[2]), kp.pt.apol_dd[isp][jsp], kp.ew, &t1, &t2);
-                const double t3 = 3.0 * t2;
-                Tp[6 * t + 0] = t3 * Rs[0] * Rs[0] - t1;
-                Tp[6 * t + 1] = t3 * Rs[1] * Rs[1] - t1;
-                Tp[6 * t + 2] = t3 * Rs[2] * Rs[2] - t1;
-                Tp[6 * t + 3] = t3 * Rs[0] * Rs[1];
-                Tp[6 * t + 4] = t3 * Rs[0] * Rs[2];
-                Tp[6 * t + 5] = t3 * Rs[1] * Rs[2];
-            }
-        if (err) atomicOr(kp.err, err);
-        double4_32a *Fb = kp.F + (size_t)b * kp.S;
-#pragma unroll
-        for (int k = 1; k <= 4; k++) {
-            const bool need_i = (MODEL == 2) ? true : (k != 1);
-            if (!need_i) continue;
-            double *fi = reinterpret_cast<double *>(Fb + (k - 1) * N + i);
-            double *fj = reinterpret_cast<double *>(Fb + (k - 1) * N + j);
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                atomicAdd(fi + c, Fi[k][c]);
-                atomicAdd(fj + c, Fj[k][c]);
-            }
-            if (k != 1) {
-                atomicAdd(fi + 3, Fi[k][3]);
-                atomicAdd(fj + 3, Fj[k][3]);
-            }
-        }
-    }
-    block_reduce_add<14, 128>(av, kp.acc + (size_t)b * NACC);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -893,11 +749,6 @@ void launch_sites(Engine &E) {
             k_sites<3, false><<<g, SITES_NT, 0, E.stream>>>(E.kp);
     }
     ++E.nlaunch;
-}
-
-void launch_pair_qq(Engine &E) {
-    dim3 g(pair_blocks(E), E.kp.P);
-    DISPATCH_TTM(E, k_pair_qq, g, 128);
 }
 
 void launch_after_qq(Engine &E) {

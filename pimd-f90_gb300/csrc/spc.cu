@@ -6,8 +6,8 @@
 //
 // Sites per bead are O(0..N-1) H1(N..2N-1) H2(2N..3N-1) with fixed charges. The neighbour
 // list and Ewald kernels are the TTM engine's (the Ewald charge sums cover all 3N sites).
-// Decomposition: one thread per (molecule, bead) for monomer/self work and the epilogue,
-// one thread per O-O pair for the real-space sums (registers, then FP64 atomics per site).
+// Decomposition: one thread per (molecule, bead) for monomer/self work and the epilogue; the
+// real-space sums are the pair kernel of pairs.cu.
 #include "engine.h"
 
 namespace pimd {
@@ -160,96 +160,6 @@ __global__ void __launch_bounds__(128) k_sites_spc(KP kp) {
     block_reduce_add<14, 128>(av, kp.acc + (size_t)b * NACC);
 }
 
-// pot_spc.f90:142-191: O-O Lennard-Jones and the 9 screened charge-charge site pairs of
-// every neighbour pair (molecule-based cutoff).
-__global__ void __launch_bounds__(128) k_pair_spc(KP kp) {
-    const int b = blockIdx.y, N = kp.N;
-    const int np = kp.npair[b];
-    const double4_32a *pos = kp.pos + (size_t)b * kp.S;
-    double4_32a *Fb = kp.F + (size_t)b * kp.S;
-    double *dRb = kp.dR + (size_t)b * kp.S * 3;
-    double av[14];
-#pragma unroll
-    for (int i = 0; i < 14; i++) av[i] = 0.0;
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < np; p += gridDim.x * blockDim.x) {
-        const int2 ij = kp.pairs[(size_t)b * kp.cap + p];
-        const int i = ij.x, j = ij.y;
-        double4_32a si[3], sj[3];
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            si[k] = pos[k * N + i];
-            sj[k] = pos[k * N + j];
-        }
-        // find_neigh.f90:76-109: the O-O separation and its square as stored in the list
-        double Rij[3];
-        Rij[0] = min_image_rn(__dsub_rn(si[0].x, sj[0].x), kp.box[0], kp.boxi[0]);
-        Rij[1] = min_image_rn(__dsub_rn(si[0].y, sj[0].y), kp.box[1], kp.boxi[1]);
-        Rij[2] = min_image_rn(__dsub_rn(si[0].z, sj[0].z), kp.box[2], kp.boxi[2]);
-        const double dRsq = dot3_rn(Rij[0], Rij[1], Rij[2]);
-        {
-            const double R2i = 1.0 / dRsq, R6i = R2i * R2i * R2i, R8i = R6i * R2i;
-            av[ACC_UVDW] += R6i * (kp.vdwA * R6i + kp.vdwC);
-            const double sc = R8i * (12.0 * kp.vdwA * R6i + 6.0 * kp.vdwC);
-            double d[3];
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                d[c] = -sc * Rij[c];
-                atomicAdd(dRb + 3 * i + c, d[c]);
-                atomicAdd(dRb + 3 * j + c, -d[c]);
-            }
-#pragma unroll
-            for (int col = 0; col < 3; col++)
-#pragma unroll
-                for (int c = 0; c < 3; c++) av[ACC_VIRT + c + 3 * col] += d[col] * Rij[c];
-        }
-        const double Rij0[3] = {Rij[0] - si[0].x + sj[0].x, Rij[1] - si[0].y + sj[0].y, Rij[2] - si[0].z + sj[0].z};
-        double Fi[3][4], Fj[3][4];
-#pragma unroll
-        for (int k = 0; k < 3; k++)
-#pragma unroll
-            for (int c = 0; c < 4; c++) Fi[k][c] = Fj[k][c] = 0.0;
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            const double Ri[3] = {si[a].x + Rij0[0], si[a].y + Rij0[1], si[a].z + Rij0[2]};
-            const double qi = si[a].w;
-#pragma unroll
-            for (int bb = 0; bb < 3; bb++) {
-                const double qj = sj[bb].w;
-                const double Rs[3] = {min_image_rn(Ri[0] - sj[bb].x, kp.box[0], kp.boxi[0]),
-                                      min_image_rn(Ri[1] - sj[bb].y, kp.box[1], kp.boxi[1]),
-                                      min_image_rn(Ri[2] - sj[bb].z, kp.box[2], kp.boxi[2])};
-                const double drsq = Rs[0] * Rs[0] + Rs[1] * Rs[1] + Rs[2] * Rs[2];
-                const double dd = sqrt(drsq);
-                const double expon = exp(-(kp.ew.a2 * drsq));
-                const double ts0 = erfc_as<double>(kp.ew.aewald * dd) / dd;
-                const double ts1 = (ts0 + kp.ew.cts1 * expon) / drsq;
-                Fi[a][3] += ts0 * qj;
-                Fj[bb][3] += ts0 * qi;
-#pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    Fi[a][c] += ts1 * qj * Rs[c];
-                    Fj[bb][c] -= ts1 * qi * Rs[c];
-                }
-#pragma unroll
-                for (int col = 0; col < 3; col++)
-#pragma unroll
-                    for (int c = 0; c < 3; c++) av[ACC_VIRT + c + 3 * col] += (-ts1 * qi * qj * Rs[col]) * Rs[c];
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            double *fi = reinterpret_cast<double *>(Fb + k * N + i);
-            double *fj = reinterpret_cast<double *>(Fb + k * N + j);
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                atomicAdd(fi + c, Fi[k][c]);
-                atomicAdd(fj + c, Fj[k][c]);
-            }
-        }
-    }
-    block_reduce_add<14, 128>(av, kp.acc + (size_t)b * NACC);
-}
-
 // pot_spc.f90:245-249, 270-275: Uelec = 1/2 sum q phi, charge forces -q Efq, and the
 // gradient in the caller's O H H atom order.
 __global__ void __launch_bounds__(128) k_finish_spc(KP kp) {
@@ -278,14 +188,6 @@ void launch_sites_spc(Engine &E) {
         k_sites_spc<4><<<g, 128, 0, E.stream>>>(E.kp);
     else
         k_sites_spc<5><<<g, 128, 0, E.stream>>>(E.kp);
-    ++E.nlaunch;
-}
-
-void launch_pair_spc(Engine &E) {
-    long nb = ((long)E.kp.N * 32 + 127) / 128;
-    nb = nb < 8 ? 8 : (nb > 4096 ? 4096 : nb);
-    dim3 g((unsigned)nb, E.kp.P);
-    k_pair_spc<<<g, 128, 0, E.stream>>>(E.kp);
     ++E.nlaunch;
 }
 
