@@ -180,7 +180,9 @@ struct DgArgs {
     uint4 *V, *Vd;
     int *vexp, *vdexp;          // scale exponents of V: [P][nslotp][2], [P][nslotp][3]
     int *zexp, *xbad;           // [P] scale of Z; a table or weight that is not finite
-    double2 *exyc;              // [P][nslot][dipole sites] e^{i(kx x + ky y)} in FP64 (may be null)
+    unsigned *fcnt;             // [P][blocks of 64 sites] slices of a dipole field pass that have arrived
+    int4 *tab;                  // [P][ntab][S] the ssincos tables in fixed point: 2^62 (cos, sin)
+    int4 *exyc;                 // [P][nslot][dipole sites] e^{i(kx x + ky y)} likewise (may be null)
 };
 
 // refresh kp.ptf from the FP64 constants (after they are set or changed)

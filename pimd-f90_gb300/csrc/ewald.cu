@@ -1061,6 +1061,7 @@ static void run_field(Engine &E, int s0, int s1) {
             launch_field_nt<MODE, 64, float>(E, s0, s1);
     } else {
         const int ns = launch_dg_field(E, MODE, s0, s1, 0);
+        if (MODE == F_D) return;  // (the update is part of the pass)
         k_field_finish<MODE, 128><<<dim3((s1 - s0 + 127) / 128, E.kp.P), 128, 0, E.stream>>>(E.kp, s0, s1, ns);
         ++E.nlaunch;
         if (MODE == F_QD) {  // the dipole half of the force pass, at the dipole sites
@@ -1253,7 +1254,7 @@ void adj_dipole_field(Engine &E, double2 *Sm_u, double *bacc, double *Dr) {
         else
             adj_field_t<64, float>(E, Dr);
     } else {
-        const int s0 = E.kp.fd, s1 = E.kp.ld, ns = launch_dg_field(E, F_D, s0, s1, 0);
+        const int s0 = E.kp.fd, s1 = E.kp.ld, ns = launch_dg_field(E, F_D, s0, s1, 1);
         k_adj_fsum<<<dim3((s1 - s0 + 127) / 128, E.kp.P), 128, 0, E.stream>>>(E.kp, s0, s1, ns, Dr);
         ++E.nlaunch;
     }

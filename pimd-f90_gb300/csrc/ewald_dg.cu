@@ -22,18 +22,22 @@
 // (weight 2^-56, resp. 2^-54): the result is nearer to the exact sum than FP64 additions in any
 // order, and it does not depend on the order of the sums.
 //
-// Measured (GB300, TTM3-F 512 x 32, |n| <= 12, before -> now): structure factor of an iteration
-// 866 -> 190 us, field 1109 -> 137 us; of the charges 2170 -> 500 us, their field 3300 -> 640 us; the
-// force pass 6800 -> 1160 us. 128 molecules, one bead: 46 -> 25 us and 111 -> 22 us an iteration.
+// Measured (GB300, TTM3-F 512 x 32, |n| <= 12; FP64 passes -> this): structure factor of an iteration
+// 866 -> 108 us (98 the product, half of it at the tensor rate, 10 forming Z), field and SOR update
+// 1109 -> 102 us; of the charges 2170 -> 260 us, their field 3300 -> 380 us; the force pass
+// 6800 -> 800 us. 128 molecules, one bead: 46 -> 22 us and 111 -> 17 us an iteration.
 //
-// The FP64 work left per (site, run) is the contraction with exy, four FMAs per T. Splitting into
-// digits and joining them are integer instructions (32 per cycle for an FP64 one's two).
+// Nearly no FP64 instruction is left: the phase tables are held in fixed point (2^62), the products
+// exy T, ex ey and w z are 64-bit integer ones (six or three 32-bit multiply-adds), digits are cut
+// and joined in integers, and a (site, run) takes two FP64 FMAs.
 #include <algorithm>
 #include <cuda_fp16.h>
 #include <type_traits>
 #include <vector>
 
+#include "dipole_check.cuh"
 #include "engine.h"
+#include "umma.cuh"
 
 namespace pimd {
 
@@ -48,9 +52,12 @@ constexpr int DG_XT = 1792, DG_ZT = 3584;  // bytes of one X (16 sites x 8 colum
 constexpr int DG_VT = 1536, DG_QT = 3072;  // the same for the field's V (8 columns) and Q (16 sites)
 constexpr int DG_BAD = 0x7fffffff;       // scale of an operand with a value that is not finite
 constexpr int DG_SW = 10;                // most warps of a structure-factor block
+constexpr int DG_SMEM = 220 * 1024;      // dynamic shared memory of a block
+constexpr int DG_FST = 4;                // tiles of the field's V ring
+constexpr int DG_ST = 3;                 // k-steps of its operand ring
 
 // ---- fixed point and digits ----------------------------------------------------------------
-// x 2^sh rounded to an integer, |x 2^sh| < 2^56, from the bits of x (an FP64 conversion costs the
+// x 2^sh rounded to an integer, |x 2^sh| < 2^63, from the bits of x (an FP64 conversion costs the
 // FP64 pipe 64 cycles a warp). A value that is not finite gives 0: the caller's scale says so.
 PIMD_D long long dg_fix(double x, int sh) {
     const unsigned long long u = (unsigned long long)__double_as_longlong(x);
@@ -115,43 +122,78 @@ PIMD_D void dg_mma(float (&d)[4], const uint4 &a, uint32_t b0, uint32_t b1) {
 }
 PIMD_D long long dg_i64(float d) { return (long long)__float2int_rn(d); }
 
-PIMD_D double2 dg_tab(const KP &kp, int b, int row, int s) { return kp.tab[((size_t)b * kp.ntab + row) * kp.S + s]; }
-PIMD_D double2 dg_exy(const KP &kp, int b, int kx, int ky, int s) {
-    const double2 ex = dg_tab(kp, b, kx, s), ey0 = dg_tab(kp, b, kp.hmax + 1 + (ky < 0 ? -ky : ky), s);
-    const double2 ey = make_double2(ey0.x, ky < 0 ? -ey0.y : ey0.y);
-    // ewald.f90:30-31: coskxky = cx cy - sx sy, sinkxky = sx cy + cx sy
-    return make_double2(ex.x * ey.x - ex.y * ey.y, ex.y * ey.x + ex.x * ey.y);
+// ---- products of fixed-point numbers -----------------------------------------------------------
+// A number in [-1, 1] as 2^62 x = hi 2^32 + lo with both halves signed, so that a product needs no
+// unsigned corrections. dg_mul: a b / 2^64 without the low halves' product (below one unit).
+PIMD_D int2 dg_split(long long v) {
+    const int lo = (int)v;
+    return make_int2((int)((v - lo) >> 32), lo);
+}
+PIMD_D long long dg_join(int2 a) { return ((long long)a.x << 32) + a.y; }
+PIMD_D long long dg_mul(int2 a, int2 b) {
+    return (long long)a.x * b.x + (((long long)a.x * b.y + (long long)a.y * b.x) >> 32);
+}
+// a1 b1 + a2 b2, a1 b1 - a2 b2 (/ 2^64)
+PIMD_D long long dg_mul2(int2 a1, int2 b1, int2 a2, int2 b2) {
+    const long long m = (long long)a1.x * b1.y + (long long)a1.y * b1.x + (long long)a2.x * b2.y + (long long)a2.y * b2.x;
+    return (long long)a1.x * b1.x + (long long)a2.x * b2.x + (m >> 32);
+}
+PIMD_D long long dg_mul2m(int2 a1, int2 b1, int2 a2, int2 b2) {
+    const long long m = (long long)a1.x * b1.y + (long long)a1.y * b1.x - (long long)a2.x * b2.y - (long long)a2.y * b2.x;
+    return (long long)a1.x * b1.x - (long long)a2.x * b2.x + (m >> 32);
+}
+// entry (cos, sin) of the fixed-point phase tables: (cos hi, lo, sin hi, lo)
+PIMD_D int4 dg_tab(const KP &kp, const DgArgs &a, int b, int row, int s) { return a.tab[((size_t)b * kp.ntab + row) * kp.S + s]; }
+PIMD_D int2 dg_re(int4 v) { return make_int2(v.x, v.y); }
+PIMD_D int2 dg_im(int4 v) { return make_int2(v.z, v.w); }
+// e^{i(kx x + ky y)} (ewald.f90:30-31: coskxky = cx cy - sx sy, sinkxky = sx cy + cx sy): one part
+PIMD_D long long dg_exy(const KP &kp, const DgArgs &a, int b, int kx, int ky, int s, int part) {
+    const int4 ex = dg_tab(kp, a, b, kx, s), ey = dg_tab(kp, a, b, kp.hmax + 1 + (ky < 0 ? -ky : ky), s);
+    const long long p = dg_mul(part ? dg_im(ex) : dg_re(ex), dg_re(ey)), r = dg_mul(part ? dg_re(ex) : dg_im(ex), dg_im(ey));
+    return ((part != 0) == (ky >= 0) ? p + r : p - r) << 2;
 }
 
 // ---- operands ------------------------------------------------------------------------------
+// The ssincos tables (ewald.f90:403-437) in fixed point, and the beads whose tables are not finite
+__global__ void __launch_bounds__(128) k_dg_tab(KP kp, DgArgs a) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
+    if (s >= kp.S) return;
+    const size_t base = (size_t)b * kp.ntab * kp.S + s;
+    bool bad = false;
+    for (int r = blockIdx.z; r < kp.ntab; r += gridDim.z) {
+        const double2 v = kp.tab[base + (size_t)r * kp.S];
+        bad |= dg_hi(v.x) >= 0x7ff00000 || dg_hi(v.y) >= 0x7ff00000;
+        const int2 c = dg_split(dg_fix(v.x, 62)), n = dg_split(dg_fix(v.y, 62));
+        a.tab[base + (size_t)r * kp.S] = make_int4(c.x, c.y, n.x, n.y);
+    }
+    if (bad) atomicOr(a.xbad + b, 1);
+}
+
 // X: one warp per tile of 4 run slots x 16 sites of a bead, every lane the fragment it holds in the
 // product (column n = lane / 4: slot n / 2, part n & 1; sites 2q, 2q + 1, 2q + 8, 2q + 9 of
-// q = lane & 3). With exyc also the FP64 values, for the field's contraction.
+// q = lane & 3). Two tiles a step, so that a block's step is one copy. With cache also the values
+// themselves, for the field's contraction.
 __global__ void __launch_bounds__(128) k_dg_x(KP kp, DgArgs a, int s0, int nsites, int nks, int b0, int cache) {
     const int u = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, xb = blockIdx.y, b = b0 + xb;
     if (u >= a.nx8 * nks) return;
     const int n8 = u / nks, ks = u - n8 * nks;
     const int n = lane >> 2, q = lane & 3, sl = 4 * n8 + (n >> 1), part = n & 1;
     long long v[4] = {0, 0, 0, 0};
-    bool bad = false;
     if (sl < a.nslot) {
         const int4 r = a.slot[sl];
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const int l = 16 * ks + 2 * q + (i & 1) + 8 * (i >> 1);
             if (l >= nsites) continue;
-            const double2 e = dg_exy(kp, b, r.x, r.y, s0 + l);
-            const double x = part ? e.y : e.x;
-            if (cache) reinterpret_cast<double *>(a.exyc)[2 * (((size_t)b * a.nslot + sl) * nsites + l) + part] = x;
-            bad |= dg_hi(x) >= 0x7ff00000;
-            v[i] = dg_fix(x, 55);
+            const long long x = dg_exy(kp, a, b, r.x, r.y, s0 + l, part);
+            if (cache) reinterpret_cast<int2 *>(a.exyc)[2 * (((size_t)b * a.nslot + sl) * nsites + l) + part] = dg_split(x);
+            v[i] = (x + 64) >> 7;
         }
     }
-    if (bad) atomicOr(a.xbad + b, 1);
     uint32_t d0[DG_SN], d1[DG_SN];
     dg_digits<DG_SB, DG_SN>(v[0], v[1], d0);
     dg_digits<DG_SB, DG_SN>(v[2], v[3], d1);
-    char *o = reinterpret_cast<char *>(a.Xd) + (((size_t)xb * a.nx8 + n8) * nks + ks) * DG_XT;
+    char *o = reinterpret_cast<char *>(a.Xd) + ((((size_t)xb * (a.nx8 / 2) + n8 / 2) * nks + ks) * 2 + (n8 & 1)) * DG_XT;
 #pragma unroll
     for (int p = 0; p < 3; p++)
         *reinterpret_cast<uint4 *>(o + 512 * p + 16 * lane) = make_uint4(d0[2 * p], d1[2 * p], d0[2 * p + 1], d1[2 * p + 1]);
@@ -177,7 +219,6 @@ __global__ void __launch_bounds__(256) k_dg_z(KP kp, DgArgs a, int s0, int nsite
     m = __reduce_max_sync(0xffffffffu, m);
     if ((threadIdx.x & 31) == 0) atomicMax(&smax, m);
     __syncthreads();
-    // a z table that is not finite has to show too: its first harmonic is looked at with the items
     const int e = dg_exp(smax);
     if (blockIdx.x == 0 && threadIdx.x == 0) a.zexp[b] = e;
     const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
@@ -192,11 +233,10 @@ __global__ void __launch_bounds__(256) k_dg_z(KP kp, DgArgs a, int s0, int nsite
                 const int l = 16 * ks + 2 * q + (i & 1) + 8 * (i >> 1);
                 if (l >= nsites) continue;
                 const size_t gs = (size_t)b * kp.S + s0 + l;
-                const double w = NC == 1 ? kp.pos[gs].w : kp.dip[3 * gs + c];
-                const double2 z = dg_tab(kp, b, kp.hmax + 1 + kp.kmax + 1 + j, s0 + l);
-                if (dg_hi(z.x) >= 0x7ff00000 || dg_hi(z.y) >= 0x7ff00000) atomicOr(a.xbad + b, 1);
-                vc[i] = dg_fix(w * z.x, 55 - e);
-                vs[i] = dg_fix(w * z.y, 55 - e);
+                const int2 w = dg_split(dg_fix(NC == 1 ? kp.pos[gs].w : kp.dip[3 * gs + c], 61 - e));
+                const int4 z = dg_tab(kp, a, b, kp.hmax + 1 + kp.kmax + 1 + j, s0 + l);
+                vc[i] = (dg_mul(w, dg_re(z)) + 8) >> 4;  // 2^(59 - e) w z -> 2^(55 - e)
+                vs[i] = (dg_mul(w, dg_im(z)) + 8) >> 4;
             }
         }
         uint32_t c0[DG_SN], c1[DG_SN], n0[DG_SN], n1[DG_SN];
@@ -204,7 +244,7 @@ __global__ void __launch_bounds__(256) k_dg_z(KP kp, DgArgs a, int s0, int nsite
         dg_digits<DG_SB, DG_SN>(vc[2], vc[3], c1);
         dg_digits<DG_SB, DG_SN>(vs[0], vs[1], n0);
         dg_digits<DG_SB, DG_SN>(vs[2], vs[3], n1);
-        uint4 *o = reinterpret_cast<uint4 *>(reinterpret_cast<char *>(a.Zd) + (((size_t)b * nmt + mt) * nks + ks) * DG_ZT);
+        uint4 *o = reinterpret_cast<uint4 *>(reinterpret_cast<char *>(a.Zd) + (((size_t)b * nks + ks) * nmt + mt) * DG_ZT);
 #pragma unroll
         for (int s = 0; s < DG_SN; s++) o[32 * s + lane] = make_uint4(c0[s], n0[s], c1[s], n1[s]);
     }
@@ -219,9 +259,9 @@ __global__ void __launch_bounds__(128) k_dg_q(KP kp, DgArgs a) {
 #pragma unroll
     for (int i = 0; i < 4; i++) {  // (site g, j), (site g + 8, j), (site g, j + 4), (site g + 8, j + 4)
         const int s = 16 * mt + g + 8 * (i & 1), j = 8 * ks + q + 4 * (i >> 1);
-        double2 z = make_double2(0.0, 0.0);
-        if (s < kp.S && j < a.jn) z = dg_tab(kp, b, kp.hmax + 1 + kp.kmax + 1 + j, s);
-        dg_digits<DG_FB, DG_FN>(dg_fix(z.x, 53), dg_fix(z.y, 53), d[i]);
+        int4 z = make_int4(0, 0, 0, 0);
+        if (s < kp.S && j < a.jn) z = dg_tab(kp, a, b, kp.hmax + 1 + kp.kmax + 1 + j, s);
+        dg_digits<DG_FB, DG_FN>((dg_join(dg_re(z)) + 256) >> 9, (dg_join(dg_im(z)) + 256) >> 9, d[i]);
     }
     uint4 *o = reinterpret_cast<uint4 *>(reinterpret_cast<char *>(a.Qd) + (((size_t)b * a.nst + mt) * a.ksf + ks) * DG_QT);
 #pragma unroll
@@ -292,76 +332,124 @@ PIMD_D void dg_build_v(const KP &kp, const DgArgs &a, int b, int slot0, int nsl,
 // ---- structure factor ------------------------------------------------------------------------
 // Block: 8 run slots of a bead, one warp per tile of 8 items (all sites), so nothing is summed
 // across blocks. The slots are sorted by kz extent, and tiles beyond the block's longest run are
-// not formed. The epilogue forms S of the slots' k-vectors and (OP_Q, OP_MU) the field's V.
+// not formed. The operands come through a ring of DG_ST k-steps in shared memory, two bulk copies a
+// step by one thread (loads straight to registers left the warps waiting on L2: 181 us an iteration
+// at 512 x 32; copies of 16 bytes a thread cost more instructions than the products: 193 us). The
+// epilogue forms S of the slots' k-vectors and (OP_Q, OP_MU) the field's V.
+PIMD_D void dg_cp16(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+PIMD_D void dg_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+PIMD_D void dg_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+// size bytes (a multiple of 16, both addresses 16-byte aligned) counted on bar
+PIMD_D void dg_bulk(void *dst, const void *src, uint32_t size, uint64_t *bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(umma::smem_u32(dst)),
+                 "l"(src), "r"(size), "r"(umma::smem_u32(bar))
+                 : "memory");
+}
+PIMD_D void dg_expect(uint64_t *bar, uint32_t size) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(umma::smem_u32(bar)), "r"(size) : "memory");
+}
+constexpr long long DG_WAIT = 1LL << 28;  // cycles (about 0.13 s) after which a wait gives up
+
 template <int OP>
-__global__ void __launch_bounds__(32 * DG_SW) k_dg_sfac(KP kp, DgArgs a, int nks, int nmt, int ksum, int b0, int skipconv) {
+__global__ void __launch_bounds__(32 * DG_SW) k_dg_sfac(KP kp, DgArgs a, int nks, int nmt, int ksum, int b0, int skipconv, int soff) {
     constexpr int NC = OP == OP_Q ? 1 : 3;
     const int xb = blockIdx.y, b = b0 + xb;
     if (skipconv && bead_converged(kp, b)) return;
     const int slot0 = blockIdx.x * DG_SLOTS, nsl = min(DG_SLOTS, a.nslot - slot0);
-    const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int LZ = 2 * kp.lmax + 1, nitem = NC * a.jn;
-    extern __shared__ double dsm[];
-    double2 *sb = reinterpret_cast<double2 *>(dsm);      // [8][nitem][2]: S_c(+j), S_c(-j)
+    extern __shared__ __align__(128) double dsm[];
+    char *ring = reinterpret_cast<char *>(dsm);          // [DG_ST][nw Z tiles, 2 X tiles]
+    const int stage = nw * DG_ZT + 2 * DG_XT;
+    // the epilogue's scratch: over the ring where the block makes one round of the tiles
+    double2 *sb = reinterpret_cast<double2 *>(ring + soff);  // [8][nitem][2]: S_c(+j), S_c(-j)
     double2 *w = sb + (size_t)DG_SLOTS * nitem * 2;      // [8][LZ]
     double *pm = reinterpret_cast<double *>(w + (size_t)DG_SLOTS * LZ);  // [8][jn][4]
+    __shared__ uint64_t full[DG_ST];
     __shared__ int vmax[DG_SLOTS * 2];
     const int4 first = a.slot[slot0];
     const int mts = min(nmt, (NC * (first.z + first.w) + 7) / 8);  // kzlo + nkz = longest |kz| + 1
     const int ze = a.zexp[b];
     const bool bad = ze == DG_BAD || a.xbad[b];
-    for (int mt = threadIdx.x >> 5; mt < mts; mt += blockDim.x >> 5) {
+    const char *Zb = reinterpret_cast<const char *>(a.Zd) + (size_t)b * nmt * nks * DG_ZT;
+    const char *X = reinterpret_cast<const char *>(a.Xd) + ((size_t)xb * (a.nx8 / 2) + blockIdx.x) * nks * (2 * DG_XT);
+    if (threadIdx.x < DG_ST) umma::mbar_init(&full[threadIdx.x], 1);
+    __syncthreads();
+    int it = 0, late = 0;  // steps taken (over all rounds), waits that gave up
+    for (int m0 = 0; m0 < mts; m0 += nw) {
+        const int nm = min(nw, mts - m0);
+        auto load = [&](int ks, int at) {  // (thread 0) step ks into the ring place of step number at
+            char *dst = ring + (at % DG_ST) * stage;
+            uint64_t *bar = &full[at % DG_ST];
+            dg_expect(bar, nm * DG_ZT + 2 * DG_XT);
+            dg_bulk(dst, Zb + ((size_t)ks * nmt + m0) * DG_ZT, nm * DG_ZT, bar);
+            dg_bulk(dst + nw * DG_ZT, X + (size_t)ks * (2 * DG_XT), 2 * DG_XT, bar);
+        };
+        if (m0 > 0) __syncthreads();
+        if (threadIdx.x == 0)
+            for (int k = 0; k < min(DG_ST - 1, nks); k++) load(k, it + k);
+        const int mt = m0 + wp;
         long long t[2][4];
+        float d[2][DG_SN][4];
 #pragma unroll
-        for (int i = 0; i < 8; i++) t[i >> 2][i & 3] = 0;
-        const uint4 *Z = reinterpret_cast<const uint4 *>(reinterpret_cast<const char *>(a.Zd) + ((size_t)b * nmt + mt) * nks * DG_ZT);
-        const char *X = reinterpret_cast<const char *>(a.Xd) + ((size_t)xb * a.nx8 + 2 * blockIdx.x) * nks * DG_XT;
-        for (int k0 = 0; k0 < nks; k0 += DG_DRAIN) {
-            float d[2][DG_SN][4];
+        for (int n = 0; n < 2; n++)
 #pragma unroll
-            for (int n = 0; n < 2; n++)
+            for (int i = 0; i < 4; i++) {
+                t[n][i] = 0;
 #pragma unroll
-                for (int s = 0; s < DG_SN; s++)
+                for (int s = 0; s < DG_SN; s++) d[n][s][i] = 0.f;
+            }
+        for (int ks = 0; ks < nks; ks++, it++) {
+            __syncthreads();  // every warp is done with the step before, whose place the next copy takes
+            if (threadIdx.x == 0 && ks + DG_ST - 1 < nks) load(ks + DG_ST - 1, it + DG_ST - 1);
+            late |= umma::mbar_wait(&full[it % DG_ST], (uint32_t)((it / DG_ST) & 1), DG_WAIT);
+            if (wp >= nm) continue;
+            const char *st = ring + (it % DG_ST) * stage;
+            uint32_t B[2][DG_SN][2];
 #pragma unroll
-                    for (int i = 0; i < 4; i++) d[n][s][i] = 0.f;
-            const int k1 = min(nks, k0 + DG_DRAIN);
-            for (int ks = k0; ks < k1; ks++) {
-                uint4 A[DG_SN];
+            for (int n = 0; n < 2; n++) {
+                const char *x = st + nw * DG_ZT + n * DG_XT;
 #pragma unroll
-                for (int s = 0; s < DG_SN; s++) A[s] = __ldg(Z + (size_t)ks * (DG_ZT / 16) + 32 * s + lane);
-                uint32_t B[2][DG_SN][2];
-#pragma unroll
-                for (int n = 0; n < 2; n++) {
-                    const char *x = X + ((size_t)n * nks + ks) * DG_XT;
-#pragma unroll
-                    for (int p = 0; p < 3; p++) {
-                        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(x + 512 * p) + lane);
-                        B[n][2 * p][0] = v.x;
-                        B[n][2 * p][1] = v.y;
-                        B[n][2 * p + 1][0] = v.z;
-                        B[n][2 * p + 1][1] = v.w;
-                    }
-                    const uint2 v = __ldg(reinterpret_cast<const uint2 *>(x + 1536) + lane);
-                    B[n][6][0] = v.x;
-                    B[n][6][1] = v.y;
+                for (int p = 0; p < 3; p++) {
+                    const uint4 v = reinterpret_cast<const uint4 *>(x + 512 * p)[lane];
+                    B[n][2 * p][0] = v.x;
+                    B[n][2 * p][1] = v.y;
+                    B[n][2 * p + 1][0] = v.z;
+                    B[n][2 * p + 1][1] = v.w;
                 }
-#pragma unroll
-                for (int i = 0; i < DG_SN; i++)
-#pragma unroll
-                    for (int j = 0; j < DG_SN - i; j++)
-#pragma unroll
-                        for (int n = 0; n < 2; n++) dg_mma(d[n][i + j], A[i], B[n][j][0], B[n][j][1]);
+                const uint2 v = reinterpret_cast<const uint2 *>(x + 1536)[lane];
+                B[n][6][0] = v.x;
+                B[n][6][1] = v.y;
             }
 #pragma unroll
-            for (int n = 0; n < 2; n++)
+            for (int i = 0; i < DG_SN; i++) {
+                const uint4 A = reinterpret_cast<const uint4 *>(st + wp * DG_ZT)[32 * i + lane];
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    // sum_d D_d 2^(40 - 8 d): z x = t 2^(ze - 54)
-                    const long long hi = (dg_i64(d[n][0][i]) << 16) + (dg_i64(d[n][1][i]) << 8) + dg_i64(d[n][2][i]);
-                    const long long lo = (dg_i64(d[n][3][i]) << 16) + (dg_i64(d[n][4][i]) << 8) + dg_i64(d[n][5][i]);
-                    t[n][i] += ((hi << 24) + lo + (dg_i64(d[n][6][i]) >> 8)) >> ksum;
-                }
+                for (int j = 0; j < DG_SN - i; j++)
+#pragma unroll
+                    for (int n = 0; n < 2; n++) dg_mma(d[n][i + j], A, B[n][j][0], B[n][j][1]);
+            }
+            if (ks % DG_DRAIN == DG_DRAIN - 1 || ks == nks - 1) {
+#pragma unroll
+                for (int n = 0; n < 2; n++)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        // sum_d D_d 2^(40 - 8 d): z x = t 2^(ze - 54)
+                        const long long hi = (dg_i64(d[n][0][i]) << 16) + (dg_i64(d[n][1][i]) << 8) + dg_i64(d[n][2][i]);
+                        const long long lo = (dg_i64(d[n][3][i]) << 16) + (dg_i64(d[n][4][i]) << 8) + dg_i64(d[n][5][i]);
+                        t[n][i] += ((hi << 24) + lo + (dg_i64(d[n][6][i]) >> 8)) >> ksum;
+#pragma unroll
+                        for (int s = 0; s < DG_SN; s++) d[n][s][i] = 0.f;
+                    }
+            }
         }
+        if (soff == 0) __syncthreads();
+        if (wp >= nm) continue;
         // e^{ik.r} = exy (cos +- i sin): S(+j) = (cc - ss) + i (sc' + cs'), S(-j) with the signs of sin turned
         const int item = 8 * mt + g;
         if (item < nitem) {
@@ -374,6 +462,7 @@ __global__ void __launch_bounds__(32 * DG_SW) k_dg_sfac(KP kp, DgArgs a, int nks
             }
         }
     }
+    if (late) atomicOr(kp.err, 8u);
     for (int i = threadIdx.x; i < DG_SLOTS * LZ; i += blockDim.x) w[i] = make_double2(0.0, 0.0);
     __syncthreads();
     const double nan = __longlong_as_double(0x7ff8000000000000LL);
@@ -434,22 +523,40 @@ __global__ void __launch_bounds__(128) k_dg_vqd(KP kp, DgArgs a) {
 //   DGF_E : dipole field (E);  DGF_Q: charge field and potential;  DGF_QG: force on the charges
 //   (-q E) and the dipoles' potential;  DGF_DG: force on the dipoles,
 //   G_a = -sum_k k_a (k.mu) Re(e W) from T0, T1, T2
-// Warp: 16 sites x the tiles of a slice, block: 4 warps on the same tiles (they share V in L1).
-// Each slice's sums go to Fpart, which k_field_finish adds in order.
+// Warp: 16 sites x the tiles of a slice, block: 4 warps on the same tiles, which come through a ring
+// in shared memory (cp.async). Each slice's sums go to Fpart. sor (DGF_E): the last slice of a block
+// of 64 sites to arrive adds the slices, in order, and runs the sites' SOR update and block end
+// (dipole_check.cuh), so that an iteration needs no finishing launch; else k_field_finish adds them.
 enum { DGF_E = 0, DGF_Q = 1, DGF_QG = 2, DGF_DG = 3 };
 template <int MODE, int KS, bool XC>
-__global__ void __launch_bounds__(128) k_dg_field(KP kp, DgArgs a, int s0, int s1, int tshift) {
+__global__ void __launch_bounds__(128, 4) k_dg_field(KP kp, DgArgs a, int s0, int s1, int tshift, int sor) {
     const int b = blockIdx.y;
-    if (MODE == DGF_E && bead_converged(kp, b)) return;
+    if (MODE == DGF_E && bead_converged(kp, b)) {
+        // (the block still counts towards the convergence test, once for its sites)
+        const double zero[2] = {0.0, 0.0};
+        if (sor && blockIdx.z == 0) dd_block_end<128>(kp, b, zero, false, gridDim.x * gridDim.y);
+        return;
+    }
     constexpr bool DG = MODE == DGF_DG;
+    extern __shared__ uint4 fring[];  // [DG_FST][ksf][96]
     const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
     const int mt = (s0 >> 4) + blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (16 * mt >= s1) return;
+    const bool work = 16 * mt < s1;
     const int nv8 = DG ? a.nvd8 : a.nv8;
     const int n0 = (int)((long)blockIdx.z * nv8 / gridDim.z), n1 = (int)((long)(blockIdx.z + 1) * nv8 / gridDim.z);
-    const uint4 *Q = reinterpret_cast<const uint4 *>(reinterpret_cast<const char *>(a.Qd) + ((size_t)b * a.nst + mt) * a.ksf * DG_QT) + lane;
-    const uint4 *V = (DG ? a.Vd : a.V) + ((size_t)b * nv8) * a.ksf * (DG_VT / 16) + lane;
+    const uint4 *Q = reinterpret_cast<const uint4 *>(reinterpret_cast<const char *>(a.Qd) + ((size_t)b * a.nst + (work ? mt : 0)) * a.ksf * DG_QT) + lane;
+    const int tile = a.ksf * (DG_VT / 16);
+    const uint4 *V = (DG ? a.Vd : a.V) + (size_t)b * nv8 * tile;
     const int *vexp = (DG ? a.vdexp : a.vexp) + (size_t)b * a.nslotp * (DG ? 3 : 2);
+    auto load = [&](int n8) {
+        uint4 *dst = fring + (n8 % DG_FST) * tile;
+        for (int i = threadIdx.x; i < tile; i += 128) dg_cp16(dst + i, V + (size_t)n8 * tile + i);
+    };
+#pragma unroll
+    for (int k = 0; k < DG_FST - 1; k++) {
+        if (n0 + k < n1) load(n0 + k);
+        dg_commit();
+    }
     uint4 A[KS > 0 ? KS : 1][DG_FN];
     if (KS > 0) {
 #pragma unroll
@@ -463,22 +570,36 @@ __global__ void __launch_bounds__(128) k_dg_field(KP kp, DgArgs a, int s0, int s
     const double kzu = TWOPI * kp.boxi[2];  // the k-vector's z component is kzu kz
     const double nan = __longlong_as_double(0x7ff8000000000000LL);
     double acc[2][3] = {{0, 0, 0}, {0, 0, 0}};
-    for (int n8 = n0; n8 < n1; n8++) {
-        // (slots past the last run and DG's fourth pair have zero digits: they add zeros)
-        const int slc = min(DG ? n8 : 2 * n8 + (q >> 1), a.nslot - 1);
-        double2 x[2];
-        if (XC) {
+    // (slots past the last run and DG's fourth pair have zero digits: they add zeros)
+    auto slot_of = [&](int n8) { return min(DG ? n8 : 2 * n8 + (q >> 1), a.nslot - 1); };
+    const int4 *xc = XC ? a.exyc + (size_t)b * a.nslot * (s1 - s0) : nullptr;
+    int4 xn[2];
+    if (XC) {
 #pragma unroll
-            for (int h = 0; h < 2; h++)
-                x[h] = a.exyc[((size_t)b * a.nslot + slc) * (s1 - s0) + (in[h] ? site[h] - s0 : 0)];
+        for (int h = 0; h < 2; h++) xn[h] = xc[(size_t)slot_of(n0) * (s1 - s0) + (in[h] ? site[h] - s0 : 0)];
+    }
+    for (int n8 = n0; n8 < n1; n8++) {
+        const int slc = slot_of(n8);
+        int4 x[2];
+        if (XC) {  // exy of the next tile while this one is worked on
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                x[h] = xn[h];
+                xn[h] = xc[(size_t)slot_of(min(n8 + 1, n1 - 1)) * (s1 - s0) + (in[h] ? site[h] - s0 : 0)];
+            }
         }
+        dg_wait<DG_FST - 2>();
+        __syncthreads();
+        if (n8 + DG_FST - 1 < n1) load(n8 + DG_FST - 1);
+        dg_commit();
+        if (!work) continue;
         long long t[4] = {0, 0, 0, 0};
-        const uint4 *v = V + (size_t)n8 * a.ksf * (DG_VT / 16);
+        const uint4 *v = fring + (n8 % DG_FST) * tile + lane;
         auto step = [&](const uint4 (&Ak)[DG_FN], int ks, float (&d)[DG_FN][4]) {
             uint32_t B[DG_FN][2];
 #pragma unroll
             for (int p = 0; p < 3; p++) {
-                const uint4 u = __ldg(v + (size_t)ks * (DG_VT / 16) + 32 * p);
+                const uint4 u = v[ks * (DG_VT / 16) + 32 * p];
                 B[2 * p][0] = u.x;
                 B[2 * p][1] = u.y;
                 B[2 * p + 1][0] = u.z;
@@ -535,20 +656,20 @@ __global__ void __launch_bounds__(128) k_dg_field(KP kp, DgArgs a, int s0, int s
         for (int h = 0; h < 2; h++) {
             if (!XC) {
                 const int4 r = a.slot[slc];
-                x[h] = dg_exy(kp, b, r.x, r.y, in[h] ? site[h] : s0);
+                const int sx = in[h] ? site[h] : s0;
+                const int2 xr = dg_split(dg_exy(kp, a, b, r.x, r.y, sx, 0)), xi = dg_split(dg_exy(kp, a, b, r.x, r.y, sx, 1));
+                x[h] = make_int4(xr.x, xr.y, xi.x, xi.y);
             }
-            double re = dg_double(t[2 * h], e - 56 + tshift), im = dg_double(t[2 * h + 1], e - 56 + tshift);
-            if (e == DG_BAD) re = im = nan;
-            const double zi = x[h].y * re + x[h].x * im;
-            if (MODE == DGF_E) {
-                acc[h][0] = fma(cf[0], zi, acc[h][0]);
-                acc[h][1] = fma(cf[1], zi, acc[h][1]);
-            } else {
-                const double zr = x[h].x * re - x[h].y * im;
-                acc[h][0] = fma(cf[0], DG ? zr : zi, acc[h][0]);
-                acc[h][1] = fma(cf[1], DG ? zr : zi, acc[h][1]);
-                acc[h][2] = fma(cf[2], zr, acc[h][2]);
-            }
+            // Im, Re of exy T in fixed point (62 bits of exy: t 2^(e - 56) -> 2^(e - 54))
+            const int2 re = dg_split(t[2 * h]), im = dg_split(t[2 * h + 1]);
+            const int ez = (e == DG_BAD ? 0 : e) - 54 + tshift;
+            double zi = 0.0, zr = 0.0;
+            if (!DG) zi = dg_double(dg_mul2(dg_im(x[h]), re, dg_re(x[h]), im), ez);
+            if (MODE != DGF_E) zr = dg_double(dg_mul2m(dg_re(x[h]), re, dg_im(x[h]), im), ez);
+            if (e == DG_BAD) zi = zr = nan;
+            acc[h][0] = fma(cf[0], DG ? zr : zi, acc[h][0]);
+            acc[h][1] = fma(cf[1], DG ? zr : zi, acc[h][1]);
+            if (MODE != DGF_E) acc[h][2] = fma(cf[2], zr, acc[h][2]);
         }
     }
     // lanes q of a row: T0 in q = 0, 2 and T1 in 1, 3 (DG: T0, T1, T2 in 0, 1, 2)
@@ -578,6 +699,40 @@ __global__ void __launch_bounds__(128) k_dg_field(KP kp, DgArgs a, int s0, int s
         }
         kp.Fpart[((size_t)blockIdx.z * kp.P + b) * (s1 - s0) + (site[h] - s0)] = make_double4_32a(o[0], o[1], o[2], o[3]);
     }
+    if (MODE != DGF_E || !sor) return;
+    __shared__ int last;
+    __threadfence();  // this thread's sums are visible before the block counts
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned *c = a.fcnt + (size_t)b * gridDim.x + blockIdx.x;
+        last = atomicAdd(c, 1u) == gridDim.z - 1;
+        if (last) *c = 0u;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    // pot_ttm.f90:371-381 for the block's 64 sites, a component a thread
+    const int iter = kp.dstep[1] + 1;
+    double av[2] = {0.0, 0.0};
+    for (int i = threadIdx.x; i < 192; i += 128) {
+        const int s = 16 * ((s0 >> 4) + (int)blockIdx.x * 4) + i / 3, c = i % 3;
+        if (s < s0 || s >= s1) continue;
+        const size_t gc = 3 * ((size_t)b * kp.S + s) + c;
+        const double mu = kp.dip[gc], efdr = kp.Efdr[gc];
+        const double efq = reinterpret_cast<const double *>(kp.F + (size_t)b * kp.S + s)[c];
+        const double pol = kp.polar_sor * kp.polar[s / kp.N + 1];
+        const double *f = reinterpret_cast<const double *>(kp.Fpart + (size_t)b * (s1 - s0) + (s - s0)) + c;
+        double e = 0.0;
+        for (int z = 0; z < (int)gridDim.z; z++) e += __ldcg(f + (size_t)z * kp.P * (s1 - s0) * 4);
+        const double efd = (efdr + e) + efq + kp.factor * mu;
+        const double mn = (1.0 - kp.polar_sor) * mu + pol * efd;
+        const double dd = (iter == 1) ? mn : mn - mu;
+        av[0] += dd * dd;
+        av[1] += mn * efq;
+        kp.dip[gc] = mn;
+        kp.Efdr[gc] = 0.0;
+    }
+    dd_block_end<128>(kp, b, av, true, gridDim.x * gridDim.y);
 }
 
 // ---- host --------------------------------------------------------------------------------------
@@ -636,6 +791,7 @@ int dg_init(Engine &E) {
         cut(d_slotkv, sizeof(double2) * a.nslot);
         cut(a.zexp, P * sizeof(int));
         cut(a.xbad, P * sizeof(int));
+        cut(a.fcnt, P * (size_t)(a.nst / 4 + 2) * sizeof(unsigned));
         cut(a.vexp, P * a.nslotp * 2 * sizeof(int));
         cut(a.vdexp, P * a.nslotp * 3 * sizeof(int));
         cut(a.Xd, (size_t)a.xsteps * per_step);
@@ -643,7 +799,8 @@ int dg_init(Engine &E) {
         cut(a.Qd, P * a.nst * a.ksf * (size_t)DG_QT);
         cut(a.V, P * a.nv8 * a.ksf * (size_t)DG_VT);
         if (nd) cut(a.Vd, P * a.nvd8 * a.ksf * (size_t)DG_VT);
-        if (nd && E.dg_xall) cut(a.exyc, P * a.nslot * (size_t)nd * sizeof(double2));
+        if (nd && E.dg_xall) cut(a.exyc, P * a.nslot * (size_t)nd * sizeof(int4));
+        cut(a.tab, P * (size_t)kp.ntab * kp.S * sizeof(int4));
         if (pass == 0) {
             if (cudaMalloc((void **)&base, used) != cudaSuccess) return 1;
             E.allocs.push_back(base);
@@ -658,7 +815,16 @@ int dg_init(Engine &E) {
     a.slotkv = d_slotkv;
     cudaMemset(a.zexp, 0, P * sizeof(int));
     cudaMemset(a.xbad, 0, P * sizeof(int));
-    const int lim = 200 * 1024;
+    cudaMemset(a.fcnt, 0, P * (size_t)(a.nst / 4 + 2) * sizeof(unsigned));
+    const int lim = DG_SMEM;
+    if ((size_t)DG_FST * a.ksf * DG_VT > 48 * 1024) {  // |kz| > 63: the field's V ring
+        cudaFuncSetAttribute(k_dg_field<DGF_E, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+        cudaFuncSetAttribute(k_dg_field<DGF_E, 0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+        cudaFuncSetAttribute(k_dg_field<DGF_DG, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+        cudaFuncSetAttribute(k_dg_field<DGF_DG, 0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+        cudaFuncSetAttribute(k_dg_field<DGF_Q, 0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+        cudaFuncSetAttribute(k_dg_field<DGF_QG, 0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+    }
     cudaFuncSetAttribute(k_dg_sfac<OP_Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
     cudaFuncSetAttribute(k_dg_sfac<OP_MU>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
     cudaFuncSetAttribute(k_dg_sfac<OP_DIP>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
@@ -676,6 +842,10 @@ static void launch_x(Engine &E, int s0, int nsites, int b0, int nb, bool cache) 
 void launch_dg_tables(Engine &E) {
     E.dg_xdip = false;
     cudaMemsetAsync(E.dg.xbad, 0, sizeof(int) * E.kp.P, E.stream);
+    const int sb = ceil_div(E.kp.S, 128);
+    const int rows = std::max(1, std::min(E.kp.ntab, (int)(608L / std::max(1L, (long)sb * E.kp.P))));
+    k_dg_tab<<<dim3(sb, E.kp.P, rows), 128, 0, E.stream>>>(E.kp, E.dg);
+    ++E.nlaunch;
     k_dg_q<<<dim3(ceil_div(E.dg.nst * E.dg.ksf, 4), E.kp.P), 128, 0, E.stream>>>(E.kp, E.dg);
     ++E.nlaunch;
 }
@@ -701,8 +871,14 @@ static void sfac(Engine &E, int s0, int nsites, int skipconv) {
     // keep the 64-bit sums of all sites below 2^61
     int ksum = 0;
     while (((long)nks * 16 >> ksum) > 128) ksum++;
-    const int nw = std::min(std::max(nmt, 4), DG_SW);
-    const size_t smem = sizeof(double2) * ((size_t)DG_SLOTS * NC * a.jn * 2 + (size_t)DG_SLOTS * (2 * kp.lmax + 1) + (size_t)DG_SLOTS * a.jn * 2);
+    // one warp a tile, at least 4 for the epilogue; with large |kz| fewer, to leave room for the
+    // epilogue's scratch, which shares the ring's place where one round of tiles is enough
+    const size_t scratch = sizeof(double2) * ((size_t)DG_SLOTS * NC * a.jn * 2 + (size_t)DG_SLOTS * (2 * kp.lmax + 1) + (size_t)DG_SLOTS * a.jn * 2);
+    int nw = std::min(std::max(nmt, 4), DG_SW);
+    auto ring = [&](int n) { return (size_t)DG_ST * (n * DG_ZT + 2 * DG_XT); };
+    while (nw > 1 && nw < nmt && scratch + ring(nw) > (size_t)DG_SMEM) nw--;
+    const int soff = nw >= nmt ? 0 : (int)ring(nw);
+    const size_t smem = soff ? scratch + ring(nw) : std::max(scratch, ring(nw));
     const bool have = OP != OP_Q && E.dg_xdip;
     const int nbmax = have ? kp.P : std::max(1, a.xsteps / nks);
     for (int b0 = 0; b0 < kp.P; b0 += nbmax) {
@@ -711,7 +887,7 @@ static void sfac(Engine &E, int s0, int nsites, int skipconv) {
             launch_x(E, s0, nsites, b0, nb, false);
             E.dg_xdip = false;
         }
-        k_dg_sfac<OP><<<dim3(a.nslotp / DG_SLOTS, nb), 32 * nw, smem, E.stream>>>(kp, a, nks, nmt, ksum, b0, skipconv);
+        k_dg_sfac<OP><<<dim3(a.nslotp / DG_SLOTS, nb), 32 * nw, smem, E.stream>>>(kp, a, nks, nmt, ksum, b0, skipconv, soff);
         ++E.nlaunch;
     }
 }
@@ -726,22 +902,29 @@ void launch_dg_sfac(Engine &E, int op, int s0, int nsites, int skipconv) {
 }
 
 template <int MODE>
-static int field(Engine &E, int s0, int s1) {
+static int field(Engine &E, int s0, int s1, int sor) {
     const KP &kp = E.kp;
     const DgArgs &a = E.dg;
     const int mb = ceil_div(ceil_div(s1, 16) - s0 / 16, 4), tiles = MODE == DGF_DG ? a.nvd8 : a.nv8;
-    // slices of the runs: about four blocks a SM
-    int ns = (int)((152L * 4 + (long)mb * kp.P - 1) / ((long)mb * kp.P));
-    ns = std::max(1, std::min(ns, std::min(E.max_slices, tiles)));
+    // slices of the runs, at least four tiles each: the count whose waves of four blocks a SM do
+    // the work soonest (512 x 32: 7 slices, 2.9 waves; 3 slices were 1.3 waves)
+    const long base = (long)mb * kp.P, room = 152L * 4;
+    int ns = 1;
+    double best = 1e300;
+    for (int c = 1; c <= std::max(1, std::min(E.max_slices, tiles / 4)); c++) {
+        const double t = (double)((base * c + room - 1) / room) / c;
+        if (t < best - 1e-12) best = t, ns = c;
+    }
+    const size_t smem = (size_t)DG_FST * a.ksf * DG_VT;
     const dim3 g(mb, kp.P, ns);
     // |T| <= sqrt(2) lmax of the run's scale: keep t below 2^62
     const int tshift = a.jn > 32 ? 3 : 0;
     const bool xc = (MODE == DGF_E || MODE == DGF_DG) && E.dg_xdip && a.exyc && s0 == kp.fd && s1 == kp.ld;
 #define PIMD_DGF(KS)                                                               \
     if (xc)                                                                        \
-        k_dg_field<MODE, KS, true><<<g, 128, 0, E.stream>>>(kp, a, s0, s1, tshift); \
+        k_dg_field<MODE, KS, MODE == DGF_E || MODE == DGF_DG><<<g, 128, smem, E.stream>>>(kp, a, s0, s1, tshift, sor); \
     else                                                                           \
-        k_dg_field<MODE, KS, false><<<g, 128, 0, E.stream>>>(kp, a, s0, s1, tshift)
+        k_dg_field<MODE, KS, false><<<g, 128, smem, E.stream>>>(kp, a, s0, s1, tshift, sor)
     if (a.ksf == 1) {
         PIMD_DGF(1);
     } else if (a.ksf == 2) {
@@ -754,17 +937,18 @@ static int field(Engine &E, int s0, int s1) {
     return ns;
 }
 
-// The slices' sums of one field pass in Fpart; returns the number of slices. part: 0 the field or
-// the charge half of the force pass, 1 its dipole half.
+// One field pass; returns the number of slices whose sums are in Fpart. F_D: part 0 runs the SOR
+// update and the convergence test too, part 1 leaves the sums; F_QD: part 0 the charge half of the
+// force pass, 1 its dipole half.
 int launch_dg_field(Engine &E, int mode, int s0, int s1, int part) {
-    if (mode == F_D) return field<DGF_E>(E, s0, s1);
-    if (mode == F_Q) return field<DGF_Q>(E, s0, s1);
-    if (part == 0) return field<DGF_QG>(E, s0, s1);
+    if (mode == F_D) return field<DGF_E>(E, s0, s1, part == 0);
+    if (mode == F_Q) return field<DGF_Q>(E, s0, s1, 0);
+    if (part == 0) return field<DGF_QG>(E, s0, s1, 0);
     const DgArgs &a = E.dg;
     const size_t smem = sizeof(double2) * ((size_t)DG_SLOTS * (2 * E.kp.lmax + 1) + (size_t)DG_SLOTS * a.jn * 2);
     k_dg_vqd<<<dim3(a.nslotp / DG_SLOTS, E.kp.P), 128, smem, E.stream>>>(E.kp, a);
     ++E.nlaunch;
-    return field<DGF_DG>(E, s0, s1);
+    return field<DGF_DG>(E, s0, s1, 0);
 }
 
 }  // namespace pimd
