@@ -31,11 +31,10 @@
 
 #include "engine.h"
 #include "nasa.cuh"
+#include "pair_math.cuh"
 
 namespace pimd {
 int run_forces(Engine &E, int t, int check_every, double *Upott, double *virialt, double *virialct, double *virt9);
-
-__constant__ double c_nasa4[4][245];  // C5ZA, CBASIS, CCORE, CREST (nasa_mod.f90)
 
 // ---------------------------------------------------------------------------------------
 // theta -> the derived parameters of the context (potential.f90:97-113, 152-160)
@@ -245,17 +244,13 @@ __global__ void __launch_bounds__(128) k_adj_cross_fold(KP kp, int s0, double *g
         for (int c = 0; c < 3; c++) grad[3 * gs + c] -= kp.dR[3 * gs + c];
 }
 
-// the forward's site-pair vector between site kinds isp of i and jsp of j (pot_ttm.f90:318-319)
+// the forward's site-pair vector between the sites a of i and c of j (pot_ttm.f90:318-319), the O sites'
+// minimum image first; images only where a component can need one
 PIMD_D void pair_vec(const KP &kp, const double4_32a &Oi, const double4_32a &Oj, const double4_32a &a,
                      const double4_32a &c, double Rs[3]) {
-    const double Rij[3] = {min_image_rn(__dsub_rn(Oi.x, Oj.x), kp.box[0], kp.boxi[0]),
-                           min_image_rn(__dsub_rn(Oi.y, Oj.y), kp.box[1], kp.boxi[1]),
-                           min_image_rn(__dsub_rn(Oi.z, Oj.z), kp.box[2], kp.boxi[2])};
-    const double Rij0[3] = {__dadd_rn(__dsub_rn(Rij[0], Oi.x), Oj.x), __dadd_rn(__dsub_rn(Rij[1], Oi.y), Oj.y),
-                            __dadd_rn(__dsub_rn(Rij[2], Oi.z), Oj.z)};
-    Rs[0] = min_image_rn(__dsub_rn(__dadd_rn(a.x, Rij0[0]), c.x), kp.box[0], kp.boxi[0]);
-    Rs[1] = min_image_rn(__dsub_rn(__dadd_rn(a.y, Rij0[1]), c.y), kp.box[1], kp.boxi[1]);
-    Rs[2] = min_image_rn(__dsub_rn(__dadd_rn(a.z, Rij0[2]), c.z), kp.box[2], kp.boxi[2]);
+    Rs[0] = min_image_near(min_image_near(Oi.x - Oj.x, kp, 0) + ((a.x - Oi.x) - (c.x - Oj.x)), kp, 0);
+    Rs[1] = min_image_near(min_image_near(Oi.y - Oj.y, kp, 1) + ((a.y - Oi.y) - (c.y - Oj.y)), kp, 1);
+    Rs[2] = min_image_near(min_image_near(Oi.z - Oj.z, kp, 2) + ((a.z - Oi.z) - (c.z - Oj.z)), kp, 2);
 }
 
 PIMD_D void atomic3(double *p, const double v[3], double s) {
@@ -285,27 +280,35 @@ __global__ void __launch_bounds__(128) k_adj_ddbil(KP kp, Polfac pf, const doubl
             double Rs[3];
             pair_vec(kp, pos[i], pos[j], pos[3 * N + i], pos[3 * N + j], Rs);
             const double d2 = dot3_rn(Rs[0], Rs[1], Rs[2]);
-            double t1, t2, t3;
-            smear3<double>(d2, a12, kp.ew, &t1, &t2, &t3);
+            PairR pr;
+            pair_r(d2, kp.ew, pr);
+            double t2 = (pr.t1 + kp.ew.cts2 * pr.g) * pr.drsqi, t3 = (t2 + kp.ew.cts3 * pr.g) * pr.drsqi;
+            const bool near = d2 < 25.0;
+            double e1 = 0.0;
+            if (near) {  // smear.f90:95-104
+                e1 = exp(-(pr.dd * d2) * a12);
+                const double s2 = (e1 * pr.dri * pr.drsqi + e1 * a12) * pr.drsqi;
+                t2 -= s2;
+                t3 -= (s2 + 0.6 * e1 * pr.dd * a12 * a12) * pr.drsqi;
+            }
             const size_t si = 3 * ((size_t)b * kp.S + 3 * N + i), sj = 3 * ((size_t)b * kp.S + 3 * N + j);
             const double ui[3] = {u[si], u[si + 1], u[si + 2]}, uj[3] = {u[sj], u[sj + 1], u[sj + 2]};
             const double vi[3] = {v[si], v[si + 1], v[si + 2]}, vj[3] = {v[sj], v[sj + 1], v[sj + 2]};
-            double dij[3] = {0, 0, 0};
-            dd_force(Rs, ui, vj, t2, t3, dij);  // -grad_R (u_i T v_j)
-            dd_force(Rs, vi, uj, t2, t3, dij);  // -grad_R (v_i T u_j)
-            atomic3(grad + si, dij, -w);
-            atomic3(grad + sj, dij, w);
-            if (d2 < 25.0) {
-                const double r = sqrt(d2), e1 = exp(-a12 * d2 * r);
-                const double rui = Rs[0] * ui[0] + Rs[1] * ui[1] + Rs[2] * ui[2];
-                const double ruj = Rs[0] * uj[0] + Rs[1] * uj[1] + Rs[2] * uj[2];
-                const double rvi = Rs[0] * vi[0] + Rs[1] * vi[1] + Rs[2] * vi[2];
-                const double rvj = Rs[0] * vj[0] + Rs[1] * vj[1] + Rs[2] * vj[2];
-                const double uv = ui[0] * vj[0] + ui[1] * vj[1] + ui[2] * vj[2];
-                const double vu = vi[0] * uj[0] + vi[1] * uj[1] + vi[2] * uj[2];
-                const double dT = 3.0 * a12 * r * e1 * (rui * rvj + rvi * ruj) - e1 * (uv + vu);
-                th[0] += w * dT * pf.v[4] * pf.v[4];  // d a12 / d a_dd = polfac_M^2
+            const double rui = Rs[0] * ui[0] + Rs[1] * ui[1] + Rs[2] * ui[2];
+            const double ruj = Rs[0] * uj[0] + Rs[1] * uj[1] + Rs[2] * uj[2];
+            const double rvi = Rs[0] * vi[0] + Rs[1] * vi[1] + Rs[2] * vi[2];
+            const double rvj = Rs[0] * vj[0] + Rs[1] * vj[1] + Rs[2] * vj[2];
+            const double uv = ui[0] * vj[0] + ui[1] * vj[1] + ui[2] * vj[2] + vi[0] * uj[0] + vi[1] * uj[1] + vi[2] * uj[2];
+            const double rr = rui * rvj + rvi * ruj;
+            // dd_force of (u_i, v_j) and (v_i, u_j): -grad_R (u_i T v_j + v_i T u_j), times -w
+            const double f0 = -w * (15.0 * t3 * rr - 3.0 * t2 * uv), f2 = 3.0 * t2 * w;
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                const double d = f0 * Rs[c] + f2 * (rui * vj[c] + rvj * ui[c] + rvi * uj[c] + ruj * vi[c]);
+                atomicAdd(grad + si + c, d);
+                atomicAdd(grad + sj + c, -d);
             }
+            if (near) th[0] += w * (3.0 * a12 * pr.dd * e1 * rr - e1 * uv) * pf.v[4] * pf.v[4];  // d a12 / d a_dd = polfac_M^2
         }
     }
     block_reduce_add<1, 128>(th, thacc + PIMD_TH_A_DD);
@@ -375,12 +378,6 @@ __global__ void __launch_bounds__(128) k_adj_ddbil_m(KP kp, double pfm2, const f
     block_reduce_add<1, 128>(tv, thacc + PIMD_TH_A_DD);
 }
 
-// Q(2/3, x) by the Numerical-Recipes series / continued fraction used by the forward
-PIMD_D double q23(double x) {
-    unsigned err = 0;
-    return gammq2_3<double>(x, &err);
-}
-
 // Real-space terms of one bead that do not involve the dipole iterations, per O-O pair:
 //   * the charge-field adjoint nu: d/dx [nu . E_q] at fixed charges for the dipole site M of
 //     one molecule and the charged sites H1, H2, M of the other (smear2 ts1, ts2 with the
@@ -391,6 +388,9 @@ PIMD_D double q23(double x) {
 //   * van der Waals: the gradient of C/r^6 + D e^{-E r} (+ A/r^12 + B/r^10) and its C, D, E
 //     derivatives (the energy's own gradient: the force-only switch of pot_ttm.f90:171 is not
 //     part of the energy).
+// Three lanes a pair, each one charged site of molecule i (and a third of the van der Waals terms'
+// atomics): the chain of a pair is bound by FP64 latency (415 us at 64 x 8 with a thread a pair and a
+// power and the tests of Q(2/3, x) a site pair).
 __global__ void __launch_bounds__(128) k_adj_pairs(KP kp, Polfac pf, const double *ebar, const double *nu,
                                                    double *grad, double *phin, double *thacc) {
     const int b = blockIdx.y, N = kp.N;
@@ -398,109 +398,129 @@ __global__ void __launch_bounds__(128) k_adj_pairs(KP kp, Polfac pf, const doubl
     const double eb = ebar[b];
     const double4_32a *pos = kp.pos + (size_t)b * kp.S;
     double th[4] = {0, 0, 0, 0};  // a_cc, C, D, E
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < np; p += gridDim.x * blockDim.x) {
+    unsigned err = 0;  // (the forward reports Q(2/3, x))
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 3 * np; t += gridDim.x * blockDim.x) {
+        const int p = t / 3, m = t - 3 * p, a = 2 + m;  // site kind of molecule i
         const int2 ij = kp.pairs[(size_t)b * kp.cap + p];
         const int i = ij.x, j = ij.y;
-        const int mol[2] = {i, j};
-        // van der Waals on the O sites
-        {
-            const double4_32a Oi = pos[i], Oj = pos[j];
-            const double R[3] = {min_image_rn(__dsub_rn(Oi.x, Oj.x), kp.box[0], kp.boxi[0]),
-                                 min_image_rn(__dsub_rn(Oi.y, Oj.y), kp.box[1], kp.boxi[1]),
-                                 min_image_rn(__dsub_rn(Oi.z, Oj.z), kp.box[2], kp.boxi[2])};
-            const double r2 = dot3_rn(R[0], R[1], R[2]), r = sqrt(r2), r2i = 1.0 / r2, r6i = r2i * r2i * r2i;
+        const double4_32a Oi = pos[i], Oj = pos[j];
+        {  // van der Waals on the O sites, a component a lane, the derivatives in lane 0
+            const double R[3] = {min_image_near(Oi.x - Oj.x, kp, 0), min_image_near(Oi.y - Oj.y, kp, 1),
+                                 min_image_near(Oi.z - Oj.z, kp, 2)};
+            const double r2 = dot3_rn(R[0], R[1], R[2]), ri = rsqrt(r2), r = r2 * ri, r2i = ri * ri, r6i = r2i * r2i * r2i;
             const double ex = exp(-kp.vdwE * r);
             const double dudr_over_r = (-12.0 * kp.vdwA * r6i * r6i - 10.0 * kp.vdwB * r6i * r2i * r2i - 6.0 * kp.vdwC * r6i) * r2i -
-                                       kp.vdwD * kp.vdwE * ex / r;
-            double gv[3] = {dudr_over_r * R[0], dudr_over_r * R[1], dudr_over_r * R[2]};
-            atomic3(grad + 3 * ((size_t)b * kp.S + i), gv, eb);
-            atomic3(grad + 3 * ((size_t)b * kp.S + j), gv, -eb);
-            th[1] += eb * r6i;
-            th[2] += eb * ex;
-            th[3] += -eb * kp.vdwD * r * ex;
-        }
-        // charged sites H1, H2, M (kinds 2..4) of both molecules
-        for (int a = 2; a <= 4; a++) {
-            for (int c = 2; c <= 4; c++) {
-                const double4_32a sa = pos[(a - 1) * N + i], sc = pos[(c - 1) * N + j];
-                double Rs[3];
-                pair_vec(kp, pos[i], pos[j], sa, sc, Rs);  // r_a(i) - r_c(j)
-                const double d2 = dot3_rn(Rs[0], Rs[1], Rs[2]);
-                const double a12 = kp.pt.apol_cd[a][c];
-                double ts1, ts2;
-                smear2<double>(d2, a12, kp.ew, &ts1, &ts2);
-                const double e1 = (d2 < 25.0) ? exp(-a12 * d2 * sqrt(d2)) : 0.0;
-                const double pfac = pf.v[a] * pf.v[c];
-                // Uelec d/da_cc (q_a q_c ts0 summed over the pair's site pairs)
-                if (d2 < 25.0) {
-                    const double x = a12 * d2 * sqrt(d2);
-                    const double dts0 = (1.0 / 3.0) * pow(a12, -2.0 / 3.0) * 1.3541179394264 * q23(x);
-                    th[0] += eb * sa.w * sc.w * dts0 * pfac;
-                }
-                // nu at M(i) in the field of charge c(j): E = q_c ts1 R, R = r_M(i) - r_c(j)
-                for (int side = 0; side < 2; side++) {
-                    const int dk = side == 0 ? a : c;  // the dipole end must be the M site
-                    if (dk != 4) continue;
-                    const int md = mol[side], mc = mol[1 - side];
-                    const int ck = side == 0 ? c : a;
-                    const double qc = side == 0 ? sc.w : sa.w;
-                    const double sg = side == 0 ? 1.0 : -1.0;  // R = sg * Rs
-                    const double R[3] = {sg * Rs[0], sg * Rs[1], sg * Rs[2]};
-                    const size_t sm = (size_t)b * kp.S + 3 * N + md, scs = (size_t)b * kp.S + (ck - 1) * N + mc;
-                    const double n[3] = {nu[3 * sm], nu[3 * sm + 1], nu[3 * sm + 2]};
-                    const double rn = R[0] * n[0] + R[1] * n[1] + R[2] * n[2];
-                    double gm[3];
-                    for (int q = 0; q < 3; q++) gm[q] = qc * (ts1 * n[q] - 3.0 * ts2 * rn * R[q]);
-                    atomic3(grad + 3 * sm, gm, 1.0);
-                    atomic3(grad + 3 * scs, gm, -1.0);
-                    atomicAdd(phin + scs, ts1 * rn);
-                    th[0] += qc * e1 * rn * pfac;
-                }
+                                       kp.vdwD * kp.vdwE * ex * ri;
+            const double gv = eb * dudr_over_r * (m == 0 ? R[0] : m == 1 ? R[1] : R[2]);
+            atomicAdd(grad + 3 * ((size_t)b * kp.S + i) + m, gv);
+            atomicAdd(grad + 3 * ((size_t)b * kp.S + j) + m, -gv);
+            if (m == 0) {
+                th[1] += eb * r6i;
+                th[2] += eb * ex;
+                th[3] += -eb * kp.vdwD * r * ex;
             }
         }
+        const double4_32a sa = pos[(a - 1) * N + i];
+        const size_t ga = (size_t)b * kp.S + (a - 1) * N + i, gM = (size_t)b * kp.S + 3 * N;
+        double gi[3] = {0, 0, 0}, pi = 0.0;
+        for (int c = 2; c <= 4; c++) {  // charged sites H1, H2, M of molecule j
+            const double4_32a sc = pos[(c - 1) * N + j];
+            double R[3];
+            pair_vec(kp, Oi, Oj, sa, sc, R);  // r_a(i) - r_c(j)
+            const double d2 = dot3_rn(R[0], R[1], R[2]);
+            const bool near = d2 < 25.0, mm = a == 4 || c == 4;
+            if (!near && !mm) continue;
+            const double a12 = kp.pt.apol_cd[a][c], pfac = pf.v[a] * pf.v[c];
+            PairR pr;
+            pair_r(d2, kp.ew, pr);
+            double t1 = pr.t1, t2 = (pr.t1 + kp.ew.cts2 * pr.g) * pr.drsqi, e1 = 0.0;
+            if (near) {
+                const double x = a12 * d2 * pr.dd, ra = kp.pt.ra_qq[a][c], rr = ra * pr.dd;
+                e1 = exp(-x);
+                const double s1 = e1 * pr.dri * pr.drsqi;
+                t1 -= s1;
+                t2 -= (s1 + e1 * a12) * pr.drsqi;
+                // Uelec d/da_cc: q_a q_c Gamma(2/3) Q(2/3, x) / (3 a12^(2/3)), a12^(1/3) = ra
+                const double q23 = thole_q23(x, e1 * (rr * rr) * kp.gq_norm, kp.gq, &err);
+                th[0] += eb * sa.w * sc.w * ((1.0 / 3.0) * 1.3541179394264) * q23 * rcp_newton(ra * ra) * pfac;
+            }
+            if (!mm) continue;
+            const size_t gc = (size_t)b * kp.S + (c - 1) * N + j;
+            double gj[3] = {0, 0, 0}, pj = 0.0;
+            // nu at M(i) in the field of charge c(j): E = q_c ts1 R; and at M(j) in that of a(i), -R
+            for (int side = 0; side < 2; side++) {
+                if ((side == 0 ? a : c) != 4) continue;
+                const double *n = nu + 3 * (gM + (side == 0 ? i : j));
+                const double qc = side == 0 ? sc.w : sa.w, n0 = n[0], n1 = n[1], n2 = n[2];
+                const double rn = R[0] * n0 + R[1] * n1 + R[2] * n2;  // (side 1: minus its R . nu)
+                const double f1 = qc * t1, f2 = -3.0 * qc * t2 * rn;
+                const double gm[3] = {f1 * n0 + f2 * R[0], f1 * n1 + f2 * R[1], f1 * n2 + f2 * R[2]};
+#pragma unroll
+                for (int q = 0; q < 3; q++) {
+                    gi[q] += side == 0 ? gm[q] : -gm[q];
+                    gj[q] -= side == 0 ? gm[q] : -gm[q];
+                }
+                if (side == 0)
+                    pj += t1 * rn;
+                else
+                    pi -= t1 * rn;
+                th[0] += (side == 0 ? qc : -qc) * e1 * rn * pfac;
+            }
+            atomic3(grad + 3 * gc, gj, 1.0);
+            if (a == 4) atomicAdd(phin + gc, pj);
+        }
+        atomic3(grad + 3 * ga, gi, 1.0);
+        atomicAdd(phin + ga, pi);
     }
     block_reduce_add<4, 128>(th, thacc + PIMD_TH_A_CC);  // slots A_CC, VDW_C, VDW_D, VDW_E (contiguous)
 }
 
-// NASA PES derivatives with respect to its four scale factors for one molecule
-// (nasa.f90:2-103): Vc = 2 c_0 + efac sum_j c_j sym_j f3_j with c_j = sum_X f_X C^X_j, and
-// deoh, phh1 proportional to f5z.
-PIMD_D void nasa_theta(const double r1[3][3], const double box[3], const double boxi[3], double f5z, double d[4]) {
-    double ROH1[3], ROH2[3], RHH[3];
-    for (int c = 0; c < 3; c++) {
-        ROH1[c] = min_image_rn(__dsub_rn(r1[1][c], r1[0][c]), box[c], boxi[c]);
-        ROH2[c] = min_image_rn(__dsub_rn(r1[2][c], r1[0][c]), box[c], boxi[c]);
-        RHH[c] = min_image_rn(__dsub_rn(r1[1][c], r1[2][c]), box[c], boxi[c]);
+// NASA PES derivatives with respect to its four scale factors (nasa.f90:2-103): Vc = 2 c_0 + efac
+// sum_j c_j sym_j f3_j with c_j = sum_X f_X C^X_j, and deoh, phh1 proportional to f5z. Four lanes a
+// molecule, one a coefficient set: per (i, j) group a Horner polynomial in x3 (a thread with all
+// four sums term by term was a chain of 1700 FP64 instructions).
+__global__ void __launch_bounds__(128) k_adj_nasa(KP kp, const double *ebar, const double *coef, double *thacc) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, w = t >> 2, x = t & 3, b = blockIdx.y, N = kp.N;
+    double d = 0.0;
+    if (w < N) {
+        const double4_32a *pos = kp.pos + (size_t)b * kp.S;
+        const double4_32a O = pos[w], H1 = pos[N + w], H2 = pos[2 * N + w];
+        const double a[3] = {min_image_near(H1.x - O.x, kp, 0), min_image_near(H1.y - O.y, kp, 1), min_image_near(H1.z - O.z, kp, 2)};
+        const double c[3] = {min_image_near(H2.x - O.x, kp, 0), min_image_near(H2.y - O.y, kp, 1), min_image_near(H2.z - O.z, kp, 2)};
+        const double hx = a[0] - c[0], hy = a[1] - c[1], hz = a[2] - c[2];
+        const double r1 = sqrt(a[0] * a[0] + a[1] * a[1] + a[2] * a[2]), r2 = sqrt(c[0] * c[0] + c[1] * c[1] + c[2] * c[2]);
+        const double costh = (a[0] * c[0] + a[1] * c[1] + a[2] * c[2]) / (r1 * r2);
+        const double reoh = PIMD_NASA_REOH, i0 = 1.0 / PIMD_NASA_REOH;
+        const double x1 = (r1 - reoh) * i0, x2 = (r2 - reoh) * i0, x3 = costh + .24780227221366464506;
+        const double efac = exp(-PIMD_NASA_B1 * ((r1 - reoh) * (r1 - reoh) + (r2 - reoh) * (r2 - reoh)));
+        double f1[16], f2[16];
+        f1[0] = f2[0] = 0.0;
+        f1[1] = f2[1] = 1.0;
+        for (int j = 2; j <= 15; j++) {
+            f1[j] = f1[j - 1] * x1;
+            f2[j] = f2[j - 1] * x2;
+        }
+        double sum = 0.0;
+        for (int g = 0; g < c_ngrp[0]; g++) {
+            const int I = c_pg[g][0], J = c_pg[g][1], s0 = c_pg[g][2], n = c_pg[g][3];
+            double pk = 0.0;
+            for (int k = 0; k < n; k++) {
+                const int j = c_ps[s0 + k];
+                pk = fma(pk, x3, j < 0 ? 0.0 : __ldg(coef + 4 * j + x));
+            }
+            sum += (f1[I] * f2[J] + f1[J] * f2[I]) * pk;
+        }
+        d = 2.0 * __ldg(coef + x) + efac * sum;
+        if (x == 0) {  // deoh = f5z DEOHA, phh1 = f5z PHH1A e^{phh2}
+            const double e1 = exp(-PIMD_NASA_ALPHAOH * (r1 - PIMD_NASA_ROH)), e2 = exp(-PIMD_NASA_ALPHAOH * (r2 - PIMD_NASA_ROH));
+            d += PIMD_NASA_DEOHA * (e1 * (e1 - 2.0) + e2 * (e2 - 2.0)) +
+                 PIMD_NASA_PHH1A * exp(PIMD_NASA_PHH2 * (1.0 - sqrt(hx * hx + hy * hy + hz * hz)));
+        }
+        d *= 0.00285914375100642899 * ebar[b];
     }
-    const double dROH1 = sqrt(ROH1[0] * ROH1[0] + ROH1[1] * ROH1[1] + ROH1[2] * ROH1[2]);
-    const double dROH2 = sqrt(ROH2[0] * ROH2[0] + ROH2[1] * ROH2[1] + ROH2[2] * ROH2[2]);
-    const double dRHH = sqrt(RHH[0] * RHH[0] + RHH[1] * RHH[1] + RHH[2] * RHH[2]);
-    const double costh = (ROH1[0] * ROH2[0] + ROH1[1] * ROH2[1] + ROH1[2] * ROH2[2]) / (dROH1 * dROH2);
-    const double reoh = PIMD_NASA_REOH, b1 = PIMD_NASA_B1, roh = PIMD_NASA_ROH, alphaoh = PIMD_NASA_ALPHAOH,
-                 phh2 = PIMD_NASA_PHH2, costhe = -.24780227221366464506;
-    const double exp1 = exp(-alphaoh * (dROH1 - roh)), exp2 = exp(-alphaoh * (dROH2 - roh));
-    const double x1 = (dROH1 - reoh) / reoh, x2 = (dROH2 - reoh) / reoh, x3 = costh - costhe;
-    double f1[16], f2[16], f3[16];
-    f1[0] = f2[0] = f3[0] = 0.0;
-    f1[1] = f2[1] = f3[1] = 1.0;
-    for (int j = 2; j <= 15; j++) {
-        f1[j] = f1[j - 1] * x1;
-        f2[j] = f2[j - 1] * x2;
-        f3[j] = f3[j - 1] * x3;
-    }
-    const double efac = exp(-b1 * ((dROH1 - reoh) * (dROH1 - reoh) + (dROH2 - reoh) * (dROH2 - reoh)));
-    double sx[4] = {0, 0, 0, 0};
-    for (int j = 1; j < 245; j++) {
-        const int inI = c_idx[j][0], inJ = c_idx[j][1], inK = c_idx[j][2];
-        const double t = (f1[inI] * f2[inJ] + f1[inJ] * f2[inI]) * f3[inK];
-        for (int x = 0; x < 4; x++) sx[x] += c_nasa4[x][j] * t;
-    }
-    const double sc = 0.00285914375100642899;
-    for (int x = 0; x < 4; x++) d[x] = sc * (2.0 * c_nasa4[x][0] + efac * sx[x]);
-    // deoh = f5z DEOHA, phh1 = f5z PHH1A e^{phh2}
-    d[0] += sc * (PIMD_NASA_DEOHA * (exp1 * (exp1 - 2.0) + exp2 * (exp2 - 2.0)) +
-                  PIMD_NASA_PHH1A * exp(phh2) * exp(-phh2 * dRHH));
-    (void)f5z;
+#pragma unroll
+    for (int o = 16; o >= 4; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+    if ((threadIdx.x & 31) < 4) atomicAdd(thacc + PIMD_TH_F5Z + x, d);
 }
 
 // Per molecule: the monomer PES gradient, the fixed-charge gradient -q E of Uelec, the
@@ -532,9 +552,6 @@ __global__ void __launch_bounds__(128) k_adj_mol(KP kp, const double *ebar, cons
                 nasa_pot(R, kp.box, kp.boxi, dr1, &e1, kp.c5z, kp.nasa_f5z);
                 for (int k = 0; k < 3; k++)
                     for (int c = 0; c < 3; c++) grad[3 * (base + k * N + w) + c] += eb * dr1[k][c];
-                double d4[4];
-                nasa_theta(R, kp.box, kp.boxi, kp.nasa_f5z, d4);
-                for (int x = 0; x < 4; x++) th[PIMD_TH_F5Z + x] += eb * d4[x];
             }
             // Uelec at fixed charges: -q E_q at the charged sites H1, H2, M
             for (int k = 1; k < 4; k++) {
@@ -712,6 +729,7 @@ int pimd_pot_backward(pimd_ctx *ctx, const double *Ebar, double *dRRt, double *d
         }
         E.adj_bytes = nbytes;
     }
+    if (!E.d_nasa4) return adj_fail(E, PIMD_ERR_NOMEM, "NASA coefficient table");
     double *g = E.d_adj, *u = g + 3 * P * nd, *v = u + sv, *Dr = v + sv, *grad = Dr + sv, *nu = grad + sv;
     double *phin = nu + sv;
     const uintptr_t sa = (reinterpret_cast<uintptr_t>(phin + P * S) + 15) & ~uintptr_t(15);  // 16-byte rows
@@ -843,6 +861,10 @@ int pimd_pot_backward(pimd_ctx *ctx, const double *Ebar, double *dRRt, double *d
         launch_adj_pairs_m(E, pf.v, ebar, nu, grad, phin, thacc);
     else
         k_adj_pairs<<<gp, 128, 0, st>>>(kp, pf, ebar, nu, grad, phin, thacc);
+    if (!kp.contraction) {
+        k_adj_nasa<<<dim3((unsigned)((4 * kp.N + 127) / 128), (unsigned)P), 128, 0, st>>>(kp, ebar, E.d_nasa4, thacc);
+        ++E.nlaunch;
+    }
     k_adj_mol<0><<<gm, 128, 0, st>>>(kp, ebar, E.d_phiq, nu, grad, phin, dR, thacc);
     k_adj_mol<1><<<gm, 128, 0, st>>>(kp, ebar, E.d_phiq, nu, grad, phin, dR, thacc);
     E.nlaunch += 5 + 8 * (long long)kmax;
@@ -866,15 +888,19 @@ namespace pimd {
 // constant tables of this translation unit: the NASA tables of nasa.cuh and the four PES
 // coefficient sets for the scale-factor derivatives
 void adjoint_init(Engine &E) {
-    (void)E;
     nasa_upload_constants();
-    static double tab[4][245];
+    double tab[245][4];  // C5ZA, CBASIS, CCORE, CREST (nasa_mod.f90)
     for (int j = 0; j < 245; j++) {
-        tab[0][j] = PIMD_NASA_C5ZA[j];
-        tab[1][j] = PIMD_NASA_CBASIS[j];
-        tab[2][j] = PIMD_NASA_CCORE[j];
-        tab[3][j] = PIMD_NASA_CREST[j];
+        tab[j][0] = PIMD_NASA_C5ZA[j];
+        tab[j][1] = PIMD_NASA_CBASIS[j];
+        tab[j][2] = PIMD_NASA_CCORE[j];
+        tab[j][3] = PIMD_NASA_CREST[j];
     }
-    cudaMemcpyToSymbol(c_nasa4, tab, sizeof(tab));
+    if (cudaMalloc((void **)&E.d_nasa4, sizeof(tab)) != cudaSuccess) {
+        E.d_nasa4 = nullptr;
+        return;
+    }
+    E.allocs.push_back(E.d_nasa4);
+    cudaMemcpy(E.d_nasa4, tab, sizeof(tab), cudaMemcpyHostToDevice);
 }
 }  // namespace pimd

@@ -334,6 +334,7 @@ struct Engine {
     // differentiation form (adjoint.cu): model parameters theta and the forward's tape
     double theta[PIMD_NTHETA];
     double *d_c5z = nullptr;     // NASA coefficients for the current theta
+    double *d_nasa4 = nullptr;   // [245][4] the four NASA coefficient sets (the scale factors' derivatives)
     bool tape_on = false;        // record the dipole iterations during the force call
     int tape_kmax = 0;           // iterations the tape holds
     double *d_tape = nullptr;    // [kmax + 1][P][N][3] dipoles of the dipole sites per iteration
@@ -495,6 +496,7 @@ void launch_dg_tables(Engine &E);        // after the ssincos tables
 void launch_dg_dipoles(Engine &E);       // X of the dipole sites, before the dipole iterations
 void launch_dg_sfac(Engine &E, int op, int s0, int nsites, int skipconv);
 int launch_dg_field(Engine &E, int mode, int s0, int s1, int part);
+int launch_dg_dforce(Engine &E, const double2 *A, const double2 *B, const double2 *A2, const double *dip2);
 // launchers (spc.cu): q-SPC/Fw and SPC/F
 void launch_sites_spc(Engine &E);
 void launch_finish_spc(Engine &E);

@@ -1261,25 +1261,30 @@ void adj_dipole_field(Engine &E, double2 *Sm_u, double *bacc, double *Dr) {
     E.kp = keep;
 }
 
-// Reciprocal-space gradients of the backward, thread per site, direct sum over the
-// k-list (c_k = 4 pi A_k / V, S raw = sum (k.mu) e^{ik.r} or sum q e^{ik.r}):
+// Reciprocal-space gradients of the backward (c_k = 4 pi A_k / V, S raw = sum (k.mu) e^{ik.r} or
+// sum q e^{ik.r}):
 //   BIL  : d/dr_s [u^T D_rec v] = sum_k c_k k [(k.u_s) Im(e_s conj S_v) + (k.v_s) Im(e_s conj S_u)]
 //   CROSS: d/dr_s [nu^T E_q,rec] = sum_k c_k k (k.nu_s) Re(e_s conj S_q) (dipole sites)
 //                                 - q_s sum_k c_k k Re(e_s conj S_nu)    (charged sites)
 //          and the potential of the nu dipoles phi_s = -sum_k c_k Im(e_s conj S_nu).
 // Derived from the forward's field formula E_s = sum_k c_k k Im(e_s conj S) (ewald.f90:45-49,
-// 114-117): the k-space operator is the Hessian of a quadratic form, so these are exact.
-// The mixed engine's instance reads the FP32 tables and forms each product in FP32; each chunk's
-// sums go to the FP64 totals. A block stages each chunk's k-vectors, weights and structure
-// factors in shared memory (converted once per block, not per site). The k-list is split over
-// gridDim.z slices of whole chunks; each slice's per-site sums (G, phi) go to Fpart, and
-// k_adj_rfin adds the slices in a fixed order.
+// 114-117): the k-space operator is the Hessian of a quadratic form, so these are exact. They are
+// minus the forward's force passes: BIL the force on u in the field of v and on v in that of u,
+// CROSS the force on nu in the field of the charges and on the charges in that of nu, which is how
+// the FP64 engine forms them (ewald_dg.cu; a site-parallel walk over the k-list took 206 us a sweep
+// at 64 x 8, the two force passes in one launch about 30). The mixed engine, where its tensor-core
+// passes do not apply: thread per site, FP32 tables and products, each chunk's sums to the FP64
+// totals. A block stages each chunk's k-vectors, weights and structure factors in shared memory
+// (converted once per block, not per site). The k-list is split over gridDim.z slices of whole
+// chunks; each slice's per-site sums (G, phi) go to Fpart, and k_adj_rfin adds the slices in a
+// fixed order.
 enum { ADJ_BIL = 0, ADJ_CROSS = 1 };
-template <int MODE, typename R>
+template <int MODE>
 __global__ void __launch_bounds__(128) k_adj_rec(KP kp, int s0, int s1, const double *a, const double *bvec,
                                                  const double2 *SA, const double2 *SB, const double *ebw,
                                                  double *grad, double *phi) {
-    using V = typename C2<R>::T;
+    using R = float;
+    using V = float2;
     __shared__ R sk[KCH][4];            // kx, ky, kz, c_k
     __shared__ R s1x[KCH][2], s2x[KCH][2];  // BIL: conj(raw S_u), conj(raw S_v); CROSS: raw S_q, conj(raw S_nu)
     const int b = blockIdx.y, s = s0 + blockIdx.x * blockDim.x + threadIdx.x;
@@ -1296,12 +1301,10 @@ __global__ void __launch_bounds__(128) k_adj_rec(KP kp, int s0, int s1, const do
             if (MODE == ADJ_BIL) bv[c] = R(bvec[3 * gs + c]);
         }
     }
-    // FP32: this site's kz table column in shared memory (dynamic, (lmax + 1) x 128), read in
+    // this site's kz table column in shared memory (dynamic, (lmax + 1) x 128), read in
     // the k loop instead of from the global table
     extern __shared__ float2 adj_ez[];
-    if constexpr (sizeof(R) == 4)
-        for (int n = 0; n <= kp.lmax; n++)
-            adj_ez[n * 128 + threadIdx.x] = valid ? tab_z<float>(kp, b, n, s) : make_float2(0.f, 0.f);
+    for (int n = 0; n <= kp.lmax; n++) adj_ez[n * 128 + threadIdx.x] = valid ? tab_z<float>(kp, b, n, s) : make_float2(0.f, 0.f);
     double G[3] = {0, 0, 0}, ph = 0.0;
     const int slice = blockIdx.z, nslice = gridDim.z;
     const int c0 = (int)((long)slice * kp.nchunk / nslice), c1 = (int)((long)(slice + 1) * kp.nchunk / nslice);
@@ -1332,17 +1335,13 @@ __global__ void __launch_bounds__(128) k_adj_rec(KP kp, int s0, int s1, const do
             const KRun run = kp.runs[r];
             const V ex = tab_x<R>(kp, b, run.kx, s);
             const V ey = tab_y<R>(kp, b, run.ky, s);
-            const V exy = C2<R>::make(ex.x * ey.x - ex.y * ey.y, ex.y * ey.x + ex.x * ey.y);
+            const V exy = make_float2(ex.x * ey.x - ex.y * ey.y, ex.y * ey.x + ex.x * ey.y);
             const int i0 = run.kbeg - ch.k0;
             for (int j = 0; j < run.nkz; j++) {
                 const int kz = run.kzlo + j, i = i0 + j;
-                V z;
-                if constexpr (sizeof(R) == 4)
-                    z = adj_ez[(kz < 0 ? -kz : kz) * 128 + threadIdx.x];
-                else
-                    z = tab_z<R>(kp, b, kz < 0 ? -kz : kz, s);
+                V z = adj_ez[(kz < 0 ? -kz : kz) * 128 + threadIdx.x];
                 if (kz < 0) z = cconj(z);
-                const V e = C2<R>::make(exy.x * z.x - exy.y * z.y, exy.y * z.x + exy.x * z.y);
+                const V e = make_float2(exy.x * z.x - exy.y * z.y, exy.y * z.x + exy.x * z.y);
                 const R kv[3] = {sk[i][0], sk[i][1], sk[i][2]}, ck = sk[i][3];
                 if (MODE == ADJ_BIL) {
                     const R imu = e.x * s1x[i][1] + e.y * s1x[i][0], imv = e.x * s2x[i][1] + e.y * s2x[i][0];
@@ -1371,10 +1370,10 @@ __global__ void __launch_bounds__(128) k_adj_rec(KP kp, int s0, int s1, const do
         kp.Fpart[((size_t)slice * kp.P + b) * (s1 - s0) + (s - s0)] = make_double4_32a(G[0], G[1], G[2], ph);
 }
 
-// grad += w (sum of the slices' G), phi += w (sum of their potentials) (CROSS), slices in order
+// grad += sg w (sum of the slices' G), phi += sg w (sum of their potentials) (CROSS), slices in order
 template <int MODE>
-__global__ void __launch_bounds__(128) k_adj_rfin(KP kp, int s0, int s1, int nslice, const double *ebw, double *grad,
-                                                  double *phi) {
+__global__ void __launch_bounds__(128) k_adj_rfin(KP kp, int s0, int s1, int nslice, const double *ebw, double sg,
+                                                  double *grad, double *phi) {
     const int b = blockIdx.y, s = s0 + blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= s1 || ebw[b] == 0.0) return;
     double G[3] = {0, 0, 0}, ph = 0.0;
@@ -1386,7 +1385,7 @@ __global__ void __launch_bounds__(128) k_adj_rfin(KP kp, int s0, int s1, int nsl
         ph += p.w;
     }
     const size_t gs = (size_t)b * kp.S + s;
-    const double w = ebw[b];  // per-bead scale
+    const double w = sg * ebw[b];  // per-bead scale
     for (int c = 0; c < 3; c++) grad[3 * gs + c] += w * G[c];
     if (MODE == ADJ_CROSS && phi) phi[gs] += w * ph;
 }
@@ -1395,27 +1394,46 @@ void adj_rec(Engine &E, int mode, const double *a, const double *bvec, const dou
              const double *ebw, double *grad, double *phi) {
     const int s0 = (mode == ADJ_BIL) ? E.kp.fd : 0, s1 = (mode == ADJ_BIL) ? E.kp.ld : E.kp.S;
     const int sblocks = (s1 - s0 + 127) / 128;
+    if (E.precision != PIMD_PREC_MIXED) {
+        // the dipole halves: (u in the field of S_v, v in that of S_u), or nu in that of the charges
+        const int d0 = E.kp.fd, d1 = E.kp.ld;
+        const dim3 gd((d1 - d0 + 127) / 128, E.kp.P);
+        const double *keep = E.kp.dip;
+        auto dipoles = [&](const double *dip, const double2 *S, const double2 *S2, const double *dip2) {
+            E.kp.dip = const_cast<double *>(dip);
+            const int ns = launch_dg_dforce(E, S, nullptr, S2, dip2);
+            E.kp.dip = const_cast<double *>(keep);
+            k_adj_rfin<ADJ_BIL><<<gd, 128, 0, E.stream>>>(E.kp, d0, d1, ns, ebw, -1.0, grad, nullptr);
+            ++E.nlaunch;
+        };
+        if (mode == ADJ_CROSS) {
+            // the charge half on the weights of S_nu, which the structure factor just formed left in V
+            const int q0 = E.kp.fq, ns = launch_dg_field(E, F_QD, q0, s1, 0);
+            k_adj_rfin<ADJ_CROSS><<<dim3((s1 - q0 + 127) / 128, E.kp.P), 128, 0, E.stream>>>(E.kp, q0, s1, ns, ebw, -1.0, grad, phi);
+            ++E.nlaunch;
+            dipoles(a, E.kp.Sq, nullptr, nullptr);
+        } else if (E.max_slices >= 2) {
+            dipoles(a, SB, SA, bvec);
+        } else {
+            dipoles(a, SB, nullptr, nullptr);
+            dipoles(bvec, SA, nullptr, nullptr);
+        }
+        return;
+    }
     const int ns = std::max(1, std::min((int)((8L * 152 + (long)sblocks * E.kp.P - 1) / ((long)sblocks * E.kp.P)),
                                         std::min(E.kp.nchunk, E.max_slices)));
     dim3 g(sblocks, E.kp.P, ns), g2(sblocks, E.kp.P);
-    const bool f = E.precision == PIMD_PREC_MIXED;
     const size_t ezb = sizeof(float2) * 128 * (E.kp.lmax + 1);  // FP32 kz column, <= 128 KB (lmax <= 127)
-    if (f && ezb > 48 * 1024) {
-        cudaFuncSetAttribute(k_adj_rec<ADJ_BIL, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ezb);
-        cudaFuncSetAttribute(k_adj_rec<ADJ_CROSS, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ezb);
+    if (ezb > 48 * 1024) {
+        cudaFuncSetAttribute(k_adj_rec<ADJ_BIL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ezb);
+        cudaFuncSetAttribute(k_adj_rec<ADJ_CROSS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ezb);
     }
     if (mode == ADJ_BIL) {
-        if (f)
-            k_adj_rec<ADJ_BIL, float><<<g, 128, ezb, E.stream>>>(E.kp, s0, s1, a, bvec, SA, SB, ebw, grad, phi);
-        else
-            k_adj_rec<ADJ_BIL, double><<<g, 128, 0, E.stream>>>(E.kp, s0, s1, a, bvec, SA, SB, ebw, grad, phi);
-        k_adj_rfin<ADJ_BIL><<<g2, 128, 0, E.stream>>>(E.kp, s0, s1, ns, ebw, grad, phi);
+        k_adj_rec<ADJ_BIL><<<g, 128, ezb, E.stream>>>(E.kp, s0, s1, a, bvec, SA, SB, ebw, grad, phi);
+        k_adj_rfin<ADJ_BIL><<<g2, 128, 0, E.stream>>>(E.kp, s0, s1, ns, ebw, 1.0, grad, phi);
     } else {
-        if (f)
-            k_adj_rec<ADJ_CROSS, float><<<g, 128, ezb, E.stream>>>(E.kp, s0, s1, a, bvec, SA, SB, ebw, grad, phi);
-        else
-            k_adj_rec<ADJ_CROSS, double><<<g, 128, 0, E.stream>>>(E.kp, s0, s1, a, bvec, SA, SB, ebw, grad, phi);
-        k_adj_rfin<ADJ_CROSS><<<g2, 128, 0, E.stream>>>(E.kp, s0, s1, ns, ebw, grad, phi);
+        k_adj_rec<ADJ_CROSS><<<g, 128, ezb, E.stream>>>(E.kp, s0, s1, a, bvec, SA, SB, ebw, grad, phi);
+        k_adj_rfin<ADJ_CROSS><<<g2, 128, 0, E.stream>>>(E.kp, s0, s1, ns, ebw, 1.0, grad, phi);
     }
     E.nlaunch += 2;
 }

@@ -31,6 +31,7 @@
 // exy T, ex ey and w z are 64-bit integer ones (six or three 32-bit multiply-adds), digits are cut
 // and joined in integers, and a (site, run) takes two FP64 FMAs.
 #include <algorithm>
+#include <cstring>
 #include <cuda_fp16.h>
 #include <type_traits>
 #include <vector>
@@ -494,13 +495,15 @@ __global__ void __launch_bounds__(32 * DG_SW) k_dg_sfac(KP kp, DgArgs a, int nks
     dg_build_v<2>(kp, a, b, slot0, DG_SLOTS, w, pm, vmax, a.V, a.vexp);
 }
 
-// V of the force pass's dipole half, from the charge and dipole structure factors together
-__global__ void __launch_bounds__(128) k_dg_vqd(KP kp, DgArgs a) {
+// V of a dipole-force pass, from the structure factor A (and B added to it, if given); the second
+// set (blockIdx.z = 1) from A2
+__global__ void __launch_bounds__(128) k_dg_vqd(KP kp, DgArgs a, const double2 *A, const double2 *B, const double2 *A2) {
     const int b = blockIdx.y, slot0 = blockIdx.x * DG_SLOTS, nsl = min(DG_SLOTS, a.nslot - slot0), LZ = 2 * kp.lmax + 1;
-    extern __shared__ double dsm[];
+    extern __shared__ __align__(128) double dsm[];
     double2 *w = reinterpret_cast<double2 *>(dsm);
     double *pm = reinterpret_cast<double *>(w + (size_t)DG_SLOTS * LZ);
     __shared__ int vmax[DG_SLOTS * 3];
+    if (blockIdx.z) A = A2, B = nullptr;
     for (int i = threadIdx.x; i < DG_SLOTS * LZ; i += blockDim.x) {
         const int sl = i / LZ, kz = i - sl * LZ - kp.lmax;
         double2 v = make_double2(0.0, 0.0);
@@ -508,15 +511,17 @@ __global__ void __launch_bounds__(128) k_dg_vqd(KP kp, DgArgs a) {
             const int4 r = a.slot[slot0 + sl];
             if (kz >= r.z && kz < r.z + r.w) {
                 const int k = a.slotk[slot0 + sl] + kz - r.z;
-                const double2 sq = kp.Sq[(size_t)b * kp.nk + k], sm = kp.Sm[(size_t)b * kp.nk + k];
+                const double2 x = A[(size_t)b * kp.nk + k], y = B ? B[(size_t)b * kp.nk + k] : make_double2(0.0, 0.0);
                 const double c = kp.kinfo[k].w;
-                v = make_double2(c * (sq.x + sm.x), -c * (sq.y + sm.y));
+                v = make_double2(c * (x.x + y.x), -c * (x.y + y.y));
             }
         }
         w[i] = v;
     }
     __syncthreads();
-    dg_build_v<3>(kp, a, b, slot0, DG_SLOTS, w, pm, vmax, a.Vd, a.vdexp);
+    const size_t set = blockIdx.z;
+    dg_build_v<3>(kp, a, b, slot0, DG_SLOTS, w, pm, vmax, a.Vd + set * kp.P * a.nvd8 * a.ksf * (DG_VT / 16),
+                  a.vdexp + set * kp.P * a.nslotp * 3);
 }
 
 // ---- field -----------------------------------------------------------------------------------
@@ -529,7 +534,8 @@ __global__ void __launch_bounds__(128) k_dg_vqd(KP kp, DgArgs a) {
 // (dipole_check.cuh), so that an iteration needs no finishing launch; else k_field_finish adds them.
 enum { DGF_E = 0, DGF_Q = 1, DGF_QG = 2, DGF_DG = 3 };
 template <int MODE, int KS, bool XC>
-__global__ void __launch_bounds__(128, 4) k_dg_field(KP kp, DgArgs a, int s0, int s1, int tshift, int sor) {
+__global__ void __launch_bounds__(128, 4) k_dg_field(KP kp, DgArgs a, int s0, int s1, int tshift, int sor,
+                                                      const double *dip2) {
     const int b = blockIdx.y;
     if (MODE == DGF_E && bead_converged(kp, b)) {
         // (the block still counts towards the convergence test, once for its sites)
@@ -543,11 +549,14 @@ __global__ void __launch_bounds__(128, 4) k_dg_field(KP kp, DgArgs a, int s0, in
     const int mt = (s0 >> 4) + blockIdx.x * 4 + (threadIdx.x >> 5);
     const bool work = 16 * mt < s1;
     const int nv8 = DG ? a.nvd8 : a.nv8;
-    const int n0 = (int)((long)blockIdx.z * nv8 / gridDim.z), n1 = (int)((long)(blockIdx.z + 1) * nv8 / gridDim.z);
+    // (DGF_DG with a second set: its slices are the upper half of the grid)
+    const int half = DG && dip2 ? gridDim.z / 2 : gridDim.z, set = (int)blockIdx.z >= half, zs = blockIdx.z - set * half;
+    const int n0 = (int)((long)zs * nv8 / half), n1 = (int)((long)(zs + 1) * nv8 / half);
     const uint4 *Q = reinterpret_cast<const uint4 *>(reinterpret_cast<const char *>(a.Qd) + ((size_t)b * a.nst + (work ? mt : 0)) * a.ksf * DG_QT) + lane;
     const int tile = a.ksf * (DG_VT / 16);
-    const uint4 *V = (DG ? a.Vd : a.V) + (size_t)b * nv8 * tile;
-    const int *vexp = (DG ? a.vdexp : a.vexp) + (size_t)b * a.nslotp * (DG ? 3 : 2);
+    const uint4 *V = (DG ? a.Vd : a.V) + ((size_t)set * kp.P + b) * nv8 * tile;
+    const int *vexp = (DG ? a.vdexp : a.vexp) + ((size_t)set * kp.P + b) * a.nslotp * (DG ? 3 : 2);
+    const double *dip = set ? dip2 : kp.dip;
     auto load = [&](int n8) {
         uint4 *dst = fring + (n8 % DG_FST) * tile;
         for (int i = threadIdx.x; i < tile; i += 128) dg_cp16(dst + i, V + (size_t)n8 * tile + i);
@@ -681,7 +690,7 @@ __global__ void __launch_bounds__(128, 4) k_dg_field(KP kp, DgArgs a, int s0, in
             const double r1x = __shfl_down_sync(0xffffffffu, acc[h][0], 1), r1y = __shfl_down_sync(0xffffffffu, acc[h][1], 1);
             const double r2 = __shfl_down_sync(0xffffffffu, acc[h][0], 2);
             if (q != 0 || !in[h]) continue;
-            const double mu[3] = {kp.dip[3 * gs], kp.dip[3 * gs + 1], kp.dip[3 * gs + 2]};
+            const double mu[3] = {dip[3 * gs], dip[3 * gs + 1], dip[3 * gs + 2]};
             o[0] = -(mu[0] * acc[h][0] + mu[1] * acc[h][1] + mu[2] * r1x);
             o[1] = -(mu[0] * acc[h][1] + mu[1] * acc[h][2] + mu[2] * r1y);
             o[2] = -(mu[0] * r1x + mu[1] * r1y + mu[2] * r2);
@@ -793,12 +802,13 @@ int dg_init(Engine &E) {
         cut(a.xbad, P * sizeof(int));
         cut(a.fcnt, P * (size_t)(a.nst / 4 + 2) * sizeof(unsigned));
         cut(a.vexp, P * a.nslotp * 2 * sizeof(int));
-        cut(a.vdexp, P * a.nslotp * 3 * sizeof(int));
+        cut(a.vdexp, 2 * P * a.nslotp * 3 * sizeof(int));
         cut(a.Xd, (size_t)a.xsteps * per_step);
         cut(a.Zd, P * zt * DG_ZT);
         cut(a.Qd, P * a.nst * a.ksf * (size_t)DG_QT);
         cut(a.V, P * a.nv8 * a.ksf * (size_t)DG_VT);
-        if (nd) cut(a.Vd, P * a.nvd8 * a.ksf * (size_t)DG_VT);
+        // (two sets where the differentiation form may run)
+        if (nd) cut(a.Vd, (kp.model == 3 ? 2 : 1) * P * a.nvd8 * a.ksf * (size_t)DG_VT);
         if (nd && E.dg_xall) cut(a.exyc, P * a.nslot * (size_t)nd * sizeof(int4));
         cut(a.tab, P * (size_t)kp.ntab * kp.S * sizeof(int4));
         if (pass == 0) {
@@ -807,15 +817,16 @@ int dg_init(Engine &E) {
         }
     }
     if (!nd || !E.dg_xall) a.exyc = nullptr;
-    cudaMemcpy(d_slot, slot.data(), sizeof(int4) * a.nslot, cudaMemcpyHostToDevice);
-    cudaMemcpy(d_slotk, slotk.data(), sizeof(int) * a.nslot, cudaMemcpyHostToDevice);
-    cudaMemcpy(d_slotkv, slotkv.data(), sizeof(double2) * a.nslot, cudaMemcpyHostToDevice);
+    // the host tables and the zeroed words after them in one copy
+    const size_t head = reinterpret_cast<char *>(a.vexp) - base;
+    std::vector<char> img(head, 0);
+    std::memcpy(img.data(), slot.data(), sizeof(int4) * a.nslot);
+    std::memcpy(img.data() + (reinterpret_cast<char *>(d_slotk) - base), slotk.data(), sizeof(int) * a.nslot);
+    std::memcpy(img.data() + (reinterpret_cast<char *>(d_slotkv) - base), slotkv.data(), sizeof(double2) * a.nslot);
+    cudaMemcpy(base, img.data(), head, cudaMemcpyHostToDevice);
     a.slot = d_slot;
     a.slotk = d_slotk;
     a.slotkv = d_slotkv;
-    cudaMemset(a.zexp, 0, P * sizeof(int));
-    cudaMemset(a.xbad, 0, P * sizeof(int));
-    cudaMemset(a.fcnt, 0, P * (size_t)(a.nst / 4 + 2) * sizeof(unsigned));
     const int lim = DG_SMEM;
     if ((size_t)DG_FST * a.ksf * DG_VT > 48 * 1024) {  // |kz| > 63: the field's V ring
         cudaFuncSetAttribute(k_dg_field<DGF_E, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
@@ -902,7 +913,7 @@ void launch_dg_sfac(Engine &E, int op, int s0, int nsites, int skipconv) {
 }
 
 template <int MODE>
-static int field(Engine &E, int s0, int s1, int sor) {
+static int field(Engine &E, int s0, int s1, int sor, const double *dip2 = nullptr) {
     const KP &kp = E.kp;
     const DgArgs &a = E.dg;
     const int mb = ceil_div(ceil_div(s1, 16) - s0 / 16, 4), tiles = MODE == DGF_DG ? a.nvd8 : a.nv8;
@@ -911,20 +922,22 @@ static int field(Engine &E, int s0, int s1, int sor) {
     const long base = (long)mb * kp.P, room = 152L * 4;
     int ns = 1;
     double best = 1e300;
-    for (int c = 1; c <= std::max(1, std::min(E.max_slices, tiles / 4)); c++) {
+    const int most = dip2 ? E.max_slices / 2 : E.max_slices;
+    for (int c = 1; c <= std::max(1, std::min(most, tiles / 4)); c++) {
         const double t = (double)((base * c + room - 1) / room) / c;
         if (t < best - 1e-12) best = t, ns = c;
     }
     const size_t smem = (size_t)DG_FST * a.ksf * DG_VT;
+    if (dip2) ns *= 2;  // (the two sets' slices, ns of each)
     const dim3 g(mb, kp.P, ns);
     // |T| <= sqrt(2) lmax of the run's scale: keep t below 2^62
     const int tshift = a.jn > 32 ? 3 : 0;
     const bool xc = (MODE == DGF_E || MODE == DGF_DG) && E.dg_xdip && a.exyc && s0 == kp.fd && s1 == kp.ld;
 #define PIMD_DGF(KS)                                                               \
     if (xc)                                                                        \
-        k_dg_field<MODE, KS, MODE == DGF_E || MODE == DGF_DG><<<g, 128, smem, E.stream>>>(kp, a, s0, s1, tshift, sor); \
+        k_dg_field<MODE, KS, MODE == DGF_E || MODE == DGF_DG><<<g, 128, smem, E.stream>>>(kp, a, s0, s1, tshift, sor, dip2); \
     else                                                                           \
-        k_dg_field<MODE, KS, false><<<g, 128, smem, E.stream>>>(kp, a, s0, s1, tshift, sor)
+        k_dg_field<MODE, KS, false><<<g, 128, smem, E.stream>>>(kp, a, s0, s1, tshift, sor, dip2)
     if (a.ksf == 1) {
         PIMD_DGF(1);
     } else if (a.ksf == 2) {
@@ -944,11 +957,18 @@ int launch_dg_field(Engine &E, int mode, int s0, int s1, int part) {
     if (mode == F_D) return field<DGF_E>(E, s0, s1, part == 0);
     if (mode == F_Q) return field<DGF_Q>(E, s0, s1, 0);
     if (part == 0) return field<DGF_QG>(E, s0, s1, 0);
+    return launch_dg_dforce(E, E.kp.Sq, E.kp.Sm, nullptr, nullptr);
+}
+
+// Force on the dipoles kp.dip in the field of the structure factor A (+ B), at the dipole sites, and
+// with A2 that on the dipoles dip2 in the field of A2: the slices' sums in Fpart, their number.
+int launch_dg_dforce(Engine &E, const double2 *A, const double2 *B, const double2 *A2, const double *dip2) {
     const DgArgs &a = E.dg;
+    if (dip2 && E.max_slices < 2) return 0;
     const size_t smem = sizeof(double2) * ((size_t)DG_SLOTS * (2 * E.kp.lmax + 1) + (size_t)DG_SLOTS * a.jn * 2);
-    k_dg_vqd<<<dim3(a.nslotp / DG_SLOTS, E.kp.P), 128, smem, E.stream>>>(E.kp, a);
+    k_dg_vqd<<<dim3(a.nslotp / DG_SLOTS, E.kp.P, A2 ? 2 : 1), 128, smem, E.stream>>>(E.kp, a, A, B, A2);
     ++E.nlaunch;
-    return field<DGF_DG>(E, s0, s1, 0);
+    return field<DGF_DG>(E, E.kp.fd, E.kp.ld, 0, dip2);
 }
 
 }  // namespace pimd
