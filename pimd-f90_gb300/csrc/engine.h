@@ -299,7 +299,6 @@ struct Engine {
     double *d_md = nullptr;   // device MD state for the host-array step (pimd_md_step)
     std::vector<void *> allocs;
     std::string last_error;
-    int last_niter_max = 0;
     long long nlaunch = 0;  // kernels launched by this context
     // CUDA-graph execution of the MD step (pimd_set_graph): captured once per set of device
     // pointers and replayed; the dipole iterations run in a conditional while node
@@ -432,6 +431,13 @@ int create_context(Engine &E, const pimd_params *p, int nrep, const int *brep);
 void timer_begin(Engine &E, const char *name);
 void timer_end(Engine &E);
 int run_forces(Engine &E, int t, int check_every, double *Upott, double *virialt, double *virialct, double *virt9);
+// the force calls of n contexts in one capture (capi.cu)
+struct AllConv {
+    const int *flag[32];
+    int n;
+};
+int capture_forces(Engine *const *ctx, int n, double *const *out, cudaStream_t st, cudaStream_t body_st, cudaEvent_t fork,
+                   const cudaEvent_t *join, std::string *why);
 
 // differentiation form (adjoint.cu)
 void tape_record(Engine &E, int iter);

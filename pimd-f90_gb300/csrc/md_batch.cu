@@ -7,8 +7,8 @@
 // those replicas in one launch; the normal-mode, thermostat and kick work of all replicas (own P,
 // own NM matrices and Langevin coefficients at its own temperature) runs in one launch per phase
 // of the step, each block on one replica's atoms. A step of the whole batch is one CUDA graph:
-// the integrator up to the force call, one branch per box group on its own stream (each with its
-// dipole loop as a conditional while node), then the integrator after it and the step outputs.
+// the integrator up to the force call, the force calls as one branch per box group before, in and
+// after one dipole loop (a conditional while node), then the integrator and the step outputs.
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -48,7 +48,7 @@ struct pimd_batch {
     std::vector<BatchReplica> reps;
     pimd_md_params mp{};
     int device = 0;
-    cudaStream_t stream = nullptr;
+    cudaStream_t stream = nullptr, body_stream = nullptr;
     cudaEvent_t ev_fork = nullptr;
     std::vector<cudaEvent_t> ev_join;
     cudaGraphExec_t gexec = nullptr;
@@ -115,23 +115,25 @@ static int capture_batch(pimd_batch *bt) {
     if (e != cudaSuccess) return bcuda(bt, e, "batch capture");
     cudaMemsetAsync(bt->d_uk, 0, sizeof(double) * bt->reps.size(), bt->stream);
     nm_launch_md_batch(0, bt->fast, bt->nblk, bt->smem, bt->stream, bt->d_reps, bt->d_blkmap);
-    cudaEventRecord(bt->ev_fork, bt->stream);
     int rc = PIMD_OK;
-    for (size_t gi = 0; gi < bt->groups.size() && !rc; gi++) {
-        BatchGroup &g = bt->groups[gi];
+    std::vector<Engine *> ctx;
+    std::vector<double *> out;
+    std::vector<char> timers;
+    for (BatchGroup &g : bt->groups) {
         Engine &E = g.ctx->E;
-        cudaStreamWaitEvent(E.stream, bt->ev_fork, 0);
         if (!E.body_stream) cudaStreamCreateWithFlags(&E.body_stream, cudaStreamNonBlocking);
-        const bool timers_on = E.timers.on;
+        timers.push_back(E.timers.on);
         E.timers.on = false;
         E.capturing = true;
-        double *d = E.d_out;  // Upott, virialt, virialct of all beads of the group
-        rc = run_forces(E, 0, 0, d, d + g.Ptot, d + 2 * g.Ptot, nullptr);
-        if (rc) bt->err = E.last_error;
+        ctx.push_back(&E);
+        out.push_back(E.d_out);  // Upott, virialt, virialct of all beads of the group
+    }
+    rc = capture_forces(ctx.data(), (int)ctx.size(), out.data(), bt->stream, bt->body_stream, bt->ev_fork, bt->ev_join.data(), &bt->err);
+    for (size_t gi = 0; gi < bt->groups.size(); gi++) {
+        Engine &E = *ctx[gi];
         E.capturing = false;
-        E.timers.on = timers_on;
-        cudaEventRecord(bt->ev_join[gi], E.stream);
-        cudaStreamWaitEvent(bt->stream, bt->ev_join[gi], 0);
+        E.kp.dd_async = 0;
+        E.timers.on = timers[gi] != 0;
     }
     nm_launch_md_batch(1, bt->fast, bt->nblk, bt->smem, bt->stream, bt->d_reps, bt->d_blkmap);
     k_md_sum_batch<<<(unsigned)bt->reps.size(), 32, 0, bt->stream>>>(bt->d_sums);
@@ -194,6 +196,7 @@ int pimd_batch_create(pimd_batch **out, const pimd_params *common, const pimd_re
         bt->reps.push_back(br);
     }
     if (!rc) rc = bcuda(bt, cudaStreamCreateWithFlags(&bt->stream, cudaStreamNonBlocking), "stream");
+    if (!rc) rc = bcuda(bt, cudaStreamCreateWithFlags(&bt->body_stream, cudaStreamNonBlocking), "stream");
     if (!rc) rc = bcuda(bt, cudaEventCreateWithFlags(&bt->ev_fork, cudaEventDisableTiming), "event");
     if (!rc) rc = balloc(bt, &bt->d_out4, 4 * (size_t)nrep);
     if (!rc) rc = balloc(bt, &bt->d_uk, (size_t)nrep);
@@ -312,6 +315,7 @@ int pimd_batch_destroy(pimd_batch *bt) {
     for (cudaEvent_t e : bt->ev_join) cudaEventDestroy(e);
     if (bt->ev_fork) cudaEventDestroy(bt->ev_fork);
     if (bt->stream) cudaStreamDestroy(bt->stream);
+    if (bt->body_stream) cudaStreamDestroy(bt->body_stream);
     delete bt;
     return PIMD_OK;
 }
