@@ -184,6 +184,16 @@ static int setup_kspace(Engine &E, const pimd_params *p) {
     return cuda_check(E, cudaGetLastError(), "k-space upload");
 }
 
+// the second stream of the force call and of the dipole iterations, with their events
+static cudaError_t overlap_init(Engine &E) {
+    cudaError_t e = cudaSuccess;
+    for (cudaStream_t *s : {&E.aux_stream, &E.loop_aux})
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(s, cudaStreamNonBlocking);
+    for (cudaEvent_t *v : {&E.ev_fork, &E.ev_join, &E.loop_fork, &E.loop_join, &E.ev_check[0], &E.ev_check[1]})
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(v, cudaEventDisableTiming);
+    return e;
+}
+
 static int create(Engine &E, const pimd_params *p, int nrep, const int *brep) {
     if (!p || p->natoms <= 0 || p->natoms % 3 || p->nbeads < 1) return fail(E, PIMD_ERR_ARG, "natoms/nbeads");
     if (p->pot_model < 2 || p->pot_model > 5) return fail(E, PIMD_ERR_ARG, "pot_model must be 2, 3, 4 or 5");
@@ -344,7 +354,7 @@ static int create(Engine &E, const pimd_params *p, int nrep, const int *brep) {
         (rc = dalloc(E, &kp.acc, P * NACC)) || (rc = dalloc(E, &kp.err, 1)) || (rc = dalloc(E, &kp.allconv, 1)) ||
         (rc = dalloc(E, &kp.dstep, 2)) || (rc = dalloc(E, &kp.fin_counter, 1)) ||
         (rc = dalloc(E, &kp.nbrtmp, P * N)) || (rc = dalloc(E, &E.d_out, 3 * P + 16)) ||
-        (rc = dalloc(E, &kp.Fpart, (size_t)E.max_slices * P * S)))
+        (rc = dalloc(E, &kp.Fpart, (size_t)E.max_slices * P * S * (E.precision == PIMD_MIXED ? 1 : 2))))
         return rc;
     if (E.precision == PIMD_MIXED) {
         kp.fcap = (int)std::min(2.0 * E.cap, (double)kp.N * (kp.N - 1));
@@ -382,7 +392,7 @@ static int create(Engine &E, const pimd_params *p, int nrep, const int *brep) {
     cudaMemset(kp.Sm, 0, sizeof(double2) * P * kp.nk);
     if (kp.Wf) cudaMemset(kp.Wf, 0, sizeof(float2) * P * 2 * kp.nk);
     cudaMemset(kp.err, 0, sizeof(unsigned));
-    if ((rc = cuda_check(E, cudaMallocHost((void **)&E.h_allconv, sizeof(int)), "cudaMallocHost"))) return rc;
+    if ((rc = cuda_check(E, cudaMallocHost((void **)&E.h_allconv, 4 * sizeof(int)), "cudaMallocHost"))) return rc;
     cudaMemset(kp.dstep, 0, sizeof(int) * 2);
     cudaMemset(kp.fin_counter, 0, sizeof(unsigned));
     if (nrep > 1) {
@@ -394,6 +404,7 @@ static int create(Engine &E, const pimd_params *p, int nrep, const int *brep) {
     pot_init_constants(E);
     ewald_init(E);
     if (E.precision != PIMD_MIXED && dg_init(E)) return fail(E, PIMD_ERR_NOMEM, "cudaMalloc");
+    if (!spc && (rc = cuda_check(E, overlap_init(E), "streams"))) return rc;
     if (E.precision == PIMD_MIXED && (rc = cuda_check(E, mixed_init(E), "mixed tables"))) return rc;
     neighbors_init(E);
     if (kp.model == 3) adjoint_init(E);
@@ -505,6 +516,20 @@ static void dipole_iteration(Engine &E, bool mixed, bool body_start = false) {
         if (E.kp.dd_async || E.dd_jpev_armed) cudaStreamWaitEvent(E.stream, E.loop_join, 0);
         return;
     }
+    if (!mixed && E.loop_aux && E.dd_overlap) {
+        // FP64: the pair field (FP64 pipe, atomics) beside the structure factor (tensor cores)
+        cudaEventRecord(E.loop_fork, E.stream);
+        cudaStreamWaitEvent(E.loop_aux, E.loop_fork, 0);
+        cudaStream_t keep = E.stream;
+        E.stream = E.loop_aux;
+        PHASE("dd_real", launch_dd_real(E));
+        E.stream = keep;
+        cudaEventRecord(E.loop_join, E.loop_aux);
+        PHASE("dd_smu", launch_ewald_smu(E));
+        cudaStreamWaitEvent(E.stream, E.loop_join, 0);
+        PHASE("dd_update", launch_dd_update(E));
+        return;
+    }
     if (mixed)
         PHASE("dd_real", launch_dd_real_m(E));
     else
@@ -564,6 +589,8 @@ static int capture_dipole_loop(Engine &E) {
 static bool force_overlap(const Engine &E) {
     return E.precision == PIMD_MIXED && E.ewald_overlap && E.aux_stream && E.kp.Fx && E.tc_ready && E.tf_ready && E.ff_tc;
 }
+
+static bool overlap64(const Engine &E) { return E.precision != PIMD_MIXED && E.ewald_overlap && E.aux_stream; }
 
 // One force call for all beads of the context (pot_ttm.f90:3-630 per bead): the part before the
 // induced-dipole iterations, and (force_after) the part after them. The SPC models have no
@@ -630,13 +657,34 @@ static void force_before(Engine &E, int t) {
         PHASE("pair_qq", launch_pair_qq_m(E));
         if (!nbe) PHASE("dd_tensors", launch_dd_tensors_m(E));
     } else {
+        // FP64: the reciprocal charge passes (tensor cores) on the second stream beside the
+        // neighbour list and the pair sums (FP64 pipe); what adds to F runs after both
+        const bool ov = overlap64(E);
+        cudaStream_t keep = E.stream;
+        if (ov) {
+            cudaEventRecord(E.ev_fork, E.stream);
+            cudaStreamWaitEvent(E.aux_stream, E.ev_fork, 0);
+            E.stream = E.aux_stream;
+            E.fin_defer = true;
+            PHASE("ewald_tables", launch_ewald_tables(E));
+            PHASE("ewald_sq", launch_ewald_sq(E));
+            PHASE("ewald_fq", launch_ewald_fq(E));
+            PHASE("dd_x", launch_dg_dipoles(E));
+            E.fin_defer = false;
+            E.stream = keep;
+            cudaEventRecord(E.ev_join, E.aux_stream);
+        }
         PHASE("neighbors", launch_neighbors(E));
         PHASE("pair_qq", launch_pair_qq(E));
+        if (ov) {
+            cudaStreamWaitEvent(E.stream, E.ev_join, 0);
+            PHASE("ewald_fin", launch_field_finish(E));
+        }
     }
     if (ovq) {
         cudaStreamWaitEvent(E.stream, E.ev_join, 0);
         kp.fx_mode = 1;
-    } else {
+    } else if (mixed || !overlap64(E)) {
         PHASE("ewald_tables", launch_ewald_tables(E));
         PHASE("ewald_sq", launch_ewald_sq(E));
         PHASE("ewald_fq", launch_ewald_fq(E));
@@ -644,7 +692,7 @@ static void force_before(Engine &E, int t) {
     PHASE("after_qq", launch_after_qq(E));
     kp.fx_mode = 0;
     if (E.tape_on) tape_record(E, 0);
-    if (!mixed) PHASE("dd_x", launch_dg_dipoles(E));
+    if (!mixed && !overlap64(E)) PHASE("dd_x", launch_dg_dipoles(E));
     kp.dd_async = (mixed && dd_async_ok(E)) ? 1 : 0;
 }
 
@@ -669,6 +717,19 @@ static void force_after(Engine &E, double *Upott, double *virialt, double *viria
             PHASE("pair_force", launch_pair_force_m(E));
             cudaStreamWaitEvent(E.stream, E.ev_join, 0);
             kp.fx_mode = 2;
+        } else if (overlap64(E)) {
+            cudaEventRecord(E.ev_fork, E.stream);
+            cudaStreamWaitEvent(E.aux_stream, E.ev_fork, 0);
+            cudaStream_t keep = E.stream;
+            E.stream = E.aux_stream;
+            E.fin_defer = true;
+            PHASE("ewald_qd", launch_ewald_qd(E));
+            E.fin_defer = false;
+            E.stream = keep;
+            cudaEventRecord(E.ev_join, E.aux_stream);
+            PHASE("pair_force", launch_pair_force(E));
+            cudaStreamWaitEvent(E.stream, E.ev_join, 0);
+            PHASE("ewald_fin", launch_field_finish(E));
         } else {
             if (mixed)
                 PHASE("pair_force", launch_pair_force_m(E));
@@ -695,17 +756,29 @@ int run_forces(Engine &E, int t, int check_every, double *Upott, double *virialt
             return rc;
         }
     } else {
-        int iter = 1;
-        for (; iter <= kp.polar_maxiter; iter++) {
+        // the convergence flag of an iteration is looked at after the next one has been launched (its
+        // kernels return at each converged bead's flag), so the GPU does not wait for the host: with a
+        // copy and a synchronisation an iteration of one bead of 128 molecules took 60 us instead of 40
+        kp.allconv_h = E.h_allconv;
+        int seen = 0;  // flags recorded so far
+        for (int iter = 1; iter <= kp.polar_maxiter; iter++) {
             dipole_iteration(E, mixed);
             if (E.tape_on) tape_record(E, iter);
             if (check_every > 0 && (iter % check_every) == 0 && iter < kp.polar_maxiter) {
-                cudaMemcpyAsync(E.h_allconv, kp.allconv, sizeof(int), cudaMemcpyDeviceToHost, E.stream);
-                cudaError_t e = cudaStreamSynchronize(E.stream);
-                if (e != cudaSuccess) return cuda_check(E, e, "dipole iteration");
-                if (*E.h_allconv) break;
+                cudaEventRecord(E.ev_check[seen & 1], E.stream);
+                if (seen > 0) {
+                    const int before = iter - check_every;
+                    cudaError_t e = cudaEventSynchronize(E.ev_check[(seen - 1) & 1]);
+                    if (e != cudaSuccess) {
+                        kp.allconv_h = nullptr;
+                        return cuda_check(E, e, "dipole iteration");
+                    }
+                    if (((volatile int *)E.h_allconv)[before & 3]) break;
+                }
+                seen++;
             }
         }
+        kp.allconv_h = nullptr;
     }
     force_after(E, Upott, virialt, virialct, virt9);
     return cuda_check(E, cudaGetLastError(), "force kernels");
@@ -840,6 +913,8 @@ int pimd_destroy(pimd_ctx *ctx) {
     if (E.ev_nbr) cudaEventDestroy(E.ev_nbr);
     if (E.loop_aux) cudaStreamDestroy(E.loop_aux);
     if (E.loop_fork) cudaEventDestroy(E.loop_fork);
+    for (cudaEvent_t ev : E.ev_check)
+        if (ev) cudaEventDestroy(ev);
     if (E.loop_pev) cudaEventDestroy(E.loop_pev);
     if (E.loop_jpev) cudaEventDestroy(E.loop_jpev);
     if (E.loop_join) cudaEventDestroy(E.loop_join);

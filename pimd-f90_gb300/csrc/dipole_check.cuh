@@ -31,6 +31,7 @@ PIMD_D void dd_check_block(const KP &kp, double eps) {
     __syncthreads();
     if (threadIdx.x == 0) {
         *kp.allconv = (nconv == kp.P) ? 1 : 0;
+        if (kp.allconv_h) *(volatile int *)(kp.allconv_h + (iter & 3)) = (nconv == kp.P) ? 1 : 0;
         kp.dstep[1] = iter;
         if (kp.cond) cudaGraphSetConditional(kp.cond, nconv == kp.P ? 0u : 1u);
     }

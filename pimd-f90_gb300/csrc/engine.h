@@ -158,6 +158,7 @@ struct KP {
     double *acc;
     unsigned *err;
     int *allconv;
+    int *allconv_h;               // eager loop: the same in host memory, by iteration modulo 4
     const int *brep;              // replica of each bead when one context holds several ring
                                   // polymers (null: one replica); RRc and posc are per replica
     int nrep;                     // replicas in this context (>= 1)
@@ -294,7 +295,8 @@ struct Engine {
     // host pinned staging
     double *h_pin = nullptr;
     size_t h_pin_bytes = 0;
-    int *h_allconv = nullptr;
+    int *h_allconv = nullptr;            // [4] pinned: all beads converged after iteration i, at i % 4
+    cudaEvent_t ev_check[2] = {nullptr, nullptr};  // the last two iterations the eager loop may look at
     double *d_out = nullptr;  // small device staging for per-bead scalar outputs
     double *d_md = nullptr;   // device MD state for the host-array step (pimd_md_step)
     std::vector<void *> allocs;
@@ -305,8 +307,15 @@ struct Engine {
     bool graph_mode = false;
     bool capturing = false;
     cudaStream_t body_stream = nullptr;
-    // mixed engine: a second stream on which the real-space dipole field of an iteration runs
-    // beside the structure factor (fork / join events; branches of the graph when captured)
+    // a second stream on which the real-space dipole field of an iteration runs beside the structure
+    // factor (fork / join events; branches of the graph when captured)
+    // FP64 field passes on the second stream leave adding their slices to F and dR for after the join
+    struct FieldFinish {
+        int mode, s0, s1, ns;
+        double4_32a *part;
+    };
+    bool fin_defer = false;
+    std::vector<FieldFinish> fin;
     cudaStream_t aux_stream = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     cudaEvent_t ev_nbr = nullptr;  // the neighbour lists built on the second stream beside k_sites
@@ -482,6 +491,7 @@ void launch_ewald_sq(Engine &E);
 void launch_ewald_fq(Engine &E);
 void launch_ewald_smu(Engine &E);
 void launch_ewald_qd(Engine &E);
+void launch_field_finish(Engine &E);  // the deferred ones (fin)
 void launch_ewald_pw(Engine &E);
 // tensor-core structure factors (ewald_tc.cu): setup once per context; per call the launch
 // writes the sums of op (OP_Q: Sq + charge weights, OP_MU: Sm + dipole weights, OP_DIP: Sdip)

@@ -1035,6 +1035,30 @@ static void launch_field_f(Engine &E, int s0, int s1) {
     E.nlaunch += 2;
 }
 
+// FP64 field passes: add the slices' sums to F and dR now, or (fin_defer) when launch_field_finish is
+// called, on the stream of then
+static void field_finish(Engine &E, const Engine::FieldFinish &f) {
+    KP kp = E.kp;
+    kp.Fpart = f.part;
+    const dim3 g((f.s1 - f.s0 + 127) / 128, kp.P);
+    if (f.mode == F_Q)
+        k_field_finish<F_Q, 128><<<g, 128, 0, E.stream>>>(kp, f.s0, f.s1, f.ns);
+    else
+        k_field_finish<F_QD, 128><<<g, 128, 0, E.stream>>>(kp, f.s0, f.s1, f.ns);
+    ++E.nlaunch;
+}
+static void finish_or_defer(Engine &E, int mode, int s0, int s1, int ns) {
+    const Engine::FieldFinish f{mode, s0, s1, ns, E.kp.Fpart};
+    if (E.fin_defer)
+        E.fin.push_back(f);
+    else
+        field_finish(E, f);
+}
+void launch_field_finish(Engine &E) {
+    for (const Engine::FieldFinish &f : E.fin) field_finish(E, f);
+    E.fin.clear();
+}
+
 template <int MODE>
 static void run_field(Engine &E, int s0, int s1) {
     const int LZ = 2 * E.kp.lmax + 1;
@@ -1062,12 +1086,13 @@ static void run_field(Engine &E, int s0, int s1) {
     } else {
         const int ns = launch_dg_field(E, MODE, s0, s1, 0);
         if (MODE == F_D) return;  // (the update is part of the pass)
-        k_field_finish<MODE, 128><<<dim3((s1 - s0 + 127) / 128, E.kp.P), 128, 0, E.stream>>>(E.kp, s0, s1, ns);
-        ++E.nlaunch;
+        finish_or_defer(E, MODE, s0, s1, ns);
         if (MODE == F_QD) {  // the dipole half of the force pass, at the dipole sites
-            const int d0 = E.kp.fd, d1 = E.kp.ld, nd = launch_dg_field(E, MODE, d0, d1, 1);
-            k_field_finish<MODE, 128><<<dim3((d1 - d0 + 127) / 128, E.kp.P), 128, 0, E.stream>>>(E.kp, d0, d1, nd);
-            ++E.nlaunch;
+            double4_32a *keep = E.kp.Fpart;
+            if (E.fin_defer) E.kp.Fpart += (size_t)ns * E.kp.P * (s1 - s0);  // (the charge half's sums wait there)
+            const int d0 = E.kp.fd, d1 = E.kp.ld;
+            finish_or_defer(E, MODE, d0, d1, launch_dg_field(E, MODE, d0, d1, 1));
+            E.kp.Fpart = keep;
         }
     }
 }
