@@ -326,12 +326,15 @@ static int create(Engine &E, const pimd_params *p, int nrep, const int *brep) {
     kp_float_tables(kp);
     kp.stath = DEBYE / CHARGECON / std::sqrt((double)kp.natoms);
     kp.factor = 4.0 * (a * a * a) / (3.0 * std::sqrt(PI));
+    const double eps = kp.polar_eps / kp.stath;
+    kp.dsq_eps = kp.polar_eps > 0 ? std::max(eps * eps, 4.9406564584124654e-324) : -1.0;
     // neighbour-list capacity: 3x the expected O-O pairs, at most all pairs
     const double shell = 4.0 / 3.0 * PI * p->rc * p->rc * p->rc / kp.volume;
     const double est = 0.5 * kp.N * (double)kp.N * shell;
     const double all = 0.5 * kp.N * (double)(kp.N - 1);
     E.cap = (size_t)std::max(1.0, std::min(all, std::max(1024.0, 3.0 * est)));
     kp.cap = (int)E.cap;
+    E.pair_est = std::min(all, est);
     const size_t P = kp.P, S = kp.S, N = kp.N;
     const int nsq = kp.S - kp.fq, nsd = kp.ld - kp.fd;
     // structure-factor partials: at most one site group per 32-site tile, at most 32 groups, and
@@ -514,6 +517,15 @@ static void dipole_iteration(Engine &E, bool mixed, bool body_start = false) {
         PHASE("dd_update", launch_dd_update(E));  // includes the convergence test (last block)
         E.field_needs_join = false;
         if (E.kp.dd_async || E.dd_jpev_armed) cudaStreamWaitEvent(E.stream, E.loop_join, 0);
+        return;
+    }
+    if (!mixed && dg_small(E)) {
+        // FP64, bound by latency: the real-space field in Z's launch, three launches an iteration, each
+        // started while the one before ends (not the first one after something else on the stream)
+        E.dg_chain = body_start ? 1 : 2;
+        PHASE("dd_smu", launch_ewald_smu(E));
+        PHASE("dd_update", launch_dd_update(E));
+        E.dg_chain = 0;
         return;
     }
     if (!mixed && E.loop_aux && E.dd_overlap) {
@@ -762,7 +774,7 @@ int run_forces(Engine &E, int t, int check_every, double *Upott, double *virialt
         kp.allconv_h = E.h_allconv;
         int seen = 0;  // flags recorded so far
         for (int iter = 1; iter <= kp.polar_maxiter; iter++) {
-            dipole_iteration(E, mixed);
+            dipole_iteration(E, mixed, !mixed && (iter == 1 || E.tape_on));
             if (E.tape_on) tape_record(E, iter);
             if (check_every > 0 && (iter % check_every) == 0 && iter < kp.polar_maxiter) {
                 cudaEventRecord(E.ev_check[seen & 1], E.stream);
@@ -1152,7 +1164,7 @@ int pimd_get_dipole_info(pimd_ctx *ctx, int bead, int *niter, double *deltadip) 
     int rc = cuda_check(E, cudaStreamSynchronize(E.stream), "get_dipole_info");
     if (rc) return rc;
     if (niter) *niter = (int)a[ACC_NITER];
-    if (deltadip) *deltadip = a[ACC_DELTADIP];
+    if (deltadip) *deltadip = ctx->E.kp.stath * std::sqrt(a[ACC_DELTADIP]);
     return PIMD_OK;
 }
 

@@ -9,7 +9,7 @@ namespace pimd {
 // is done at convergence (1) or at polar_maxiter (2). The iteration number comes from the
 // device step word, which this advances; inside a CUDA graph it also sets the conditional of
 // the dipole loop (continue while some bead is not done).
-PIMD_D void dd_check_block(const KP &kp, double eps) {
+PIMD_D void dd_check_block(const KP &kp) {
     __shared__ int nconv;
     const int iter = kp.dstep[1] + 1;
     if (threadIdx.x == 0) nconv = 0;
@@ -18,11 +18,12 @@ PIMD_D void dd_check_block(const KP &kp, double eps) {
         // the sums arrived by atomics from other blocks: read through L2
         double *a = kp.acc + (size_t)b * NACC;
         if (__ldcg(a + ACC_CONV) == 0.0) {
-            const double dd = kp.stath * sqrt(__ldcg(a + ACC_DSQ));
+            const double dsq = __ldcg(a + ACC_DSQ);  // (compared squared: no square root here)
+            const bool conv = dsq < kp.dsq_eps;
             a[ACC_UIND] = -0.5 * __ldcg(a + ACC_MUEFQ);
             a[ACC_NITER] = (double)iter;
-            a[ACC_DELTADIP] = dd;
-            if (dd < eps || iter >= kp.polar_maxiter) a[ACC_CONV] = (dd < eps) ? 1.0 : 2.0;
+            a[ACC_DELTADIP] = dsq;  // pimd_get_dipole_info takes stath sqrt of it
+            if (conv || iter >= kp.polar_maxiter) a[ACC_CONV] = conv ? 1.0 : 2.0;
             a[ACC_DSQ] = 0.0;
             a[ACC_MUEFQ] = 0.0;
         }
@@ -121,7 +122,7 @@ PIMD_D void dd_block_end(const KP &kp, int b, const double (&av)[2], bool add, u
         __syncthreads();
         if (last) {
             __threadfence();
-            dd_check_block(kp, kp.polar_eps);
+            dd_check_block(kp);
             if (threadIdx.x == 0) *kp.fin_counter = 0u;
         }
     }

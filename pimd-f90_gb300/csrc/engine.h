@@ -78,6 +78,7 @@ struct KP {
     int ndd;             // dipole site pairs per molecule pair (TTM3 1, TTM2 9)
     int contraction, guess, t, polar_maxiter, same_acd;
     double polar_eps;
+    double dsq_eps;      // |dmu|^2 below which stath |dmu| < polar_eps (negative: never)
     double box[3], boxi[3], volume, rc2, rc1;
     float boxq[3];  // box / 2^32 (FP32): the length of one unit of ofix
     double vdwA, vdwB, vdwC, vdwD, vdwE, shiftA, shiftB;
@@ -287,7 +288,9 @@ struct Engine {
     DgArgs dg;                 // FP64 engine: digit operands of the reciprocal sums
     bool dg_xall = false;      // the X buffer holds the dipole sites of every bead
     bool dg_xdip = false;      // ... and does so for this force call's positions
+    int dg_chain = 0;          // small system's iteration: 1 the first of a loop (body), 2 after another
     size_t cap = 0;
+    double pair_est = 0;       // O-O pairs expected per bead
     std::vector<KRun> h_runs;
     std::vector<KChunk> h_chunks;
     std::vector<int> h_khkl;
@@ -509,6 +512,7 @@ int launch_field_qd_tc(Engine &E, int s0, int s1);  // ewald_std_qd force pass o
 // digit-product reciprocal sums of the FP64 engine (ewald_dg.cu)
 int dg_init(Engine &E);                  // 0, or 1 when a buffer could not be allocated
 void launch_dg_tables(Engine &E);        // after the ssincos tables
+bool dg_small(const Engine &E);          // its dipole iterations run as chained launches
 void launch_dg_dipoles(Engine &E);       // X of the dipole sites, before the dipole iterations
 void launch_dg_sfac(Engine &E, int op, int s0, int nsites, int skipconv);
 int launch_dg_field(Engine &E, int mode, int s0, int s1, int part);

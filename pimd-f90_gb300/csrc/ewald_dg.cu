@@ -36,6 +36,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "dd_real.cuh"
 #include "dipole_check.cuh"
 #include "engine.h"
 #include "umma.cuh"
@@ -201,12 +202,27 @@ __global__ void __launch_bounds__(128) k_dg_x(KP kp, DgArgs a, int s0, int nsite
     *reinterpret_cast<uint2 *>(o + 1536 + 8 * lane) = make_uint2(d0[6], d1[6]);
 }
 
+// ---- programmatic dependent launch ---------------------------------------------------------------
+// In small systems an iteration's kernels are chained so: a kernel starts while the one before ends,
+// does what does not depend on it, and waits (no effect on a launch without the attribute).
+PIMD_D void dg_after_prior() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+PIMD_D void dg_next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Z: the weights of a bead's sites times the kz tables. Items (j, c), eight a tile, cos in the rows
 // 0-7 and sin in 8-15. The scale is the bead's largest weight, which every block finds for itself.
-template <int NC>
-__global__ void __launch_bounds__(256) k_dg_z(KP kp, DgArgs a, int s0, int nsites, int nks, int nmt, int skipconv) {
+// REAL (2 TTM2.1-F, 3 TTM3-F): the blocks from nzb on take the iteration's real-space dipole field,
+// which needs the same dipoles (small systems: one launch less).
+template <int NC, int REAL>
+__global__ void __launch_bounds__(256) k_dg_z(KP kp, DgArgs a, int s0, int nsites, int nks, int nmt, int skipconv, int nzb) {
     const int b = blockIdx.y;
+    dg_next_may_start();
+    dg_after_prior();
     if (skipconv && bead_converged(kp, b)) return;
+    if (REAL && (int)blockIdx.x >= nzb) {
+        // (half a block's threads: FP64 instructions wait for their sub-partition, more blocks spread them)
+        if (threadIdx.x < 128) dd_real_pairs<REAL ? REAL : 3>(kp, b, (blockIdx.x - nzb) * 128 + threadIdx.x, (gridDim.x - nzb) * 128);
+        return;
+    }
     __shared__ int smax;
     if (threadIdx.x == 0) smax = 0;
     __syncthreads();
@@ -223,7 +239,7 @@ __global__ void __launch_bounds__(256) k_dg_z(KP kp, DgArgs a, int s0, int nsite
     const int e = dg_exp(smax);
     if (blockIdx.x == 0 && threadIdx.x == 0) a.zexp[b] = e;
     const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-    const int units = nmt * nks, step = gridDim.x * 8;
+    const int units = nmt * nks, step = nzb * 8;
     for (int u = blockIdx.x * 8 + (threadIdx.x >> 5); u < units; u += step) {
         const int mt = u / nks, ks = u - mt * nks;
         const int item = 8 * mt + g, j = NC == 1 ? item : item / NC, c = NC == 1 ? 0 : item - NC * j;
@@ -360,7 +376,7 @@ template <int OP>
 __global__ void __launch_bounds__(32 * DG_SW) k_dg_sfac(KP kp, DgArgs a, int nks, int nmt, int ksum, int b0, int skipconv, int soff) {
     constexpr int NC = OP == OP_Q ? 1 : 3;
     const int xb = blockIdx.y, b = b0 + xb;
-    if (skipconv && bead_converged(kp, b)) return;
+    dg_next_may_start();
     const int slot0 = blockIdx.x * DG_SLOTS, nsl = min(DG_SLOTS, a.nslot - slot0);
     const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int LZ = 2 * kp.lmax + 1, nitem = NC * a.jn;
@@ -375,11 +391,19 @@ __global__ void __launch_bounds__(32 * DG_SW) k_dg_sfac(KP kp, DgArgs a, int nks
     __shared__ int vmax[DG_SLOTS * 2];
     const int4 first = a.slot[slot0];
     const int mts = min(nmt, (NC * (first.z + first.w) + 7) / 8);  // kzlo + nkz = longest |kz| + 1
+    if (threadIdx.x < DG_ST) umma::mbar_init(&full[threadIdx.x], 1);
+    for (int i = threadIdx.x; i < nsl * LZ; i += blockDim.x) {  // the epilogue's reads, to L2 / L1
+        const int sl = i / LZ, kz = i - sl * LZ - kp.lmax;
+        const int4 r = a.slot[slot0 + sl];
+        if (kz >= r.z && kz < r.z + r.w)
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(kp.kinfo + a.slotk[slot0 + sl] + kz - r.z));
+    }
+    dg_after_prior();
+    if (skipconv && bead_converged(kp, b)) return;
     const int ze = a.zexp[b];
     const bool bad = ze == DG_BAD || a.xbad[b];
     const char *Zb = reinterpret_cast<const char *>(a.Zd) + (size_t)b * nmt * nks * DG_ZT;
     const char *X = reinterpret_cast<const char *>(a.Xd) + ((size_t)xb * (a.nx8 / 2) + blockIdx.x) * nks * (2 * DG_XT);
-    if (threadIdx.x < DG_ST) umma::mbar_init(&full[threadIdx.x], 1);
     __syncthreads();
     int it = 0, late = 0;  // steps taken (over all rounds), waits that gave up
     for (int m0 = 0; m0 < mts; m0 += nw) {
@@ -537,12 +561,7 @@ template <int MODE, int KS, bool XC>
 __global__ void __launch_bounds__(128, 4) k_dg_field(KP kp, DgArgs a, int s0, int s1, int tshift, int sor,
                                                       const double *dip2) {
     const int b = blockIdx.y;
-    if (MODE == DGF_E && bead_converged(kp, b)) {
-        // (the block still counts towards the convergence test, once for its sites)
-        const double zero[2] = {0.0, 0.0};
-        if (sor && blockIdx.z == 0) dd_block_end<128>(kp, b, zero, false, gridDim.x * gridDim.y);
-        return;
-    }
+    dg_next_may_start();
     constexpr bool DG = MODE == DGF_DG;
     extern __shared__ uint4 fring[];  // [DG_FST][ksf][96]
     const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
@@ -561,11 +580,6 @@ __global__ void __launch_bounds__(128, 4) k_dg_field(KP kp, DgArgs a, int s0, in
         uint4 *dst = fring + (n8 % DG_FST) * tile;
         for (int i = threadIdx.x; i < tile; i += 128) dg_cp16(dst + i, V + (size_t)n8 * tile + i);
     };
-#pragma unroll
-    for (int k = 0; k < DG_FST - 1; k++) {
-        if (n0 + k < n1) load(n0 + k);
-        dg_commit();
-    }
     uint4 A[KS > 0 ? KS : 1][DG_FN];
     if (KS > 0) {
 #pragma unroll
@@ -586,6 +600,18 @@ __global__ void __launch_bounds__(128, 4) k_dg_field(KP kp, DgArgs a, int s0, in
     if (XC) {
 #pragma unroll
         for (int h = 0; h < 2; h++) xn[h] = xc[(size_t)slot_of(n0) * (s1 - s0) + (in[h] ? site[h] - s0 : 0)];
+    }
+    dg_after_prior();
+    if (MODE == DGF_E && bead_converged(kp, b)) {
+        // (the block still counts towards the convergence test, once for its sites)
+        const double zero[2] = {0.0, 0.0};
+        if (sor && blockIdx.z == 0) dd_block_end<128>(kp, b, zero, false, gridDim.x * gridDim.y);
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < DG_FST - 1; k++) {
+        if (n0 + k < n1) load(n0 + k);
+        dg_commit();
     }
     for (int n8 = n0; n8 < n1; n8++) {
         const int slc = slot_of(n8);
@@ -747,6 +773,32 @@ __global__ void __launch_bounds__(128, 4) k_dg_field(KP kp, DgArgs a, int s0, in
 // ---- host --------------------------------------------------------------------------------------
 static int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
+// a launch that may start while the one before it on the stream ends (dg_after_prior)
+template <typename K, typename... A>
+static void launch_pdl(bool on, K kernel, dim3 g, int nt, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = g;
+    c.blockDim = dim3(nt);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = on ? 1 : 0;
+    cudaLaunchKernelEx(&c, kernel, args...);
+}
+
+// Small systems, whose iterations are bound by latency: one launch for Z and the real-space field, the
+// three launches of an iteration chained (one bead of 128 molecules 1.40 -> 1.24 ms a call; not inside
+// a graph, whose plain edges are faster: 101 x 7 0.52 ms a step, 0.59 with programmatic ones). By the
+// pairs' work: at 100 thousand tensors the real-space
+// field takes about 8 us, as long as Z; beyond, it runs on the second stream beside the structure
+// factor (512 x 32: 850 thousand, 58 us).
+bool dg_small(const Engine &E) {
+    return E.precision != PIMD_PREC_MIXED && E.kp.model < 4 && E.dg_xall && E.pair_est * E.kp.P * E.kp.ndd <= 1.0e5;
+}
+
 // Buffers of the context's size. X holds as many beads as fit the limit (a pass over more beads
 // forms X in several parts); the FP64 exy values are kept where X holds all dipole sites.
 int dg_init(Engine &E) {
@@ -877,7 +929,19 @@ static void sfac(Engine &E, int s0, int nsites, int skipconv) {
     // blocks of the Z kernel: enough to fill the chip, few enough that finding the bead's largest
     // weight (each block reads all of them) stays small
     const int upb = std::max(1, (int)((long)nmt * nks * kp.P / (8L * 608)));
-    k_dg_z<NC><<<dim3(ceil_div(ceil_div(nmt * nks, 8), upb), kp.P), 256, 0, E.stream>>>(kp, a, s0, nsites, nks, nmt, skipconv);
+    const int nzb = ceil_div(ceil_div(nmt * nks, 8), upb);
+    const bool chain = OP == OP_MU && E.dg_chain;
+    if (chain) {
+        const int nrb = std::max(1, ceil_div((int)E.pair_est, 128));
+        const dim3 g(nzb + nrb, kp.P);
+        if (kp.model == 2)
+            launch_pdl(E.dg_chain == 2 && !E.capturing, k_dg_z<NC, 2>, g, 256, 0, E.stream, kp, a, s0, nsites, nks, nmt, skipconv, nzb);
+        else
+            launch_pdl(E.dg_chain == 2 && !E.capturing, k_dg_z<NC, 3>, g, 256, 0, E.stream, kp, a, s0, nsites, nks, nmt, skipconv, nzb);
+        E.dg_chain = 2;
+    } else {
+        k_dg_z<NC, 0><<<dim3(nzb, kp.P), 256, 0, E.stream>>>(kp, a, s0, nsites, nks, nmt, skipconv, nzb);
+    }
     ++E.nlaunch;
     // keep the 64-bit sums of all sites below 2^61
     int ksum = 0;
@@ -898,7 +962,7 @@ static void sfac(Engine &E, int s0, int nsites, int skipconv) {
             launch_x(E, s0, nsites, b0, nb, false);
             E.dg_xdip = false;
         }
-        k_dg_sfac<OP><<<dim3(a.nslotp / DG_SLOTS, nb), 32 * nw, smem, E.stream>>>(kp, a, nks, nmt, ksum, b0, skipconv, soff);
+        launch_pdl(chain && !E.capturing, k_dg_sfac<OP>, dim3(a.nslotp / DG_SLOTS, nb), 32 * nw, smem, E.stream, kp, a, nks, nmt, ksum, b0, skipconv, soff);
         ++E.nlaunch;
     }
 }
@@ -933,11 +997,13 @@ static int field(Engine &E, int s0, int s1, int sor, const double *dip2 = nullpt
     // |T| <= sqrt(2) lmax of the run's scale: keep t below 2^62
     const int tshift = a.jn > 32 ? 3 : 0;
     const bool xc = (MODE == DGF_E || MODE == DGF_DG) && E.dg_xdip && a.exyc && s0 == kp.fd && s1 == kp.ld;
-#define PIMD_DGF(KS)                                                               \
-    if (xc)                                                                        \
-        k_dg_field<MODE, KS, MODE == DGF_E || MODE == DGF_DG><<<g, 128, smem, E.stream>>>(kp, a, s0, s1, tshift, sor, dip2); \
-    else                                                                           \
-        k_dg_field<MODE, KS, false><<<g, 128, smem, E.stream>>>(kp, a, s0, s1, tshift, sor, dip2)
+    const bool chain = MODE == DGF_E && sor && E.dg_chain && !E.capturing;
+#define PIMD_DGF(KS)                                                                                                      \
+    if (xc)                                                                                                               \
+        launch_pdl(chain, k_dg_field<MODE, KS, MODE == DGF_E || MODE == DGF_DG>, g, 128, smem, E.stream, kp, a, s0, s1, tshift, \
+                   sor, dip2);                                                                                            \
+    else                                                                                                                  \
+        launch_pdl(chain, k_dg_field<MODE, KS, false>, g, 128, smem, E.stream, kp, a, s0, s1, tshift, sor, dip2)
     if (a.ksf == 1) {
         PIMD_DGF(1);
     } else if (a.ksf == 2) {
