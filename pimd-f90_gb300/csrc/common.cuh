@@ -27,6 +27,21 @@ constexpr double HBAR = 6.35077993041;
 PIMD_D double min_image_rn(double r, double box, double boxi) {
     return __dsub_rn(r, __dmul_rn(box, round(__dmul_rn(r, boxi))));
 }
+PIMD_D int hi_abs(double x) { return __double2hiint(x) & 0x7fffffff; }
+// The same value with the test first: where |r| < box / 2 (the high words compared, exponents one
+// apart) anint(r / box) is 0 and the image is r itself; four FP64 instructions saved, which cost
+// this part 64 cycles a warp each.
+PIMD_D double min_image_fast(double r, double box, double boxi) {
+    return hi_abs(r) < __double2hiint(box) - 0x100000 ? r : min_image_rn(r, box, boxi);
+}
+// 1 / v of a normal v by two Newton iterations r <- r + r (1 - v r) from the hardware's
+// approximation (about 20 bits); below an ulp off
+PIMD_D double rcp_newton(double v) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(v));
+    r = fma(r, fma(-v, r, 1.0), r);
+    return fma(r, fma(-v, r, 1.0), r);
+}
 // Round to the nearest integer, ties to even, for |x| < 2^22: adding and subtracting 1.5 x 2^23
 // leaves an FP32 value whose last place is 1, so the addition rounds x to an integer (the
 // classic magic-number rounding). The same value as rintf(x) on that range, in two FP32 adds.
@@ -261,18 +276,47 @@ PIMD_D void dd_force_f(const float R[3], const float di[3], const float dj[3], f
 }
 
 // ---------------------------------------------------------------------------------------
+// Warp sums of W (a power of two <= 16) doubles a lane: in each of the first steps a lane keeps half of
+// its values and gives the other half away, so that W + 4 - log2 W additions do instead of 5 W (an FP64
+// addition takes a warp 64 cycles here). Returns the sum of value number `at`; lanes differing only in
+// the bits below 32 / W hold the same one.
+template <int W>
+PIMD_D double warp_sums(double (&x)[W], int &at) {
+    const int lane = threadIdx.x & 31;
+    at = 0;
+    int m = W;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if (m > 1) {
+            m >>= 1;
+            const bool up = lane & o;
+            at += up ? m : 0;
+#pragma unroll
+            for (int i = 0; i < W / 2; i++)
+                if (i < m) {
+                    const double give = up ? x[i] : x[i + m], keep = up ? x[i + m] : x[i];
+                    x[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                }
+        } else {
+            x[0] += __shfl_xor_sync(0xffffffffu, x[0], o);
+        }
+    }
+    return x[0];
+}
+
 // block-wide sum of NV doubles into per-bead accumulators (one atomic per value per block)
 template <int NV, int NT>
 PIMD_D void block_reduce_add(double (&v)[NV], double *dst) {
-    __shared__ double red[NT / 32][NV];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int W = NV > 8 ? 16 : NV > 4 ? 8 : NV > 2 ? 4 : NV > 1 ? 2 : 1;
+    static_assert(NV <= 16, "values a lane");
+    __shared__ double red[NT / 32][W];
+    const int warp = threadIdx.x >> 5;
+    double x[W];
 #pragma unroll
-    for (int i = 0; i < NV; i++) {
-        double x = v[i];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-        if (lane == 0) red[warp][i] = x;
-    }
+    for (int i = 0; i < W; i++) x[i] = i < NV ? v[i] : 0.0;
+    int at;
+    const double sum = warp_sums<W>(x, at);
+    if ((threadIdx.x & (32 / W - 1)) == 0) red[warp][at] = sum;
     __syncthreads();
     if (threadIdx.x < NV) {
         double s = 0;

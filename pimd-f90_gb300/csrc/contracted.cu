@@ -5,7 +5,8 @@
 // every bead; the intermolecular (slow) ones on the centroid only, through a one-bead context of
 // the centroid (contraction set for contracted_MD, so pot_ttm skips the monomer PES there,
 // pot_ttm.f90:92-132; unset for monomer_PIMD, whose centroid call keeps it, as the reference's
-// does). The bead monomer kernel is one thread per (molecule, bead); the inner MTS steps are the
+// does). The bead monomer kernel is one thread, in small systems four lanes, per (molecule, bead);
+// the inner MTS steps are the
 // fast kicks, EvolveRing with the normal modes made for deltfast, and the monomer kernel again.
 // The thermostats, kinetic energies and estimators are the MD step's (nm.cu).
 #include <cmath>
@@ -68,18 +69,24 @@ __global__ void k_centroid_pbc(double *RRt, double *RRc, int natoms, int P, doub
 // pot_nasa on every (molecule, bead): the gradient rows into g; with acc, the energies into
 // Upott[bead] and the monomer virials, bead separations into vir2[0] and centroid separations
 // (RRc) into vir2[1] (MD.f90:348-378 / 182-217)
+// L lanes a molecule (lanes_per_molecule)
+template <int L>
 __global__ void __launch_bounds__(128) k_monomer_beads(KP kp, int P, const double *RRt, const double *RRc, double *g,
                                                        double *Upott, double *vir2, int acc) {
-    const int iw = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, N = kp.N, na = 3 * N;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, l = t % L, j = blockIdx.y, N = kp.N, na = 3 * N;
+    const int iw = min(t / L, N - 1);
+    const bool in = t / L < N;
     double e1 = 0.0, v[2] = {0.0, 0.0};
-    if (iw < N) {
-        const double *rb = RRt + (size_t)3 * na * j + 9 * (size_t)iw;
-        double r1[3][3], dr1[3][3];
+    const double *rb = RRt + (size_t)3 * na * j + 9 * (size_t)iw;
+    double r1[3][3], dr1[3][3];
 #pragma unroll
-        for (int a = 0; a < 3; a++)
+    for (int a = 0; a < 3; a++)
 #pragma unroll
-            for (int c = 0; c < 3; c++) r1[a][c] = rb[3 * a + c];
-        nasa_pot(r1, kp.box, kp.boxi, dr1, &e1, kp.c5z, kp.nasa_f5z);
+        for (int c = 0; c < 3; c++) r1[a][c] = rb[3 * a + c];
+    nasa_pot<L>(r1, kp.box, kp.boxi, dr1, &e1, kp.c5z, kp.nasa_f5z, false, l);
+    if (!in || l != 0) {
+        e1 = 0.0;
+    } else {
         double *gb = g + (size_t)3 * na * j + 9 * (size_t)iw;
 #pragma unroll
         for (int a = 0; a < 3; a++)
@@ -92,8 +99,8 @@ __global__ void __launch_bounds__(128) k_monomer_beads(KP kp, int P, const doubl
                 double d1 = 0.0, d2 = 0.0;
 #pragma unroll
                 for (int c = 0; c < 3; c++) {
-                    const double roh1 = min_image_rn(__dsub_rn(rr[3 + c], rr[c]), kp.box[c], kp.boxi[c]);
-                    const double roh2 = min_image_rn(__dsub_rn(rr[6 + c], rr[c]), kp.box[c], kp.boxi[c]);
+                    const double roh1 = min_image_fast(__dsub_rn(rr[3 + c], rr[c]), kp.box[c], kp.boxi[c]);
+                    const double roh2 = min_image_fast(__dsub_rn(rr[6 + c], rr[c]), kp.box[c], kp.boxi[c]);
                     d1 = __dadd_rn(d1, __dmul_rn(roh1, dr1[1][c]));
                     d2 = __dadd_rn(d2, __dmul_rn(roh2, dr1[2][c]));
                 }
@@ -114,24 +121,35 @@ __global__ void __launch_bounds__(128) k_monomer_beads(KP kp, int P, const doubl
     }
 }
 
+static void monomer_beads(const KP &kp, int P, const double *RRt, const double *RRc, double *g, double *Upott, double *vir2,
+                          int acc, cudaStream_t st) {
+    if (lanes_per_molecule(kp.N, P) == 4)
+        k_monomer_beads<4><<<dim3((4 * kp.N + 127) / 128, P), 128, 0, st>>>(kp, P, RRt, RRc, g, Upott, vir2, acc);
+    else
+        k_monomer_beads<1><<<dim3((kp.N + 127) / 128, P), 128, 0, st>>>(kp, P, RRt, RRc, g, Upott, vir2, acc);
+}
+
 // calc_monomer_dip_moments (force_calc.f90:205-264): DMS charges of every bead's monomer, the
 // dipole about the M site (TTM3-F) or the O atom, plus the centroid's induced dipoles dE
+template <int L>
 __global__ void __launch_bounds__(128) k_monomer_dipoles(KP kp, int P, int model, double gammaM, const double *RRt,
                                                          const double *dE, double *dipI, double *dipE) {
-    const int iw = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, N = kp.N, na = 3 * N;
-    if (iw >= N) return;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, l = t % L, j = blockIdx.y, N = kp.N, na = 3 * N;
+    const int iw = min(t / L, N - 1);
     const double *rb = RRt + (size_t)3 * na * j + 9 * (size_t)iw;
     double r1[3][3], q3[3], dq3[3][3][3];
 #pragma unroll
     for (int a = 0; a < 3; a++)
 #pragma unroll
         for (int c = 0; c < 3; c++) r1[a][c] = rb[3 * a + c];
-    nasa_dms(r1, kp.box, kp.boxi, kp.dms1, kp.dms2, kp.dms3, q3, dq3);
+    nasa_dms<L>(r1, kp.box, kp.boxi, kp.dms1, kp.dms2, kp.dms3, q3, dq3, false, l);
+    if (t / L >= N) return;
     const double tmp = 0.5 * gammaM / (1.0 - gammaM);
     for (int a = 0; a < 3; a++) q3[a] = q3[a] * CHARGECON;
     const double cH1 = q3[1] + tmp * (q3[1] + q3[2]), cH2 = q3[2] + tmp * (q3[1] + q3[2]);
 #pragma unroll
     for (int c = 0; c < 3; c++) {
+        if (L > 1 && c != l) continue;  // (a component a lane)
         const double roh1 = min_image_rn(__dsub_rn(rb[3 + c], rb[c]), kp.box[c], kp.boxi[c]);
         const double roh2 = min_image_rn(__dsub_rn(rb[6 + c], rb[c]), kp.box[c], kp.boxi[c]);
         double d;
@@ -248,7 +266,7 @@ int pimd_contracted_step_device(pimd_ctx *ctx, const pimd_md_params *mp, double 
     const double delt = mp->delt, delt2 = delt / 2.0;
     const double deltfast = mode == 0 ? delt / nin : delt, delt2fast = deltfast / 2.0;
     const unsigned gb = (unsigned)std::min<size_t>((nall + 255) / 256, 4096);
-    const dim3 gm((N + 127) / 128, P);
+    const dim3 gm((N + 127) / 128, P), g4((4 * N + 127) / 128, P);
     cudaMemsetAsync(s.Upott, 0, sizeof(double) * (P + 2), st);
     // bead thermostat, global chain, slow half kick, then (monomer PIMD) the drift, and the
     // centroid with its PBC shift
@@ -270,7 +288,7 @@ int pimd_contracted_step_device(pimd_ctx *ctx, const pimd_md_params *mp, double 
             else
                 k_free_flight<<<(3 * na + 255) / 256, 256, 0, st>>>(RRt, PPt, na, mp->massO, mp->massH, deltfast);
             if (ti == nin) cudaMemsetAsync(s.vir2, 0, 2 * sizeof(double), st);
-            k_monomer_beads<<<gm, 128, 0, st>>>(E.kp, P, RRt, RRc, dRRfast, s.Upott, s.vir2, ti == nin);
+            monomer_beads(E.kp, P, RRt, RRc, dRRfast, s.Upott, s.vir2, ti == nin, st);
             k_kick<<<gb, 256, 0, st>>>(PPt, dRRfast, nall, delt2fast);
             E.nlaunch += 3;
         }
@@ -286,13 +304,17 @@ int pimd_contracted_step_device(pimd_ctx *ctx, const pimd_md_params *mp, double 
     }
     if (mode == 1) {  // Upott(:) = Upot, then the monomer PES on the beads
         k_fill<<<1, 32, 0, st>>>(s.Upott, s.cen3, P);
-        k_monomer_beads<<<gm, 128, 0, st>>>(E.kp, P, RRt, RRc, s.dRRmon, s.Upott, s.vir2, 1);
+        monomer_beads(E.kp, P, RRt, RRc, s.dRRmon, s.Upott, s.vir2, 1, st);
         E.nlaunch += 2;
     }
     k_con_totals<<<1, 32, 0, st>>>(P, mode, s.cen3, s.Upott, s.vir2, s.uvv);
     k_broadcast_grad<<<gb, 256, 0, st>>>(dRRt, s.dRRc, mode == 1 ? s.dRRmon : nullptr, na, P);
-    if (dip_momIt || dip_momEt)
-        k_monomer_dipoles<<<gm, 128, 0, st>>>(E.kp, P, E.kp.model, E.kp.gammaM, RRt, s.dE, dip_momIt, dip_momEt);
+    if (dip_momIt || dip_momEt) {
+        if (lanes_per_molecule(E.kp.N, P) == 4)
+            k_monomer_dipoles<4><<<g4, 128, 0, st>>>(E.kp, P, E.kp.model, E.kp.gammaM, RRt, s.dE, dip_momIt, dip_momEt);
+        else
+            k_monomer_dipoles<1><<<gm, 128, 0, st>>>(E.kp, P, E.kp.model, E.kp.gammaM, RRt, s.dE, dip_momIt, dip_momEt);
+    }
     nm_launch_ring_sums(a, st, RRt, PPt, E.d_nh + 5);
     // slow half kick, bead thermostat, kinetic energy, global chain
     double *uk = E.d_out + 3 * P;

@@ -92,7 +92,7 @@ struct KP {
     PairTables pt;
     GqBounds gq;     // FP64 pair kernels: Q(2/3, x)'s numbers of terms, 1 / Gamma(2/3)
     double gq_norm;
-    int box49[3];    // high words of 0.49 box edges: |r| below needs no minimum image
+    int box49[3], box51[3], box149[3];  // high words of 0.49, 0.51, 1.49 box edges (min_image_near)
     // buffers
     const double *RRt, *RRc;
     double *dRRt, *dipI, *dipE, *chg;
@@ -466,6 +466,10 @@ void adj_rec(Engine &E, int mode, const double *a, const double *bvec, const dou
 void neighbors_init(Engine &E);
 void launch_neighbors(Engine &E);
 bool nbr_from_inputs(const Engine &E);
+// Lanes per molecule of the FP64 monomer kernels: with a lane each, 608 sub-partitions of 32 lanes
+// take 19456 molecules; up to a quarter of that four lanes are shorter (measured: 128 x 1, 101 x 7,
+// 128 x 16; at 128 x 32 and 512 x 32 one lane)
+inline int lanes_per_molecule(int N, int P) { return (long)N * P <= 4096 ? 4 : 1; }
 // launchers (pot.cu)
 void pot_init_constants(Engine &E);
 void launch_sites(Engine &E);

@@ -6,21 +6,13 @@
 
 namespace pimd {
 
-PIMD_D int hi_abs(double x) { return __double2hiint(x) & 0x7fffffff; }
-
-// min_image_rn(r, box) where |r| may reach half the box, r itself where it cannot (the same value:
-// there anint(r / box) is 0)
+// min_image_rn(r, box) by the cell r lies in, where that is beyond doubt: anint(r / box) is 0 below 0.49
+// box edges and +-1 between 0.51 and 1.49, so the same value with at most one FP64 operation
 PIMD_D double min_image_near(double r, const KP &kp, int c) {
-    return hi_abs(r) >= kp.box49[c] ? min_image_rn(r, kp.box[c], kp.boxi[c]) : r;
-}
-
-// 1 / v of a normal v by two Newton iterations r <- r + r (1 - v r) from the hardware's
-// approximation (about 20 bits); below an ulp off
-PIMD_D double rcp_newton(double v) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(v));
-    r = fma(r, fma(-v, r, 1.0), r);
-    return fma(r, fma(-v, r, 1.0), r);
+    const int h = hi_abs(r);
+    if (h < kp.box49[c]) return r;
+    if (h >= kp.box51[c] && h < kp.box149[c]) return __dsub_rn(r, copysign(kp.box[c], r));
+    return min_image_rn(r, kp.box[c], kp.boxi[c]);
 }
 
 // the undamped screened interaction at r^2 = d2 (smear.f90:10-18): 1/r, r, 1/r^2, exp(-a^2 r^2),
@@ -82,13 +74,12 @@ PIMD_D void pair_block_sums(const double (&vt)[6], double vc, double uv, double 
     long long any = 0;
 #pragma unroll
     for (int i = 0; i < 8; i++) any |= __double_as_longlong(v[i]) << 1;
-    const bool some = __any_sync(0xffffffffu, any != 0);
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        if (some)
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
-        if (lane == 0) red[wp][i] = v[i];
+    if (__any_sync(0xffffffffu, any != 0)) {
+        int at;
+        const double s = warp_sums<8>(v, at);
+        if ((lane & 3) == 0) red[wp][at] = s;
+    } else if (lane < 8) {
+        red[wp][lane] = 0.0;
     }
     __syncthreads();
     if (threadIdx.x < 8) {

@@ -1,6 +1,7 @@
-// pairs.cu -- real-space charge sums of the FP64 engine: O-O van der Waals and the site pairs of
-// every neighbour pair (pot_ttm.f90:159-228, pot_spc.f90:142-191), and the dipole tensors of the
-// induced-dipole iterations (pot_ttm.f90:311-342).
+// pairs.cu -- real-space sums of the FP64 engine: O-O van der Waals and the charges' site pairs of
+// every neighbour pair (pot_ttm.f90:159-228, pot_spc.f90:142-191) with the dipole tensors of the
+// induced-dipole iterations (pot_ttm.f90:311-342), and the forces on charges and dipoles
+// (pot_ttm.f90:399-542).
 //
 // Bound by FP64 instructions (two lanes a cycle and SM; conversions, compares and shuffled adds
 // count too), so the kernel is built to issue few of them:
@@ -306,12 +307,12 @@ __global__ void __launch_bounds__(PQ_NT) k_pair_qq(KP kp) {
 }
 
 // Chunks of NI rounds where they fill the chip, of one round where they do not; blocks for one
-// pass over the expected pairs (a third of the list capacity), at most about five a SM, so that a
+// pass over the expected pairs, at most about five a SM, so that a
 // block's closing sums are few.
 template <int MODEL>
 static void pair_qq(Engine &E) {
     constexpr int NI = MODEL == 2 ? 4 : 3, PW = 32 / NI;
-    const long est = std::max(1L, (long)(E.cap / 3)), P = E.kp.P;
+    const long est = std::max(1L, (long)E.pair_est), P = E.kp.P;
     const long full = (est + 4L * PW * NI - 1) / (4L * PW * NI);
     if (full * P >= 2 * 152) {
         const long nb = std::max(1L, std::min(full, (152L * 5 + P - 1) / P));
@@ -330,6 +331,201 @@ void launch_pair_qq(Engine &E) {
         pair_qq<3>(E);
     else
         pair_qq<4>(E);
+}
+
+// pot_ttm.f90:399-542: real-space forces on charges and dipoles (charge-dipole and dipole-dipole), the
+// dipole part of phi, and the intramolecular terms. A lane takes one site pair: TTM3-F five a molecule
+// pair (H1 M, H2 M, M M, M H1, M H2: six pairs a warp), TTM2.1-F sixteen (two pairs a warp, M M idle);
+// the sites' sums are formed by shuffles and added with one atomic a component. Bound by FP64
+// instructions like the charge sums; a thread per pair, with exponentials and divisions of its own for
+// each term, took 1520 us at TTM3-F 512 x 32, 917 us at TTM2.1-F 128 x 32 and 80 us at 128 x 1.
+template <int MODEL>
+PIMD_D void force_term(const KP &kp, const double (&R)[3], double d2, int ka, int kb, double q1, double q2, const double (&m1)[3],
+                       const double (&m2)[3], double (&f)[3], double &p1, double &p2) {
+    const bool dd = MODEL == 2 ? (ka < 3 && kb < 3) : (ka == 3 && kb == 3);
+    PairR pr;
+    pair_r(d2, kp.ew, pr);
+    const double t2 = (pr.t1 + kp.ew.cts2 * pr.g) * pr.drsqi;
+    double c1 = pr.t1, c2 = t2, d2t = t2, d3t = (t2 + kp.ew.cts3 * pr.g) * pr.drsqi;
+    if (__double2hiint(d2) < 0x40390000) {  // r < 5 A: the Thole factors (smear.f90:36-107)
+        const double r3 = pr.dd * d2, r3i = pr.dri * pr.drsqi;
+        const double a = kp.pt.apol_cd[ka + 1][kb + 1], e = exp(-r3 * a), s2 = (e * r3i + e * a) * pr.drsqi;
+        c1 -= e * r3i;
+        c2 -= s2;
+        if (dd) {
+            const double ad = kp.pt.apol_dd[ka + 1][kb + 1], ed = kp.same_acd ? e : exp(-r3 * ad);
+            const double sd = kp.same_acd ? s2 : (ed * r3i + ed * ad) * pr.drsqi;
+            d2t -= sd;
+            d3t -= (sd + 0.6 * ed * pr.dd * ad * ad) * pr.drsqi;
+        }
+    }
+    f[0] = f[1] = f[2] = p1 = p2 = 0.0;
+    if (dd) dd_force(R, m1, m2, d2t, d3t, f);
+    const double qd[3] = {q2 * m1[0] - q1 * m2[0], q2 * m1[1] - q1 * m2[1], q2 * m1[2] - q1 * m2[2]};
+    if (qd[0] * qd[0] + qd[1] * qd[1] + qd[2] * qd[2] > 1.e-9) {
+        const double w = 3.0 * c2 * (R[0] * qd[0] + R[1] * qd[1] + R[2] * qd[2]);
+#pragma unroll
+        for (int c = 0; c < 3; c++) f[c] += w * R[c] - c1 * qd[c];
+        p1 = c1 * (R[0] * m2[0] + R[1] * m2[1] + R[2] * m2[2]);
+        p2 = -c1 * (R[0] * m1[0] + R[1] * m1[1] + R[2] * m1[2]);
+    }
+}
+
+template <int MODEL>
+__global__ void __launch_bounds__(PQ_NT) k_pair_force(KP kp) {
+    constexpr int NL = MODEL == 2 ? 16 : 5, PW = 32 / NL;  // lanes a pair, pairs a warp
+    const int b = blockIdx.y, N = kp.N, lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int np = kp.npair[b], nwarp = gridDim.x * (PQ_NT / 32), w0 = blockIdx.x * (PQ_NT / 32) + wp;
+    const double4_32a *pos = kp.pos + (size_t)b * kp.S, *posc = posc_of(kp, b);
+    const double *dip = kp.dip + (size_t)b * kp.S * 3;
+    double *dR = kp.dR + (size_t)b * kp.S * 3;
+    double4_32a *Fb = kp.F + (size_t)b * kp.S;
+    double av[14];
+#pragma unroll
+    for (int i = 0; i < 14; i++) av[i] = 0.0;
+    auto isdip = [](int k) { return MODEL == 2 ? k < 3 : k == 3; };
+    auto site = [&](int k, int mol, double &q, double (&m)[3]) {
+        const size_t s = (size_t)k * N + mol;
+        const double4_32a r = pos[s];
+        q = r.w;
+        m[0] = m[1] = m[2] = 0.0;
+        if (isdip(k))
+#pragma unroll
+            for (int c = 0; c < 3; c++) m[c] = dip[3 * s + c];
+        return r;
+    };
+    auto virial = [&](const double (&f)[3], const double (&R)[3], const double (&Rc)[3]) {
+        av[ACC_VIRIALC] += Rc[0] * f[0] + Rc[1] * f[1] + Rc[2] * f[2];
+#pragma unroll
+        for (int col = 0; col < 3; col++)
+#pragma unroll
+            for (int c = 0; c < 3; c++) av[ACC_VIRT + c + 3 * col] += f[c] * R[col];
+    };
+    const int r = lane % NL;
+    const int ka = MODEL == 2 ? r >> 2 : r < 2 ? r + 1 : 3, kb = MODEL == 2 ? r & 3 : r < 3 ? 3 : r - 2;
+    for (int base = w0 * PW; base < np; base += nwarp * PW) {
+        const int p = base + lane / NL;
+        const bool act = lane < PW * NL && p < np && !(MODEL == 2 && r == 15);
+        int i = 0, j = 0;
+        double f[3] = {0, 0, 0}, p1 = 0.0, p2 = 0.0;
+        if (act) {
+            const int2 ij = kp.pairs[(size_t)b * kp.cap + p];
+            i = ij.x, j = ij.y;
+            double q1, q2, m1[3], m2[3];
+            const double4_32a oi = pos[i], oj = pos[j], s1 = site(ka, i, q1, m1), s2 = site(kb, j, q2, m2);
+            // the separation from the O sites' image (a second one only where a component can need it)
+            const double R[3] = {min_image_near(min_image_near(oi.x - oj.x, kp, 0) + ((s1.x - oi.x) - (s2.x - oj.x)), kp, 0),
+                                 min_image_near(min_image_near(oi.y - oj.y, kp, 1) + ((s1.y - oi.y) - (s2.y - oj.y)), kp, 1),
+                                 min_image_near(min_image_near(oi.z - oj.z, kp, 2) + ((s1.z - oi.z) - (s2.z - oj.z)), kp, 2)};
+            force_term<MODEL>(kp, R, dot3_rn(R[0], R[1], R[2]), ka, kb, q1, q2, m1, m2, f, p1, p2);
+            // (the reference takes the centroids' separation as it is, pot_ttm.f90:468)
+            const double4_32a ca = posc[(size_t)ka * N + i], cb = posc[(size_t)kb * N + j];
+            const double Rc[3] = {ca.x - cb.x, ca.y - cb.y, ca.z - cb.z};
+            virial(f, R, Rc);
+        }
+        double g[4] = {f[0], f[1], f[2], p1}, h[4] = {-f[0], -f[1], -f[2], p2};
+        if (MODEL == 2) {
+#pragma unroll
+            for (int x = 0; x < 4; x++) {
+                g[x] += __shfl_xor_sync(0xffffffffu, g[x], 1);
+                g[x] += __shfl_xor_sync(0xffffffffu, g[x], 2);
+                h[x] += __shfl_xor_sync(0xffffffffu, h[x], 4);
+                h[x] += __shfl_xor_sync(0xffffffffu, h[x], 8);
+            }
+            // sums of site ka of i in the lanes of a row, of site kb of j in those of a column; the lanes
+            // of the diagonal add one of each
+            if (lane / NL + base < np && ka == kb) {
+                const int2 ij = kp.pairs[(size_t)b * kp.cap + base + lane / NL];
+                const size_t s1 = (size_t)ka * N + ij.x, s2 = (size_t)ka * N + ij.y;
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    atomicAdd(dR + 3 * s1 + c, g[c]);
+                    atomicAdd(dR + 3 * s2 + c, h[c]);
+                }
+                if (ka != 0) {
+                    atomicAdd(&Fb[s1].w, g[3]);
+                    atomicAdd(&Fb[s2].w, h[3]);
+                }
+            }
+        } else {
+            // M of i takes lanes 2, 3, 4 of its pair, M of j lanes 0, 1, 2; both in lane 2 (the forces only:
+            // the other lanes have a potential at their own H site or none)
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                const double a = __shfl_down_sync(0xffffffffu, f[c], 1), d = __shfl_down_sync(0xffffffffu, f[c], 2);
+                const double u = __shfl_up_sync(0xffffffffu, f[c], 1), v = __shfl_up_sync(0xffffffffu, f[c], 2);
+                if (r == 2) {
+                    g[c] = f[c] + (a + d);
+                    h[c] = -(f[c] + (u + v));
+                }
+            }
+            const double a = __shfl_down_sync(0xffffffffu, p1, 1), d = __shfl_down_sync(0xffffffffu, p1, 2);
+            const double u = __shfl_up_sync(0xffffffffu, p2, 1), v = __shfl_up_sync(0xffffffffu, p2, 2);
+            if (r == 2) {
+                g[3] = p1 + (a + d);
+                h[3] = p2 + (u + v);
+            }
+            if (act && r <= 2) {
+                const size_t s1 = (size_t)ka * N + i;
+#pragma unroll
+                for (int c = 0; c < 3; c++) atomicAdd(dR + 3 * s1 + c, g[c]);
+                atomicAdd(&Fb[s1].w, g[3]);
+            }
+            if (act && r >= 2) {
+                const size_t s2 = (size_t)kb * N + j;
+#pragma unroll
+                for (int c = 0; c < 3; c++) atomicAdd(dR + 3 * s2 + c, h[c]);
+                atomicAdd(&Fb[s2].w, h[3]);
+            }
+        }
+    }
+    // intramolecular (pot_ttm.f90:482-542): a lane a site pair, six a molecule, five molecules a warp
+    for (int base = w0 * 5; base < N; base += nwarp * 5) {
+        const int w = base + lane / 6, t = lane % 6;
+        if (lane >= 30 || w >= N) continue;
+        const int k1 = t < 3 ? 0 : t < 5 ? 1 : 2, k2 = t < 3 ? t + 1 : t < 5 ? t - 1 : 3;
+        double q1, q2, m1[3], m2[3];
+        const double4_32a s1 = site(k1, w, q1, m1), s2 = site(k2, w, q2, m2);
+        const double4_32a ca = posc[(size_t)k1 * N + w], cb = posc[(size_t)k2 * N + w];
+        const double R[3] = {min_image_near(s1.x - s2.x, kp, 0), min_image_near(s1.y - s2.y, kp, 1), min_image_near(s1.z - s2.z, kp, 2)};
+        const double Rc[3] = {min_image_near(ca.x - cb.x, kp, 0), min_image_near(ca.y - cb.y, kp, 1), min_image_near(ca.z - cb.z, kp, 2)};
+        const double d2 = dot3_rn(R[0], R[1], R[2]);
+        double f[3] = {0, 0, 0};
+        if (isdip(k1) && isdip(k2)) {
+            double t1, t2, t3;
+            smear3<double>(d2, kp.pt.apol_dd[k1 + 1][k2 + 1], kp.ew, &t1, &t2, &t3);
+            dd_force(R, m1, m2, t2, t3, f);
+        }
+        // self2 (smear.f90:133-156): the screened interaction less the whole one
+        PairR pr;
+        pair_r(d2, kp.ew, pr);
+        const double r3i = pr.dri * pr.drsqi, ts1 = pr.t1 - r3i, ts2 = (pr.t1 + kp.ew.cts2 * pr.g) * pr.drsqi - r3i * pr.drsqi;
+        const double qd[3] = {q2 * m1[0] - q1 * m2[0], q2 * m1[1] - q1 * m2[1], q2 * m1[2] - q1 * m2[2]};
+        const double x = 3.0 * ts2 * (R[0] * qd[0] + R[1] * qd[1] + R[2] * qd[2]);
+        const size_t a1 = (size_t)k1 * N + w, a2 = (size_t)k2 * N + w;
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            f[c] += x * R[c] - ts1 * qd[c];
+            atomicAdd(dR + 3 * a1 + c, f[c]);
+            atomicAdd(dR + 3 * a2 + c, -f[c]);
+        }
+        if (k1 != 0) atomicAdd(&Fb[a1].w, ts1 * (R[0] * m2[0] + R[1] * m2[1] + R[2] * m2[2]));
+        atomicAdd(&Fb[a2].w, -ts1 * (R[0] * m1[0] + R[1] * m1[1] + R[2] * m1[2]));
+        virial(f, R, Rc);
+    }
+    block_reduce_add<14, PQ_NT>(av, kp.acc + (size_t)b * NACC);
+}
+
+// Blocks for one pass over the expected pairs, at most about four a SM
+void launch_pair_force(Engine &E) {
+    const long P = E.kp.P, pw = E.kp.model == 2 ? 2 : 6;
+    const long full = std::max((long)(E.kp.N + 19) / 20, (long)(E.pair_est / (4 * pw)) + 1);
+    const dim3 g((unsigned)std::max(1L, std::min(full, (152L * 4 + P - 1) / P)), (unsigned)P);
+    if (E.kp.model == 2)
+        k_pair_force<2><<<g, PQ_NT, 0, E.stream>>>(E.kp);
+    else
+        k_pair_force<3><<<g, PQ_NT, 0, E.stream>>>(E.kp);
+    ++E.nlaunch;
 }
 
 // ---- Q(2/3, x): where the reference's iterations stop --------------------------------------
@@ -393,12 +589,14 @@ void pair_math_init(Engine &E) {
     static const GqBounds bounds = q23_bounds();  // of the reference's algorithm alone
     kp.gq = bounds;
     kp.gq_norm = std::exp(-0.303150275147547);  // 1 / Gamma(2/3) as the reference's gln has it
-    for (int c = 0; c < 3; c++) {
-        const double h = 0.49 * kp.box[c];
-        unsigned long long u;
-        std::memcpy(&u, &h, sizeof u);
-        kp.box49[c] = (int)(u >> 32);
-    }
+    const double at[3] = {0.49, 0.51, 1.49};
+    for (int c = 0; c < 3; c++)
+        for (int i = 0; i < 3; i++) {
+            const double h = at[i] * kp.box[c];
+            unsigned long long u;
+            std::memcpy(&u, &h, sizeof u);
+            (i == 0 ? kp.box49 : i == 1 ? kp.box51 : kp.box149)[c] = (int)(u >> 32);
+        }
 }
 
 }  // namespace pimd

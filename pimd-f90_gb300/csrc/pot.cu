@@ -1,16 +1,15 @@
 // pot.cu -- real-space, monomer and bookkeeping kernels of the TTM2.1-F / TTM3-F force call
 // for all beads at once (FP64). Restates pot_ttm/pot_ttm.f90:3-630 and find_neigh.f90.
 //
-// Work decomposition: the bead is blockIdx.y (or .z) everywhere. Monomer and intramolecular
-// work is one thread per molecule; intermolecular work is one thread per O-O pair of the
-// half neighbour list, accumulating the pair's 4+4 site contributions in registers and
-// issuing one atomic per site component. Energies and virials are reduced per block and
-// added once per block to the per-bead accumulators.
+// Work decomposition: the bead is blockIdx.y (or .z) everywhere. Monomer work is one thread (small
+// FP64 systems: four lanes) per molecule; the pairs' sums are in pairs.cu (FP64) and mixed.cu.
+// Energies and virials are reduced per block and added once per block to the per-bead accumulators.
 #include <cstdio>
 
 #include "dd_real.cuh"
 #include "engine.h"
 #include "nasa.cuh"
+#include "pair_math.cuh"
 
 namespace pimd {
 
@@ -29,9 +28,10 @@ void pot_init_constants(Engine &E) {
 // warps per SM at 512 x 32, spread over every SM.
 constexpr int SITES_NT = 64;
 
-// FSUM: the NASA polynomial sums in FP32 (the mixed engine)
-template <int MODEL, bool FSUM>
+// The mixed engine: the NASA polynomial sums in FP32 (k_sites64 is the FP64 engine's)
+template <int MODEL>
 __global__ void __launch_bounds__(SITES_NT) k_sites(KP kp) {
+    constexpr bool FSUM = true;
     const int w = blockIdx.x * (SITES_NT / 2) + (threadIdx.x & 31);
     const bool pes = threadIdx.x < 32;  // warp-uniform roles
     const int b = blockIdx.y;
@@ -249,6 +249,156 @@ __global__ void __launch_bounds__(SITES_NT) k_sites(KP kp) {
     block_reduce_add<14, SITES_NT>(av, kp.acc + (size_t)b * NACC);
 }
 
+// The same in FP64 (the FP64 engine). A molecule is some 2500 FP64 instructions of 64 cycles a warp,
+// so in small systems a molecule takes L = 4 lanes: they share the polynomial sums, and each does the
+// self energy, exclusions and rows of one site (each exclusion pair twice, its virial at half
+// weight); with enough molecules to fill the chip one lane takes them all. Few FP64 instructions:
+// reciprocals for divisions, minimum images only where needed, the screened interaction of the
+// pair kernels. 128 molecules, one bead: 97 -> 36 us; 512 x 32: 149 -> 95 us.
+template <int MODEL, int L>
+__global__ void __launch_bounds__(SITES_NT) k_sites64(KP kp) {
+    const int lane = threadIdx.x & 31, l = lane % L, b = blockIdx.y, N = kp.N, S = kp.S;
+    const int wm = blockIdx.x * (32 / L) + lane / L, w = min(wm, N - 1);
+    const bool in = wm < N, pes = threadIdx.x < 32;  // warp-uniform roles
+    double av[14];
+#pragma unroll
+    for (int i = 0; i < 14; i++) av[i] = 0.0;
+    const double *RR = kp.RRt + (size_t)b * kp.natoms * 3 + 9 * w;
+    const int rep = rep_of(kp, b);
+    const double *RC = kp.RRc + (size_t)rep * kp.natoms * 3 + 9 * w;
+    const bool first_bead = (b == 0) || (kp.brep && kp.brep[b - 1] != rep);
+    double R[4][3], Rc[4][3], oh[2][3], ohc[2][3];
+    const double hg = 0.5 * kp.gammaM;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            R[k][c] = RR[3 * k + c];
+            Rc[k][c] = RC[3 * k + c];
+        }
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            oh[h][c] = min_image_fast(__dsub_rn(R[1 + h][c], R[0][c]), kp.box[c], kp.boxi[c]);
+            ohc[h][c] = min_image_fast(__dsub_rn(Rc[1 + h][c], Rc[0][c]), kp.box[c], kp.boxi[c]);
+        }
+        R[3][c] = __dadd_rn(__dmul_rn(hg, __dadd_rn(oh[0][c], oh[1][c])), R[0][c]);
+        Rc[3][c] = __dadd_rn(__dmul_rn(hg, __dadd_rn(ohc[0][c], ohc[1][c])), Rc[0][c]);
+    }
+    if (pes) {
+        double dr1[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, e1 = 0.0;
+        if (!kp.contraction) {
+            nasa_pot<L>(R, kp.box, kp.boxi, dr1, &e1, kp.c5z, kp.nasa_f5z, false, l);
+            if (in && l == 0) {
+                av[ACC_UMON] = e1;
+#pragma unroll
+                for (int col = 0; col < 3; col++) {
+#pragma unroll
+                    for (int c = 0; c < 3; c++) av[ACC_VIRT + c + 3 * col] = oh[0][c] * dr1[1][col] + oh[1][c] * dr1[2][col];
+                    av[ACC_VIRIALC] += ohc[0][col] * dr1[1][col] + ohc[1][col] * dr1[2][col];
+                }
+            }
+        }
+        if (in)
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (L > 1 && k != l) continue;
+                const size_t s = (size_t)b * S + k * N + w;
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    kp.dR[3 * s + c] = (k < 3) ? dr1[k < 3 ? k : 0][c] : 0.0;
+                    kp.dip[3 * s + c] = 0.0;
+                    kp.Efdr[3 * s + c] = 0.0;
+                }
+            }
+    } else {
+        double q3[3], dq3[3][3][3];
+        nasa_dms<L>(R, kp.box, kp.boxi, kp.dms1, kp.dms2, kp.dms3, q3, dq3, false, l);
+#pragma unroll
+        for (int k = 0; k < 3; k++) q3[k] *= CHARGECON;
+        const double ig = rcp_newton(1.0 - kp.gammaM), tmp = hg * ig;
+        const double q[4] = {0.0, q3[1] + tmp * (q3[1] + q3[2]), q3[2] + tmp * (q3[1] + q3[2]), q3[0] * ig};
+        if (in) {
+            double *g = kp.grdq + ((size_t)b * N + w) * 27;
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                if (L > 1 && a != l) continue;
+                kp.chg[(size_t)b * kp.natoms + 3 * w + a] = q3[a];
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    const double g0 = dq3[a][0][c] * CHARGECON, g1 = dq3[a][1][c] * CHARGECON, s01 = g0 + g1;
+                    g[9 * a + 0 + c] = g0 + tmp * s01;
+                    g[9 * a + 3 + c] = g1 + tmp * s01;
+                    g[9 * a + 6 + c] = dq3[a][2][c] * CHARGECON - 2.0 * tmp * s01;
+                }
+            }
+            // self energy and intramolecular exclusions (pot_ttm.f90:232-261): site k's row
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (L > 1 && k != l) continue;
+                double Ef[3] = {0, 0, 0}, ph = k == 0 ? 0.0 : -kp.ew.aewald * TSP * q[k];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    if (j == k) continue;
+                    if (MODEL == 3 && (k == 0 || j == 0)) continue;  // O: no charge, and no dipole to see a field
+                    double Rs[3], Rcs[3];
+#pragma unroll
+                    for (int c = 0; c < 3; c++) {
+                        Rs[c] = min_image_fast(__dsub_rn(R[k][c], R[j][c]), kp.box[c], kp.boxi[c]);
+                        Rcs[c] = min_image_fast(__dsub_rn(Rc[k][c], Rc[j][c]), kp.box[c], kp.boxi[c]);
+                    }
+                    PairR pr;
+                    pair_r(dot3_rn(Rs[0], Rs[1], Rs[2]), kp.ew, pr);
+                    const double ts0 = pr.t0 - pr.dri, ts1 = pr.t1 - pr.dri * pr.drsqi;
+                    ph += ts0 * q[j];
+                    const double a = ts1 * q[j], h = -0.5 * a * q[k];
+                    double d[3];
+#pragma unroll
+                    for (int c = 0; c < 3; c++) {
+                        Ef[c] += a * Rs[c];
+                        d[c] = h * Rs[c];
+                        av[ACC_VIRIALC] += Rcs[c] * d[c];
+                    }
+                    av[ACC_VIRT + 0] += d[0] * Rs[0];
+                    av[ACC_VIRT + 4] += d[1] * Rs[1];
+                    av[ACC_VIRT + 8] += d[2] * Rs[2];
+                    av[ACC_VIRT + 1] += d[0] * Rs[1];
+                    av[ACC_VIRT + 2] += d[0] * Rs[2];
+                    av[ACC_VIRT + 5] += d[1] * Rs[2];
+                }
+                const size_t s = (size_t)b * S + k * N + w;
+                kp.pos[s] = make_double4_32a(R[k][0], R[k][1], R[k][2], q[k]);
+                if (first_bead) kp.posc[(size_t)rep * S + k * N + w] = make_double4_32a(Rc[k][0], Rc[k][1], Rc[k][2], 0.0);
+                kp.F[s] = make_double4_32a(Ef[0], Ef[1], Ef[2], ph);
+            }
+            av[ACC_VIRT + 3] = av[ACC_VIRT + 1];  // (symmetric)
+            av[ACC_VIRT + 6] = av[ACC_VIRT + 2];
+            av[ACC_VIRT + 7] = av[ACC_VIRT + 5];
+            if (MODEL == 2) {  // intramolecular dipole tensors (pot_ttm.f90:344-365), cached per molecule
+                int t = 0;
+#pragma unroll
+                for (int i = 0; i < 2; i++)
+#pragma unroll
+                    for (int j = i + 1; j < 3; j++, t++) {
+                        if (L > 1 && t != l) continue;
+                        double Rs[3];
+#pragma unroll
+                        for (int c = 0; c < 3; c++) Rs[c] = min_image_fast(__dsub_rn(R[i][c], R[j][c]), kp.box[c], kp.boxi[c]);
+                        double t1, t2;
+                        smear2<double>(dot3_rn(Rs[0], Rs[1], Rs[2]), kp.pt.apol_dd[i + 1][j + 1], kp.ew, &t1, &t2);
+                        double *T = kp.Tself + (((size_t)b * N + w) * 3 + t) * 6;
+                        T[0] = 3.0 * t2 * Rs[0] * Rs[0] - t1;
+                        T[1] = 3.0 * t2 * Rs[1] * Rs[1] - t1;
+                        T[2] = 3.0 * t2 * Rs[2] * Rs[2] - t1;
+                        T[3] = 3.0 * t2 * Rs[0] * Rs[1];
+                        T[4] = 3.0 * t2 * Rs[0] * Rs[2];
+                        T[5] = 3.0 * t2 * Rs[1] * Rs[2];
+                    }
+            }
+        }
+    }
+    block_reduce_add<14, SITES_NT>(av, kp.acc + (size_t)b * NACC);
+}
+
 // ---------------------------------------------------------------------------------------
 // pot_ttm.f90:273-297: charge forces -q Efq, Uelec, and the initial induced dipoles
 // (polarisability times the charge field, or the 4-step predictor from the history).
@@ -328,181 +478,6 @@ __global__ void k_set_step(int *dstep, int t) {
 }
 
 // ---------------------------------------------------------------------------------------
-
-// pot_ttm.f90:399-542: real-space forces on charges and dipoles (charge-dipole and
-// dipole-dipole), the dipole part of phi, and the intramolecular terms.
-template <int MODEL>
-__global__ void __launch_bounds__(128) k_pair_force(KP kp) {
-    using T = TT<MODEL>;
-    const int b = blockIdx.y, N = kp.N;
-    const int np = kp.npair[b];
-    const double4_32a *pos = kp.pos + (size_t)b * kp.S;
-    const double *dip = kp.dip + (size_t)b * kp.S * 3;
-    double *dR = kp.dR + (size_t)b * kp.S * 3;
-    double4_32a *Fb = kp.F + (size_t)b * kp.S;
-    const bool same_a = kp.same_acd != 0;  // |aCCaCD - aDD| < 1e-12 (pot_ttm.f90:443)
-    double av[14];
-#pragma unroll
-    for (int i = 0; i < 14; i++) av[i] = 0.0;
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < np; p += gridDim.x * blockDim.x) {
-        const int2 ij = kp.pairs[(size_t)b * kp.cap + p];
-        const int i = ij.x, j = ij.y;
-        double4_32a si[5], sj[5];
-#pragma unroll
-        for (int k = 1; k <= 4; k++) {
-            si[k] = pos[(k - 1) * N + i];
-            sj[k] = pos[(k - 1) * N + j];
-        }
-        const double Rij[3] = {min_image_rn(__dsub_rn(si[1].x, sj[1].x), kp.box[0], kp.boxi[0]),
-                               min_image_rn(__dsub_rn(si[1].y, sj[1].y), kp.box[1], kp.boxi[1]),
-                               min_image_rn(__dsub_rn(si[1].z, sj[1].z), kp.box[2], kp.boxi[2])};
-        double Rw[3];
-        Rw[0] = min_image_rn(__dadd_rn(__dsub_rn(Rij[0], si[1].x), sj[1].x), kp.box[0], kp.boxi[0]);
-        Rw[1] = min_image_rn(__dadd_rn(__dsub_rn(Rij[1], si[1].y), sj[1].y), kp.box[1], kp.boxi[1]);
-        Rw[2] = min_image_rn(__dadd_rn(__dsub_rn(Rij[2], si[1].z), sj[1].z), kp.box[2], kp.boxi[2]);
-        double gi[5][3], gj[5][3], pi[5], pj[5];
-#pragma unroll
-        for (int k = 0; k < 5; k++) {
-            gi[k][0] = gi[k][1] = gi[k][2] = gj[k][0] = gj[k][1] = gj[k][2] = 0.0;
-            pi[k] = pj[k] = 0.0;
-        }
-#pragma unroll
-        for (int isp = 1; isp <= 4; isp++) {
-#pragma unroll
-            for (int jsp = 1; jsp <= 4; jsp++) {
-                if (!T::f_active(isp, jsp)) continue;
-                const double Rs[3] = {
-                    min_image_rn(__dsub_rn(__dadd_rn(si[isp].x, Rw[0]), sj[jsp].x), kp.box[0], kp.boxi[0]),
-                    min_image_rn(__dsub_rn(__dadd_rn(si[isp].y, Rw[1]), sj[jsp].y), kp.box[1], kp.boxi[1]),
-                    min_image_rn(__dsub_rn(__dadd_rn(si[isp].z, Rw[2]), sj[jsp].z), kp.box[2], kp.boxi[2])};
-                const double d2 = dot3_rn(Rs[0], Rs[1], Rs[2]);
-                const double qi = si[isp].w, qj = sj[jsp].w;
-                double di[3] = {0, 0, 0}, dj[3] = {0, 0, 0};
-                if (T::dip(isp)) {
-                    const double3 m = ld3(dip + 3 * ((isp - 1) * N + i));
-                    di[0] = m.x, di[1] = m.y, di[2] = m.z;
-                }
-                if (T::dip(jsp)) {
-                    const double3 m = ld3(dip + 3 * ((jsp - 1) * N + j));
-                    dj[0] = m.x, dj[1] = m.y, dj[2] = m.z;
-                }
-                double qd[3];
-#pragma unroll
-                for (int c = 0; c < 3; c++) qd[c] = qj * di[c] - qi * dj[c];
-                const double qd2 = qd[0] * qd[0] + qd[1] * qd[1] + qd[2] * qd[2];
-                double dij[3] = {0, 0, 0};
-                double ts1 = 0.0, ts2 = 0.0;
-                bool have = false;
-                if (T::dip(isp) && T::dip(jsp)) {
-                    double t1, t2, t3;
-                    smear3<double>(d2, kp.pt.apol_dd[isp][jsp], kp.ew, &t1, &t2, &t3);
-                    dd_force(Rs, di, dj, t2, t3, dij);
-                    if (same_a) {
-                        ts1 = t1, ts2 = t2;
-                        have = true;
-                    }
-                }
-                if (qd2 > 1.e-9) {
-                    if (!have) smear2<double>(d2, kp.pt.apol_cd[isp][jsp], kp.ew, &ts1, &ts2);
-                    const double rq = Rs[0] * qd[0] + Rs[1] * qd[1] + Rs[2] * qd[2];
-#pragma unroll
-                    for (int c = 0; c < 3; c++) dij[c] += 3.0 * ts2 * rq * Rs[c] - ts1 * qd[c];
-                    if (isp != 1) pi[isp] += ts1 * (Rs[0] * dj[0] + Rs[1] * dj[1] + Rs[2] * dj[2]);
-                    if (jsp != 1) pj[jsp] -= ts1 * (Rs[0] * di[0] + Rs[1] * di[1] + Rs[2] * di[2]);
-                }
-#pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    gi[isp][c] += dij[c];
-                    gj[jsp][c] -= dij[c];
-                }
-                const double4_32a ca = posc_of(kp, b)[(isp - 1) * N + i], cb = posc_of(kp, b)[(jsp - 1) * N + j];
-                const double Rc[3] = {ca.x - cb.x + Rw[0], ca.y - cb.y + Rw[1], ca.z - cb.z + Rw[2]};
-                av[ACC_VIRIALC] += Rc[0] * dij[0] + Rc[1] * dij[1] + Rc[2] * dij[2];
-#pragma unroll
-                for (int col = 0; col < 3; col++)
-#pragma unroll
-                    for (int c = 0; c < 3; c++) av[ACC_VIRT + c + 3 * col] += dij[c] * Rs[col];
-            }
-        }
-#pragma unroll
-        for (int k = 1; k <= 4; k++) {
-            const bool any = (MODEL == 2) || k != 1;
-            if (!any) continue;
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                atomicAdd(dR + 3 * ((k - 1) * N + i) + c, gi[k][c]);
-                atomicAdd(dR + 3 * ((k - 1) * N + j) + c, gj[k][c]);
-            }
-            if (k != 1) {
-                atomicAdd(&Fb[(k - 1) * N + i].w, pi[k]);
-                atomicAdd(&Fb[(k - 1) * N + j].w, pj[k]);
-            }
-        }
-    }
-    // intramolecular (pot_ttm.f90:482-542), one molecule per thread
-    for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < N; w += gridDim.x * blockDim.x) {
-        double4_32a s[5], c4[5];
-        double mu[5][3];
-#pragma unroll
-        for (int k = 1; k <= 4; k++) {
-            s[k] = pos[(k - 1) * N + w];
-            c4[k] = posc_of(kp, b)[(k - 1) * N + w];
-            const double3 m = ld3(dip + 3 * ((k - 1) * N + w));
-            mu[k][0] = T::dip(k) ? m.x : 0.0;
-            mu[k][1] = T::dip(k) ? m.y : 0.0;
-            mu[k][2] = T::dip(k) ? m.z : 0.0;
-        }
-        double g[5][3], ph[5];
-#pragma unroll
-        for (int k = 0; k < 5; k++) g[k][0] = g[k][1] = g[k][2] = ph[k] = 0.0;
-#pragma unroll
-        for (int isp = 1; isp <= 3; isp++)
-#pragma unroll
-            for (int jsp = isp + 1; jsp <= 4; jsp++) {
-                const double Rs[3] = {min_image_rn(__dsub_rn(s[isp].x, s[jsp].x), kp.box[0], kp.boxi[0]),
-                                      min_image_rn(__dsub_rn(s[isp].y, s[jsp].y), kp.box[1], kp.boxi[1]),
-                                      min_image_rn(__dsub_rn(s[isp].z, s[jsp].z), kp.box[2], kp.boxi[2])};
-                const double Rc[3] = {min_image_rn(__dsub_rn(c4[isp].x, c4[jsp].x), kp.box[0], kp.boxi[0]),
-                                      min_image_rn(__dsub_rn(c4[isp].y, c4[jsp].y), kp.box[1], kp.boxi[1]),
-                                      min_image_rn(__dsub_rn(c4[isp].z, c4[jsp].z), kp.box[2], kp.boxi[2])};
-                const double d2 = dot3_rn(Rs[0], Rs[1], Rs[2]);
-                double dij[3] = {0, 0, 0};
-                if (T::dip(isp) && T::dip(jsp)) {
-                    double t1, t2, t3;
-                    smear3<double>(d2, kp.pt.apol_dd[isp][jsp], kp.ew, &t1, &t2, &t3);
-                    dd_force(Rs, mu[isp], mu[jsp], t2, t3, dij);
-                }
-                const double qi = s[isp].w, qj = s[jsp].w;
-                double qd[3];
-#pragma unroll
-                for (int c = 0; c < 3; c++) qd[c] = qj * mu[isp][c] - qi * mu[jsp][c];
-                double ts1, ts2;
-                self2(d2, kp.ew, &ts1, &ts2);
-                const double rq = Rs[0] * qd[0] + Rs[1] * qd[1] + Rs[2] * qd[2];
-#pragma unroll
-                for (int c = 0; c < 3; c++) dij[c] += 3.0 * ts2 * rq * Rs[c] - ts1 * qd[c];
-                ph[isp] += ts1 * (Rs[0] * mu[jsp][0] + Rs[1] * mu[jsp][1] + Rs[2] * mu[jsp][2]);
-                ph[jsp] -= ts1 * (Rs[0] * mu[isp][0] + Rs[1] * mu[isp][1] + Rs[2] * mu[isp][2]);
-#pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    g[isp][c] += dij[c];
-                    g[jsp][c] -= dij[c];
-                }
-                av[ACC_VIRIALC] += Rc[0] * dij[0] + Rc[1] * dij[1] + Rc[2] * dij[2];
-#pragma unroll
-                for (int col = 0; col < 3; col++)
-#pragma unroll
-                    for (int c = 0; c < 3; c++) av[ACC_VIRT + c + 3 * col] += dij[c] * Rs[col];
-            }
-#pragma unroll
-        for (int k = 1; k <= 4; k++) {
-#pragma unroll
-            for (int c = 0; c < 3; c++) atomicAdd(dR + 3 * ((k - 1) * N + w) + c, g[k][c]);
-            if (k != 1) atomicAdd(&Fb[(k - 1) * N + w].w, ph[k]);
-        }
-    }
-    block_reduce_add<14, 128>(av, kp.acc + (size_t)b * NACC);
-}
 
 // ---------------------------------------------------------------------------------------
 // pot_ttm.f90:556-627: charge-derivative forces grdq*phi, their virials, M-site force
@@ -652,18 +627,23 @@ static int pair_blocks(const Engine &E) {
 }
 
 void launch_sites(Engine &E) {
-    dim3 g((2 * E.kp.N + SITES_NT - 1) / SITES_NT, E.kp.P);
-    const bool f = E.precision == PIMD_PREC_MIXED;
-    if (E.kp.model == 2) {
-        if (f)
-            k_sites<2, true><<<g, SITES_NT, 0, E.stream>>>(E.kp);
+    const int N = E.kp.N, P = E.kp.P;
+    const dim3 g((2 * N + SITES_NT - 1) / SITES_NT, P);
+    if (E.precision == PIMD_PREC_MIXED) {
+        if (E.kp.model == 2)
+            k_sites<2><<<g, SITES_NT, 0, E.stream>>>(E.kp);
         else
-            k_sites<2, false><<<g, SITES_NT, 0, E.stream>>>(E.kp);
+            k_sites<3><<<g, SITES_NT, 0, E.stream>>>(E.kp);
+    } else if (lanes_per_molecule(N, P) == 4) {
+        const dim3 g4((N + 7) / 8, P);
+        if (E.kp.model == 2)
+            k_sites64<2, 4><<<g4, SITES_NT, 0, E.stream>>>(E.kp);
+        else
+            k_sites64<3, 4><<<g4, SITES_NT, 0, E.stream>>>(E.kp);
+    } else if (E.kp.model == 2) {
+        k_sites64<2, 1><<<g, SITES_NT, 0, E.stream>>>(E.kp);
     } else {
-        if (f)
-            k_sites<3, true><<<g, SITES_NT, 0, E.stream>>>(E.kp);
-        else
-            k_sites<3, false><<<g, SITES_NT, 0, E.stream>>>(E.kp);
+        k_sites64<3, 1><<<g, SITES_NT, 0, E.stream>>>(E.kp);
     }
     ++E.nlaunch;
 }
@@ -683,11 +663,6 @@ void launch_dd_real(Engine &E) {
     DISPATCH_TTM(E, k_dd_real, g, 128);
 }
 
-
-void launch_pair_force(Engine &E) {
-    dim3 g(pair_blocks(E), E.kp.P);
-    DISPATCH_TTM(E, k_pair_force, g, 128);
-}
 
 void launch_finish(Engine &E) {
     dim3 g((E.kp.N + 127) / 128, E.kp.P);
