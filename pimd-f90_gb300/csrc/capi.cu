@@ -187,10 +187,11 @@ static int setup_kspace(Engine &E, const pimd_params *p) {
 // the second stream of the force call and of the dipole iterations, with their events
 static cudaError_t overlap_init(Engine &E) {
     cudaError_t e = cudaSuccess;
+    const bool loop = E.kp.model < 4;  // (the SPC models have no dipole iterations)
     for (cudaStream_t *s : {&E.aux_stream, &E.loop_aux})
-        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(s, cudaStreamNonBlocking);
+        if (e == cudaSuccess && (loop || s == &E.aux_stream)) e = cudaStreamCreateWithFlags(s, cudaStreamNonBlocking);
     for (cudaEvent_t *v : {&E.ev_fork, &E.ev_join, &E.loop_fork, &E.loop_join, &E.ev_check[0], &E.ev_check[1]})
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(v, cudaEventDisableTiming);
+        if (e == cudaSuccess && (loop || v == &E.ev_fork || v == &E.ev_join)) e = cudaEventCreateWithFlags(v, cudaEventDisableTiming);
     return e;
 }
 
@@ -407,7 +408,7 @@ static int create(Engine &E, const pimd_params *p, int nrep, const int *brep) {
     pot_init_constants(E);
     ewald_init(E);
     if (E.precision != PIMD_MIXED && dg_init(E)) return fail(E, PIMD_ERR_NOMEM, "cudaMalloc");
-    if (!spc && (rc = cuda_check(E, overlap_init(E), "streams"))) return rc;
+    if ((rc = cuda_check(E, overlap_init(E), "streams"))) return rc;
     if (E.precision == PIMD_MIXED && (rc = cuda_check(E, mixed_init(E), "mixed tables"))) return rc;
     neighbors_init(E);
     if (kp.model == 3) adjoint_init(E);
@@ -618,11 +619,25 @@ static void force_before(Engine &E, int t) {
         launch_set_step(E, t);
     const bool mixed = E.precision == PIMD_MIXED;
     if (kp.model >= 4) {  // pot_spc.f90: no induced dipoles
+        // the reciprocal passes on the second stream beside the pair sums (32 x 8: 71 us a step in one
+        // stream, with the site kernel's old form; 47 us so)
+        const bool ov = overlap64(E);
+        cudaStream_t keep = E.stream;
         PHASE("sites", launch_sites_spc(E));
-        PHASE("neighbors", launch_neighbors(E));
-        PHASE("pair_qq", launch_pair_qq(E));
+        if (ov) {
+            cudaEventRecord(E.ev_fork, E.stream);
+            cudaStreamWaitEvent(E.aux_stream, E.ev_fork, 0);
+            E.stream = E.aux_stream;
+        }
+        E.fin_defer = true;
         PHASE("ewald_tables", launch_ewald_tables(E));
         PHASE("ewald_pw", launch_ewald_pw(E));
+        E.fin_defer = false;
+        if (ov) cudaEventRecord(E.ev_join, E.aux_stream);
+        E.stream = keep;
+        PHASE("neighbors", launch_neighbors(E));
+        PHASE("pair_qq", launch_pair_qq(E));
+        if (ov) cudaStreamWaitEvent(E.stream, E.ev_join, 0);
         PHASE("finish", launch_finish_spc(E));
         return;
     }
