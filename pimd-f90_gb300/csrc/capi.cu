@@ -187,11 +187,12 @@ static int setup_kspace(Engine &E, const pimd_params *p) {
 // the second stream of the force call and of the dipole iterations, with their events
 static cudaError_t overlap_init(Engine &E) {
     cudaError_t e = cudaSuccess;
-    const bool loop = E.kp.model < 4;  // (the SPC models have no dipole iterations)
+    const bool loop = E.kp.model < 4;  // (the SPC models have no dipole iterations; they fork twice)
     for (cudaStream_t *s : {&E.aux_stream, &E.loop_aux})
         if (e == cudaSuccess && (loop || s == &E.aux_stream)) e = cudaStreamCreateWithFlags(s, cudaStreamNonBlocking);
     for (cudaEvent_t *v : {&E.ev_fork, &E.ev_join, &E.loop_fork, &E.loop_join, &E.ev_check[0], &E.ev_check[1]})
         if (e == cudaSuccess && (loop || v == &E.ev_fork || v == &E.ev_join)) e = cudaEventCreateWithFlags(v, cudaEventDisableTiming);
+    if (e == cudaSuccess && !loop) e = cudaEventCreateWithFlags(&E.ev_nbr, cudaEventDisableTiming);
     return e;
 }
 
@@ -349,10 +350,10 @@ static int create(Engine &E, const pimd_params *p, int nrep, const int *brep) {
         (rc = dalloc(E, &kp.dipE, P * N * 3)) || (rc = dalloc(E, &kp.chg, P * kp.natoms)) ||
         (rc = dalloc(E, &kp.pos, P * S)) || (rc = dalloc(E, &kp.posc, (size_t)kp.nrep * S)) || (rc = dalloc(E, &kp.F, P * S)) ||
         (rc = dalloc(E, &kp.dR, P * S * 3)) || (rc = dalloc(E, &kp.dip, P * S * 3)) || (rc = dalloc(E, &kp.Efdr, P * S * 3)) ||
-        (rc = dalloc(E, &kp.txdip, P * 4 * S * 3)) || (rc = dalloc(E, &kp.grdq, P * N * 27)) ||
-        (rc = dalloc(E, &kp.Tdd, P * E.cap * kp.ndd * 6)) || (rc = dalloc(E, &kp.Tself, P * N * 18)) ||
+        (rc = dalloc(E, &kp.txdip, P * 4 * S * 3)) ||
+        (!spc && ((rc = dalloc(E, &kp.grdq, P * N * 27)) || (rc = dalloc(E, &kp.Tdd, P * E.cap * kp.ndd * 6)) ||
+                  (rc = dalloc(E, &kp.Tself, P * N * 18)))) ||
         (rc = dalloc(E, &kp.pairs, P * E.cap)) || (rc = dalloc(E, &kp.npair, P)) ||
-        (rc = dalloc(E, &kp.tab, P * kp.ntab * S)) ||
         (E.precision == PIMD_MIXED && (rc = dalloc(E, &kp.Spart, P * maxgroups * kp.nk * 3))) ||
         (rc = dalloc(E, &kp.Sq, P * kp.nk)) || (rc = dalloc(E, &kp.Sm, P * kp.nk)) || (rc = dalloc(E, &kp.Sdip, P * kp.nk * 3)) ||
         (rc = dalloc(E, &kp.acc, P * NACC)) || (rc = dalloc(E, &kp.err, 1)) || (rc = dalloc(E, &kp.allconv, 1)) ||
@@ -396,7 +397,7 @@ static int create(Engine &E, const pimd_params *p, int nrep, const int *brep) {
     cudaMemset(kp.Sm, 0, sizeof(double2) * P * kp.nk);
     if (kp.Wf) cudaMemset(kp.Wf, 0, sizeof(float2) * P * 2 * kp.nk);
     cudaMemset(kp.err, 0, sizeof(unsigned));
-    if ((rc = cuda_check(E, cudaMallocHost((void **)&E.h_allconv, 4 * sizeof(int)), "cudaMallocHost"))) return rc;
+    if (!spc && (rc = cuda_check(E, cudaMallocHost((void **)&E.h_allconv, 4 * sizeof(int)), "cudaMallocHost"))) return rc;
     cudaMemset(kp.dstep, 0, sizeof(int) * 2);
     cudaMemset(kp.fin_counter, 0, sizeof(unsigned));
     if (nrep > 1) {
@@ -611,32 +612,42 @@ static bool overlap64(const Engine &E) { return E.precision != PIMD_MIXED && E.e
 static void force_before(Engine &E, int t) {
     KP &kp = E.kp;
     kp.t = t;
-    cudaMemsetAsync(kp.acc, 0, sizeof(double) * kp.P * NACC, E.stream);
-    cudaMemsetAsync(kp.err, 0, sizeof(unsigned), E.stream);
-    if (E.capturing)
-        cudaMemsetAsync(kp.dstep + 1, 0, sizeof(int), E.stream);  // t is set before each graph launch
-    else
-        launch_set_step(E, t);
+    launch_begin(E, t);
     const bool mixed = E.precision == PIMD_MIXED;
     if (kp.model >= 4) {  // pot_spc.f90: no induced dipoles
-        // the reciprocal passes on the second stream beside the pair sums (32 x 8: 71 us a step in one
-        // stream, with the site kernel's old form; 47 us so)
+        // the reciprocal passes on the second stream: the tables, which need only the input atoms, beside
+        // the site kernel, the rest beside the pair sums, and the virial beside the field
+        // (32 x 8: 71 us a step in one stream with the site kernel's old form; 41 us so)
         const bool ov = overlap64(E);
         cudaStream_t keep = E.stream;
-        PHASE("sites", launch_sites_spc(E));
-        if (ov) {
-            cudaEventRecord(E.ev_fork, E.stream);
-            cudaStreamWaitEvent(E.aux_stream, E.ev_fork, 0);
-            E.stream = E.aux_stream;
-        }
-        E.fin_defer = true;
+        auto on_aux = [&](bool aux) {
+            if (ov) E.stream = aux ? E.aux_stream : keep;
+        };
+        auto wait = [&](cudaEvent_t ev, cudaStream_t from, cudaStream_t to) {
+            if (!ov) return;
+            cudaEventRecord(ev, from);
+            cudaStreamWaitEvent(to, ev, 0);
+        };
+        wait(E.ev_fork, keep, E.aux_stream);
+        on_aux(true);
         PHASE("ewald_tables", launch_ewald_tables(E));
-        PHASE("ewald_pw", launch_ewald_pw(E));
+        on_aux(false);
+        PHASE("sites", launch_sites_spc(E));
+        if (ov) cudaEventRecord(E.ev_nbr, keep);
+        on_aux(true);
+        E.dg_after_x = ov ? E.ev_nbr : nullptr;
+        PHASE("ewald_sq", launch_ewald_sq(E));
+        E.dg_after_x = nullptr;
+        if (ov) cudaEventRecord(E.ev_fork, E.aux_stream);
+        E.fin_defer = true;
+        PHASE("ewald_fq", launch_ewald_fq(E));
         E.fin_defer = false;
         if (ov) cudaEventRecord(E.ev_join, E.aux_stream);
-        E.stream = keep;
+        on_aux(false);
         PHASE("neighbors", launch_neighbors(E));
         PHASE("pair_qq", launch_pair_qq(E));
+        if (ov) cudaStreamWaitEvent(E.stream, E.ev_fork, 0);
+        PHASE("ewald_virial", launch_ewald_virial(E));
         if (ov) cudaStreamWaitEvent(E.stream, E.ev_join, 0);
         PHASE("finish", launch_finish_spc(E));
         return;

@@ -15,7 +15,6 @@
 //   Efdr  [P][S][3]   real-space dipole field of the current iteration
 //   pairs [P][cap]    int2 half neighbour list of O-O pairs (i < j), ordered as find_neigh
 //   Tdd   [P][cap][ND][6]  cached dipole-dipole tensors for the iterations
-//   tab   [P][nx+ny+nz][S]  double2 e^{i 2pi n x/L} recurrence tables (ssincos)
 //   Spart [P][tiles][nk]    double2 per-site-tile structure-factor partials
 //   Sq, Sm [P][nk]          double2 charge / dipole structure factors
 //   Sdip  [P][nk][3]        double2 sum mu_c e^{ik.r} for the reciprocal virial
@@ -100,7 +99,7 @@ struct KP {
     double *dR, *dip, *Efdr, *txdip, *grdq, *Tdd, *Tself;
     int2 *pairs;
     int *npair;
-    double2 *tab, *Spart, *Sq, *Sm, *Sdip;
+    double2 *Spart, *Sq, *Sm, *Sdip;
     const KRun *runs;
     const KChunk *chunks;
     const double4_32a *kinfo;  // (kx, ky, kz) vector, 4pi Ak / V
@@ -321,7 +320,8 @@ struct Engine {
     std::vector<FieldFinish> fin;
     cudaStream_t aux_stream = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-    cudaEvent_t ev_nbr = nullptr;  // the neighbour lists built on the second stream beside k_sites
+    cudaEvent_t ev_nbr = nullptr;  // the neighbour lists built on the second stream beside k_sites (SPC: the sites done)
+    cudaEvent_t dg_after_x = nullptr;  // what a structure factor waits for after its site tables (null: nothing)
     bool nbr_overlap = true;       // (knob)
     // the dipole iterations' own pair (inside a graph they are captured into the conditional
     // loop's body, a graph of its own, which must not share a stream with the outer capture)
@@ -479,6 +479,7 @@ void launch_after_qq(Engine &E);
 void launch_dd_real(Engine &E);
 void launch_dd_update(Engine &E);
 void launch_set_step(Engine &E, int t);
+void launch_begin(Engine &E, int t);         // start of a force call
 void launch_pair_force(Engine &E);
 void launch_finish(Engine &E);
 void launch_totals(Engine &E, double *Upott, double *virialt, double *virialct, double *virt9);
@@ -499,7 +500,7 @@ void launch_ewald_fq(Engine &E);
 void launch_ewald_smu(Engine &E);
 void launch_ewald_qd(Engine &E);
 void launch_field_finish(Engine &E);  // the deferred ones (fin)
-void launch_ewald_pw(Engine &E);
+void launch_ewald_virial(Engine &E);
 // tensor-core structure factors (ewald_tc.cu): setup once per context; per call the launch
 // writes the sums of op (OP_Q: Sq + charge weights, OP_MU: Sm + dipole weights, OP_DIP: Sdip)
 // and returns 1, or returns 0 (not applicable)
@@ -515,7 +516,7 @@ bool field_pdl_ok(const Engine &E);
 int launch_field_qd_tc(Engine &E, int s0, int s1);  // ewald_std_qd force pass on the tensor cores
 // digit-product reciprocal sums of the FP64 engine (ewald_dg.cu)
 int dg_init(Engine &E);                  // 0, or 1 when a buffer could not be allocated
-void launch_dg_tables(Engine &E);        // after the ssincos tables
+void launch_dg_tables(Engine &E);        // site tables and their digits
 bool dg_small(const Engine &E);          // its dipole iterations run as chained launches
 void launch_dg_dipoles(Engine &E);       // X of the dipole sites, before the dipole iterations
 void launch_dg_sfac(Engine &E, int op, int s0, int nsites, int skipconv);

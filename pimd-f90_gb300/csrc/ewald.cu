@@ -52,46 +52,11 @@ PIMD_D V cconj(V a) {
 template <typename R>
 PIMD_D typename C2<R>::T *tab_base(const KP &kp);
 template <>
-PIMD_D double2 *tab_base<double>(const KP &kp) {
-    return kp.tab;
-}
-template <>
 PIMD_D float2 *tab_base<float>(const KP &kp) {
     return kp.tabf;
 }
 
-// ewald.f90:403-437 ssincos: cos/sin(2 pi n x / L) for n = 0..nmax by the angle-addition
-// recurrence from n = 1, each product and sum rounded separately like the reference.
-template <typename R>
-__global__ void __launch_bounds__(128) k_ewald_tables(KP kp) {
-    using V = typename C2<R>::T;
-    const int s = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
-    if (s >= kp.S) return;
-    const double4_32a r = kp.pos[(size_t)b * kp.S + s];
-    const double xyz[3] = {r.x, r.y, r.z};
-    const int nmx[3] = {kp.hmax, kp.kmax, kp.lmax};
-    int off = 0;
-    V *T = tab_base<R>(kp) + (size_t)b * kp.ntab * kp.S + s;
-    for (int d = 0; d < 3; d++) {
-        T[(size_t)off * kp.S] = C2<R>::make(R(1), R(0));
-        if (nmx[d] >= 1) {
-            const double arg = __dmul_rn(__dmul_rn(TWOPI, kp.boxi[d]), xyz[d]);
-            const double c1 = cos(arg), s1 = sin(arg);
-            double c = c1, sn = s1;
-            T[(size_t)(off + 1) * kp.S] = C2<R>::make(R(c1), R(s1));
-            for (int n = 2; n <= nmx[d]; n++) {
-                const double cn = __dsub_rn(__dmul_rn(c, c1), __dmul_rn(sn, s1));
-                const double snn = __dadd_rn(__dmul_rn(c, s1), __dmul_rn(sn, c1));
-                c = cn;
-                sn = snn;
-                T[(size_t)(off + n) * kp.S] = C2<R>::make(R(c), R(sn));
-            }
-        }
-        off += nmx[d] + 1;
-    }
-}
-
-// The FP32 tables of the mixed engine without the FP64 recurrence: the site's coordinate as a
+// ewald.f90:403-437 ssincos, cos/sin(2 pi n x / L) for n = 0..nmax, without the recurrence: the site's coordinate as a
 // 32-bit fraction u of the box edge (wrapped, rounded once from FP64), n u modulo 2^32 is the
 // exact phase fraction of harmonic n (a wrapping integer multiply), read as signed it is the
 // angle pi ph / 2^31 in [-pi, pi) for sincospif. Each entry carries only FP32 rounding (of the
@@ -1165,13 +1130,9 @@ void ewald_init(Engine &E) {
 }
 
 void launch_ewald_tables(Engine &E) {
-    dim3 g((E.kp.S + 127) / 128, E.kp.P);
-    if (E.precision == PIMD_PREC_MIXED)
-        k_ewald_tables_m<<<g, 128, 0, E.stream>>>(E.kp);
-    else
-        k_ewald_tables<double><<<g, 128, 0, E.stream>>>(E.kp);
+    if (E.precision != PIMD_PREC_MIXED) return launch_dg_tables(E);
+    k_ewald_tables_m<<<dim3((E.kp.S + 127) / 128, E.kp.P), 128, 0, E.stream>>>(E.kp);
     ++E.nlaunch;
-    if (E.precision != PIMD_PREC_MIXED) launch_dg_tables(E);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1479,12 +1440,8 @@ void launch_ewald_qd(Engine &E) {
     launch_qd_virial(E, true);
     run_field<F_QD>(E, field_s0(E), E.kp.S);
 }
-// ewald_pw_std_qq (ewald.f90:230-291): charge structure factor over all sites, field and
-// potential at all sites, reciprocal virial
-void launch_ewald_pw(Engine &E) {
-    launch_ewald_sq(E);
-    launch_ewald_fq(E);
-    launch_qd_virial(E, false);
-}
+// ewald_pw_std_qq (ewald.f90:230-291) is launch_ewald_sq and launch_ewald_fq, over all sites, and the
+// reciprocal virial of the charges alone
+void launch_ewald_virial(Engine &E) { launch_qd_virial(E, false); }
 
 }  // namespace pimd

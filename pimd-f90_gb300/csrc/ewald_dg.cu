@@ -156,17 +156,43 @@ PIMD_D long long dg_exy(const KP &kp, const DgArgs &a, int b, int kx, int ky, in
 }
 
 // ---- operands ------------------------------------------------------------------------------
-// The ssincos tables (ewald.f90:403-437) in fixed point, and the beads whose tables are not finite
-__global__ void __launch_bounds__(128) k_dg_tab(KP kp, DgArgs a) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
+// ewald.f90:403-437 ssincos: cos/sin(2 pi n x / L) for n = 0..nmax by the angle-addition recurrence from
+// n = 1, each product and sum rounded separately like the reference, left in fixed point; and the
+// beads whose tables are not finite. A thread takes one coordinate of a site: bound by the
+// recurrence's chain of FP64 instructions, 15 us at 96 sites with all three in a thread and a
+// conversion pass after it, 7.8 us so. The SPC models' sites are the input atoms (atoms, O H H).
+__global__ void __launch_bounds__(128) k_dg_tab(KP kp, DgArgs a, const double *atoms) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y, d = blockIdx.z;
     if (s >= kp.S) return;
-    const size_t base = (size_t)b * kp.ntab * kp.S + s;
+    double x;
+    if (atoms) {
+        const int k = s / kp.N, w = s - k * kp.N;
+        x = atoms[((size_t)b * kp.natoms + 3 * w + k) * 3 + d];
+    } else {
+        x = reinterpret_cast<const double *>(kp.pos + (size_t)b * kp.S + s)[d];
+    }
+    const int nmax = d == 0 ? kp.hmax : d == 1 ? kp.kmax : kp.lmax;
+    const int row = d == 0 ? 0 : d == 1 ? kp.hmax + 1 : kp.hmax + kp.kmax + 2;
+    int4 *T = a.tab + ((size_t)b * kp.ntab + row) * kp.S + s;
     bool bad = false;
-    for (int r = blockIdx.z; r < kp.ntab; r += gridDim.z) {
-        const double2 v = kp.tab[base + (size_t)r * kp.S];
-        bad |= dg_hi(v.x) >= 0x7ff00000 || dg_hi(v.y) >= 0x7ff00000;
-        const int2 c = dg_split(dg_fix(v.x, 62)), n = dg_split(dg_fix(v.y, 62));
-        a.tab[base + (size_t)r * kp.S] = make_int4(c.x, c.y, n.x, n.y);
+    auto put = [&](int n, double c, double sn) {
+        bad |= dg_hi(c) >= 0x7ff00000 || dg_hi(sn) >= 0x7ff00000;
+        const int2 u = dg_split(dg_fix(c, 62)), v = dg_split(dg_fix(sn, 62));
+        T[(size_t)n * kp.S] = make_int4(u.x, u.y, v.x, v.y);
+    };
+    put(0, 1.0, 0.0);
+    if (nmax >= 1) {
+        const double arg = __dmul_rn(__dmul_rn(TWOPI, kp.boxi[d]), x);
+        const double c1 = cos(arg), s1 = sin(arg);
+        double c = c1, sn = s1;
+        put(1, c1, s1);
+        for (int n = 2; n <= nmax; n++) {
+            const double cn = __dsub_rn(__dmul_rn(c, c1), __dmul_rn(sn, s1));
+            const double snn = __dadd_rn(__dmul_rn(c, s1), __dmul_rn(sn, c1));
+            c = cn;
+            sn = snn;
+            put(n, c, sn);
+        }
     }
     if (bad) atomicOr(a.xbad + b, 1);
 }
@@ -901,13 +927,10 @@ static void launch_x(Engine &E, int s0, int nsites, int b0, int nb, bool cache) 
     ++E.nlaunch;
 }
 
-// Site tables in digits (after the ssincos tables of a force call): the field's Q for every site
+// Site tables of a force call, and their digits for the field (Q, every site)
 void launch_dg_tables(Engine &E) {
     E.dg_xdip = false;
-    cudaMemsetAsync(E.dg.xbad, 0, sizeof(int) * E.kp.P, E.stream);
-    const int sb = ceil_div(E.kp.S, 128);
-    const int rows = std::max(1, std::min(E.kp.ntab, (int)(608L / std::max(1L, (long)sb * E.kp.P))));
-    k_dg_tab<<<dim3(sb, E.kp.P, rows), 128, 0, E.stream>>>(E.kp, E.dg);
+    k_dg_tab<<<dim3(ceil_div(E.kp.S, 128), E.kp.P, 3), 128, 0, E.stream>>>(E.kp, E.dg, E.kp.model >= 4 ? E.kp.RRt : nullptr);
     ++E.nlaunch;
     k_dg_q<<<dim3(ceil_div(E.dg.nst * E.dg.ksf, 4), E.kp.P), 128, 0, E.stream>>>(E.kp, E.dg);
     ++E.nlaunch;
@@ -930,6 +953,15 @@ static void sfac(Engine &E, int s0, int nsites, int skipconv) {
     // weight (each block reads all of them) stays small
     const int upb = std::max(1, (int)((long)nmt * nks * kp.P / (8L * 608)));
     const int nzb = ceil_div(ceil_div(nmt * nks, 8), upb);
+    const bool have = OP != OP_Q && E.dg_xdip;
+    const int nbmax = have ? kp.P : std::max(1, a.xsteps / nks);
+    auto form_x = [&](int b0) {  // X of the beads from b0 that fit
+        if (have) return;
+        launch_x(E, s0, nsites, b0, std::min(nbmax, kp.P - b0), false);
+        E.dg_xdip = false;
+    };
+    form_x(0);
+    if (E.dg_after_x) cudaStreamWaitEvent(E.stream, E.dg_after_x, 0);
     const bool chain = OP == OP_MU && E.dg_chain;
     if (chain) {
         const int nrb = std::max(1, ceil_div((int)E.pair_est, 128));
@@ -954,14 +986,9 @@ static void sfac(Engine &E, int s0, int nsites, int skipconv) {
     while (nw > 1 && nw < nmt && scratch + ring(nw) > (size_t)DG_SMEM) nw--;
     const int soff = nw >= nmt ? 0 : (int)ring(nw);
     const size_t smem = soff ? scratch + ring(nw) : std::max(scratch, ring(nw));
-    const bool have = OP != OP_Q && E.dg_xdip;
-    const int nbmax = have ? kp.P : std::max(1, a.xsteps / nks);
     for (int b0 = 0; b0 < kp.P; b0 += nbmax) {
         const int nb = std::min(nbmax, kp.P - b0);
-        if (!have) {
-            launch_x(E, s0, nsites, b0, nb, false);
-            E.dg_xdip = false;
-        }
+        if (b0) form_x(b0);
         launch_pdl(chain && !E.capturing, k_dg_sfac<OP>, dim3(a.nslotp / DG_SLOTS, nb), 32 * nw, smem, E.stream, kp, a, nks, nmt, ksum, b0, skipconv, soff);
         ++E.nlaunch;
     }

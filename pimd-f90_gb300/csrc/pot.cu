@@ -653,6 +653,23 @@ void launch_after_qq(Engine &E) {
     DISPATCH_TTM(E, k_after_qq, g, 128);
 }
 
+// The force call's accumulators, error word, bad-table flags and iteration count to zero, and the step
+// (set: not inside a graph, where its caller sets it): one launch, which took three or four memory sets of about
+// 1.5 us each on the call's critical path
+__global__ void __launch_bounds__(256) k_begin(KP kp, int *xbad, int t, int set) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < kp.P * NACC) kp.acc[i] = 0.0;
+    if (xbad && i < kp.P) xbad[i] = 0;
+    if (i == 0) {
+        *kp.err = 0u;
+        if (set) kp.dstep[0] = t;
+        kp.dstep[1] = 0;
+    }
+}
+void launch_begin(Engine &E, int t) {
+    k_begin<<<(E.kp.P * NACC + 255) / 256, 256, 0, E.stream>>>(E.kp, E.dg.xbad, t, E.capturing ? 0 : 1);
+    ++E.nlaunch;
+}
 void launch_set_step(Engine &E, int t) {
     k_set_step<<<1, 32, 0, E.stream>>>(E.kp.dstep, t);
     ++E.nlaunch;
