@@ -409,6 +409,7 @@ static int create(Engine &E, const pimd_params *p, int nrep, const int *brep) {
     pot_init_constants(E);
     ewald_init(E);
     if (E.precision != PIMD_MIXED && dg_init(E)) return fail(E, PIMD_ERR_NOMEM, "cudaMalloc");
+    if (dm_init(E)) return fail(E, PIMD_ERR_NOMEM, "cudaMalloc");
     if ((rc = cuda_check(E, overlap_init(E), "streams"))) return rc;
     if (E.precision == PIMD_MIXED && (rc = cuda_check(E, mixed_init(E), "mixed tables"))) return rc;
     neighbors_init(E);
@@ -604,6 +605,10 @@ static bool force_overlap(const Engine &E) {
     return E.precision == PIMD_MIXED && E.ewald_overlap && E.aux_stream && E.kp.Fx && E.tc_ready && E.tf_ready && E.ff_tc;
 }
 
+// small boxes iterate with the matrix of the dipole field; a taped forward keeps the passes, whose
+// structure factors the backward reads
+static bool dipole_matrix(const Engine &E) { return E.dm.M && !E.tape_on; }
+
 static bool overlap64(const Engine &E) { return E.precision != PIMD_MIXED && E.ewald_overlap && E.aux_stream; }
 
 // One force call for all beads of the context (pot_ttm.f90:3-630 per bead): the part before the
@@ -684,7 +689,10 @@ static void force_before(Engine &E, int t) {
             kp.fx_mode = 0;
             // the iterations' dipole-pair scalars fill this stream's slack beside the charge
             // gather (after the full lists this stream built)
-            if (nbe) PHASE("dd_tensors", launch_dd_tensors_m(E));
+            if (dipole_matrix(E))
+                PHASE("dd_matrix", launch_dm_build(E));
+            else if (nbe)
+                PHASE("dd_tensors", launch_dd_tensors_m(E));
             E.stream = keep;
             cudaEventRecord(E.ev_join, E.aux_stream);
         }
@@ -693,7 +701,7 @@ static void force_before(Engine &E, int t) {
         else
             PHASE("neighbors", launch_neighbors(E));
         PHASE("pair_qq", launch_pair_qq_m(E));
-        if (!nbe) PHASE("dd_tensors", launch_dd_tensors_m(E));
+        if (!nbe && !dipole_matrix(E)) PHASE("dd_tensors", launch_dd_tensors_m(E));
     } else {
         // FP64: the reciprocal charge passes (tensor cores) on the second stream beside the
         // neighbour list and the pair sums (FP64 pipe); what adds to F runs after both
@@ -708,6 +716,7 @@ static void force_before(Engine &E, int t) {
             PHASE("ewald_sq", launch_ewald_sq(E));
             PHASE("ewald_fq", launch_ewald_fq(E));
             PHASE("dd_x", launch_dg_dipoles(E));
+            if (dipole_matrix(E)) PHASE("dd_matrix", launch_dm_build(E));
             E.fin_defer = false;
             E.stream = keep;
             cudaEventRecord(E.ev_join, E.aux_stream);
@@ -726,12 +735,20 @@ static void force_before(Engine &E, int t) {
         PHASE("ewald_tables", launch_ewald_tables(E));
         PHASE("ewald_sq", launch_ewald_sq(E));
         PHASE("ewald_fq", launch_ewald_fq(E));
+        if (dipole_matrix(E)) PHASE("dd_matrix", launch_dm_build(E));
     }
     PHASE("after_qq", launch_after_qq(E));
     kp.fx_mode = 0;
     if (E.tape_on) tape_record(E, 0);
     if (!mixed && !overlap64(E)) PHASE("dd_x", launch_dg_dipoles(E));
-    kp.dd_async = (mixed && dd_async_ok(E)) ? 1 : 0;
+    kp.dd_async = (mixed && !dipole_matrix(E) && dd_async_ok(E)) ? 1 : 0;
+    if (dipole_matrix(E)) PHASE("dd_solve", launch_dm_solve(E));
+}
+
+// the reciprocal force pass; it takes the structure factor of the last iteration's input dipoles
+static void ewald_qd(Engine &E) {
+    if (dipole_matrix(E)) PHASE("dd_smu", launch_ewald_smu_before(E));
+    PHASE("ewald_qd", launch_ewald_qd(E));
 }
 
 static void force_after(Engine &E, double *Upott, double *virialt, double *virialct, double *virt9) {
@@ -748,7 +765,7 @@ static void force_after(Engine &E, double *Upott, double *virialt, double *viria
             cudaStream_t keep = E.stream;
             E.stream = E.aux_stream;
             kp.fx_mode = 2;
-            PHASE("ewald_qd", launch_ewald_qd(E));
+            ewald_qd(E);
             kp.fx_mode = 0;
             E.stream = keep;
             cudaEventRecord(E.ev_join, E.aux_stream);
@@ -761,7 +778,7 @@ static void force_after(Engine &E, double *Upott, double *virialt, double *viria
             cudaStream_t keep = E.stream;
             E.stream = E.aux_stream;
             E.fin_defer = true;
-            PHASE("ewald_qd", launch_ewald_qd(E));
+            ewald_qd(E);
             E.fin_defer = false;
             E.stream = keep;
             cudaEventRecord(E.ev_join, E.aux_stream);
@@ -773,7 +790,7 @@ static void force_after(Engine &E, double *Upott, double *virialt, double *viria
                 PHASE("pair_force", launch_pair_force_m(E));
             else
                 PHASE("pair_force", launch_pair_force(E));
-            PHASE("ewald_qd", launch_ewald_qd(E));
+            ewald_qd(E);
         }
         PHASE("finish", launch_finish(E));
         kp.fx_mode = 0;
@@ -785,8 +802,8 @@ int run_forces(Engine &E, int t, int check_every, double *Upott, double *virialt
     KP &kp = E.kp;
     force_before(E, t);
     const bool mixed = E.precision == PIMD_MIXED;
-    if (kp.model >= 4) {
-        ;
+    if (kp.model >= 4 || dipole_matrix(E)) {
+        // no iterations, or all of them done
     } else if (E.capturing) {
         int rc = capture_dipole_loop(E);
         if (rc) {
@@ -853,28 +870,30 @@ int capture_forces(Engine *const *ctx, int n, double *const *out, cudaStream_t s
             cudaStreamWaitEvent(from, join[i], 0);
         }
     };
-    bool loops = false;
     branches(st, [&](int i, bool which) {
         Engine &E = *ctx[i];
         if (!which) force_before(E, 0);
-        loops |= E.kp.model < 4;
         return E.stream;
     });
-    for (int i0 = 0; i0 < n && loops; i0 += 32) {  // (one loop per 32 contexts: the flags' warp)
-        const int m = std::min(32, n - i0);
+    std::vector<int> loop;  // the contexts with iterations of their own
+    for (int i = 0; i < n; i++)
+        if (ctx[i]->kp.model < 4 && !dipole_matrix(*ctx[i])) loop.push_back(i);
+    for (int i0 = 0; i0 < (int)loop.size(); i0 += 32) {  // (one loop per 32 contexts: the flags' warp)
+        const int m = std::min(32, (int)loop.size() - i0);
         cudaGraphConditionalHandle h;
         if (bad(capture_while(st, body_st, &h), "batch dipole loop")) return PIMD_ERR_CUDA;
         AllConv f{};
         f.n = m;
         branches(body_st, [&](int i, bool which) -> cudaStream_t {
             Engine &E = *ctx[i];
-            if (i < i0 || i >= i0 + m) return nullptr;
+            const int at = (int)(std::find(loop.begin() + i0, loop.begin() + i0 + m, i) - loop.begin()) - i0;
+            if (at == m) return nullptr;
             if (!which) {
                 cudaStream_t keep = E.stream;
                 E.stream = E.body_stream;
                 dipole_body(E);
                 E.stream = keep;
-                f.flag[i - i0] = E.kp.allconv;
+                f.flag[at] = E.kp.allconv;
             }
             return E.body_stream;
         });

@@ -186,6 +186,22 @@ struct DgArgs {
     int4 *exyc;                 // [P][nslot][dipole sites] e^{i(kx x + ky y)} likewise (may be null)
 };
 
+// The dipole field's matrix of small boxes (dipole_matrix.cu); M null: not used
+struct DmArgs {
+    int nd, ndp;            // dipole sites of a bead, the same rounded up to a row's pitch
+    int nqmax;              // groups of four kz of the longest run
+    int nkx;                // entries of the kx list
+    // the host's tables: (kx, first run, ky of it, part) of the kx, largest first; from at[0] [run] groups of
+    // four kz and shifts to the kx's scales; at[1] [kx][8] exponents of its six sums; at[2], at[3]
+    // [run][4 nqmax] fixed-point weights (w, w kz^2), (w kz) (FP64), or at[2] w in FP32 (mixed)
+    const int4 *tables;
+    int words, at[4];       // 16-byte words
+    int phase;              // shared memory of a build block before the tables
+    double gk[3];           // 2 pi / box
+    int c16;                // clusters of 16 CTAs the device holds at once
+    void *M;                // [P][nd][6][ndp] xx yy zz xy xz yz (FP64 engine double, mixed float)
+};
+
 // refresh kp.ptf from the FP64 constants (after they are set or changed)
 inline void kp_float_tables(KP &kp) {
     for (int i = 0; i < 5; i++)
@@ -285,6 +301,7 @@ struct Engine {
     const int2 *d_tfkpm = nullptr;    // per (run slot, j): k-vectors of kz = +j, -j
     alignas(64) unsigned char tc_map[128];  // CUtensorMap of the FP32 tables tabf
     DgArgs dg;                 // FP64 engine: digit operands of the reciprocal sums
+    DmArgs dm{};               // small boxes: the dipole field as a matrix
     bool dg_xall = false;      // the X buffer holds the dipole sites of every bead
     bool dg_xdip = false;      // ... and does so for this force call's positions
     int dg_chain = 0;          // small system's iteration: 1 the first of a loop (body), 2 after another
@@ -477,6 +494,7 @@ void launch_pair_qq(Engine &E);       // pairs.cu
 void pair_math_init(Engine &E);
 void launch_after_qq(Engine &E);
 void launch_dd_real(Engine &E);
+void launch_ewald_smu_before(Engine &E);
 void launch_dd_update(Engine &E);
 void launch_set_step(Engine &E, int t);
 void launch_begin(Engine &E, int t);         // start of a force call
@@ -523,6 +541,10 @@ void launch_dg_sfac(Engine &E, int op, int s0, int nsites, int skipconv);
 int launch_dg_field(Engine &E, int mode, int s0, int s1, int part);
 int launch_dg_dforce(Engine &E, const double2 *A, const double2 *B, const double2 *A2, const double *dip2);
 // launchers (spc.cu): q-SPC/Fw and SPC/F
+// dipole_matrix.cu
+int dm_init(Engine &E);                    // 1: out of memory
+void launch_dm_build(Engine &E);           // after the site tables
+void launch_dm_solve(Engine &E);           // all dipole iterations
 void launch_sites_spc(Engine &E);
 void launch_finish_spc(Engine &E);
 

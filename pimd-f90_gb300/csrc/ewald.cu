@@ -1433,6 +1433,16 @@ void launch_ewald_sq(Engine &E) { run_spass<OP_Q>(E, E.kp.fq, E.kp.S - E.kp.fq, 
 void launch_ewald_fq(Engine &E) { run_field<F_Q>(E, field_s0(E), E.kp.S); }
 // one induced-dipole iteration's reciprocal part (ewald_std_dd) fused with the update
 void launch_ewald_smu(Engine &E) { run_spass<OP_MU>(E, E.kp.fd, E.kp.ld - E.kp.fd, 1); }
+// the same of the dipoles before the last iteration, where that left them (dipole_matrix.cu)
+void launch_ewald_smu_before(Engine &E) {
+    KP &kp = E.kp;
+    const KP keep = kp;
+    kp.dip = kp.Efdr;
+    if (kp.dipf) kp.dipf = kp.dipf_alt;
+    run_spass<OP_MU>(E, kp.fd, kp.ld - kp.fd, 0);
+    kp.dip = keep.dip;
+    kp.dipf = keep.dipf;
+}
 void launch_dd_update(Engine &E) { run_field<F_D>(E, E.kp.fd, E.kp.ld); }
 // ewald_std_qd
 void launch_ewald_qd(Engine &E) {

@@ -19,6 +19,7 @@
 
 #include "engine.h"
 #include "dipole_check.cuh"
+#include "mixed_pair.cuh"
 
 namespace pimd {
 
@@ -35,8 +36,6 @@ struct TM {
         return (dip(i) && dip(j)) || (dip(i) && chg(j)) || (chg(i) && dip(j));
     }
 };
-
-PIMD_D float wrapf(float v, float L, float Li) { return v - L * rint_small(__fmul_rn(v, Li)); }
 
 // ---------------------------------------------------------------------------------------
 // Q(2/3, x) of the Thole-smeared charge pairs (smear.f90:2-34 calls math.f90:188-285 with
@@ -174,14 +173,6 @@ __global__ void __launch_bounds__(128) k_site_offsets(KP kp) {
     }
     kp.posf[gs] = d;
     kp.rhof[gs] = make_float4((float)(C.x - O.x), (float)(C.y - O.y), (float)(C.z - O.z), 0.f);
-}
-
-// O_i - O_j, minimum image, from the fixed-point sites: the unsigned difference wraps modulo the
-// box, read as signed it is the nearest image; one rounding to FP32 (relative 2^-24) and the scale
-PIMD_D void oo_min_image(const KP &kp, uint4 oi, uint4 oj, float R[3]) {
-    R[0] = (float)(int)(oi.x - oj.x) * kp.boxq[0];
-    R[1] = (float)(int)(oi.y - oj.y) * kp.boxq[1];
-    R[2] = (float)(int)(oi.z - oj.z) * kp.boxq[2];
 }
 
 // sum over the QL lanes of one molecule's group (QL divides 32; every lane of the warp calls it)
