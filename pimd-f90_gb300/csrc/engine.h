@@ -291,14 +291,17 @@ struct Engine {
     bool ewald_overlap = true;        // reciprocal charge / force passes beside the pair gathers
     bool dd_otf = false;              // real-space dipole tensors formed in each iteration (no cache)
     bool l2_keep = false;             // the iterations' cached operands (X blocks, dipole-pair scalars) loaded evict-last in L2
-    bool ff_tc = true;                // tensor-core dipole field pass (k_field_tc) when tf_ready
+    bool ff_tc = true;                // tensor-core field passes (k_field_v, k_field_p) when tf_ready
     bool tf_ready = false;
-    int tf_nr = 0, tf_nph = 0, tf_jm = 0, tf_ncol = 0, tf_kq = 0;
     bool tf_qd_ready = false;         // the force-pass modes (charge / dipole halves of ewald_std_qd)
-    int tf_nphd = 0, tf_ncold = 0;    // runs per pass and V rows of the dipole-force mode
-    int tf_vpp = 0, tf_wglob = 0;     // field passes: V built per pass (> 2 passes), weights read from global
-    int tf_wglob_d = 0;               // the same for the dipole-force mode's weights
-    const int2 *d_tfkpm = nullptr;    // per (run slot, j): k-vectors of kz = +j, -j
+    // tables and V of the field passes (ewald_tc.cu): [0] 8 rows a run pair, [1] 12 (the dipole force)
+    struct TpSet {
+        const int4 *pair, *kidx;
+        const int2 *chunk;
+        void *V;
+        int vstride, nchunk, rp, kcm;
+    } tp[2] = {};
+    alignas(64) unsigned char tp_mapxy[128], tp_mapz[128];  // CUtensorMaps of tabf's ex and ey rows, and ez rows
     alignas(64) unsigned char tc_map[128];  // CUtensorMap of the FP32 tables tabf
     DgArgs dg;                 // FP64 engine: digit operands of the reciprocal sums
     DmArgs dm{};               // small boxes: the dipole field as a matrix

@@ -42,6 +42,10 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <map>
+#include <utility>
 #include <vector>
 
 #include <cuda_fp16.h>
@@ -619,8 +623,8 @@ __global__ void __maxnreg__(64) k_sfac_tc(const __grid_constant__ CUtensorMap tm
 }
 
 // ---------------------------------------------------------------------------------------
-// Tensor-core dipole field of the mixed engine (the per-iteration k_field_f<F_D> sum,
-// ewald.f90:114-117): at every dipole site s of a bead,
+// Tensor-core field passes of the mixed engine (the per-iteration k_field_f<F_D> sum,
+// ewald.f90:114-117, and the charge field and the force pass): at every site s of a bead,
 //   E_x,y(s) = sum_run k_x,y Im(exy(s) T0(s)),   E_z(s) = sum_run Im(exy(s) T1(s)),
 //   T0(s) = sum_kz W(kz) ez(s, kz),   T1(s) = sum_kz k_z W(kz) ez(s, kz),
 // with W the FP32 weights 4 pi Ak / V conj(S) of the run's k-vectors. Folding +-j as in the
@@ -629,370 +633,40 @@ __global__ void __maxnreg__(64) k_sfac_tc(const __grid_constant__ CUtensorMap tm
 //   T1 = sum_j k_z(j) [(Wm.x c_j - Wp.y s_j) + i (Wm.y c_j + Wp.x s_j)]
 // so T0, T1 of every run at every site are one GEMM per bead,
 //   D[s][(run, comp)] = sum_q Q[s][q] V[(run, comp)][q],  comp = T0re|T0im|T1re|T1im,  q = (j, cos|sin),
-// with the sites on M (128 per CTA), runs x components on N (two passes of half the runs, each
-// component-major in <= 512 TMEM columns) and only 2 (max |kz| + 1) terms on K (FP16 hi + lo
-// split, three MMAs per 16-term K step). V is built by every CTA of a bead from
-// the bead's weights Wf (one bulk copy into shared memory; scaled by 2^10, exact, to keep small
-// weights normal in FP16). The epilogue contracts each TMEM row with exy(s, run) from the
-// TMA-staged tables (16 warps = 4 lane quarters x 4 run quarters, 16 runs x 4 components per
-// TMEM wait), then applies the iteration's
-// FP64 SOR update at the CTA's dipole sites and the convergence test in the last CTA
-// (dipole_check.cuh, as k_field_finish<F_D> does).
+// with the sites on M (128 per CTA), runs x components on N and only 2 (max |kz| + 1) terms on K (FP16
+// hi + lo split, three MMAs per 16-term K step); each TMEM row is then contracted with exy(s, run).
+//
+// V is formed from the weights once a pass (k_field_v; every CTA of a bead did it before, each pass of
+// runs one phase after the other: V, MMAs, contraction), and
+// the runs are taken in pairs (kx, +ky), (kx, -ky). With T+, T- the pair's sums, Ts = T+ + T-, Td = T+ - T- and
+// e(kx x +- ky y) = ex (cy +- i sy),
+//   e+ T+ + e- T- = ex U,  U = cy Ts + i sy Td;   e+ T+ - e- T- = ex V,  V = cy Td + i sy Ts,
+// so a pair's contraction is U0, V0 (T0) and U1 (T1) and three products with ex: 20 FMAs and one load
+// each of ex and ey for two runs, where one run took 15 and both loads. The rows of V are Ts, Td of T0 and T1
+// (8 a pair) and, for the dipole force, of T2 and with V1 (12 a pair: the force is -G mu with
+// G = (kx^2 S0, kx ky D0, ky^2 S0, kx S1, ky D1, S2), S and D the real parts of ex U and ex V).
+//
+// A chunk is the pairs of one accumulator (256 columns at most, half of TMEM), sorted by their largest |kz| so
+// that later chunks have fewer K steps. The control warp copies chunk c + 1 of V (one bulk copy) while the MMAs
+// of chunk c run into one half of TMEM and 16 warps contract chunk c - 1 from the other.
 constexpr int TF_NT = 512;
 constexpr int TF_SITES = 128;             // sites per CTA (M)
-constexpr float TF_WS = 1024.f;           // power-of-two scale of V
-
-struct TfArgs {
-    const int4 *slot;     // per run slot: packed kx/ky, local k offset, kzlo, nkz
-    const float2 *skv;    // per run slot: FP32 (k_x, k_y)
-    const int2 *kpm;      // per (slot, j): k-vector of kz = +j and of kz = -j (-1: none)
-    const float *kzv;     // k_z by kz + lmax
-    int nr, nph, ncol, kq, jm;  // runs, runs per pass (rounded up to 8), V rows (8 nph), K terms (x16), kz rows
-    int sbase, s_lo, s_hi;
-    int pdl;  // launched as a programmatic dependent of the structure factor (pdl_wait before W)
-    int vpp;    // more than two passes: V of each pass built before it (4 nph rows), as TF_DG does
-    int wglob;  // the bead's weights read from global memory (too many k-vectors for shared memory)
-};
-
-struct TfSmem {
-    int boxb, A, B, W, total;
-    __host__ __device__ TfSmem(int ntab, int ncol, int kq, int nk, int nslot = 1) {
-        boxb = ((ntab * 128 + 1023) / 1024) * 1024;
-        A = 8 * boxb;                      // tables of 128 sites: 8 TMA boxes of 16 sites
-        B = A + 2 * TF_SITES * kq * 2;     // Q hi, lo: 128 rows x kq halves
-        W = B + 2 * ncol * kq * 2;         // V hi, lo: ncol rows x kq halves
-        total = W + ((nslot * nk * 8 + 127) / 128) * 128 + 1024;  // the bead's weights Wf (1 or 2 slots)
-    }
-};
-
 // byte offset of the 16-byte chunk jc (halves 8 jc .. 8 jc + 7) of row n in a K-major operand
 // with kcm core matrices along K
 PIMD_D int rowchunk_k(int n, int jc, int kcm) { return (((n >> 3) * kcm + jc) << 7) + ((n & 7) << 4); }
 
-// VPP: V built before each pass (more than two passes); a template argument so that the
-// two-pass form keeps its registers (118 against 127 with a run-time choice)
-template <int MODE, bool VPP>
-__global__ void __launch_bounds__(TF_NT, 1) k_field_tc(const __grid_constant__ CUtensorMap tmap, KP kp, TfArgs a) {
-    // TF_DG: 6 components per run (T0, T1 and T2 = sum kz^2 W ez, complex), V rebuilt for each
-    // pass of nph runs; the other modes: 4 components, V of both passes built once (or, with
-    // a.vpp, V of each pass before it, for more than two passes)
-    constexpr bool DG = MODE == TF_DG;
-    constexpr int NC = DG ? 6 : 4;
-    constexpr bool vpp = DG || VPP;
-    const int t = blockIdx.x, b = blockIdx.y;
-    // the next iteration's structure factor may be scheduled now; it waits for this grid
-    if (MODE == TF_D) pdl_launch_dependents();
-    if (MODE == TF_D && bead_converged(kp, b)) {
-        // converged bead: no update, but the block still counts towards the convergence test
-        const double zero[2] = {0.0, 0.0};
-        if (kp.dd_async) {  // (a unit's arrivals still complete it)
-            const float z[3] = {0.f, 0.f, 0.f};
-            if (dd_unit_arrive(kp, b, t)) dd_unit_sor<TF_NT>(kp, b, t, false, z);
-            return;
-        }
-        dd_block_end<TF_NT>(kp, b, zero, false);
-        return;
-    }
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const TfSmem L(kp.ntab, a.ncol, a.kq, kp.nk, a.wglob ? 0 : (DG ? 2 : 1));
-    extern __shared__ __align__(1024) unsigned char sm_raw[];
-    unsigned char *sm = sm_raw + ((1024u - (umma::smem_u32(sm_raw) & 1023u)) & 1023u);
-    __shared__ uint64_t tbar, wbar, mbar;
-    __shared__ uint32_t tslot;
-    // per run of the current pass: byte offsets of the ex and ey table rows in a stage and their
-    // swizzle keys (16 x (row & 7)); bit 0 of the ey key: ky < 0 (conjugate ey)
-    __shared__ int4 sroff[TC_MAXRUN];
-    __shared__ float2 sskv[TC_MAXRUN];
-    const int sb = a.sbase + t * TF_SITES;
-    // the copies go out first: the bead's weights (one bulk copy) and the tables of 128 sites
-    if (tid == 0) {
-        umma::mbar_init(&tbar, 1);
-        umma::mbar_init(&wbar, 1);
-        umma::mbar_init(&mbar, 1);
-        // weight slots: charge (0), dipole (1); TF_DG takes both (adjacent in Wf)
-        if (!a.pdl && !a.wglob) {
-            const int slot = (MODE == TF_D || MODE == TF_QG) ? 1 : 0;
-            const uint32_t wbytes = (uint32_t)kp.nk * 8u * (DG ? 2u : 1u);
-            mbar_expect_tx(&wbar, wbytes);
-            bulk_load(sm + L.W, kp.Wf + ((size_t)b * 2 + slot) * kp.nk, wbytes, &wbar);
-        }
-        const uint32_t box_tx = (uint32_t)(kp.ntab * 128);
-        mbar_expect_tx(&tbar, 8 * box_tx);
-        for (int i = 0; i < 8; i++) tma_load_2d(sm + i * L.boxb, &tmap, 2 * (sb + 16 * i), b * kp.ntab, &tbar);
-    }
-    const int iter = kp.dstep[1] + 1;  // dipole iteration of this update
-    const int kcm = a.kq / 8, nr = a.nr, nph = a.nph, jm = a.jm;
-    const int npass = vpp ? (nr + nph - 1) / nph : 2;
-    const int yrow = kp.hmax + 1, zrow = yrow + kp.kmax + 1;
-    // the runs' table offsets: all of them once when they fit the arrays, else those of each
-    // pass before it (index p - rbase; the caller syncs before the epilogue reads them)
-    const bool rall = nr <= TC_MAXRUN;
-    auto load_runs = [&](int pass) {
-        const int p = (rall ? 0 : pass * nph) + tid;
-        if (tid < (rall ? nr : nph) && p < nr) {
-            const int kxy = a.slot[p].x, kx = kxy & 255, ky = (kxy >> 8) - 128;
-            const int ry = yrow + (ky < 0 ? -ky : ky);
-            sroff[tid] = make_int4(kx * 128, (kx & 7) << 4, ry * 128, ((ry & 7) << 4) | (ky < 0 ? 1 : 0));
-            const float ws = DG ? 1.f : 1.f / TF_WS;  // TF_DG scales its sums once at the end
-            sskv[tid] = make_float2(a.skv[p].x * ws, a.skv[p].y * ws);
-        }
-    };
-    load_runs(0);
-    if (warp == 0) umma::tmem_alloc(&tslot, 512);
-    // the (k(+j), k(-j)) pairs and k_z of a V item (run p0 + it % nrow, j = 4 (it / nrow) + e):
-    // this thread's first item of each early V build is fetched now, before the weights land
-    auto fetch_km = [&](int p0, int nrow, int it, int2 (&km)[4], float (&kz)[4]) {
-        const int p = p0 + it % nrow, jc = it / nrow;
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const int j = 4 * jc + e;
-            const bool ok = it < nrow * kcm && p < nr && j < jm;
-            km[e] = ok ? a.kpm[p * jm + j] : make_int2(-1, -1);
-            kz[e] = ok ? a.kzv[kp.lmax + j] : 0.f;
-        }
-    };
-    int2 km0[4], km1[4];
-    float kz0[4], kz1[4];
-    fetch_km(0, nph, tid, km0, kz0);
-    fetch_km(vpp ? 0 : nph, nph, tid, km1, kz1);
-    umma::fence_before_sync();
-    __syncthreads();
-    umma::fence_after_sync();
-    const uint32_t tm = tslot;
-    unsigned char *Vh = sm + L.B, *Vl = Vh + a.ncol * a.kq * 2;
-    unsigned char *Qh = sm + L.A, *Ql = Qh + TF_SITES * a.kq * 2;
-    // Q = ez rows of the CTA's sites, 8 halves (4 j: c_j, s_j) per item, zero for j >= jm
-    uint32_t err = (uint32_t)umma::mbar_wait(&tbar, 0, TC_WAIT);
-    for (int it = tid; it < TF_SITES * kcm; it += TF_NT) {
-        const int s = it % TF_SITES, jc = it / TF_SITES;
-        float v[8];
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const int j = 4 * jc + e;
-            const float2 z = j < jm ? tab_elem(sm, L.boxb, zrow + j, s) : make_float2(0.f, 0.f);
-            v[2 * e] = z.x;
-            v[2 * e + 1] = z.y;
-        }
-        uint4 hi, lo;
-        split8_h(v, hi, lo);
-        const int o = rowchunk_k(s, jc, kcm);
-        *reinterpret_cast<uint4 *>(Qh + o) = hi;
-        *reinterpret_cast<uint4 *>(Ql + o) = lo;
-    }
-    // everything above reads only the positions; from here on the structure factor's weights
-    // and the iteration's dipoles and fields (a programmatic launch waits for them here)
-    if (a.pdl) {
-        pdl_wait();
-        if (tid == 0 && !a.wglob) {
-            const int slot = (MODE == TF_D || MODE == TF_QG) ? 1 : 0;
-            const uint32_t wbytes = (uint32_t)kp.nk * 8u * (DG ? 2u : 1u);
-            mbar_expect_tx(&wbar, wbytes);
-            bulk_load(sm + L.W, kp.Wf + ((size_t)b * 2 + slot) * kp.nk, wbytes, &wbar);
-        }
-    }
-    // the SOR inputs of the CTA's dipole sites
-    const int s_own = sb + tid;
-    const bool own = tid < TF_SITES && s_own >= a.s_lo && s_own < a.s_hi;
-    DdSite din;
-    if (MODE == TF_D && own && !kp.dd_async) dd_sor_load(kp, b, s_own, din);
-    if (!a.wglob) err |= (uint32_t)umma::mbar_wait(&wbar, 0, TC_WAIT);
-    const float2 *W = a.wglob ? kp.Wf + ((size_t)b * 2 + ((MODE == TF_D || MODE == TF_QG) ? 1 : 0)) * kp.nk
-                              : reinterpret_cast<const float2 *>(sm + L.W);
-    // V of runs [p0, p0 + nrow): run p0 + pl, component c at row vrow0 + c nrow + pl; 8 halves
-    // (4 j) per item, zero for runs >= nr and j >= jm
-    auto build_v = [&](int p0, int nrow, int vrow0, const int2 (&kmf)[4], const float (&kzf)[4]) {
-        for (int it = tid; it < nrow * kcm; it += TF_NT) {
-            const int pl = it % nrow, jc = it / nrow;
-            int2 km[4];
-            float kzz[4];
-            if (it == tid) {
-#pragma unroll
-                for (int e = 0; e < 4; e++) km[e] = kmf[e], kzz[e] = kzf[e];
-            } else {
-                fetch_km(p0, nrow, it, km, kzz);
-            }
-            float v[NC][8];
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                float2 wp = make_float2(0.f, 0.f), wm = wp;
-                const float kz = kzz[e];
-                {
-                    float2 wpl = km[e].x >= 0 ? W[km[e].x] : make_float2(0.f, 0.f);
-                    float2 wmi = km[e].y >= 0 ? W[km[e].y] : make_float2(0.f, 0.f);
-                    if (DG) {  // total weights W_q + W_mu
-                        if (km[e].x >= 0) wpl = make_float2(wpl.x + W[kp.nk + km[e].x].x, wpl.y + W[kp.nk + km[e].x].y);
-                        if (km[e].y >= 0) wmi = make_float2(wmi.x + W[kp.nk + km[e].y].x, wmi.y + W[kp.nk + km[e].y].y);
-                    }
-                    wp = make_float2(TF_WS * (wpl.x + wmi.x), TF_WS * (wpl.y + wmi.y));
-                    wm = make_float2(TF_WS * (wpl.x - wmi.x), TF_WS * (wpl.y - wmi.y));
-                }
-                // (cos, sin) coefficients of T0re, T0im, T1re, T1im (, T2re, T2im)
-                v[0][2 * e] = wp.x;
-                v[0][2 * e + 1] = -wm.y;
-                v[1][2 * e] = wp.y;
-                v[1][2 * e + 1] = wm.x;
-                v[2][2 * e] = kz * wm.x;
-                v[2][2 * e + 1] = -kz * wp.y;
-                v[3][2 * e] = kz * wm.y;
-                v[3][2 * e + 1] = kz * wp.x;
-                if constexpr (DG) {
-                    const float k2 = kz * kz;
-                    v[4][2 * e] = k2 * wp.x;
-                    v[4][2 * e + 1] = -k2 * wm.y;
-                    v[5][2 * e] = k2 * wp.y;
-                    v[5][2 * e + 1] = k2 * wm.x;
-                }
-            }
-#pragma unroll
-            for (int c = 0; c < NC; c++) {
-                uint4 hi, lo;
-                split8_h(v[c], hi, lo);
-                const int o = rowchunk_k(vrow0 + c * nrow + pl, jc, kcm);
-                *reinterpret_cast<uint4 *>(Vh + o) = hi;
-                *reinterpret_cast<uint4 *>(Vl + o) = lo;
-            }
-        }
-    };
-    if (!vpp) {  // both passes: pass q's rows from q 4 nph
-        build_v(0, nph, 0, km0, kz0);
-        build_v(nph, nph, 4 * nph, km1, kz1);
-    }
-    // passes of nph runs, NC nph <= 512 TMEM columns each: column c nph + pl for component c
-    // of the pass's run pl
-    float Ex = 0.f, Ey = 0.f, Ez = 0.f, phi = 0.f;
-    const int lq = warp & 3, part = warp >> 2, sl = 32 * lq + lane;
-    const int q4 = nph / 4;  // runs per run quarter
-    // the epilogue lane's site in the staged tables: its box and float2 slot, and its 16-byte
-    // chunk (before the swizzle) times 16
-    const unsigned char *tsite = sm + (sl >> 4) * L.boxb + (sl & 1) * 8;
-    const int cs4 = ((sl & 15) >> 1) << 4;
-    // TF_DG: the dipole of the epilogue lane's site (scaled by nothing; zero outside the range)
-    float mu[3] = {0.f, 0.f, 0.f};
-    if (DG && sb + sl >= a.s_lo && sb + sl < a.s_hi) {
-        const float4 m = kp.dipf[(size_t)b * kp.S + sb + sl];
-        mu[0] = m.x, mu[1] = m.y, mu[2] = m.z;
-    }
-    bool bad = err != 0;
-    for (int pass = 0; pass < npass; pass++) {
-        if (pass > 0 && !rall) load_runs(pass);  // (the previous pass's epilogue is past its last sync)
-        const int rbase = rall ? 0 : pass * nph;
-        if (vpp) {
-            if (pass == 0) {
-                build_v(0, nph, 0, km0, kz0);
-            } else {
-                fetch_km(pass * nph, nph, tid, km1, kz1);
-                build_v(pass * nph, nph, 0, km1, kz1);
-            }
-        }
-        umma::fence_smem_to_async();
-        umma::fence_before_sync();
-        bad = __syncthreads_or((int)bad) != 0;
-        umma::fence_after_sync();
-        if (bad) break;
-        if (tid == 0) {
-            const uint32_t idesc_base = umma::idesc_f16(128, 16) & ~(0x3Fu << 17);
-            const uint32_t qh = umma::smem_u32(Qh), ql = umma::smem_u32(Ql);
-            const uint32_t vh = umma::smem_u32(Vh), vl = umma::smem_u32(Vl);
-            for (int c0 = 0; c0 < NC * nph; c0 += 256) {
-                const int N = min(256, NC * nph - c0);
-                const uint32_t id = idesc_base | ((uint32_t)(N >> 3) << 17);
-                const uint32_t d = tm + (uint32_t)c0;
-                const int vr = (vpp ? 0 : pass * 4 * nph) + c0;  // first V row of the MMA
-                const uint32_t vo = (uint32_t)((vr >> 3) * kcm * 128);
-                for (int ks = 0; ks < a.kq / 16; ks++) {
-                    const uint64_t dq_h = umma::sdesc(qh + ks * 256, 128, kcm * 128), dq_l = umma::sdesc(ql + ks * 256, 128, kcm * 128);
-                    const uint64_t dv_h = umma::sdesc(vh + vo + ks * 256, 128, kcm * 128), dv_l = umma::sdesc(vl + vo + ks * 256, 128, kcm * 128);
-                    umma::mma_f16(d, dq_h, dv_h, id, ks > 0);
-                    umma::mma_f16(d, dq_h, dv_l, id, 1);
-                    umma::mma_f16(d, dq_l, dv_h, id, 1);
-                }
-            }
-            umma::commit(&mbar);
-        }
-        __syncwarp();
-        int to = umma::mbar_wait(&mbar, (uint32_t)(pass & 1), TC_WAIT);
-        if (to) to = umma::mbar_wait(&mbar, (uint32_t)(pass & 1), TC_WAIT);
-        umma::fence_after_sync();
-        bad = __syncthreads_or(to) != 0;
-        if (bad) break;
-        // this warp's run quarter in groups of 16 runs x 4 (6) components (one TMEM wait each)
-        for (int pl0 = part * q4; pl0 < (part + 1) * q4; pl0 += 16) {
-            if (pass * nph + pl0 >= nr) break;
-            float v[64];
-            const uint32_t tl = tm + ((uint32_t)(32 * lq) << 16) + (uint32_t)pl0;
-            umma::tmem_ld16x4(tl, tl + (uint32_t)nph, tl + (uint32_t)(2 * nph), tl + (uint32_t)(3 * nph), v);
-            float w[32];
-            if constexpr (DG) umma::tmem_ld16x2(tl + (uint32_t)(4 * nph), tl + (uint32_t)(5 * nph), w);
-#pragma unroll
-            for (int e = 0; e < 16; e++) {
-                const int pl = pl0 + e, p = pass * nph + pl;
-                if (pl >= (part + 1) * q4 || p >= nr) break;
-                // tab_elem(sm, boxb, row, sl) with the run's row offsets and keys precomputed
-                const int4 ro = sroff[p - rbase];
-                const float2 ex = *reinterpret_cast<const float2 *>(tsite + ro.x + (cs4 ^ ro.y));
-                float2 ey = *reinterpret_cast<const float2 *>(tsite + ro.z + (cs4 ^ (ro.w & ~1)));
-                if (ro.w & 1) ey.y = -ey.y;
-                // ewald.f90:30-31: coskxky = cx cy - sx sy, sinkxky = sx cy + cx sy
-                const float er = ex.x * ey.x - ex.y * ey.y, ei = ex.y * ey.x + ex.x * ey.y;
-                const float2 kv = sskv[p - rbase];
-                if constexpr (DG) {
-                    // sum_k k (k . mu) Re(e W) with the run's kz sums (ewald.f90:146-187)
-                    const float R0 = fmaf(er, v[e], -ei * v[16 + e]);       // Re(exy T0)
-                    const float R1 = fmaf(er, v[32 + e], -ei * v[48 + e]);  // Re(exy T1)
-                    const float R2 = fmaf(er, w[e], -ei * w[16 + e]);       // Re(exy T2)
-                    const float aa = kv.x * mu[0] + kv.y * mu[1];
-                    const float tt = fmaf(aa, R0, mu[2] * R1);
-                    Ex = fmaf(-kv.x, tt, Ex);
-                    Ey = fmaf(-kv.y, tt, Ey);
-                    Ez -= fmaf(aa, R1, mu[2] * R2);
-                } else {
-                    const float t0 = fmaf(er, v[16 + e], ei * v[e]);       // Im(exy T0)
-                    const float t1 = fmaf(er, v[48 + e], ei * v[32 + e]);  // Im(exy T1)
-                    Ex = fmaf(kv.x, t0, Ex);
-                    Ey = fmaf(kv.y, t0, Ey);
-                    Ez = fmaf(1.f / TF_WS, t1, Ez);
-                    if (MODE == TF_Q || MODE == TF_QG) phi = fmaf(1.f / TF_WS, fmaf(er, v[e], -ei * v[16 + e]), phi);  // Re(exy T0)
-                }
-            }
-        }
-        umma::fence_before_sync();
-        __syncthreads();
-        umma::fence_after_sync();
-    }
-    if (DG) {
-        Ex *= 1.f / TF_WS;
-        Ey *= 1.f / TF_WS;
-        Ez *= 1.f / TF_WS;
-    }
-    // the four run quarters of each site, in order
-    float *red = reinterpret_cast<float *>(Qh);  // [4][128][4]
-    red[(part * TF_SITES + sl) * 4 + 0] = Ex;
-    red[(part * TF_SITES + sl) * 4 + 1] = Ey;
-    red[(part * TF_SITES + sl) * 4 + 2] = Ez;
-    red[(part * TF_SITES + sl) * 4 + 3] = phi;
-    umma::fence_before_sync();
-    __syncthreads();
-    if (warp == 0) {
-        umma::fence_after_sync();
-        umma::tmem_dealloc(tm, 512);
-        umma::tmem_relinquish();
-    }
-    float e[4] = {0.f, 0.f, 0.f, 0.f};
-    if (own && !bad) {
-#pragma unroll
-        for (int rq = 0; rq < 4; rq++)
-#pragma unroll
-            for (int c = 0; c < 4; c++) e[c] += red[(rq * TF_SITES + tid) * 4 + c];
-    }
-    if (bad && tid == 0) atomicOr(kp.err, 8u);
+// What a field pass does with the field e (and potential, e[3]) of its sites: thread tid < 128 of the
+// block holds site s_own (own: in the pass's range and its sums are good; bad: the block gave up).
+template <int MODE, int NT>
+PIMD_D void field_out(const KP &kp, int b, int t, int s_own, bool own, bool bad, const float (&e)[4], const DdSite &din, int iter) {
     if (MODE == TF_Q && (kp.fx_mode & 1)) {  // into the scratch (this pass runs beside the pair kernels)
-        if (own && !bad)
+        if (own)
             kp.Fx[(size_t)b * kp.S + s_own] =
                 make_double4_32a((double)e[0], (double)e[1], (double)e[2], s_own >= kp.fq ? (double)e[3] : 0.0);
         return;
     }
     if ((MODE == TF_QG || MODE == TF_DG) && (kp.fx_mode & 2)) {
-        if (own && !bad) {
+        if (own) {
             const size_t gs = (size_t)b * kp.S + s_own;
             if (MODE == TF_QG) {
                 const double q = kp.pos[gs].w;
@@ -1010,7 +684,7 @@ __global__ void __launch_bounds__(TF_NT, 1) k_field_tc(const __grid_constant__ C
     }
     if (MODE == TF_Q) {
         // ewald.f90:45-49 as k_field_finish<F_Q>: Efq += E, phi += (charged sites)
-        if (own && !bad) {
+        if (own) {
             const size_t gs = (size_t)b * kp.S + s_own;
             double4_32a f = kp.F[gs];
             f.x += (double)e[0];
@@ -1024,7 +698,7 @@ __global__ void __launch_bounds__(TF_NT, 1) k_field_tc(const __grid_constant__ C
     if (MODE == TF_QG || MODE == TF_DG) {
         // as k_field_finish<F_QD>: dR += -q E (charge part) or the dipole force; phi of the
         // dipole structure factor at the charged sites
-        if (own && !bad) {
+        if (own) {
             const size_t gs = (size_t)b * kp.S + s_own;
             const double q = MODE == TF_QG ? kp.pos[gs].w : -1.0;
             kp.dR[3 * gs + 0] -= q * (double)e[0];
@@ -1037,18 +711,348 @@ __global__ void __launch_bounds__(TF_NT, 1) k_field_tc(const __grid_constant__ C
     if (kp.dd_async) {
         // the real-space field runs beside this pass: store the reciprocal field, arrive, and
         // run the unit's SOR update if the real-space blocks of its molecules are done
-        if (own && !bad) kp.Erec[(size_t)b * kp.S + s_own] = make_float4(e[0], e[1], e[2], 0.f);
+        if (own) kp.Erec[(size_t)b * kp.S + s_own] = make_float4(e[0], e[1], e[2], 0.f);
         const float er[3] = {e[0], e[1], e[2]};
-        if (dd_unit_arrive(kp, b, t)) dd_unit_sor<TF_NT>(kp, b, t, own && !bad, er);
+        if (dd_unit_arrive(kp, b, t)) dd_unit_sor<NT>(kp, b, t, own, er);
         return;
     }
     // the iteration's FP64 SOR update at the CTA's dipole sites, then the block's end
     double av[2] = {0.0, 0.0};
-    if (own && !bad) {
+    if (own) {
         const double E[3] = {(double)e[0], (double)e[1], (double)e[2]};
         dd_sor_apply(kp, b, s_own, din, E, iter, av);
     }
-    dd_block_end<TF_NT, TF_SITES / 32>(kp, b, av, !bad);  // own sites: threads < TF_SITES
+    dd_block_end<NT, TF_SITES / 32>(kp, b, av, !bad);  // own sites: threads < TF_SITES
+}
+
+constexpr int TP_NT = TF_NT + 32;         // 16 contracting warps, one for copies and MMAs
+constexpr int TP_VT = 128;                // threads of a k_field_v block
+constexpr int TP_RP = 32;                 // pairs a chunk at most (8 rows each)
+constexpr int TP_RPD = 20;                // the same with 12 rows each
+constexpr int TP_RING = 8;                // pair tables in shared memory
+constexpr float TP_WS = 512.f;            // power-of-two scale of V (a row adds up to four weights)
+
+struct TpArgs {
+    const int4 *pair;    // [chunk][rp] ex row offset + 65536 key, ey row offset + 65536 key, k_x, k_y (float bits)
+    const int2 *chunk;   // K row blocks (4 |kz| each, even) of the chunk, its offset in a bead's V (16-byte words)
+    const int4 *kidx;    // [chunk rp + pair][4 TP jmax blocks] k-vectors of (+ky, +kz), (+ky, -kz), (-ky, +kz), (-ky, -kz)
+    const float *kzv;    // k_z by kz + lmax
+    uint4 *V;            // [P][vstride] per chunk: hi rows, lo rows
+    int vstride, nchunk, rp, kcm;  // kcm: K row blocks of Q (the longest)
+    int sbase, s_lo, s_hi;
+    int skipconv, pdl;
+};
+
+template <bool DG>
+__global__ void __launch_bounds__(TP_VT) k_field_v(KP kp, TpArgs a, int slot) {
+    constexpr int NC = DG ? 12 : 8;
+    const int c = blockIdx.x, b = blockIdx.y;
+    const int2 ch = a.chunk[c];
+    const int kc = ch.x;
+    // the field pass may set up; it waits for this grid, which waits for the structure factor here
+    pdl_launch_dependents();
+    if (a.pdl) pdl_wait();
+    if (a.skipconv && bead_converged(kp, b)) return;
+    uint4 *Vh = a.V + (size_t)b * a.vstride + ch.y, *Vl = Vh + NC * a.rp * kc;
+    const float2 *W = kp.Wf + ((size_t)b * 2 + slot) * kp.nk;
+    for (int it = threadIdx.x; it < a.rp * kc; it += blockDim.x) {
+        const int pl = it / kc, jc = it - pl * kc;
+        const int4 *ki = a.kidx + (size_t)(c * a.rp + pl) * 4 * a.kcm + 4 * jc;
+        float v[NC][8];
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const int4 k = ki[e];
+            auto w = [&](int i) {
+                if (i < 0) return make_float2(0.f, 0.f);
+                float2 x = W[i];
+                if (DG) {  // both weight slots
+                    const float2 y = W[kp.nk + i];
+                    x = make_float2(x.x + y.x, x.y + y.y);
+                }
+                return make_float2(TP_WS * x.x, TP_WS * x.y);
+            };
+            const float2 pp = w(k.x), pm = w(k.y), mp = w(k.z), mm = w(k.w);
+            const int j = 4 * jc + e;
+            const float kz = j <= kp.lmax ? a.kzv[kp.lmax + j] : 0.f;
+            // W(+kz) + W(-kz) and their difference for both signs of ky
+            const float2 wpp = make_float2(pp.x + pm.x, pp.y + pm.y), wmp = make_float2(pp.x - pm.x, pp.y - pm.y);
+            const float2 wpm = make_float2(mp.x + mm.x, mp.y + mm.y), wmm = make_float2(mp.x - mm.x, mp.y - mm.y);
+#pragma unroll
+            for (int d = 0; d < 2; d++) {  // Ts, Td
+                const float2 wp = d ? make_float2(wpp.x - wpm.x, wpp.y - wpm.y) : make_float2(wpp.x + wpm.x, wpp.y + wpm.y);
+                const float2 wm = d ? make_float2(wmp.x - wmm.x, wmp.y - wmm.y) : make_float2(wmp.x + wmm.x, wmp.y + wmm.y);
+                v[2 * d][2 * e] = wp.x;
+                v[2 * d][2 * e + 1] = -wm.y;
+                v[2 * d + 1][2 * e] = wp.y;
+                v[2 * d + 1][2 * e + 1] = wm.x;
+                v[4 + 2 * d][2 * e] = kz * wm.x;
+                v[4 + 2 * d][2 * e + 1] = -kz * wp.y;
+                v[5 + 2 * d][2 * e] = kz * wm.y;
+                v[5 + 2 * d][2 * e + 1] = kz * wp.x;
+                if constexpr (DG) {
+                    const float k2 = kz * kz;
+                    v[8 + 2 * d][2 * e] = k2 * wp.x;
+                    v[8 + 2 * d][2 * e + 1] = -k2 * wm.y;
+                    v[9 + 2 * d][2 * e] = k2 * wp.y;
+                    v[9 + 2 * d][2 * e + 1] = k2 * wm.x;
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < NC; r++) {
+            uint4 hi, lo;
+            split8_h(v[r], hi, lo);
+            const int n = NC * pl + r, o = ((n >> 3) * kc + jc) * 8 + (n & 7);
+            Vh[o] = hi;
+            Vl[o] = lo;
+        }
+    }
+}
+
+// Shared memory (from a 1024-aligned base): ex and ey tables of 128 sites (8 TMA boxes), Q hi and lo, two V
+// buffers; the ez tables, read for Q before the second buffer is filled, lie in that one.
+struct TpSmem {
+    int boxxy, boxz, Q, V, vbuf, total;
+    __host__ __device__ TpSmem(int rowsxy, int rowsz, int kcm, int rows) {
+        boxxy = ((rowsxy * 128 + 1023) / 1024) * 1024;
+        boxz = ((rowsz * 128 + 1023) / 1024) * 1024;
+        Q = 8 * boxxy;
+        V = Q + 2 * TF_SITES * kcm * 16;
+        vbuf = ((2 * rows * kcm * 16 + 1023) / 1024) * 1024;
+        total = V + vbuf + (vbuf > 8 * boxz ? vbuf : 8 * boxz) + 1024;
+    }
+};
+
+template <int MODE>
+__global__ void __launch_bounds__(TP_NT, 1)
+    k_field_p(const __grid_constant__ CUtensorMap mapxy, const __grid_constant__ CUtensorMap mapz, KP kp, TpArgs a) {
+    constexpr bool DG = MODE == TF_DG;
+    constexpr int NC = DG ? 12 : 8, EP = (DG ? TP_RPD : TP_RP) / 4;  // pairs a warp at most
+    const int t = blockIdx.x, b = blockIdx.y;
+    if (MODE == TF_D) pdl_launch_dependents();
+    if (MODE == TF_D && bead_converged(kp, b)) {
+        if (a.pdl) pdl_wait();
+        const double zero[2] = {0.0, 0.0};
+        if (kp.dd_async) {
+            const float z[3] = {0.f, 0.f, 0.f};
+            if (dd_unit_arrive(kp, b, t)) dd_unit_sor<TP_NT>(kp, b, t, false, z);
+            return;
+        }
+        dd_block_end<TP_NT>(kp, b, zero, false);
+        return;
+    }
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rowsxy = kp.hmax + kp.kmax + 2, rp = a.rp, kcm = a.kcm, nch = a.nchunk;
+    const TpSmem L(rowsxy, kp.lmax + 1, kcm, NC * rp);
+    extern __shared__ __align__(1024) unsigned char sm_raw[];
+    unsigned char *sm = sm_raw + ((1024u - (umma::smem_u32(sm_raw) & 1023u)) & 1023u);
+    __shared__ uint64_t tbar, vfull[2], mdone[2], tfree[2], pfull[TP_RING];
+    __shared__ uint32_t tslot;
+    // the chunks' pairs, a ring: the copy of chunk c + 5 follows the MMAs of c + 3, which follow every warp's
+    // TMEM load of c + 1 and with it the warp's contraction of c
+    __shared__ __align__(16) int4 sp[TP_RING][TP_RP];
+    const int sb = a.sbase + t * TF_SITES;
+    const uint4 *Vb = a.V + (size_t)b * a.vstride;
+    unsigned char *zt = sm + L.V + L.vbuf;
+    auto copy_chunk = [&](int c) {
+        const int2 ch = a.chunk[c];
+        const uint32_t vb = (uint32_t)(2 * NC * rp * ch.x * 16);
+        mbar_expect_tx(&vfull[c & 1], vb);
+        bulk_load(sm + L.V + (c & 1) * L.vbuf, Vb + ch.y, vb, &vfull[c & 1]);
+        mbar_expect_tx(&pfull[c % TP_RING], (uint32_t)rp * 16u);
+        bulk_load(sp[c % TP_RING], a.pair + (size_t)c * rp, (uint32_t)rp * 16u, &pfull[c % TP_RING]);
+    };
+    if (tid == TF_NT) {
+        umma::mbar_init(&tbar, 1);
+        for (int i = 0; i < 2; i++) {
+            umma::mbar_init(&vfull[i], 1);
+            umma::mbar_init(&mdone[i], 1);
+            umma::mbar_init(&tfree[i], TF_NT / 32);
+        }
+        for (int i = 0; i < TP_RING; i++) umma::mbar_init(&pfull[i], 1);
+        mbar_expect_tx(&tbar, 8u * (uint32_t)((rowsxy + kp.lmax + 1) * 128));
+        for (int i = 0; i < 8; i++) {
+            tma_load_2d(zt + i * L.boxz, &mapz, 2 * (sb + 16 * i), b * kp.ntab + rowsxy, &tbar);
+            tma_load_2d(sm + i * L.boxxy, &mapxy, 2 * (sb + 16 * i), b * kp.ntab, &tbar);
+        }
+    }
+    if (warp == 0) umma::tmem_alloc(&tslot, 512);
+    const int iter = kp.dstep[1] + 1;
+    umma::fence_before_sync();
+    __syncthreads();
+    umma::fence_after_sync();
+    const uint32_t tm = tslot;
+    uint32_t err = 0;
+    int issued = 0;
+    if (tid == TF_NT) {  // the first chunk, beside Q
+        if (a.pdl) pdl_wait();
+        copy_chunk(0);
+        issued = 1;
+    }
+    __syncwarp();
+    unsigned char *Qh = sm + L.Q, *Ql = Qh + TF_SITES * kcm * 16;
+    if (warp < TF_NT / 32) {
+        err |= (uint32_t)umma::mbar_wait(&tbar, 0, TC_WAIT);
+        for (int it = tid; it < TF_SITES * kcm; it += TF_NT) {
+            const int s = it % TF_SITES, jc = it / TF_SITES;
+            float v[8];
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const int j = 4 * jc + e;
+                const float2 z = j <= kp.lmax ? tab_elem(zt, L.boxz, j, s) : make_float2(0.f, 0.f);
+                v[2 * e] = z.x;
+                v[2 * e + 1] = z.y;
+            }
+            uint4 hi, lo;
+            split8_h(v, hi, lo);
+            const int o = rowchunk_k(s, jc, kcm);
+            *reinterpret_cast<uint4 *>(Qh + o) = hi;
+            *reinterpret_cast<uint4 *>(Ql + o) = lo;
+        }
+    }
+    // everything above reads only the positions; from here on V and the iteration's fields (a programmatic
+    // launch waits for them here); the SOR inputs of the CTA's dipole sites
+    if (a.pdl) pdl_wait();
+    const int s_own = sb + tid;
+    const bool own = tid < TF_SITES && s_own >= a.s_lo && s_own < a.s_hi;
+    DdSite din;
+    if (MODE == TF_D && own && !kp.dd_async) dd_sor_load(kp, b, s_own, din);
+    umma::fence_smem_to_async();
+    umma::fence_before_sync();
+    bool bad = __syncthreads_or((int)err) != 0;
+    umma::fence_after_sync();
+    constexpr int NA = DG ? 6 : 4;
+    float acc[NA];
+#pragma unroll
+    for (int i = 0; i < NA; i++) acc[i] = 0.f;
+    const int lq = warp & 3, part = warp >> 2, sl = 32 * lq + lane;
+    err = 0;
+    if (warp == TF_NT / 32) {
+        if (lane == 0 && !bad) {
+            const uint32_t idesc = (umma::idesc_f16(128, 16) & ~(0x3Fu << 17)) | ((uint32_t)(NC * rp >> 3) << 17);
+            const uint32_t qh = umma::smem_u32(Qh), ql = umma::smem_u32(Ql);
+            int mma = 0;  // chunks whose MMAs are issued
+            for (int c = 0; c < nch; c++) {
+                const int h = c & 1;
+                // the next chunk's copy goes out once the MMAs that read its buffer are done
+                if (c + 1 < nch) {
+                    if (c >= 1) err |= (uint32_t)umma::mbar_wait(&mdone[h ^ 1], (uint32_t)(((c - 1) >> 1) & 1), TC_WAIT);
+                    if (err) break;
+                    copy_chunk(c + 1);
+                    issued = c + 2;
+                }
+                err |= (uint32_t)umma::mbar_wait(&vfull[h], (uint32_t)((c >> 1) & 1), TC_WAIT);
+                if (c >= 2) err |= (uint32_t)umma::mbar_wait(&tfree[h], (uint32_t)(((c - 2) >> 1) & 1), TC_WAIT);
+                if (err) break;
+                umma::fence_after_sync();
+                const int kc = a.chunk[c].x;
+                const uint32_t vh = umma::smem_u32(sm + L.V + h * L.vbuf), vl = vh + (uint32_t)(NC * rp * kc * 16);
+                const uint32_t d = tm + (uint32_t)(256 * h);
+                for (int ks = 0; ks < kc / 2; ks++) {
+                    const uint64_t dq_h = umma::sdesc(qh + ks * 256, 128, kcm * 128), dq_l = umma::sdesc(ql + ks * 256, 128, kcm * 128);
+                    const uint64_t dv_h = umma::sdesc(vh + ks * 256, 128, kc * 128), dv_l = umma::sdesc(vl + ks * 256, 128, kc * 128);
+                    umma::mma_f16(d, dq_h, dv_h, idesc, ks > 0);
+                    umma::mma_f16(d, dq_h, dv_l, idesc, 1);
+                    umma::mma_f16(d, dq_l, dv_h, idesc, 1);
+                }
+                umma::commit(&mdone[h]);
+                mma = c + 1;
+            }
+            // MMAs and copies still in flight end before the CTA leaves
+            for (int c = max(0, mma - 2); c < mma; c++) err |= (uint32_t)umma::mbar_wait(&mdone[c & 1], (uint32_t)((c >> 1) & 1), TC_WAIT);
+            for (int c = mma; c < issued; c++) umma::mbar_wait(&vfull[c & 1], (uint32_t)((c >> 1) & 1), TC_WAIT);
+            for (int c = max(0, issued - TP_RING); c < issued; c++) umma::mbar_wait(&pfull[c % TP_RING], (uint32_t)((c / TP_RING) & 1), TC_WAIT);
+        } else if (lane == 0 && issued) {
+            umma::mbar_wait(&vfull[0], 0, TC_WAIT);
+            umma::mbar_wait(&pfull[0], 0, TC_WAIT);
+        }
+        __syncwarp();
+    } else if (!bad) {
+        const int q4 = rp / 4;
+        // the lane's site in the staged tables: its box and float2 slot, and its 16-byte chunk (before the swizzle) times 16
+        const unsigned char *tsite = sm + (sl >> 4) * L.boxxy + (sl & 1) * 8;
+        const int cs4 = ((sl & 15) >> 1) << 4;
+        const uint32_t tl = tm + ((uint32_t)(32 * lq) << 16) + (uint32_t)(part * q4 * NC);
+        for (int c = 0; c < nch; c++) {
+            const int h = c & 1;
+            err |= (uint32_t)umma::mbar_wait(&pfull[c % TP_RING], (uint32_t)((c / TP_RING) & 1), TC_WAIT);
+            err |= (uint32_t)umma::mbar_wait(&mdone[h], (uint32_t)((c >> 1) & 1), TC_WAIT);
+            if (__any_sync(0xffffffffu, err != 0)) break;
+            umma::fence_after_sync();
+            float v[64];
+            const uint32_t tc = tl + (uint32_t)(256 * h);
+            umma::tmem_ld16x4(tc, tc + 16, tc + 32, tc + 48, v);
+            umma::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tfree[h]);  // chunk c + 2's MMAs may overwrite it
+            const int4 *pp = sp[c % TP_RING] + part * q4;
+#pragma unroll
+            for (int e = 0; e < EP; e++) {
+                if (e >= q4) break;
+                const int4 P = pp[e];
+                const float kx = __int_as_float(P.z), ky = __int_as_float(P.w);
+                const float2 ex = *reinterpret_cast<const float2 *>(tsite + (P.x & 0xffff) + (cs4 ^ (P.x >> 16)));
+                const float2 ey = *reinterpret_cast<const float2 *>(tsite + (P.y & 0xffff) + (cs4 ^ (P.y >> 16)));
+                const float *w = v + NC * e;  // Ts, Td of T0, of T1 (, of T2): re, im
+                const float u0r = fmaf(ey.x, w[0], -ey.y * w[3]), u0i = fmaf(ey.x, w[1], ey.y * w[2]);
+                const float v0r = fmaf(ey.x, w[2], -ey.y * w[1]), v0i = fmaf(ey.x, w[3], ey.y * w[0]);
+                const float u1r = fmaf(ey.x, w[4], -ey.y * w[7]), u1i = fmaf(ey.x, w[5], ey.y * w[6]);
+                if constexpr (DG) {
+                    const float v1r = fmaf(ey.x, w[6], -ey.y * w[5]), v1i = fmaf(ey.x, w[7], ey.y * w[4]);
+                    const float u2r = fmaf(ey.x, w[8], -ey.y * w[11]), u2i = fmaf(ey.x, w[9], ey.y * w[10]);
+                    const float S0 = kx * fmaf(ex.x, u0r, -ex.y * u0i), D0 = ky * fmaf(ex.x, v0r, -ex.y * v0i);
+                    acc[0] = fmaf(kx, S0, acc[0]);
+                    acc[1] = fmaf(kx, D0, acc[1]);
+                    acc[2] = fmaf(ky * ky, fmaf(ex.x, u0r, -ex.y * u0i), acc[2]);
+                    acc[3] = fmaf(kx, fmaf(ex.x, u1r, -ex.y * u1i), acc[3]);
+                    acc[4] = fmaf(ky, fmaf(ex.x, v1r, -ex.y * v1i), acc[4]);
+                    acc[5] += fmaf(ex.x, u2r, -ex.y * u2i);
+                } else {
+                    acc[0] = fmaf(kx, fmaf(ex.x, u0i, ex.y * u0r), acc[0]);
+                    acc[1] = fmaf(ky, fmaf(ex.x, v0i, ex.y * v0r), acc[1]);
+                    acc[2] += fmaf(ex.x, u1i, ex.y * u1r);
+                    if (MODE == TF_Q || MODE == TF_QG) acc[3] += fmaf(ex.x, u0r, -ex.y * u0i);
+                }
+            }
+        }
+    }
+    float e[4] = {0.f, 0.f, 0.f, 0.f};
+    if constexpr (DG) {  // the dipole of the lane's site, zero outside the range
+        float mx = 0.f, my = 0.f, mz = 0.f;
+        if (warp < TF_NT / 32 && sb + sl >= a.s_lo && sb + sl < a.s_hi) {
+            const float4 m = kp.dipf[(size_t)b * kp.S + sb + sl];
+            mx = m.x, my = m.y, mz = m.z;
+        }
+        e[0] = -fmaf(acc[0], mx, fmaf(acc[1], my, acc[3] * mz));
+        e[1] = -fmaf(acc[1], mx, fmaf(acc[2], my, acc[4] * mz));
+        e[2] = -fmaf(acc[3], mx, fmaf(acc[4], my, acc[5] * mz));
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; i++) e[i] = acc[i];
+    }
+    bad = __syncthreads_or((int)(bad || err)) != 0;  // (every MMA is done: Q may be written)
+    float *red = reinterpret_cast<float *>(Qh);      // the four pair quarters of each site, in order
+    if (warp < TF_NT / 32) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) red[(part * TF_SITES + sl) * 4 + i] = e[i] * (1.f / TP_WS);
+    }
+    umma::fence_before_sync();
+    __syncthreads();
+    if (warp == 0) {
+        umma::fence_after_sync();
+        umma::tmem_dealloc(tm, 512);
+        umma::tmem_relinquish();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) e[i] = 0.f;
+    if (own && !bad) {
+#pragma unroll
+        for (int rq = 0; rq < 4; rq++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) e[i] += red[(rq * TF_SITES + tid) * 4 + i];
+    }
+    if (bad && tid == 0) atomicOr(kp.err, 8u);
+    field_out<MODE, TP_NT>(kp, b, t, s_own, own && !bad, bad, e, din, iter);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1066,6 +1070,130 @@ static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
             fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
     }
     return fn;
+}
+
+// Pairs, chunks, k-vector indices and V of the prepared passes: which 0 the 8-row form, 1 the 12-row one.
+static bool tp_init(Engine &E, int which, const std::vector<int> &jr, int dmax) {
+    KP &kp = E.kp;
+    Engine::TpSet &T = E.tp[which];
+    const int NC = which ? 12 : 8, rowsxy = kp.hmax + kp.kmax + 2, jmax = kp.lmax + 1;
+    const int kcm = ((2 * jmax + 15) / 16) * 2;  // K row blocks of Q: 8 halves (4 |kz|: cos, sin) each, an even number
+    if (rowsxy > 256 || rowsxy * 128 > 0xffff || jmax > 256) return false;
+    int rp = which ? TP_RPD : TP_RP;
+    while (rp >= 4 && TpSmem(rowsxy, jmax, kcm, NC * rp).total > dmax) rp -= 4;
+    if (rp < 4) return false;
+    struct Pair {
+        int kx, ky, r[2], jm;
+    };
+    std::vector<Pair> pairs;
+    std::map<std::pair<int, int>, int> at;
+    for (int r = 0; r < kp.nrun; r++) {
+        const KRun &run = E.h_runs[r];
+        const std::pair<int, int> key(run.kx, std::abs(run.ky));
+        if (!at.count(key)) {
+            at[key] = (int)pairs.size();
+            pairs.push_back(Pair{run.kx, key.second, {-1, -1}, 0});
+        }
+        Pair &p = pairs[at[key]];
+        int &slot = p.r[run.ky < 0 ? 1 : 0];
+        if (run.kx < 0 || slot >= 0) return false;
+        slot = r;
+        p.jm = std::max(p.jm, jr[r]);
+    }
+    std::stable_sort(pairs.begin(), pairs.end(), [](const Pair &x, const Pair &y) { return x.jm > y.jm; });
+    const int np = (int)pairs.size(), nch = (np + rp - 1) / rp;
+    std::vector<int4> pr((size_t)nch * rp, make_int4(0, 0, 0, 0)), ki((size_t)nch * rp * 4 * kcm, make_int4(-1, -1, -1, -1));
+    std::vector<int2> chunk(nch);
+    int words = 0;
+    auto bits = [](float f) {
+        int i;
+        std::memcpy(&i, &f, 4);
+        return i;
+    };
+    for (int c = 0; c < nch; c++) {
+        const int kc = ((2 * pairs[c * rp].jm + 15) / 16) * 2;
+        chunk[c] = make_int2(kc, words);
+        words += 2 * NC * rp * kc;
+        for (int q = 0; q < rp; q++) {
+            // the last chunk's missing pairs: zero rows of V against the (0, 0) tables
+            const int ry0 = kp.hmax + 1;
+            if (c * rp + q >= np) {
+                pr[c * rp + q] = make_int4(0, ry0 * 128 | ((ry0 & 7) << 4) << 16, 0, 0);
+                continue;
+            }
+            const Pair &p = pairs[c * rp + q];
+            const int ry = ry0 + p.ky, r0 = p.r[0] >= 0 ? p.r[0] : p.r[1];
+            const float kx = (float)E.h_kvec[3 * E.h_runs[r0].kbeg], ky = std::fabs((float)E.h_kvec[3 * E.h_runs[r0].kbeg + 1]);
+            pr[c * rp + q] = make_int4(p.kx * 128 | ((p.kx & 7) << 4) << 16, ry * 128 | ((ry & 7) << 4) << 16, bits(kx), bits(ky));
+            for (int j = 0; j < p.jm; j++) {
+                int k[4] = {-1, -1, -1, -1};
+                for (int s = 0; s < 2; s++) {
+                    if (p.r[s] < 0) continue;
+                    const KRun &run = E.h_runs[p.r[s]];
+                    if (j >= run.kzlo && j < run.kzlo + run.nkz) k[2 * s] = run.kbeg + j - run.kzlo;
+                    if (j > 0 && -j >= run.kzlo && -j < run.kzlo + run.nkz) k[2 * s + 1] = run.kbeg - j - run.kzlo;
+                }
+                ki[((size_t)c * rp + q) * 4 * kcm + j] = make_int4(k[0], k[1], k[2], k[3]);
+            }
+        }
+    }
+    const size_t n[4] = {sizeof(int4) * pr.size(), sizeof(int2) * chunk.size(), sizeof(int4) * ki.size(), 16 * (size_t)words * kp.P};
+    const void *src[3] = {pr.data(), chunk.data(), ki.data()};
+    void *d[4] = {nullptr, nullptr, nullptr, nullptr};
+    for (int i = 0; i < 4; i++) {
+        if (cudaMalloc(&d[i], n[i]) != cudaSuccess) {
+            cudaGetLastError();
+            for (int q = 0; q < i; q++) cudaFree(d[q]);
+            return false;
+        }
+    }
+    for (int i = 0; i < 4; i++) {
+        E.allocs.push_back(d[i]);
+        if (i < 3) cudaMemcpy(d[i], src[i], n[i], cudaMemcpyHostToDevice);
+    }
+    T.pair = reinterpret_cast<const int4 *>(d[0]);
+    T.chunk = reinterpret_cast<const int2 *>(d[1]);
+    T.kidx = reinterpret_cast<const int4 *>(d[2]);
+    T.V = d[3];
+    T.vstride = words;
+    T.nchunk = nch;
+    T.rp = rp;
+    T.kcm = kcm;
+    return true;
+}
+
+static void tp_setup(Engine &E, PFN_cuTensorMapEncodeTiled_v12000 enc, const std::vector<int> &jr, int optin) {
+    KP &kp = E.kp;
+    const void *fk[4] = {(const void *)k_field_p<TF_Q>, (const void *)k_field_p<TF_D>, (const void *)k_field_p<TF_QG>,
+                         (const void *)k_field_p<TF_DG>};
+    size_t fstat = 0;
+    for (const void *f : fk) {
+        cudaFuncAttributes fa;
+        if (cudaFuncGetAttributes(&fa, f) != cudaSuccess) {
+            cudaGetLastError();
+            return;
+        }
+        fstat = std::max(fstat, fa.sharedSizeBytes);
+    }
+    const int dmax = optin - (int)fstat;
+    for (const void *f : fk)
+        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, dmax) != cudaSuccess) {
+            cudaGetLastError();
+            return;
+        }
+    // the ex and ey rows, and the ez rows, of 16 sites
+    const cuuint64_t dims[2] = {(cuuint64_t)2 * kp.S, (cuuint64_t)kp.P * kp.ntab};
+    const cuuint64_t strides[1] = {(cuuint64_t)kp.S * 8};
+    const cuuint32_t es[2] = {1, 1};
+    for (int z = 0; z < 2; z++) {
+        const cuuint32_t box[2] = {32, (cuuint32_t)(z ? kp.lmax + 1 : kp.hmax + kp.kmax + 2)};
+        if (box[1] > 256 || enc(reinterpret_cast<CUtensorMap *>(z ? E.tp_mapz : E.tp_mapxy), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, kp.tabf,
+                                dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return;
+    }
+    E.tf_ready = tp_init(E, 0, jr, dmax);
+    E.tf_qd_ready = E.tf_ready && tp_init(E, 1, jr, dmax);
 }
 
 void tc_init(Engine &E) {
@@ -1241,165 +1369,81 @@ void tc_init(Engine &E) {
     E.tc_ncolmax = ncolmax;
     E.tc_nabuf = nabuf;
     E.tc_ready = true;
-    // field kernel: every run once (the first kp.nrun slots, in the same order), K over its
-    // whole |kz| range; per (run, j) the k-vectors of kz = +j and -j
     E.tf_ready = false;
-    const int nr = kp.nrun, jm = jr[order[0]], kq = ((2 * jm + 15) / 16) * 16;
-    const void *fk[7] = {(const void *)k_field_tc<TF_Q, false>, (const void *)k_field_tc<TF_D, false>,
-                         (const void *)k_field_tc<TF_QG, false>, (const void *)k_field_tc<TF_Q, true>,
-                         (const void *)k_field_tc<TF_D, true>, (const void *)k_field_tc<TF_QG, true>,
-                         (const void *)k_field_tc<TF_DG, true>};
-    size_t fstat = 0;
-    for (const void *f : fk) {
-        cudaFuncAttributes fa;
-        if (cudaFuncGetAttributes(&fa, f) != cudaSuccess) {
-            cudaGetLastError();
-            return;
-        }
-        fstat = std::max(fstat, fa.sharedSizeBytes);
-    }
-    const int dmaxf = optin - (int)fstat;
-    for (const void *f : fk)
-        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, dmaxf) != cudaSuccess) {
-            cudaGetLastError();
-            return;
-        }
-    // passes: two passes of nph runs (a multiple of 8) x 4 components in TMEM with V of both built
-    // once, when that fits (plus the 16 columns the last 16-run load of a run quarter reaches past
-    // a pass); else passes of nph runs with V of each built before it. The bead's weights sit in
-    // shared memory (one bulk copy: 8 nk bytes, a multiple of 16) when they fit, else the V
-    // builders read them from global memory.
-    auto fits = [&](int nph_, int vpp_, int wglob_, int ncomp, int nslot_) {
-        return ncomp * nph_ + 16 <= 512 && TfSmem(kp.ntab, (vpp_ ? ncomp : 2 * ncomp) * nph_, kq, kp.nk, wglob_ ? 0 : nslot_).total <= dmaxf;
-    };
-    const bool w_ok = (kp.nk & 1) == 0;
-    int nph = ((nr + 1) / 2 + 7) / 8 * 8, vpp = 0, wglob = w_ok ? 0 : 1;
-    if (!fits(nph, 0, wglob, 4, 1)) {
-        vpp = 1;
-        for (wglob = w_ok ? 0 : 1; wglob < 2; wglob++) {
-            for (nph = std::min(120, (nr + 7) / 8 * 8); nph > 8 && !fits(nph, 1, wglob, 4, 1); nph -= 8) {
-            }
-            if (fits(nph, 1, wglob, 4, 1)) break;
-        }
-        if (wglob == 2) return;
-    }
-    const int ncolf = (vpp ? 4 : 8) * nph;
-    if (kp.ntab > 128) return;
-    std::vector<int2> kpm((size_t)nr * jm, make_int2(-1, -1));
-    for (int p = 0; p < nr; p++) {
-        const KRun &run = E.h_runs[order[p]];
-        for (int j = 0; j < jm; j++) {
-            int2 v = make_int2(-1, -1);
-            if (j >= run.kzlo && j < run.kzlo + run.nkz) v.x = run.kbeg + j - run.kzlo;
-            if (j > 0 && -j >= run.kzlo && -j < run.kzlo + run.nkz) v.y = run.kbeg - j - run.kzlo;
-            kpm[(size_t)p * jm + j] = v;
-        }
-    }
-    int2 *d_kpm = nullptr;
-    if (cudaMalloc((void **)&d_kpm, sizeof(int2) * kpm.size()) != cudaSuccess) {
-        cudaGetLastError();
-        return;
-    }
-    E.allocs.push_back(d_kpm);
-    cudaMemcpy(d_kpm, kpm.data(), sizeof(int2) * kpm.size(), cudaMemcpyHostToDevice);
-    E.d_tfkpm = d_kpm;
-    E.tf_nr = nr;
-    E.tf_nph = nph;
-    E.tf_jm = jm;
-    E.tf_ncol = ncolf;
-    E.tf_kq = kq;
-    E.tf_vpp = vpp;
-    E.tf_wglob = wglob;
-    E.tf_ready = true;
-    // dipole-force mode: 6 components per run, passes of nphd runs (a multiple of 8) with
-    // 6 nphd + 16 <= 512 TMEM columns, V of one pass at a time, both weight slots in shared
-    // memory when they fit
-    const int npd = (nr + 79) / 80;
-    int nphd = ((nr + npd - 1) / npd + 7) / 8 * 8, wgd = w_ok ? 0 : 1;
-    for (; wgd < 2; wgd++) {
-        for (nphd = ((nr + npd - 1) / npd + 7) / 8 * 8; nphd > 8 && !fits(nphd, 1, wgd, 6, 2); nphd -= 8) {
-        }
-        if (fits(nphd, 1, wgd, 6, 2)) break;
-    }
-    E.tf_qd_ready = wgd < 2;
-    E.tf_nphd = nphd;
-    E.tf_ncold = 6 * nphd;
-    E.tf_wglob_d = wgd;
+    tp_setup(E, enc, jr, optin);
 }
 
 // whether the iterations' field pass is launched as a programmatic dependent (griddepcontrol.wait
 // before it reads the iteration's fields)
-bool field_pdl_ok(const Engine &E) { return E.tc_ready && E.tf_ready && E.ff_tc && E.tc_pdl && E.sf_tc; }
+bool field_pdl_ok(const Engine &E) {
+    return E.tc_ready && E.tf_ready && E.ff_tc && E.tc_pdl && E.sf_tc;
+}
+
+// One of the prepared passes (k_field_v, then k_field_p).
+template <int MODE>
+static void launch_field_p(Engine &E, int s0, int s1) {
+    const KP &kp = E.kp;
+    constexpr bool DG = MODE == TF_DG;
+    const Engine::TpSet &T = E.tp[DG ? 1 : 0];
+    TpArgs a;
+    a.pair = T.pair;
+    a.chunk = T.chunk;
+    a.kidx = T.kidx;
+    a.kzv = E.d_tckzv;
+    a.V = reinterpret_cast<uint4 *>(T.V);
+    a.vstride = T.vstride;
+    a.nchunk = T.nchunk;
+    a.rp = T.rp;
+    a.kcm = T.kcm;
+    a.sbase = s0 & ~(TC_SS - 1);  // TMA x coordinates 2 (sbase + 16 i): 128-byte aligned
+    a.s_lo = s0;
+    a.s_hi = s1;
+    a.skipconv = MODE == TF_D ? 1 : 0;
+    a.pdl = E.tc_pdl ? 1 : 0;
+    const int slot = (MODE == TF_D || MODE == TF_QG) ? 1 : 0;
+    const TpSmem L(kp.hmax + kp.kmax + 2, kp.lmax + 1, T.kcm, (DG ? 12 : 8) * T.rp);
+    const CUtensorMap *xy = reinterpret_cast<const CUtensorMap *>(E.tp_mapxy), *z = reinterpret_cast<const CUtensorMap *>(E.tp_mapz);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cv = {}, cf = {};
+    cv.gridDim = dim3(T.nchunk, kp.P);
+    cv.blockDim = dim3(TP_VT);
+    cf.gridDim = dim3((s1 - a.sbase + TF_SITES - 1) / TF_SITES, kp.P);
+    cf.blockDim = dim3(TP_NT);
+    cf.dynamicSmemBytes = L.total;
+    // both as programmatic dependents: V's grid of the structure factor, the field pass of V's
+    auto run = [&](cudaLaunchConfig_t &cfg, auto &&launch) {
+        cfg.stream = E.stream;
+        cfg.attrs = at;
+        cfg.numAttrs = a.pdl;
+        if (launch() == cudaSuccess || !a.pdl) return;
+        cudaGetLastError();
+        a.pdl = 0;
+        cfg.numAttrs = 0;
+        E.tc_pdl = false;  // not available: plain launches from now on
+        if (E.field_needs_join) cudaStreamWaitEvent(E.stream, E.loop_join, 0);
+        launch();
+    };
+    run(cv, [&] { return cudaLaunchKernelEx(&cv, k_field_v<DG>, kp, a, slot); });
+    run(cf, [&] { return cudaLaunchKernelEx(&cf, k_field_p<MODE>, *xy, *z, kp, a); });
+    E.nlaunch += 2;
+}
 
 // mode TF_D: dipole field, SOR update and convergence test of one iteration at the dipole sites
 // [s0, s1) (k_field_f<F_D> + k_field_finish<F_D>); TF_Q: charge field and potential added to F at
 // [s0, s1) (k_field_f<F_Q> + k_field_finish<F_Q>); TF_QG, TF_DG: the halves of the force pass
 // (launch_field_qd_tc). 1 when launched, else 0.
 int launch_field_tc(Engine &E, int mode, int s0, int s1) {
-    if (!E.tc_ready || !E.tf_ready || !E.ff_tc || s1 <= s0) return 0;
-    const KP &kp = E.kp;
-    TfArgs a;
-    a.slot = E.d_tcslot;
-    a.skv = E.d_tcskv;
-    a.kpm = E.d_tfkpm;
-    a.kzv = E.d_tckzv;
-    a.nr = E.tf_nr;
-    a.nph = E.tf_nph;
-    a.ncol = E.tf_ncol;
-    a.kq = E.tf_kq;
-    a.jm = E.tf_jm;
-    a.sbase = s0 & ~(TC_SS - 1);  // TMA x coordinates 2 (sbase + 16 i): 128-byte aligned
-    a.s_lo = s0;
-    a.s_hi = s1;
-    a.vpp = E.tf_vpp;
-    a.wglob = E.tf_wglob;
-    if (mode == TF_DG) {
-        a.nph = E.tf_nphd;
-        a.ncol = E.tf_ncold;
-        a.vpp = 1;
-        a.wglob = E.tf_wglob_d;
-    }
-    const TfSmem L(kp.ntab, a.ncol, a.kq, kp.nk, a.wglob ? 0 : (mode == TF_DG ? 2 : 1));
-    dim3 g((s1 - a.sbase + TF_SITES - 1) / TF_SITES, kp.P);
-    const CUtensorMap *map = reinterpret_cast<const CUtensorMap *>(E.tc_map);
-    a.pdl = 0;
-    if (mode == TF_D && E.tc_pdl && E.sf_tc) {
-        // a programmatic dependent of the iteration's structure factor: its set-up (tables,
-        // Q) runs while that grid finishes; it waits (pdl_wait) before reading the weights
-        a.pdl = 1;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = g;
-        cfg.blockDim = dim3(TF_NT);
-        cfg.dynamicSmemBytes = L.total;
-        cfg.stream = E.stream;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        const cudaError_t le = a.vpp ? cudaLaunchKernelEx(&cfg, k_field_tc<TF_D, true>, *map, kp, a)
-                                     : cudaLaunchKernelEx(&cfg, k_field_tc<TF_D, false>, *map, kp, a);
-        if (le == cudaSuccess) {
-            ++E.nlaunch;
-            return 1;
-        }
-        cudaGetLastError();
-        a.pdl = 0;
-        E.tc_pdl = false;  // not available: plain launches from now on
-        if (E.field_needs_join) cudaStreamWaitEvent(E.stream, E.loop_join, 0);
-    }
+    if (!E.tc_ready || !E.tf_ready || !E.ff_tc || s1 <= s0 || (mode == TF_DG && !E.tf_qd_ready)) return 0;
     if (mode == TF_D)
-        a.vpp ? k_field_tc<TF_D, true><<<g, TF_NT, L.total, E.stream>>>(*map, kp, a)
-              : k_field_tc<TF_D, false><<<g, TF_NT, L.total, E.stream>>>(*map, kp, a);
+        launch_field_p<TF_D>(E, s0, s1);
     else if (mode == TF_Q)
-        a.vpp ? k_field_tc<TF_Q, true><<<g, TF_NT, L.total, E.stream>>>(*map, kp, a)
-              : k_field_tc<TF_Q, false><<<g, TF_NT, L.total, E.stream>>>(*map, kp, a);
+        launch_field_p<TF_Q>(E, s0, s1);
     else if (mode == TF_QG)
-        a.vpp ? k_field_tc<TF_QG, true><<<g, TF_NT, L.total, E.stream>>>(*map, kp, a)
-              : k_field_tc<TF_QG, false><<<g, TF_NT, L.total, E.stream>>>(*map, kp, a);
+        launch_field_p<TF_QG>(E, s0, s1);
     else
-        k_field_tc<TF_DG, true><<<g, TF_NT, L.total, E.stream>>>(*map, kp, a);
-    ++E.nlaunch;
+        launch_field_p<TF_DG>(E, s0, s1);
     return 1;
 }
 
