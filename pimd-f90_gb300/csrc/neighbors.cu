@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(NB_MAXN) k_nbr_block(KP kp) {
 // Boxes of more than NB_MAXN molecules with at least 4 cells of width >= Rc per edge: cell lists.
 // The O sites of a bead are binned into cells; a warp owns row i, tests the members of the 27
 // surrounding cells (FP32 prefilter, FP64 near the cutoff: the same decisions as above), collects
-// the hits of the full row in shared memory and sorts them by j (bitonic), so the half and full
+// the hits of the full row in shared memory and puts them in order of j, so the half and full
 // lists written afterwards are the reference's lists bit for bit.
 constexpr int CL_ROWCAP = 256;  // neighbours of one molecule in the full list (about 100 at water density and 9 A)
 
@@ -301,14 +301,25 @@ __global__ void __launch_bounds__(128) k_cell_fill(KP kp) {
     kp.cl_list[(size_t)b * kp.N + kp.cl_start[(size_t)b * (kp.cl_ncell + 1) + cell] + slot] = i;
 }
 
-// warp per (row, bead): sorted full row into cl_row, counts of the half / full rows
-template <bool FULL>
+// warp per (row, bead): sorted full row into cl_row, counts of the half / full rows. The hits are put in order
+// by setting their bits of a row of N bits in shared memory and reading it back word by word (BITS): 200
+// instructions at 4096 molecules where a bitonic sort of 256 takes 3500. The reading grows with N and takes
+// as long as the sort at about 100000 molecules, where the sort stays. Cells along x are contiguous in the list,
+// so the 27 cells are 9 ranges of members (10 or more at the box faces).
+constexpr int CL_BITN = 65536;
+
+template <bool FULL, bool BITS>
 __global__ void __launch_bounds__(128) k_cell_rows(KP kp) {
-    __shared__ int buf[4][CL_ROWCAP];
+    extern __shared__ int cl_buf[];  // a warp's bits, or its hits
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, b = blockIdx.y;
     if (i >= kp.N) return;
-    int *row = buf[wib];
+    const int words = BITS ? ((kp.N + 31) / 32 + 31) / 32 * 32 : CL_ROWCAP;
+    int *row = cl_buf + wib * words;
+    if (BITS) {
+        for (int w = lane; w < words; w += 32) row[w] = 0;
+        __syncwarp();
+    }
     const float4 *pf = kp.cl_posf + (size_t)b * kp.N;
     const double4_32a *O = kp.pos + (size_t)b * kp.S;
     const float4 fi = pf[i];
@@ -316,56 +327,86 @@ __global__ void __launch_bounds__(128) k_cell_rows(KP kp) {
     const float rc2f = (float)kp.rc2;
     const float3 Lf = make_float3((float)kp.box[0], (float)kp.box[1], (float)kp.box[2]);
     const float3 Lif = make_float3((float)kp.boxi[0], (float)kp.boxi[1], (float)kp.boxi[2]);
+    const int nx = kp.cl_n[0];
     const int ci = kp.cl_mol[(size_t)b * kp.N + i];
-    const int c0 = ci % kp.cl_n[0], c1 = (ci / kp.cl_n[0]) % kp.cl_n[1], c2 = ci / (kp.cl_n[0] * kp.cl_n[1]);
+    const int c0 = ci % nx, c1 = (ci / nx) % kp.cl_n[1], c2 = ci / (nx * kp.cl_n[1]);
     const int *start = kp.cl_start + (size_t)b * (kp.cl_ncell + 1);
     const int *list = kp.cl_list + (size_t)b * kp.N;
     int n = 0;
-    for (int d = 0; d < 27; d++) {
-        const int x = (c0 + d % 3 - 1 + kp.cl_n[0]) % kp.cl_n[0];
-        const int y = (c1 + (d / 3) % 3 - 1 + kp.cl_n[1]) % kp.cl_n[1];
-        const int z = (c2 + d / 9 - 1 + kp.cl_n[2]) % kp.cl_n[2];
-        const int cell = (z * kp.cl_n[1] + y) * kp.cl_n[0] + x;
-        const int m0 = start[cell], m1 = start[cell + 1];
+    auto members = [&](int m0, int m1) {
         for (int m = m0; m < m1; m += 32) {
             const int mm = m + lane;
             const int j = mm < m1 ? list[mm] : -1;
             const bool hit = j >= 0 && j != i && oo_test_sm(fi, pf[max(j, 0)], di, O[max(j, 0)], kp, rc2f, Lf, Lif);
             const unsigned msk = __ballot_sync(0xffffffffu, hit);
             if (hit) {
-                const int slot = n + __popc(msk & ((1u << lane) - 1u));
-                if (slot < CL_ROWCAP) row[slot] = j;
+                if (BITS) {
+                    atomicOr(row + (j >> 5), 1 << (j & 31));
+                } else {
+                    const int slot = n + __popc(msk & ((1u << lane) - 1u));
+                    if (slot < CL_ROWCAP) row[slot] = j;
+                }
             }
             n += __popc(msk);
         }
+    };
+    for (int d = 0; d < 9; d++) {
+        const int y = (c1 + d % 3 - 1 + kp.cl_n[1]) % kp.cl_n[1];
+        const int z = (c2 + d / 3 - 1 + kp.cl_n[2]) % kp.cl_n[2];
+        const int *at = start + (z * kp.cl_n[1] + y) * nx;
+        members(at[max(c0 - 1, 0)], at[min(c0 + 1, nx - 1) + 1]);
+        if (c0 == 0) members(at[nx - 1], at[nx]);
+        if (c0 == nx - 1) members(at[0], at[1]);
     }
-    if (n > CL_ROWCAP) {
-        if (lane == 0) atomicOr(kp.err, 1u);
-        n = CL_ROWCAP;
-    }
-    for (int s = n + lane; s < CL_ROWCAP; s += 32) row[s] = 0x7fffffff;
-    __syncwarp();
-    // bitonic sort of the row (ascending j)
-    for (int k = 2; k <= CL_ROWCAP; k <<= 1)
-        for (int jj = k >> 1; jj > 0; jj >>= 1) {
-            for (int t = lane; t < CL_ROWCAP; t += 32) {
-                const int p = t ^ jj;
-                if (p > t) {
-                    const int a = row[t], c = row[p];
-                    const bool up = (t & k) == 0;
-                    if ((a > c) == up) {
-                        row[t] = c;
-                        row[p] = a;
-                    }
-                }
-            }
-            __syncwarp();
-        }
+    if (n > CL_ROWCAP && lane == 0) atomicOr(kp.err, 1u);
     int nh = 0;
     int *out = kp.cl_row + ((size_t)b * kp.N + i) * CL_ROWCAP;
-    for (int s = lane; s < n; s += 32) {
-        out[s] = row[s];
-        nh += row[s] > i;
+    if (BITS) {
+        __syncwarp();
+        int base = 0;
+        for (int w0 = 0; w0 < words; w0 += 32) {
+            const int w = w0 + lane;
+            unsigned bits = (unsigned)row[w];
+            const int c = __popc(bits);
+            int x = c;  // inclusive sum over the lanes
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            for (int s = base + x - c; bits; s++, bits &= bits - 1) {
+                const int j = 32 * w + __ffs((int)bits) - 1;
+                if (s >= CL_ROWCAP) break;
+                out[s] = j;
+                nh += j > i;
+            }
+            base += __shfl_sync(0xffffffffu, x, 31);
+        }
+        n = min(n, CL_ROWCAP);
+    } else {
+        n = min(n, CL_ROWCAP);
+        for (int s = n + lane; s < CL_ROWCAP; s += 32) row[s] = 0x7fffffff;
+        __syncwarp();
+        // bitonic sort of the row (ascending j)
+        for (int k = 2; k <= CL_ROWCAP; k <<= 1)
+            for (int jj = k >> 1; jj > 0; jj >>= 1) {
+                for (int t = lane; t < CL_ROWCAP; t += 32) {
+                    const int p = t ^ jj;
+                    if (p > t) {
+                        const int a = row[t], c = row[p];
+                        const bool up = (t & k) == 0;
+                        if ((a > c) == up) {
+                            row[t] = c;
+                            row[p] = a;
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+        for (int s = lane; s < n; s += 32) {
+            out[s] = row[s];
+            nh += row[s] > i;
+        }
     }
     for (int o = 16; o > 0; o >>= 1) nh += __shfl_xor_sync(0xffffffffu, nh, o);
     if (lane == 0) {
@@ -425,10 +466,10 @@ void launch_neighbors(Engine &E) {
         k_cell_bin<<<g1, 128, 0, E.stream>>>(kp);
         k_cell_scan<<<kp.P, 1024, 0, E.stream>>>(kp);
         k_cell_fill<<<g1, 128, 0, E.stream>>>(kp);
-        if (full)
-            k_cell_rows<true><<<gw, 128, 0, E.stream>>>(kp);
-        else
-            k_cell_rows<false><<<gw, 128, 0, E.stream>>>(kp);
+        const bool bits = kp.N <= CL_BITN;
+        const size_t smem = 4 * sizeof(int) * (bits ? ((size_t)(kp.N + 31) / 32 + 31) / 32 * 32 : (size_t)CL_ROWCAP);
+        (full ? (bits ? k_cell_rows<true, true> : k_cell_rows<true, false>)
+              : (bits ? k_cell_rows<false, true> : k_cell_rows<false, false>))<<<gw, 128, smem, E.stream>>>(kp);
         k_scan_counts<<<kp.P, 1024, 0, E.stream>>>(kp.nbrtmp, kp.npair, kp.N, kp.cap, kp.err);
         if (full) k_scan_counts<<<kp.P, 1024, 0, E.stream>>>(kp.foff, kp.fntot, kp.N, kp.fcap, kp.err);
         if (full)
