@@ -107,6 +107,7 @@ struct TcArgs {
     int xsub, xblock;     // 16-site blocks per bead and run group, bytes per block
     int xkeep;            // load the cached X blocks with the L2 evict-last policy
     int pdl;              // launched as a programmatic dependent of the previous iteration's field pass
+    int npt;              // dipole-component partials held at a time: 3, or 1
 };
 
 // Shared-memory carve-up (bytes from a 1024-aligned base), used by the kernel and the launcher.
@@ -330,9 +331,9 @@ __global__ void __maxnreg__(64) k_sfac_tc(const __grid_constant__ CUtensorMap tm
             it_ys[u] = ky < 0 ? -1.f : 1.f;
         }
         // Z items: one row (c, j, cos|sin) x 8 sites each, on the whole warps after the X items
-        // (else on the last warp), at most TC_ZMAX per thread; row decoded once here
+        // (or as many of the last as TC_ZMAX items per thread need); row decoded once here
         const int nzi = 2 * NCZ * jm * 2;
-        const int zwarps = xm == 2 ? TC_NB : max(1, TC_NB - (2 * nr + 31) / 32);
+        const int zwarps = xm == 2 ? TC_NB : max((nzi + 32 * TC_ZMAX - 1) / (32 * TC_ZMAX), TC_NB - (2 * nr + 31) / 32);
         const int zthreads = 32 * zwarps, zbase = 32 * TC_NB - zthreads;
         int zn = 0, zoff[TC_ZMAX], zmo[TC_ZMAX], zer[TC_ZMAX], zcs[TC_ZMAX], zq[TC_ZMAX];
 #pragma unroll
@@ -510,115 +511,121 @@ __global__ void __maxnreg__(64) k_sfac_tc(const __grid_constant__ CUtensorMap tm
     }
     // epilogue: TMEM -> shared, 64 runs (128 columns) at a time -> partial S of every k of the group
     float *stg = reinterpret_cast<float *>(sm);                       // [128][TC_LD]
-    float2 *pt = reinterpret_cast<float2 *>(sm + 128 * TC_LD * 4);    // [nkl]
-    for (int ch = 0; ch * TC_CH < nr && !bad; ch++) {
-        if (warp < 16) {
-            const int lq = warp & 3, part = warp >> 2;  // 4 lane quarters x 4 column quarters
-            const int c0 = ch * 2 * TC_CH + 32 * part;
-            float v[8];
-            float *row = stg + (32 * lq + lane) * TC_LD + 32 * part;
-#pragma unroll
-            for (int hh = 0; hh < 4; hh++) {
-                if (nsub > 0) {
-                    umma::tmem_ld8(tm + ((uint32_t)(32 * lq) << 16) + (uint32_t)(c0 + 8 * hh), v);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 8; j++) v[j] = 0.f;
-                }
-                *reinterpret_cast<float4 *>(row + 8 * hh) = make_float4(v[0], v[1], v[2], v[3]);
-                *reinterpret_cast<float4 *>(row + 8 * hh + 4) = make_float4(v[4], v[5], v[6], v[7]);
-            }
-        }
-        __syncthreads();
-        for (int i = tid; i < TC_CH * jm; i += TC_NT) {
-            const int q = i % TC_CH, jj = i / TC_CH, p = ch * TC_CH + q, j = G.j0 + jj;  // row jj: |kz| = j
-            if (p >= nr) continue;
-            const int4 sl = sslot[p];  // run, local offset, kzlo, nkz
-            const bool plus = j >= sl.z && j < sl.z + sl.w;
-            const bool minus = j > 0 && -j >= sl.z && -j < sl.z + sl.w;
-            if (!plus && !minus) continue;
-            float2 gp[NCZ], gm[NCZ];
-#pragma unroll
-            for (int c = 0; c < NCZ; c++) {
-                const int rc = (c * jm + jj) * 2;
-                // (x, y) = (Re exy, Im exy) against mu_c c_j (row rc) and mu_c s_j (row rc + 1)
-                const float2 dc = *reinterpret_cast<const float2 *>(stg + rc * TC_LD + 2 * q);
-                const float2 ds = *reinterpret_cast<const float2 *>(stg + (rc + 1) * TC_LD + 2 * q);
-                gp[c] = make_float2(dc.x - ds.y, ds.x + dc.y);
-                gm[c] = make_float2(dc.x + ds.y, dc.y - ds.x);
-            }
-            const float zs = 1.f / TC_ZS;
-            if (OP == TC_OP_MU) {
-                const float2 kv = make_float2(sskv[p].x * zs, sskv[p].y * zs);
-                if (plus) {
-                    const float kz = skz[kp.lmax + j] * zs;
-                    pt[sl.y + j - sl.z] = make_float2(fmaf(kz, gp[NCZ - 1].x, fmaf(kv.y, gp[1 % NCZ].x, kv.x * gp[0].x)),
-                                                      fmaf(kz, gp[NCZ - 1].y, fmaf(kv.y, gp[1 % NCZ].y, kv.x * gp[0].y)));
-                }
-                if (minus) {
-                    const float kz = skz[kp.lmax - j] * zs;
-                    pt[sl.y - j - sl.z] = make_float2(fmaf(kz, gm[NCZ - 1].x, fmaf(kv.y, gm[1 % NCZ].x, kv.x * gm[0].x)),
-                                                      fmaf(kz, gm[NCZ - 1].y, fmaf(kv.y, gm[1 % NCZ].y, kv.x * gm[0].y)));
-                }
-            } else {
-                // charges: S itself; dipole components: the three G_c
-#pragma unroll
-                for (int c = 0; c < NPT; c++) {
-                    if (plus) pt[NPT * (sl.y + j - sl.z) + c] = make_float2(zs * gp[c].x, zs * gp[c].y);
-                    if (minus) pt[NPT * (sl.y - j - sl.z) + c] = make_float2(zs * gm[c].x, zs * gm[c].y);
-                }
-            }
-        }
-        __syncthreads();
-    }
-    umma::fence_before_sync();
-    __syncthreads();
-    if (warp == 0) {
-        umma::fence_after_sync();
-        umma::tmem_dealloc(tm, 512);
-        umma::tmem_relinquish();
-    }
-    // cluster: add the partials of all site groups over this CTA's slice of the k-vectors
-    // (groups in order), then Sm = (-Im, Re) and the FP32 weights 4 pi Ak / V conj(S)
-    cluster_sync();
-    if (!bad) {
-        const uint32_t pbase = umma::smem_u32(pt);
-        auto reduce_one = [&](int i, const TcKW &kw) {
-            if (kw.k < 0) return;  // a k-vector of the run that another (band) group sums
-#pragma unroll
-            for (int e = 0; e < NPT; e++) {
-                float2 v[TC_CLMAX];
-#pragma unroll
-                for (int c = 0; c < TC_CLMAX; c++)
-                    if (c < cn) v[c] = ld_cluster_f2(pbase + 8u * (uint32_t)(NPT * i + e), (uint32_t)c);
-                // FP32 in a fixed order: FP64 arithmetic is slow on this part, and the partials
-                // carry only the split operands' ~2^-21 anyway
-                float sx = 0.f, sy = 0.f;
-#pragma unroll
-                for (int c = 0; c < TC_CLMAX; c++)
-                    if (c < cn) {
-                        sx += v[c].x;
-                        sy += v[c].y;
+    float2 *pt = reinterpret_cast<float2 *>(sm + 128 * TC_LD * 4);    // [nkl][npt]
+    // (dipole components: one at a time where the three partials of a group's k-vectors do not fit)
+    const int npt = (OP == TC_OP_DIP) ? a.npt : 1;
+    for (int c0 = 0; c0 < NPT; c0 += npt) {
+        for (int ch = 0; ch * TC_CH < nr && !bad; ch++) {
+            if (warp < 16) {
+                const int lq = warp & 3, part = warp >> 2;  // 4 lane quarters x 4 column quarters
+                const int col = ch * 2 * TC_CH + 32 * part;
+                float v[8];
+                float *row = stg + (32 * lq + lane) * TC_LD + 32 * part;
+    #pragma unroll
+                for (int hh = 0; hh < 4; hh++) {
+                    if (nsub > 0) {
+                        umma::tmem_ld8(tm + ((uint32_t)(32 * lq) << 16) + (uint32_t)(col + 8 * hh), v);
+                    } else {
+    #pragma unroll
+                        for (int j = 0; j < 8; j++) v[j] = 0.f;
                     }
-                if (OP == TC_OP_MU) {  // (-Im, Re) as the reference's rQm, iQm (ewald.f90:106-107)
-                    kp.Sm[(size_t)b * kp.nk + kw.k] = make_double2(-(double)sy, (double)sx);
-                    kp.Wf[((size_t)b * 2 + 1) * kp.nk + kw.k] = make_float2(-kw.w * sy, -kw.w * sx);
-                } else if (OP == TC_OP_Q) {
-                    kp.Sq[(size_t)b * kp.nk + kw.k] = make_double2((double)sx, (double)sy);
-                    kp.Wf[((size_t)b * 2) * kp.nk + kw.k] = make_float2(kw.w * sx, -kw.w * sy);
-                } else {
-                    kp.Sdip[((size_t)b * kp.nk + kw.k) * 3 + e] = make_double2((double)sx, (double)sy);
+                    *reinterpret_cast<float4 *>(row + 8 * hh) = make_float4(v[0], v[1], v[2], v[3]);
+                    *reinterpret_cast<float4 *>(row + 8 * hh + 4) = make_float4(v[4], v[5], v[6], v[7]);
                 }
             }
-        };
-#pragma unroll
-        for (int u = 0; u < TC_PF; u++) {
-            const int i = i0 + tid + u * TC_NT;
-            if (i < i1) reduce_one(i, pf[u]);
+            __syncthreads();
+            for (int i = tid; i < TC_CH * jm; i += TC_NT) {
+                const int q = i % TC_CH, jj = i / TC_CH, p = ch * TC_CH + q, j = G.j0 + jj;  // row jj: |kz| = j
+                if (p >= nr) continue;
+                const int4 sl = sslot[p];  // run, local offset, kzlo, nkz
+                const bool plus = j >= sl.z && j < sl.z + sl.w;
+                const bool minus = j > 0 && -j >= sl.z && -j < sl.z + sl.w;
+                if (!plus && !minus) continue;
+                float2 gp[NCZ], gm[NCZ];
+    #pragma unroll
+                for (int c = 0; c < NCZ; c++) {
+                    const int rc = (c * jm + jj) * 2;
+                    // (x, y) = (Re exy, Im exy) against mu_c c_j (row rc) and mu_c s_j (row rc + 1)
+                    const float2 dc = *reinterpret_cast<const float2 *>(stg + rc * TC_LD + 2 * q);
+                    const float2 ds = *reinterpret_cast<const float2 *>(stg + (rc + 1) * TC_LD + 2 * q);
+                    gp[c] = make_float2(dc.x - ds.y, ds.x + dc.y);
+                    gm[c] = make_float2(dc.x + ds.y, dc.y - ds.x);
+                }
+                const float zs = 1.f / TC_ZS;
+                if (OP == TC_OP_MU) {
+                    const float2 kv = make_float2(sskv[p].x * zs, sskv[p].y * zs);
+                    if (plus) {
+                        const float kz = skz[kp.lmax + j] * zs;
+                        pt[sl.y + j - sl.z] = make_float2(fmaf(kz, gp[NCZ - 1].x, fmaf(kv.y, gp[1 % NCZ].x, kv.x * gp[0].x)),
+                                                          fmaf(kz, gp[NCZ - 1].y, fmaf(kv.y, gp[1 % NCZ].y, kv.x * gp[0].y)));
+                    }
+                    if (minus) {
+                        const float kz = skz[kp.lmax - j] * zs;
+                        pt[sl.y - j - sl.z] = make_float2(fmaf(kz, gm[NCZ - 1].x, fmaf(kv.y, gm[1 % NCZ].x, kv.x * gm[0].x)),
+                                                          fmaf(kz, gm[NCZ - 1].y, fmaf(kv.y, gm[1 % NCZ].y, kv.x * gm[0].y)));
+                    }
+                } else {
+                    // charges: S itself; dipole components: the three G_c
+    #pragma unroll
+                    for (int c = 0; c < NPT; c++) {
+                        if (c < c0 || c >= c0 + npt) continue;
+                        if (plus) pt[npt * (sl.y + j - sl.z) + c - c0] = make_float2(zs * gp[c].x, zs * gp[c].y);
+                        if (minus) pt[npt * (sl.y - j - sl.z) + c - c0] = make_float2(zs * gm[c].x, zs * gm[c].y);
+                    }
+                }
+            }
+            __syncthreads();
         }
-        for (int i = i0 + tid + TC_PF * TC_NT; i < i1; i += TC_NT) reduce_one(i, a.kw[G.kgoff + i]);
+        umma::fence_before_sync();
+        __syncthreads();
+        if (warp == 0 && c0 + npt >= NPT) {
+            umma::fence_after_sync();
+            umma::tmem_dealloc(tm, 512);
+            umma::tmem_relinquish();
+        }
+        // cluster: add the partials of all site groups over this CTA's slice of the k-vectors
+        // (groups in order), then Sm = (-Im, Re) and the FP32 weights 4 pi Ak / V conj(S)
+        cluster_sync();
+        if (!bad) {
+            const uint32_t pbase = umma::smem_u32(pt);
+            auto reduce_one = [&](int i, const TcKW &kw) {
+                if (kw.k < 0) return;  // a k-vector of the run that another (band) group sums
+    #pragma unroll
+                for (int e = 0; e < NPT; e++) {
+                    if (e >= npt) break;
+                    float2 v[TC_CLMAX];
+    #pragma unroll
+                    for (int c = 0; c < TC_CLMAX; c++)
+                        if (c < cn) v[c] = ld_cluster_f2(pbase + 8u * (uint32_t)(npt * i + e), (uint32_t)c);
+                    // FP32 in a fixed order: FP64 arithmetic is slow on this part, and the partials
+                    // carry only the split operands' ~2^-21 anyway
+                    float sx = 0.f, sy = 0.f;
+    #pragma unroll
+                    for (int c = 0; c < TC_CLMAX; c++)
+                        if (c < cn) {
+                            sx += v[c].x;
+                            sy += v[c].y;
+                        }
+                    if (OP == TC_OP_MU) {  // (-Im, Re) as the reference's rQm, iQm (ewald.f90:106-107)
+                        kp.Sm[(size_t)b * kp.nk + kw.k] = make_double2(-(double)sy, (double)sx);
+                        kp.Wf[((size_t)b * 2 + 1) * kp.nk + kw.k] = make_float2(-kw.w * sy, -kw.w * sx);
+                    } else if (OP == TC_OP_Q) {
+                        kp.Sq[(size_t)b * kp.nk + kw.k] = make_double2((double)sx, (double)sy);
+                        kp.Wf[((size_t)b * 2) * kp.nk + kw.k] = make_float2(kw.w * sx, -kw.w * sy);
+                    } else {
+                        kp.Sdip[((size_t)b * kp.nk + kw.k) * 3 + c0 + e] = make_double2((double)sx, (double)sy);
+                    }
+                }
+            };
+    #pragma unroll
+            for (int u = 0; u < TC_PF; u++) {
+                const int i = i0 + tid + u * TC_NT;
+                if (i < i1) reduce_one(i, pf[u]);
+            }
+            for (int i = i0 + tid + TC_PF * TC_NT; i < i1; i += TC_NT) reduce_one(i, a.kw[G.kgoff + i]);
+        }
+        cluster_sync();  // remote reads done before any CTA of the cluster leaves (or writes the next component)
     }
-    cluster_sync();  // remote reads done before any CTA of the cluster leaves
     if (bad && tid == 0) atomicOr(kp.err, 8u);
 }
 
@@ -1250,17 +1257,13 @@ void tc_init(Engine &E) {
     for (int r = 0; r < kp.nrun; r++)
         runkf[r] = make_float2((float)E.h_kvec[3 * E.h_runs[r].kbeg], (float)E.h_kvec[3 * E.h_runs[r].kbeg + 1]);
     int ncolmax = 16, nklmax = 0, nvalid = 0;
-    // while a group's X is built, its 2 nr X items take whole builder warps first and the Z items
-    // (12 jm at most) the warps left over, TC_ZMAX per thread: the most runs a group of jm rows holds
-    auto zfit = [](int nr, int jm) {
-        const int zw = std::max(1, TC_NB - (2 * nr + 31) / 32);
-        return (12 * jm + 32 * zw - 1) / (32 * zw) <= TC_ZMAX;
-    };
+    // groups of one band hold equally many runs: the bead's CTAs of all groups run side by side, and a last
+    // group of one run (897 runs in groups of 224) would take a CTA's time for it
     for (int p0 = 0; p0 < nslot;) {
         const int j0 = src[p0].y, jmg = std::min(TC_JB, jr[src[p0].x] - j0);
-        int nr = 0;
-        while (p0 + nr < nslot && nr < TC_MAXRUN && src[p0 + nr].y == j0 && zfit(nr + 1, jmg)) nr++;
-        if (nr == 0) return;
+        int left = 0;
+        while (p0 + left < nslot && src[p0 + left].y == j0) left++;
+        const int ng = (left + TC_MAXRUN - 1) / TC_MAXRUN, nr = (left + ng - 1) / ng;
         TcGroup g{p0, nr, 0, jmg, 0, (int)kloc.size(), j0, 0};
         g.ncol = ((2 * g.nr + 15) / 16) * 16;
         for (int p = p0; p < p0 + g.nr; p++) {
@@ -1306,8 +1309,8 @@ void tc_init(Engine &E) {
         cudaGetLastError();
         return;
     }
-    // the component sums keep three partials per k-vector
-    E.tc_dip_ok = 128 * TC_LD * 4 + 3 * 8 * nklmax <= L.total - 1024;
+    // the component sums keep three partials per k-vector, or one at a time
+    E.tc_npt = 128 * TC_LD * 4 + 3 * 8 * nklmax <= L.total - 1024 ? 3 : 1;
     int4 *d_slots = nullptr;
     float2 *d_skv = nullptr;
     TcGroup *d_groups = nullptr;
@@ -1368,6 +1371,24 @@ void tc_init(Engine &E) {
     E.tc_ntg = (int)groups.size();
     E.tc_ncolmax = ncolmax;
     E.tc_nabuf = nabuf;
+    // clusters of n CTAs the device holds at once
+    int nsm = 0;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, E.device);
+    for (int n = 1; n <= TC_CLMAX; n++) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(n, E.tc_ntg, kp.P);
+        cfg.blockDim = dim3(TC_NT);
+        cfg.dynamicSmemBytes = L.total;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = n;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int c = 0;
+        if (cudaOccupancyMaxActiveClusters(&c, k_sfac_tc<TC_OP_MU>, &cfg) != cudaSuccess) cudaGetLastError();
+        E.tc_ncl[n] = c > 0 ? c : std::max(1, nsm / n);
+    }
     E.tc_ready = true;
     E.tf_ready = false;
     tp_setup(E, enc, jr, optin);
@@ -1479,7 +1500,7 @@ int launch_field_qd_tc(Engine &E, int s0, int s1) {
 // Returns 1 when the launch wrote the structure factor of `op` (Sq and the charge weights, Sm
 // and the dipole weights, or Sdip; no k_sreduce needed), else 0.
 int launch_sfac_tc(Engine &E, int op, int s0, int nsites, int skipconv) {
-    if (!E.tc_ready || !E.sf_tc || nsites <= 0 || (op == TC_OP_DIP && !E.tc_dip_ok)) return 0;
+    if (!E.tc_ready || !E.sf_tc || nsites <= 0) return 0;
     const KP &kp = E.kp;
     TcArgs a;
     a.slot = E.d_tcslot;
@@ -1499,23 +1520,23 @@ int launch_sfac_tc(Engine &E, int op, int s0, int nsites, int skipconv) {
     a.xsub = E.tc_xsub;
     a.xblock = E.tc_xblock;
     a.xkeep = E.l2_keep ? 1 : 0;
+    a.npt = E.tc_npt;
     // the iterations' structure factor follows the previous iteration's field pass on the stream
     // (or the charge passes, which need no overlap): its CTAs are scheduled as that grid drains
     a.pdl = (op == TC_OP_MU && skipconv && E.tc_pdl && E.tf_ready && E.ff_tc) ? 1 : 0;
-    // one CTA per SM (shared memory); site groups (= cluster size) so that one wave fills the GPU
-    static int nsm_cache[64] = {0};
-    int &nsm = nsm_cache[E.device & 63];
-    if (!nsm) {
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, E.device);
-        if (nsm <= 0) nsm = 152;
-    }
+    // one CTA per SM (shared memory). Site groups (= cluster size) with the fewest waves x stages a CTA; a
+    // CTA's set-up and epilogue take about as long as 6 stages (512 x 32: 4 stages a CTA in 19 us, 4096 x 32:
+    // 128 in 225 us). One group whenever a wave was full took two waves of 152 and 40 CTAs at 4096 x 32
     const int nst = (a.s_hi - a.sbase + TC_SS - 1) / TC_SS;
     const long per = (long)E.tc_ntg * kp.P;
-    int ng = (int)std::max(1L, (long)nsm / per);
-    ng = std::max(1, std::min(ng, std::min(nst, TC_CLMAX)));
-    const int spg = (nst + ng - 1) / ng;
+    int ng = 1, spg = nst;
+    long best = -1;
+    for (int n = 1; n <= std::min(nst, TC_CLMAX); n++) {
+        const int sp = (nst + n - 1) / n, used = (nst + sp - 1) / sp;
+        const long cost = (per + E.tc_ncl[used] - 1) / E.tc_ncl[used] * (sp + 6);
+        if (best < 0 || cost < best) best = cost, ng = used, spg = sp;
+    }
     a.tsg = spg * TC_SS;
-    ng = (nst + spg - 1) / spg;
     const TcSmem L(kp.ntab, a.ncolmax, a.nabuf);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ng, E.tc_ntg, kp.P);
