@@ -802,6 +802,7 @@ int pimd_pot_backward(pimd_ctx *ctx, const double *Ebar, double *dRRt, double *d
             // d/dx [u^T D_rec v] = -(dipole force of u in E_v + dipole force of v in E_u)
             const dim3 gk((unsigned)((kp.nk + 255) / 256), (unsigned)P);
             k_adj_wslots<0><<<gk, 256, 0, st>>>(kp, nullptr);
+            if (E.tp_vslot == 1) E.tp_vslot = 0;  // (the field passes' operand of S_u)
             KP kq = kp;
             kq.acc = bacc;
             kq.dd_async = 0;
@@ -814,6 +815,7 @@ int pimd_pot_backward(pimd_ctx *ctx, const double *Ebar, double *dRRt, double *d
             E.kp.dipf = vf;
             launch_adj_dforce_tc(E);
             k_adj_wslots<1><<<gk, 256, 0, st>>>(kp, Smv);
+            E.tp_vslot = -1;
             E.kp.dipf = uf;
             launch_adj_dforce_tc(E);
             E.kp = keep;
@@ -845,6 +847,7 @@ int pimd_pot_backward(pimd_ctx *ctx, const double *Ebar, double *dRRt, double *d
         launch_adj_qforce_tc(E);
         const dim3 gk((unsigned)((kp.nk + 255) / 256), (unsigned)P);
         k_adj_wslots<2><<<gk, 256, 0, st>>>(kp, kp.Sq);
+        E.tp_vslot = -1;
         cudaMemsetAsync(kp.dR, 0, sizeof(double) * sv, st);
         E.kp.fx_mode = 0;
         E.kp.dipf = uf;

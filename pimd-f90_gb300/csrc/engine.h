@@ -302,6 +302,8 @@ struct Engine {
         void *V;
         int vstride, nchunk, rp, kcm;
     } tp[2] = {};
+    int tp_vslot = -1;                // weight slot whose operand tp[0].V holds (-1: none)
+    const int4 *d_tcvp = nullptr;     // run pairs of the structure factor's groups
     alignas(64) unsigned char tp_mapxy[128], tp_mapz[128];  // CUtensorMaps of tabf's ex and ey rows, and ez rows
     alignas(64) unsigned char tc_map[128];  // CUtensorMap of the FP32 tables tabf
     DgArgs dg;                 // FP64 engine: digit operands of the reciprocal sums

@@ -890,6 +890,7 @@ static void run_spass_t(Engine &E, int s0, int nsites, int skipconv) {
     ++E.nlaunch;
     dim3 g2((E.kp.nk + 255) / 256, E.kp.P);
     k_sreduce<OP, R><<<g2, 256, 0, E.stream>>>(E.kp, ngr, skipconv);
+    if (OP != OP_DIP) E.tp_vslot = -1;
     ++E.nlaunch;
 }
 
@@ -919,6 +920,7 @@ static void run_sfac_f(Engine &E, int s0, int nsites, int skipconv) {
     ++E.nlaunch;
     dim3 g2((kp.nk + 255) / 256, kp.P);
     k_sreduce<OP, float><<<g2, 256, 0, E.stream>>>(E.kp, ngr, skipconv);
+    if (OP != OP_DIP) E.tp_vslot = -1;
     ++E.nlaunch;
 }
 

@@ -35,7 +35,7 @@
 // TMEM (tcgen05.ld) 64 runs at a time, combines each k-vector's 12 sums, and keeps the CTA's FP32
 // partial S in shared memory; after a cluster barrier each CTA adds the partials of all CTAs of
 // its cluster over a slice of the k-vectors (distributed shared memory, FP32, site groups in a
-// fixed order) and writes Sm and the FP32 weights Wf.
+// fixed order) and writes Sm, the FP32 weights Wf and the field pass's operand V.
 // Every mbarrier wait is bounded (~0.13 s); after a timeout a role stops, the CTA waits (bounded)
 // for its copies and MMAs in flight, frees its TMEM, still meets its cluster barriers, and bit 8
 // of the context's error word is set.
@@ -45,6 +45,7 @@
 #include <cmath>
 #include <cstring>
 #include <map>
+#include <tuple>
 #include <utility>
 #include <vector>
 
@@ -69,6 +70,7 @@ constexpr int TC_CLMAX = 8;               // site groups per cluster (portable c
 constexpr int TC_MAXRUN = 256;            // runs per group: 512 TMEM columns
 constexpr int TC_CH = 64;                 // runs per epilogue chunk
 constexpr int TC_LD = 2 * TC_CH + 4;      // staging row pitch (floats)
+constexpr float TP_WS = 512.f;            // power-of-two scale of the field passes' V (a row adds up to four weights)
 constexpr long long TC_WAIT = 1LL << 28;  // cycles before a wait gives up (~0.13 s)
 
 // structure-factor sums (values as in ewald.cu): charge q e, dipole (k.mu) e, dipole components mu_c e
@@ -80,9 +82,10 @@ enum { TF_Q = 0, TF_D = 1, TF_QG = 2, TF_DG = 3 };
 
 // A run group: slots [p0, p0 + nr), MMA columns, the |kz| rows j0 .. j0 + jm - 1 of its Z
 // operand (6 jm <= 128: |kz| above 20 goes to band groups, j0 = 21, of the same runs), k-vectors
-// (local indices; those of a run outside the group's |kz| rows are entries with k = -1)
+// (local indices; those of a run outside the group's |kz| rows are entries with k = -1), and np pairs of runs
+// (kx, +-ky) from vp0 of the pair table
 struct TcGroup {
-    int p0, nr, ncol, jm, nkl, kgoff, j0, pad1;
+    int p0, nr, ncol, jm, nkl, kgoff, j0, np, vp0;
 };
 
 // k-vector of a local index and its 4 pi Ak / V
@@ -108,6 +111,10 @@ struct TcArgs {
     int xkeep;            // load the cached X blocks with the L2 evict-last policy
     int pdl;              // launched as a programmatic dependent of the previous iteration's field pass
     int npt;              // dipole-component partials held at a time: 3, or 1
+    const int4 *vp;       // per pair: group slots of its +ky | -ky << 16 runs (0xffff: none), where its rows of
+                          // the field pass's V begin and how far the lo rows are from there (16-byte words), |kz| rows
+    uint4 *V;             // [P][vstride] that operand (null: none)
+    int vstride;
 };
 
 // Shared-memory carve-up (bytes from a 1024-aligned base), used by the kernel and the launcher.
@@ -211,6 +218,33 @@ PIMD_D void split8_h(const float (&x)[8], uint4 &hi, uint4 &lo) {
 // byte offset of the 16-byte chunk c (sites 8 c .. 8 c + 7) of row n in a K-major operand of 16
 // FP16 sites (two core matrices along K)
 PIMD_D int rowchunk(int n, int c) { return (((n >> 3) * 2 + c) << 7) + ((n & 7) << 4); }
+
+// The rows of the field passes' V of a run pair at one |kz|: w the weights of (+ky, +kz), (+ky, -kz), (-ky, +kz),
+// (-ky, -kz); out(row, cos part, sin part) for T0's Ts re, im, Td re, im, the same of T1, and with T2 of T2.
+template <bool T2 = false, typename F>
+PIMD_D void v_rows(const float2 (&w)[4], float kz, F &&out) {
+    float2 p[2], m[2];  // W(+kz) + W(-kz) and W(+kz) - W(-kz), by the sign of ky
+#pragma unroll
+    for (int y = 0; y < 2; y++) {
+        const float2 a = make_float2(TP_WS * w[2 * y].x, TP_WS * w[2 * y].y), c = make_float2(TP_WS * w[2 * y + 1].x, TP_WS * w[2 * y + 1].y);
+        p[y] = make_float2(a.x + c.x, a.y + c.y);
+        m[y] = make_float2(a.x - c.x, a.y - c.y);
+    }
+#pragma unroll
+    for (int d = 0; d < 2; d++) {
+        const float2 wp = d ? make_float2(p[0].x - p[1].x, p[0].y - p[1].y) : make_float2(p[0].x + p[1].x, p[0].y + p[1].y);
+        const float2 wm = d ? make_float2(m[0].x - m[1].x, m[0].y - m[1].y) : make_float2(m[0].x + m[1].x, m[0].y + m[1].y);
+        out(2 * d, wp.x, -wm.y);
+        out(2 * d + 1, wp.y, wm.x);
+        out(4 + 2 * d, kz * wm.x, -kz * wp.y);
+        out(5 + 2 * d, kz * wm.y, kz * wp.x);
+        if (T2) {
+            const float k2 = kz * kz;
+            out(8 + 2 * d, k2 * wp.x, -k2 * wm.y);
+            out(9 + 2 * d, k2 * wp.y, k2 * wm.x);
+        }
+    }
+}
 
 // 64 registers a thread (a few bytes spill): one CTA of 576 threads then leaves 28 K registers
 // of the SM to the real-space dipole field running beside it on the second stream (4 blocks
@@ -499,16 +533,32 @@ __global__ void __maxnreg__(64) k_sfac_tc(const __grid_constant__ CUtensorMap tm
     umma::fence_after_sync();
     const bool bad = __syncthreads_or((int)err) != 0;
 
-    // this CTA's slice of the cluster reduction; its (k, w) pairs are fetched now, under the epilogue
+    // this CTA's slice of the cluster reduction: k-vectors of the dipole components, else items (run pair, |kz|);
+    // the thread's first item is fetched now, under the epilogue
     const int cr = (int)cluster_rank(), cn = gridDim.x;
-    const int i0 = (int)((long)cr * G.nkl / cn), i1 = (int)((long)(cr + 1) * G.nkl / cn);
-    constexpr int TC_PF = 4;
-    TcKW pf[TC_PF];
+    const int ni = (OP == TC_OP_DIP) ? G.nkl : G.np * jm;
+    const int i0 = (int)((long)cr * ni / cn), i1 = (int)((long)(cr + 1) * ni / cn);
+    struct Item {
+        int4 vp;
+        TcKW kw[4];  // (+ky, +kz), (+ky, -kz), (-ky, +kz), (-ky, -kz); k < 0: none
+    };
+    auto local_k = [&](const int4 &vp, int j, int u) {  // the k-vector's local index, -1: none
+        const int p = (u & 2) ? (vp.x >> 16) & 0xffff : vp.x & 0xffff, kz = (u & 1) ? -j : j;
+        if (p == 0xffff || ((u & 1) && j == 0)) return -1;
+        const int4 sl = sslot[p];
+        return kz >= sl.z && kz < sl.z + sl.w ? sl.y + kz - sl.z : -1;
+    };
+    auto fetch = [&](int it, Item &x) {
+        const int q = it / jm, j = G.j0 + it - q * jm;
+        x.vp = a.vp[G.vp0 + q];
 #pragma unroll
-    for (int u = 0; u < TC_PF; u++) {
-        const int i = i0 + tid + u * TC_NT;
-        pf[u] = i < i1 ? a.kw[G.kgoff + i] : TcKW{0, 0.f};
-    }
+        for (int u = 0; u < 4; u++) {
+            const int i = local_k(x.vp, j, u);
+            x.kw[u] = i >= 0 ? a.kw[G.kgoff + i] : TcKW{-1, 0.f};
+        }
+    };
+    Item first;
+    if (OP != TC_OP_DIP && i0 + tid < i1) fetch(i0 + tid, first);
     // epilogue: TMEM -> shared, 64 runs (128 columns) at a time -> partial S of every k of the group
     float *stg = reinterpret_cast<float *>(sm);                       // [128][TC_LD]
     float2 *pt = reinterpret_cast<float2 *>(sm + 128 * TC_LD * 4);    // [nkl][npt]
@@ -583,46 +633,67 @@ __global__ void __maxnreg__(64) k_sfac_tc(const __grid_constant__ CUtensorMap tm
             umma::tmem_dealloc(tm, 512);
             umma::tmem_relinquish();
         }
-        // cluster: add the partials of all site groups over this CTA's slice of the k-vectors
-        // (groups in order), then Sm = (-Im, Re) and the FP32 weights 4 pi Ak / V conj(S)
+            // cluster: add the partials of all site groups over this CTA's slice (groups in order, in FP32: FP64
+        // arithmetic is slow on this part, and the partials carry only the split operands' ~2^-21 anyway)
         cluster_sync();
-        if (!bad) {
-            const uint32_t pbase = umma::smem_u32(pt);
-            auto reduce_one = [&](int i, const TcKW &kw) {
-                if (kw.k < 0) return;  // a k-vector of the run that another (band) group sums
-    #pragma unroll
-                for (int e = 0; e < NPT; e++) {
-                    if (e >= npt) break;
-                    float2 v[TC_CLMAX];
-    #pragma unroll
-                    for (int c = 0; c < TC_CLMAX; c++)
-                        if (c < cn) v[c] = ld_cluster_f2(pbase + 8u * (uint32_t)(npt * i + e), (uint32_t)c);
-                    // FP32 in a fixed order: FP64 arithmetic is slow on this part, and the partials
-                    // carry only the split operands' ~2^-21 anyway
-                    float sx = 0.f, sy = 0.f;
-    #pragma unroll
-                    for (int c = 0; c < TC_CLMAX; c++)
-                        if (c < cn) {
-                            sx += v[c].x;
-                            sy += v[c].y;
-                        }
-                    if (OP == TC_OP_MU) {  // (-Im, Re) as the reference's rQm, iQm (ewald.f90:106-107)
-                        kp.Sm[(size_t)b * kp.nk + kw.k] = make_double2(-(double)sy, (double)sx);
-                        kp.Wf[((size_t)b * 2 + 1) * kp.nk + kw.k] = make_float2(-kw.w * sy, -kw.w * sx);
-                    } else if (OP == TC_OP_Q) {
-                        kp.Sq[(size_t)b * kp.nk + kw.k] = make_double2((double)sx, (double)sy);
-                        kp.Wf[((size_t)b * 2) * kp.nk + kw.k] = make_float2(kw.w * sx, -kw.w * sy);
-                    } else {
-                        kp.Sdip[((size_t)b * kp.nk + kw.k) * 3 + c0 + e] = make_double2((double)sx, (double)sy);
-                    }
+        const uint32_t pbase = umma::smem_u32(pt);
+        auto total = [&](int i) {
+            float2 v[TC_CLMAX];
+#pragma unroll
+            for (int c = 0; c < TC_CLMAX; c++)
+                if (c < cn) v[c] = ld_cluster_f2(pbase + 8u * (uint32_t)i, (uint32_t)c);
+            float sx = 0.f, sy = 0.f;
+#pragma unroll
+            for (int c = 0; c < TC_CLMAX; c++)
+                if (c < cn) {
+                    sx += v[c].x;
+                    sy += v[c].y;
                 }
-            };
-    #pragma unroll
-            for (int u = 0; u < TC_PF; u++) {
-                const int i = i0 + tid + u * TC_NT;
-                if (i < i1) reduce_one(i, pf[u]);
+            return make_float2(sx, sy);
+        };
+        if (OP == TC_OP_DIP && !bad) {
+            for (int i = i0 + tid; i < i1; i += TC_NT) {
+                const TcKW kw = a.kw[G.kgoff + i];
+                if (kw.k < 0) continue;  // a k-vector of the run that another (band) group sums
+                for (int e = 0; e < npt; e++) {
+                    const float2 t = total(npt * i + e);
+                    kp.Sdip[((size_t)b * kp.nk + kw.k) * 3 + c0 + e] = make_double2((double)t.x, (double)t.y);
+                }
             }
-            for (int i = i0 + tid + TC_PF * TC_NT; i < i1; i += TC_NT) reduce_one(i, a.kw[G.kgoff + i]);
+        }
+        // charges and dipoles: Sq = S or Sm = (-Im, Re), the reference's rQm, iQm (ewald.f90:106-107), the FP32
+        // weights 4 pi Ak / V conj(S), and a pair's rows of the field pass's V (k_field_v's job, which took a
+        // launch of 5 us an iteration at 512 x 32)
+        for (int it = i0 + tid; OP != TC_OP_DIP && it < i1 && !bad; it += TC_NT) {
+            Item x = first;
+            if (it != i0 + tid) fetch(it, x);
+            const int j = G.j0 + it % jm;
+            float2 w[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                w[u] = make_float2(0.f, 0.f);
+                const TcKW kw = x.kw[u];
+                if (kw.k < 0) continue;
+                const float2 t = total(local_k(x.vp, j, u));
+                if (OP == TC_OP_MU) {
+                    kp.Sm[(size_t)b * kp.nk + kw.k] = make_double2(-(double)t.y, (double)t.x);
+                    w[u] = make_float2(-kw.w * t.y, -kw.w * t.x);
+                } else {
+                    kp.Sq[(size_t)b * kp.nk + kw.k] = make_double2((double)t.x, (double)t.y);
+                    w[u] = make_float2(kw.w * t.x, -kw.w * t.y);
+                }
+                kp.Wf[((size_t)b * 2 + (OP == TC_OP_MU ? 1 : 0)) * kp.nk + kw.k] = w[u];
+            }
+            if (!a.V || j >= x.vp.w) continue;
+            uint32_t *hi = reinterpret_cast<uint32_t *>(a.V + (size_t)b * a.vstride + x.vp.y) + (j >> 2) * 32 + (j & 3);
+            uint32_t *lo = hi + 4 * x.vp.z;
+            v_rows(w, skz[kp.lmax + j], [&](int r, float c, float sn) {
+                const __half2 h = __floats2half2_rn(c, sn);
+                const float2 hf = __half22float2(h);
+                const __half2 l = __floats2half2_rn(c - hf.x, sn - hf.y);
+                hi[4 * r] = *reinterpret_cast<const uint32_t *>(&h);
+                lo[4 * r] = *reinterpret_cast<const uint32_t *>(&l);
+            });
         }
         cluster_sync();  // remote reads done before any CTA of the cluster leaves (or writes the next component)
     }
@@ -643,9 +714,9 @@ __global__ void __maxnreg__(64) k_sfac_tc(const __grid_constant__ CUtensorMap tm
 // with the sites on M (128 per CTA), runs x components on N and only 2 (max |kz| + 1) terms on K (FP16
 // hi + lo split, three MMAs per 16-term K step); each TMEM row is then contracted with exy(s, run).
 //
-// V is formed from the weights once a pass (k_field_v; every CTA of a bead did it before, each pass of
-// runs one phase after the other: V, MMAs, contraction), and
-// the runs are taken in pairs (kx, +ky), (kx, -ky). With T+, T- the pair's sums, Ts = T+ + T-, Td = T+ - T- and
+// V is formed from the weights once a pass, by the structure factor that makes them or by k_field_v (every CTA
+// of a bead formed it before, and V, MMAs and contraction followed one another: 492 us a pass at 4096 x 32
+// against 188), and the runs are taken in pairs (kx, +ky), (kx, -ky). With T+, T- the pair's sums, Ts = T+ + T-, Td = T+ - T- and
 // e(kx x +- ky y) = ex (cy +- i sy),
 //   e+ T+ + e- T- = ex U,  U = cy Ts + i sy Td;   e+ T+ - e- T- = ex V,  V = cy Td + i sy Ts,
 // so a pair's contraction is U0, V0 (T0) and U1 (T1) and three products with ex: 20 FMAs and one load
@@ -737,7 +808,6 @@ constexpr int TP_VT = 128;                // threads of a k_field_v block
 constexpr int TP_RP = 32;                 // pairs a chunk at most (8 rows each)
 constexpr int TP_RPD = 20;                // the same with 12 rows each
 constexpr int TP_RING = 8;                // pair tables in shared memory
-constexpr float TP_WS = 512.f;            // power-of-two scale of V (a row adds up to four weights)
 
 struct TpArgs {
     const int4 *pair;    // [chunk][rp] ex row offset + 65536 key, ey row offset + 65536 key, k_x, k_y (float bits)
@@ -769,41 +839,21 @@ __global__ void __launch_bounds__(TP_VT) k_field_v(KP kp, TpArgs a, int slot) {
 #pragma unroll
         for (int e = 0; e < 4; e++) {
             const int4 k = ki[e];
-            auto w = [&](int i) {
+            auto weight = [&](int i) {
                 if (i < 0) return make_float2(0.f, 0.f);
                 float2 x = W[i];
                 if (DG) {  // both weight slots
                     const float2 y = W[kp.nk + i];
                     x = make_float2(x.x + y.x, x.y + y.y);
                 }
-                return make_float2(TP_WS * x.x, TP_WS * x.y);
+                return x;
             };
-            const float2 pp = w(k.x), pm = w(k.y), mp = w(k.z), mm = w(k.w);
+            const float2 w[4] = {weight(k.x), weight(k.y), weight(k.z), weight(k.w)};
             const int j = 4 * jc + e;
-            const float kz = j <= kp.lmax ? a.kzv[kp.lmax + j] : 0.f;
-            // W(+kz) + W(-kz) and their difference for both signs of ky
-            const float2 wpp = make_float2(pp.x + pm.x, pp.y + pm.y), wmp = make_float2(pp.x - pm.x, pp.y - pm.y);
-            const float2 wpm = make_float2(mp.x + mm.x, mp.y + mm.y), wmm = make_float2(mp.x - mm.x, mp.y - mm.y);
-#pragma unroll
-            for (int d = 0; d < 2; d++) {  // Ts, Td
-                const float2 wp = d ? make_float2(wpp.x - wpm.x, wpp.y - wpm.y) : make_float2(wpp.x + wpm.x, wpp.y + wpm.y);
-                const float2 wm = d ? make_float2(wmp.x - wmm.x, wmp.y - wmm.y) : make_float2(wmp.x + wmm.x, wmp.y + wmm.y);
-                v[2 * d][2 * e] = wp.x;
-                v[2 * d][2 * e + 1] = -wm.y;
-                v[2 * d + 1][2 * e] = wp.y;
-                v[2 * d + 1][2 * e + 1] = wm.x;
-                v[4 + 2 * d][2 * e] = kz * wm.x;
-                v[4 + 2 * d][2 * e + 1] = -kz * wp.y;
-                v[5 + 2 * d][2 * e] = kz * wm.y;
-                v[5 + 2 * d][2 * e + 1] = kz * wp.x;
-                if constexpr (DG) {
-                    const float k2 = kz * kz;
-                    v[8 + 2 * d][2 * e] = k2 * wp.x;
-                    v[8 + 2 * d][2 * e + 1] = -k2 * wm.y;
-                    v[9 + 2 * d][2 * e] = k2 * wp.y;
-                    v[9 + 2 * d][2 * e + 1] = k2 * wm.x;
-                }
-            }
+            v_rows<DG>(w, j <= kp.lmax ? a.kzv[kp.lmax + j] : 0.f, [&](int r, float c, float sn) {
+                v[r][2 * e] = c;
+                v[r][2 * e + 1] = sn;
+            });
         }
 #pragma unroll
         for (int r = 0; r < NC; r++) {
@@ -1080,7 +1130,7 @@ static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 }
 
 // Pairs, chunks, k-vector indices and V of the prepared passes: which 0 the 8-row form, 1 the 12-row one.
-static bool tp_init(Engine &E, int which, const std::vector<int> &jr, int dmax) {
+static bool tp_init(Engine &E, int which, const std::vector<int> &jr, int dmax, std::vector<int4> *place) {
     KP &kp = E.kp;
     Engine::TpSet &T = E.tp[which];
     const int NC = which ? 12 : 8, rowsxy = kp.hmax + kp.kmax + 2, jmax = kp.lmax + 1;
@@ -1103,14 +1153,15 @@ static bool tp_init(Engine &E, int which, const std::vector<int> &jr, int dmax) 
         }
         Pair &p = pairs[at[key]];
         int &slot = p.r[run.ky < 0 ? 1 : 0];
-        if (run.kx < 0 || slot >= 0) return false;
+        if (run.kx < 0 || slot >= 0 || (p.jm && p.jm != jr[r])) return false;  // (the structure factor keeps a pair together)
         slot = r;
-        p.jm = std::max(p.jm, jr[r]);
+        p.jm = jr[r];
     }
     std::stable_sort(pairs.begin(), pairs.end(), [](const Pair &x, const Pair &y) { return x.jm > y.jm; });
     const int np = (int)pairs.size(), nch = (np + rp - 1) / rp;
     std::vector<int4> pr((size_t)nch * rp, make_int4(0, 0, 0, 0)), ki((size_t)nch * rp * 4 * kcm, make_int4(-1, -1, -1, -1));
     std::vector<int2> chunk(nch);
+    std::vector<int4> where(kp.nrun);
     int words = 0;
     auto bits = [](float f) {
         int i;
@@ -1120,7 +1171,6 @@ static bool tp_init(Engine &E, int which, const std::vector<int> &jr, int dmax) 
     for (int c = 0; c < nch; c++) {
         const int kc = ((2 * pairs[c * rp].jm + 15) / 16) * 2;
         chunk[c] = make_int2(kc, words);
-        words += 2 * NC * rp * kc;
         for (int q = 0; q < rp; q++) {
             // the last chunk's missing pairs: zero rows of V against the (0, 0) tables
             const int ry0 = kp.hmax + 1;
@@ -1129,6 +1179,8 @@ static bool tp_init(Engine &E, int which, const std::vector<int> &jr, int dmax) 
                 continue;
             }
             const Pair &p = pairs[c * rp + q];
+            for (int r : p.r)
+                if (r >= 0) where[r] = make_int4(words + NC * q * kc, NC * rp * kc, p.jm, 0);
             const int ry = ry0 + p.ky, r0 = p.r[0] >= 0 ? p.r[0] : p.r[1];
             const float kx = (float)E.h_kvec[3 * E.h_runs[r0].kbeg], ky = std::fabs((float)E.h_kvec[3 * E.h_runs[r0].kbeg + 1]);
             pr[c * rp + q] = make_int4(p.kx * 128 | ((p.kx & 7) << 4) << 16, ry * 128 | ((ry & 7) << 4) << 16, bits(kx), bits(ky));
@@ -1143,6 +1195,7 @@ static bool tp_init(Engine &E, int which, const std::vector<int> &jr, int dmax) 
                 ki[((size_t)c * rp + q) * 4 * kcm + j] = make_int4(k[0], k[1], k[2], k[3]);
             }
         }
+        words += 2 * NC * rp * kc;
     }
     const size_t n[4] = {sizeof(int4) * pr.size(), sizeof(int2) * chunk.size(), sizeof(int4) * ki.size(), 16 * (size_t)words * kp.P};
     const void *src[3] = {pr.data(), chunk.data(), ki.data()};
@@ -1158,6 +1211,8 @@ static bool tp_init(Engine &E, int which, const std::vector<int> &jr, int dmax) 
         E.allocs.push_back(d[i]);
         if (i < 3) cudaMemcpy(d[i], src[i], n[i], cudaMemcpyHostToDevice);
     }
+    cudaMemset(d[3], 0, n[3]);  // (rows past a pair's |kz| stay zero)
+    if (place) *place = where;
     T.pair = reinterpret_cast<const int4 *>(d[0]);
     T.chunk = reinterpret_cast<const int2 *>(d[1]);
     T.kidx = reinterpret_cast<const int4 *>(d[2]);
@@ -1169,8 +1224,10 @@ static bool tp_init(Engine &E, int which, const std::vector<int> &jr, int dmax) 
     return true;
 }
 
-static void tp_setup(Engine &E, PFN_cuTensorMapEncodeTiled_v12000 enc, const std::vector<int> &jr, int optin) {
+static void tp_setup(Engine &E, PFN_cuTensorMapEncodeTiled_v12000 enc, const std::vector<int> &jr, std::vector<int4> *place) {
     KP &kp = E.kp;
+    int optin = 0;
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, E.device);
     const void *fk[4] = {(const void *)k_field_p<TF_Q>, (const void *)k_field_p<TF_D>, (const void *)k_field_p<TF_QG>,
                          (const void *)k_field_p<TF_DG>};
     size_t fstat = 0;
@@ -1199,8 +1256,7 @@ static void tp_setup(Engine &E, PFN_cuTensorMapEncodeTiled_v12000 enc, const std
                                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return;
     }
-    E.tf_ready = tp_init(E, 0, jr, dmax);
-    E.tf_qd_ready = E.tf_ready && tp_init(E, 1, jr, dmax);
+    if (tp_init(E, 0, jr, dmax, place)) tp_init(E, 1, jr, dmax, nullptr);
 }
 
 void tc_init(Engine &E) {
@@ -1235,7 +1291,18 @@ void tc_init(Engine &E) {
         jr[r] = std::max(std::abs(run.kzlo), std::abs(run.kzlo + run.nkz - 1)) + 1;
         order[r] = r;
     }
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return jr[x] > jr[y]; });
+    // ... the runs (kx, +-ky) of a pair side by side
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
+        const KRun &a = E.h_runs[x], &c = E.h_runs[y];
+        return std::make_tuple(-jr[x], a.kx, std::abs(a.ky)) < std::make_tuple(-jr[y], c.kx, std::abs(c.ky));
+    });
+    auto paired = [&](int x, int y) {
+        const KRun &a = E.h_runs[x], &c = E.h_runs[y];
+        return a.kx == c.kx && a.ky == -c.ky;
+    };
+    // the field passes' tables, and where their V has the rows of each run's pair (its offset, to the lo rows, |kz| rows)
+    std::vector<int4> place;
+    tp_setup(E, enc, jr, &place);
     // slots: every run once with its |kz| rows below TC_JB, then the runs reaching beyond once
     // per further band of TC_JB rows (j0 = TC_JB, 2 TC_JB, ...), each band in groups of <= 256
     // slots; a slot's k-vectors outside its group's rows are local entries with k = -1
@@ -1253,6 +1320,7 @@ void tc_init(Engine &E) {
     std::vector<float2> skv(nslot);
     std::vector<TcGroup> groups;
     std::vector<TcKW> kloc;
+    std::vector<int4> vp;
     std::vector<float2> runkf(kp.nrun);
     for (int r = 0; r < kp.nrun; r++)
         runkf[r] = make_float2((float)E.h_kvec[3 * E.h_runs[r].kbeg], (float)E.h_kvec[3 * E.h_runs[r].kbeg + 1]);
@@ -1263,8 +1331,11 @@ void tc_init(Engine &E) {
         const int j0 = src[p0].y, jmg = std::min(TC_JB, jr[src[p0].x] - j0);
         int left = 0;
         while (p0 + left < nslot && src[p0 + left].y == j0) left++;
-        const int ng = (left + TC_MAXRUN - 1) / TC_MAXRUN, nr = (left + ng - 1) / ng;
-        TcGroup g{p0, nr, 0, jmg, 0, (int)kloc.size(), j0, 0};
+        // (a pair stays in one group)
+        const int ng = (left + TC_MAXRUN - 2) / (TC_MAXRUN - 1);
+        int nr = (left + ng - 1) / ng;
+        if (nr < left && paired(src[p0 + nr - 1].x, src[p0 + nr].x)) nr++;
+        TcGroup g{p0, nr, 0, jmg, 0, (int)kloc.size(), j0, 0, (int)vp.size()};
         g.ncol = ((2 * g.nr + 15) / 16) * 16;
         for (int p = p0; p < p0 + g.nr; p++) {
             const int r = src[p].x;
@@ -1278,7 +1349,16 @@ void tc_init(Engine &E) {
                 kloc.push_back(TcKW{mine ? run.kbeg + j : -1, (float)(FOURPI * E.h_Ak[run.kbeg + j] / kp.volume)});
             }
             g.nkl += run.nkz;
+            const int4 at = place.empty() ? make_int4(0, 0, 0, 0) : place[r];
+            const int q = p - p0, ip = run.ky < 0 ? 0xffff : q, im = run.ky < 0 ? q : 0xffff;
+            if (q > 0 && paired(src[p - 1].x, r) && run.ky != 0) {  // the pair's second run
+                int4 &v = vp.back();
+                v.x = run.ky < 0 ? (v.x & 0xffff) | im << 16 : ip | (v.x & ~0xffff);
+            } else {
+                vp.push_back(make_int4(ip | im << 16, at.x, at.y, at.z));
+            }
         }
+        g.np = (int)vp.size() - g.vp0;
         groups.push_back(g);
         ncolmax = std::max(ncolmax, g.ncol);
         nklmax = std::max(nklmax, g.nkl);
@@ -1316,22 +1396,25 @@ void tc_init(Engine &E) {
     TcGroup *d_groups = nullptr;
     TcKW *d_kloc = nullptr;
     float *d_kzv = nullptr;
+    int4 *d_vp = nullptr;
     if (cudaMalloc((void **)&d_slots, sizeof(int4) * slots.size()) != cudaSuccess ||
         cudaMalloc((void **)&d_skv, sizeof(float2) * skv.size()) != cudaSuccess ||
         cudaMalloc((void **)&d_groups, sizeof(TcGroup) * groups.size()) != cudaSuccess ||
         cudaMalloc((void **)&d_kloc, sizeof(TcKW) * kloc.size()) != cudaSuccess ||
+        cudaMalloc((void **)&d_vp, sizeof(int4) * vp.size()) != cudaSuccess ||
         cudaMalloc((void **)&d_kzv, sizeof(float) * kzv.size()) != cudaSuccess) {
         cudaGetLastError();
-        for (void *p : {(void *)d_slots, (void *)d_skv, (void *)d_groups, (void *)d_kloc, (void *)d_kzv})
+        for (void *p : {(void *)d_slots, (void *)d_skv, (void *)d_groups, (void *)d_kloc, (void *)d_kzv, (void *)d_vp})
             if (p) cudaFree(p);
         return;
     }
-    for (void *p : {(void *)d_slots, (void *)d_skv, (void *)d_groups, (void *)d_kloc, (void *)d_kzv}) E.allocs.push_back(p);
+    for (void *p : {(void *)d_slots, (void *)d_skv, (void *)d_groups, (void *)d_kloc, (void *)d_kzv, (void *)d_vp}) E.allocs.push_back(p);
     cudaMemcpy(d_slots, slots.data(), sizeof(int4) * slots.size(), cudaMemcpyHostToDevice);
     cudaMemcpy(d_skv, skv.data(), sizeof(float2) * skv.size(), cudaMemcpyHostToDevice);
     cudaMemcpy(d_groups, groups.data(), sizeof(TcGroup) * groups.size(), cudaMemcpyHostToDevice);
     cudaMemcpy(d_kloc, kloc.data(), sizeof(TcKW) * kloc.size(), cudaMemcpyHostToDevice);
     cudaMemcpy(d_kzv, kzv.data(), sizeof(float) * kzv.size(), cudaMemcpyHostToDevice);
+    cudaMemcpy(d_vp, vp.data(), sizeof(int4) * vp.size(), cudaMemcpyHostToDevice);
     // tables [P][ntab][S] float2 as a 2-D FP32 tensor (x = 2 S values, y = P ntab rows); a box
     // is 16 sites (128 bytes) x ntab rows, written to shared memory with the 128-byte swizzle
     CUtensorMap *map = reinterpret_cast<CUtensorMap *>(E.tc_map);
@@ -1347,6 +1430,7 @@ void tc_init(Engine &E) {
     E.d_tcgrp = d_groups;
     E.d_tckloc = d_kloc;
     E.d_tckzv = d_kzv;
+    E.d_tcvp = d_vp;
     // X-operand cache of the dipole sites (k_sfac_tc, TC_OP_MU): per bead and run group, one
     // block per 16 sites from the first site group's base, hi and lo rows [0, 2 nr) rounded to
     // 8-row groups; zero-filled once (the padding rows are never written)
@@ -1390,8 +1474,8 @@ void tc_init(Engine &E) {
         E.tc_ncl[n] = c > 0 ? c : std::max(1, nsm / n);
     }
     E.tc_ready = true;
-    E.tf_ready = false;
-    tp_setup(E, enc, jr, optin);
+    E.tf_ready = E.tp[0].V != nullptr;
+    E.tf_qd_ready = E.tf_ready && E.tp[1].V != nullptr;
 }
 
 // whether the iterations' field pass is launched as a programmatic dependent (griddepcontrol.wait
@@ -1433,7 +1517,8 @@ static void launch_field_p(Engine &E, int s0, int s1) {
     cf.gridDim = dim3((s1 - a.sbase + TF_SITES - 1) / TF_SITES, kp.P);
     cf.blockDim = dim3(TP_NT);
     cf.dynamicSmemBytes = L.total;
-    // both as programmatic dependents: V's grid of the structure factor, the field pass of V's
+    // V where the structure factor has not written it, and the field pass, each as a programmatic dependent of
+    // the kernel before it
     auto run = [&](cudaLaunchConfig_t &cfg, auto &&launch) {
         cfg.stream = E.stream;
         cfg.attrs = at;
@@ -1446,9 +1531,13 @@ static void launch_field_p(Engine &E, int s0, int s1) {
         if (E.field_needs_join) cudaStreamWaitEvent(E.stream, E.loop_join, 0);
         launch();
     };
-    run(cv, [&] { return cudaLaunchKernelEx(&cv, k_field_v<DG>, kp, a, slot); });
+    if (DG || E.tp_vslot != slot) {
+        run(cv, [&] { return cudaLaunchKernelEx(&cv, k_field_v<DG>, kp, a, slot); });
+        if (!DG) E.tp_vslot = slot;
+        ++E.nlaunch;
+    }
     run(cf, [&] { return cudaLaunchKernelEx(&cf, k_field_p<MODE>, *xy, *z, kp, a); });
-    E.nlaunch += 2;
+    ++E.nlaunch;
 }
 
 // mode TF_D: dipole field, SOR update and convergence test of one iteration at the dipole sites
@@ -1521,6 +1610,9 @@ int launch_sfac_tc(Engine &E, int op, int s0, int nsites, int skipconv) {
     a.xblock = E.tc_xblock;
     a.xkeep = E.l2_keep ? 1 : 0;
     a.npt = E.tc_npt;
+    a.vp = E.d_tcvp;
+    a.V = reinterpret_cast<uint4 *>(E.tp[0].V);
+    a.vstride = E.tp[0].vstride;
     // the iterations' structure factor follows the previous iteration's field pass on the stream
     // (or the charge passes, which need no overlap): its CTAs are scheduled as that grid drains
     a.pdl = (op == TC_OP_MU && skipconv && E.tc_pdl && E.tf_ready && E.ff_tc) ? 1 : 0;
@@ -1596,6 +1688,7 @@ int launch_sfac_tc(Engine &E, int op, int s0, int nsites, int skipconv) {
         E.sf_tc = false;  // e.g. no room for the cluster: the FP32-pipe kernel from now on
         return 0;
     }
+    if (op != TC_OP_DIP && a.V) E.tp_vslot = op == TC_OP_MU ? 1 : 0;
     ++E.nlaunch;
     return 1;
 }
