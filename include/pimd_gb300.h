@@ -97,6 +97,8 @@ int pimd_full_bead_forces_device(pimd_ctx *ctx, const double *RRt, const double 
 int pimd_get_energies(pimd_ctx *ctx, int bead, double U[4]);
 int pimd_get_virial(pimd_ctx *ctx, int bead, double virt[9]);
 int pimd_get_dipole_info(pimd_ctx *ctx, int bead, int *niter, double *deltadip);
+/* the energies and the dipole information in one copy (any of the three may be null) */
+int pimd_get_bead_info(pimd_ctx *ctx, int bead, double *U, int *niter, double *deltadip);
 
 /* The half neighbour list of bead `bead` from the last force call: O-O pairs (i, j), 0-based,
  * i < j, in find_neigh's order (find_neigh.f90:75-117). Writes min(npairs, cap) pairs to

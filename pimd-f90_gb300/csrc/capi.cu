@@ -910,10 +910,42 @@ int capture_forces(Engine *const *ctx, int n, double *const *out, cudaStream_t s
     return bad(cudaGetLastError(), "force kernels") ? PIMD_ERR_CUDA : PIMD_OK;
 }
 
-static int read_err(Engine &E) {
+HostCopies::HostCopies(Engine &e) : E(e) {
+    if (!E.h_pin && cudaMallocHost((void **)&E.h_pin, ROOM) != cudaSuccess) {
+        cudaGetLastError();  // (plain copies then)
+        E.h_pin = nullptr;
+    }
+}
+char *HostCopies::part(size_t n) {
+    if (!E.h_pin || n > SMALL || used + n > ROOM) return nullptr;
+    char *p = E.h_pin + used;
+    used += (n + 63) & ~(size_t)63;
+    return p;
+}
+void HostCopies::in(void *dev, const void *host, size_t n) {
+    char *p = part(n);
+    if (p) std::memcpy(p, host, n);
+    cudaMemcpyAsync(dev, p ? p : host, n, cudaMemcpyHostToDevice, E.stream);
+}
+void HostCopies::out(void *host, const void *dev, size_t n) {
+    if (!host) return;
+    char *p = part(n);
+    if (p) outs.push_back(Out{host, p, n});
+    cudaMemcpyAsync(p ? p : host, dev, n, cudaMemcpyDeviceToHost, E.stream);
+}
+cudaError_t HostCopies::done() {
+    const cudaError_t e = cudaStreamSynchronize(E.stream);
+    if (e == cudaSuccess)
+        for (const Out &o : outs) std::memcpy(o.host, o.from, o.n);
+    outs.clear();
+    return e;
+}
+
+// the end of a force call on host arrays: its outputs and the error word
+static int finish_copies(Engine &E, HostCopies &hc) {
     unsigned err = 0;
-    cudaError_t e = cudaMemcpyAsync(&err, E.kp.err, sizeof(unsigned), cudaMemcpyDeviceToHost, E.stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(E.stream);
+    hc.out(&err, E.kp.err, sizeof(unsigned));
+    const cudaError_t e = hc.done();
     if (e != cudaSuccess) return cuda_check(E, e, "force call");
     if (err & 1u) return fail(E, PIMD_ERR_NEIGHBOR_OVERFLOW, "neighbour list capacity exceeded");
     if (err & 4u) return fail(E, PIMD_ERR_GAMMQ, "gammq2_3 did not converge");
@@ -1045,25 +1077,26 @@ int pimd_full_bead_forces(pimd_ctx *ctx, const double *RRt, const double *RRc, d
     cudaSetDevice(E.device);
     KP &kp = E.kp;
     const size_t P = kp.P, na = kp.natoms, nw = kp.N;
-    cudaMemcpyAsync((void *)kp.RRt, RRt, sizeof(double) * P * na * 3, cudaMemcpyHostToDevice, E.stream);
-    cudaMemcpyAsync((void *)kp.RRc, RRc, sizeof(double) * na * 3, cudaMemcpyHostToDevice, E.stream);
+    HostCopies hc(E);
+    hc.in((void *)kp.RRt, RRt, sizeof(double) * P * na * 3);
+    hc.in((void *)kp.RRc, RRc, sizeof(double) * na * 3);
     double *d_out = E.d_out;  // Upott, virialt, virialct staged on the device
     int rc = run_forces(E, t, ctx->check_every, d_out, d_out + P, d_out + 2 * P, nullptr);
     if (!rc) {
         std::vector<double> h(3 * P);
-        cudaMemcpyAsync(h.data(), d_out, sizeof(double) * 3 * P, cudaMemcpyDeviceToHost, E.stream);
-        if (dRRt) cudaMemcpyAsync(dRRt, kp.dRRt, sizeof(double) * P * na * 3, cudaMemcpyDeviceToHost, E.stream);
-        if (dip_momIt) cudaMemcpyAsync(dip_momIt, kp.dipI, sizeof(double) * P * nw * 3, cudaMemcpyDeviceToHost, E.stream);
-        if (dip_momEt) cudaMemcpyAsync(dip_momEt, kp.dipE, sizeof(double) * P * nw * 3, cudaMemcpyDeviceToHost, E.stream);
-        if (chg) cudaMemcpyAsync(chg, kp.chg + (P - 1) * na, sizeof(double) * na, cudaMemcpyDeviceToHost, E.stream);
-        rc = read_err(E);
+        hc.out(h.data(), d_out, sizeof(double) * 3 * P);
+        hc.out(dRRt, kp.dRRt, sizeof(double) * P * na * 3);
+        hc.out(dip_momIt, kp.dipI, sizeof(double) * P * nw * 3);
+        hc.out(dip_momEt, kp.dipE, sizeof(double) * P * nw * 3);
+        hc.out(chg, kp.chg + (P - 1) * na, sizeof(double) * na);
+        rc = finish_copies(E, hc);
         if (!rc) {
             if (Upott) std::copy(h.begin(), h.begin() + P, Upott);
             if (virialt) std::copy(h.begin() + P, h.begin() + 2 * P, virialt);
             if (virialct) std::copy(h.begin() + 2 * P, h.end(), virialct);
         }
     }
-    cudaStreamSynchronize(E.stream);
+    if (rc) cudaStreamSynchronize(E.stream);
     return rc;
 }
 
@@ -1075,25 +1108,26 @@ int pimd_pot_ttm(pimd_ctx *ctx, const double *RR, const double *RRc, double *En,
     KP saved = E.kp;
     E.kp.P = 1;  // bead-0 view of the context
     const size_t na = E.kp.natoms, nw = E.kp.N;
-    cudaMemcpyAsync((void *)E.kp.RRt, RR, sizeof(double) * na * 3, cudaMemcpyHostToDevice, E.stream);
-    cudaMemcpyAsync((void *)E.kp.RRc, RRc, sizeof(double) * na * 3, cudaMemcpyHostToDevice, E.stream);
+    HostCopies hc(E);
+    hc.in((void *)E.kp.RRt, RR, sizeof(double) * na * 3);
+    hc.in((void *)E.kp.RRc, RRc, sizeof(double) * na * 3);
     double *d_out = E.d_out;  // En, virialc, virt(9)
     int rc = run_forces(E, t, ctx->check_every, d_out, nullptr, d_out + 1, d_out + 2);
     if (!rc) {
         double h[12];
-        cudaMemcpyAsync(h, d_out, sizeof(h) - sizeof(double), cudaMemcpyDeviceToHost, E.stream);
-        if (dRR) cudaMemcpyAsync(dRR, E.kp.dRRt, sizeof(double) * na * 3, cudaMemcpyDeviceToHost, E.stream);
-        if (dip_momI) cudaMemcpyAsync(dip_momI, E.kp.dipI, sizeof(double) * nw * 3, cudaMemcpyDeviceToHost, E.stream);
-        if (Edip_mom) cudaMemcpyAsync(Edip_mom, E.kp.dipE, sizeof(double) * nw * 3, cudaMemcpyDeviceToHost, E.stream);
-        if (chg) cudaMemcpyAsync(chg, E.kp.chg, sizeof(double) * na, cudaMemcpyDeviceToHost, E.stream);
-        rc = read_err(E);
+        hc.out(h, d_out, sizeof(h) - sizeof(double));
+        hc.out(dRR, E.kp.dRRt, sizeof(double) * na * 3);
+        hc.out(dip_momI, E.kp.dipI, sizeof(double) * nw * 3);
+        hc.out(Edip_mom, E.kp.dipE, sizeof(double) * nw * 3);
+        hc.out(chg, E.kp.chg, sizeof(double) * na);
+        rc = finish_copies(E, hc);
         if (!rc) {
             if (En) *En = h[0];
             if (virialc) *virialc = h[1];
             if (virt) std::copy(h + 2, h + 11, virt);
         }
     }
-    cudaStreamSynchronize(E.stream);
+    if (rc) cudaStreamSynchronize(E.stream);
     E.kp = saved;
     return rc;
 }
@@ -1107,38 +1141,53 @@ int pimd_pot_spc(pimd_ctx *ctx, const double *RR, double *En, double *dRR, doubl
     KP saved = E.kp;
     E.kp.P = 1;  // bead-0 view of the context
     const size_t na = E.kp.natoms, nw = E.kp.N;
-    cudaMemcpyAsync((void *)E.kp.RRt, RR, sizeof(double) * na * 3, cudaMemcpyHostToDevice, E.stream);
+    HostCopies hc(E);
+    hc.in((void *)E.kp.RRt, RR, sizeof(double) * na * 3);
     double *d_out = E.d_out;  // En, (unused), virt(9)
     int rc = run_forces(E, 0, ctx->check_every, d_out, nullptr, nullptr, d_out + 2);
     if (!rc) {
         double h[11];
-        cudaMemcpyAsync(h, d_out, sizeof(h), cudaMemcpyDeviceToHost, E.stream);
-        if (dRR) cudaMemcpyAsync(dRR, E.kp.dRRt, sizeof(double) * na * 3, cudaMemcpyDeviceToHost, E.stream);
-        if (dip_momI) cudaMemcpyAsync(dip_momI, E.kp.dipI, sizeof(double) * nw * 3, cudaMemcpyDeviceToHost, E.stream);
-        if (chg) cudaMemcpyAsync(chg, E.kp.chg, sizeof(double) * na, cudaMemcpyDeviceToHost, E.stream);
-        rc = read_err(E);
+        hc.out(h, d_out, sizeof(h));
+        hc.out(dRR, E.kp.dRRt, sizeof(double) * na * 3);
+        hc.out(dip_momI, E.kp.dipI, sizeof(double) * nw * 3);
+        hc.out(chg, E.kp.chg, sizeof(double) * na);
+        rc = finish_copies(E, hc);
         if (!rc) {
             if (En) *En = h[0];
             if (virt) std::copy(h + 2, h + 11, virt);
         }
     }
-    cudaStreamSynchronize(E.stream);
+    if (rc) cudaStreamSynchronize(E.stream);
     E.kp = saved;
     return rc;
 }
 
-int pimd_get_energies(pimd_ctx *ctx, int bead, double U[4]) {
-    if (!ctx || bead < 0 || bead >= ctx->E.kp.P || !U) return PIMD_ERR_ARG;
-    Engine &E = ctx->E;
+// a bead's accumulators in one copy
+static int read_acc(Engine &E, int bead, double (&a)[NACC], const char *what) {
+    HostCopies hc(E);
+    hc.out(a, E.kp.acc + (size_t)bead * NACC, sizeof(a));
+    return cuda_check(E, hc.done(), what);
+}
+
+int pimd_get_bead_info(pimd_ctx *ctx, int bead, double *U, int *niter, double *deltadip) {
+    if (!ctx || bead < 0 || bead >= ctx->E.kp.P) return PIMD_ERR_ARG;
     double a[NACC];
-    cudaMemcpyAsync(a, E.kp.acc + (size_t)bead * NACC, sizeof(a), cudaMemcpyDeviceToHost, E.stream);
-    int rc = cuda_check(E, cudaStreamSynchronize(E.stream), "get_energies");
+    const int rc = read_acc(ctx->E, bead, a, "get_bead_info");
     if (rc) return rc;
-    U[0] = a[ACC_UMON];
-    U[1] = a[ACC_UVDW];
-    U[2] = 0.5 * a[ACC_UELEC2];
-    U[3] = a[ACC_UIND];
+    if (U) {
+        U[0] = a[ACC_UMON];
+        U[1] = a[ACC_UVDW];
+        U[2] = 0.5 * a[ACC_UELEC2];
+        U[3] = a[ACC_UIND];
+    }
+    if (niter) *niter = (int)a[ACC_NITER];
+    if (deltadip) *deltadip = ctx->E.kp.stath * std::sqrt(a[ACC_DELTADIP]);
     return PIMD_OK;
+}
+
+int pimd_get_energies(pimd_ctx *ctx, int bead, double U[4]) {
+    if (!U) return PIMD_ERR_ARG;
+    return pimd_get_bead_info(ctx, bead, U, nullptr, nullptr);
 }
 
 int pimd_get_virial(pimd_ctx *ctx, int bead, double virt[9]) {
@@ -1202,15 +1251,7 @@ int pimd_get_neighbors(pimd_ctx *ctx, int bead, int *ij, int cap, int *npairs) {
 }
 
 int pimd_get_dipole_info(pimd_ctx *ctx, int bead, int *niter, double *deltadip) {
-    if (!ctx || bead < 0 || bead >= ctx->E.kp.P) return PIMD_ERR_ARG;
-    Engine &E = ctx->E;
-    double a[NACC];
-    cudaMemcpyAsync(a, E.kp.acc + (size_t)bead * NACC, sizeof(a), cudaMemcpyDeviceToHost, E.stream);
-    int rc = cuda_check(E, cudaStreamSynchronize(E.stream), "get_dipole_info");
-    if (rc) return rc;
-    if (niter) *niter = (int)a[ACC_NITER];
-    if (deltadip) *deltadip = ctx->E.kp.stath * std::sqrt(a[ACC_DELTADIP]);
-    return PIMD_OK;
+    return pimd_get_bead_info(ctx, bead, nullptr, niter, deltadip);
 }
 
 // ---------------------------------------------------------------------------------------

@@ -254,6 +254,31 @@ struct PhaseTimers {
     int cur = -1;
 };
 
+struct Engine;
+// The copies of one call between the caller's host arrays and the device. Arrays of up to 64 KB go by way of a
+// pinned buffer of the context: a copy from or to pageable memory waits for itself (10-11 us each, also
+// for a few bytes; 2 us pinned), and a force call has nine. Larger ones go straight: 1.2 MB takes 19 us.
+// The buffer's parts are used once a call; done() waits for the stream and gives the arrays their values.
+class HostCopies {
+  public:
+    explicit HostCopies(Engine &e);
+    void in(void *dev, const void *host, size_t n);
+    void out(void *host, const void *dev, size_t n);  // (nothing for a null host)
+    cudaError_t done();
+
+  private:
+    static constexpr size_t SMALL = 64 << 10, ROOM = 256 << 10;
+    char *part(size_t n);
+    struct Out {
+        void *host;
+        const char *from;
+        size_t n;
+    };
+    Engine &E;
+    size_t used = 0;
+    std::vector<Out> outs;
+};
+
 struct Engine {
     KP kp;
     PhaseTimers timers;
@@ -318,12 +343,12 @@ struct Engine {
     std::vector<int> h_khkl;
     std::vector<double> h_kvec, h_Ak;
     // host pinned staging
-    double *h_pin = nullptr;
-    size_t h_pin_bytes = 0;
+    char *h_pin = nullptr;               // HostCopies
     int *h_allconv = nullptr;            // [4] pinned: all beads converged after iteration i, at i % 4
     cudaEvent_t ev_check[2] = {nullptr, nullptr};  // the last two iterations the eager loop may look at
     double *d_out = nullptr;  // small device staging for per-bead scalar outputs
     double *d_md = nullptr;   // device MD state for the host-array step (pimd_md_step)
+    double *d_con = nullptr;  // the same for the contracted step (pimd_contracted_step)
     std::vector<void *> allocs;
     std::string last_error;
     long long nlaunch = 0;  // kernels launched by this context

@@ -1501,20 +1501,24 @@ static int md_step_host(pimd_ctx *ctx, const pimd_md_params *mp, double *RRt, do
         E.allocs.push_back(E.d_md);
     }
     double *dR = E.d_md, *dP = dR + n, *dG = dP + n, *dx1 = dG + n, *dx2 = dx1 + n, *dC = dx2 + n, *dO = dC + nc;
-    cudaMemcpyAsync(dR, RRt, sizeof(double) * n, cudaMemcpyHostToDevice, E.stream);
-    cudaMemcpyAsync(dP, PPt, sizeof(double) * n, cudaMemcpyHostToDevice, E.stream);
-    cudaMemcpyAsync(dG, dRRt, sizeof(double) * n, cudaMemcpyHostToDevice, E.stream);
-    if (xi1) cudaMemcpyAsync(dx1, xi1, sizeof(double) * n, cudaMemcpyHostToDevice, E.stream);
-    if (xi2) cudaMemcpyAsync(dx2, xi2, sizeof(double) * n, cudaMemcpyHostToDevice, E.stream);
+    HostCopies hc(E);
+    hc.in(dR, RRt, sizeof(double) * n);
+    hc.in(dP, PPt, sizeof(double) * n);
+    hc.in(dG, dRRt, sizeof(double) * n);
+    if (xi1) hc.in(dx1, xi1, sizeof(double) * n);
+    if (xi2) hc.in(dx2, xi2, sizeof(double) * n);
     int rc = md_step_any(ctx, mp, dR, dP, dG, dC, xi1 ? dx1 : nullptr, xi2 ? dx2 : nullptr, t,
                          nout == 4 ? dO : nullptr, nout == 4 ? nullptr : dO);
-    if (rc) return rc;
-    cudaMemcpyAsync(RRt, dR, sizeof(double) * n, cudaMemcpyDeviceToHost, E.stream);
-    cudaMemcpyAsync(PPt, dP, sizeof(double) * n, cudaMemcpyDeviceToHost, E.stream);
-    cudaMemcpyAsync(dRRt, dG, sizeof(double) * n, cudaMemcpyDeviceToHost, E.stream);
-    if (RRc) cudaMemcpyAsync(RRc, dC, sizeof(double) * nc, cudaMemcpyDeviceToHost, E.stream);
-    if (out) cudaMemcpyAsync(out, dO, sizeof(double) * nout, cudaMemcpyDeviceToHost, E.stream);
-    return nm_err(E, cudaStreamSynchronize(E.stream), "md_step");
+    if (rc) {
+        cudaStreamSynchronize(E.stream);  // (the copies in flight)
+        return rc;
+    }
+    hc.out(RRt, dR, sizeof(double) * n);
+    hc.out(PPt, dP, sizeof(double) * n);
+    hc.out(dRRt, dG, sizeof(double) * n);
+    hc.out(RRc, dC, sizeof(double) * nc);
+    hc.out(out, dO, sizeof(double) * nout);
+    return nm_err(E, hc.done(), "md_step");
 }
 
 int pimd_md_step(pimd_ctx *ctx, const pimd_md_params *mp, double *RRt, double *PPt, double *dRRt, double *RRc,
