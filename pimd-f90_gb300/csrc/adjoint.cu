@@ -772,11 +772,28 @@ int pimd_pot_backward(pimd_ctx *ctx, const double *Ebar, double *dRRt, double *d
     // structure factor, the field pass and the force pass's dipole half)
     const bool tcs = mixed && kp.model == 3 && E.tc_ready && E.sf_tc && E.tf_ready && E.ff_tc && E.tf_qd_ready &&
                      kp.Fx && kp.ld - kp.fd == kp.N;
+    // The real-space part of a sweep (the field of u, the bilinear term) runs on the second stream beside the
+    // reciprocal passes, and the PES's scale-factor derivatives, which need only the positions, on the third
+    // beside the sweeps (in one stream: forward + backward 4.84 ms at 512 x 32 mixed, 3.84 ms at 64 x 8 FP64)
+    const bool ov = E.ewald_overlap && E.aux_stream && E.loop_aux;
+    const cudaStream_t aux = ov ? E.aux_stream : st, aux2 = ov ? E.loop_aux : st;
+    auto order = [&](cudaEvent_t ev, cudaStream_t from, cudaStream_t to) {  // what follows on `to` after what is on `from`
+        if (!ov) return;
+        cudaEventRecord(ev, from);
+        cudaStreamWaitEvent(to, ev, 0);
+    };
+    if (!kp.contraction) {
+        order(E.ev_fork, st, aux2);
+        k_adj_nasa<<<dim3((unsigned)((4 * kp.N + 127) / 128), (unsigned)P), 128, 0, aux2>>>(kp, ebar, E.d_nasa4, thacc);
+        if (ov) cudaEventRecord(E.loop_join, aux2);
+        ++E.nlaunch;
+    }
     k_adj_init<<<gd, 128, 0, st>>>(kp, ebar, g, nu);
     for (int k = kmax; k >= 1; k--) {
         k_adj_u<<<gd, 128, 0, st>>>(kp, k, iters, E.d_tape, g, u, v, nu, bacc, bw, thacc, omega, mixed ? uf : nullptr,
                                     mixed ? vf : nullptr);
         cudaMemsetAsync(Dr, 0, sizeof(double) * sv, st);
+        order(E.ev_fork, st, aux);
         {  // D_real u: the forward's cached Thole tensors (FP64), or its per-entry smear scalars
            // with u in the molecule records (mixed)
             KP kq = kp;
@@ -786,50 +803,54 @@ int pimd_pot_backward(pimd_ctx *ctx, const double *Ebar, double *dRRt, double *d
             kq.dd_async = 0;
             const KP keep = E.kp;
             E.kp = kq;
+            E.stream = aux;
             if (mixed)
                 launch_dd_real_m(E);
             else
                 launch_dd_real(E);
+            E.stream = st;
             E.kp = keep;
         }
+        if (ov) cudaEventRecord(E.ev_check[0], aux);
+        if (mixed)
+            k_adj_ddbil_m<<<gw, 128, 0, aux>>>(kp, pf.v[4] * pf.v[4], uf, vf, bw, grad, thacc);
+        else
+            k_adj_ddbil<<<gp, 128, 0, aux>>>(kp, pf, u, v, bw, grad, thacc);
+        if (ov) cudaEventRecord(E.ev_join, aux);
         // S(v) = S(mu_{k-1}) is on the tape (the forward's iteration k formed it)
         const double2 *Smv = E.d_tapeS + (size_t)(k - 1) * P * kp.nk;
         adj_structure_factor(E, u, mixed ? uf : nullptr, Smu, bacc);
         if (tcs) {
-            // tensor-core sweep: the field of u (TF_Q on the weights of S_u moved to slot 0) into
-            // Fx, then the reciprocal bilinear term as the dipole force of v in the field of u
-            // plus that of u in the field of v (TF_DG, slot 1 zero) into dR:
-            // d/dx [u^T D_rec v] = -(dipole force of u in E_v + dipole force of v in E_u)
+            // tensor-core sweep: the reciprocal bilinear term as the dipole force of v in the field of u plus
+            // that of u in the field of v (TF_DG, the one weight slot in use at a time, the other zero) into dR:
+            // d/dx [u^T D_rec v] = -(dipole force of u in E_v + dipole force of v in E_u).
+            // The first pass has the sums of the field of u at hand and leaves it in Fx.
             const dim3 gk((unsigned)((kp.nk + 255) / 256), (unsigned)P);
             k_adj_wslots<0><<<gk, 256, 0, st>>>(kp, nullptr);
-            if (E.tp_vslot == 1) E.tp_vslot = 0;  // (the field passes' operand of S_u)
+            E.tp_vslot = -1;
             KP kq = kp;
             kq.acc = bacc;
             kq.dd_async = 0;
-            kq.fx_mode = 1;
+            kq.fx_mode = 0;
             const KP keep = E.kp;
             E.kp = kq;
-            launch_adj_field_tc(E);
             cudaMemsetAsync(kp.dR, 0, sizeof(double) * sv, st);
-            E.kp.fx_mode = 0;
             E.kp.dipf = vf;
-            launch_adj_dforce_tc(E);
+            launch_adj_dforce_tc(E, true);
             k_adj_wslots<1><<<gk, 256, 0, st>>>(kp, Smv);
-            E.tp_vslot = -1;
             E.kp.dipf = uf;
-            launch_adj_dforce_tc(E);
+            launch_adj_dforce_tc(E, false);
             E.kp = keep;
             E.nlaunch += 2;
+            if (ov) cudaStreamWaitEvent(st, E.ev_join, 0);
             k_adj_g<<<gd, 128, 0, st>>>(kp, k, iters, g, u, Dr, omega, kp.Fx, kp.dR, bw, grad);
         } else {
+            if (ov) cudaStreamWaitEvent(st, E.ev_check[0], 0);
             adj_dipole_field(E, Smu, bacc, Dr);
             k_adj_g<<<gd, 128, 0, st>>>(kp, k, iters, g, u, Dr, omega, nullptr, nullptr, bw, grad);
+            if (ov) cudaStreamWaitEvent(st, E.ev_join, 0);
+            adj_rec(E, 0, u, v, Smu, Smv, bw, grad, nullptr);
         }
-        if (mixed)
-            k_adj_ddbil_m<<<gw, 128, 0, st>>>(kp, pf.v[4] * pf.v[4], uf, vf, bw, grad, thacc);
-        else
-            k_adj_ddbil<<<gp, 128, 0, st>>>(kp, pf, u, v, bw, grad, thacc);
-        if (!tcs) adj_rec(E, 0, u, v, Smu, Smv, bw, grad, nullptr);
     }
     k_adj_final<<<gd, 128, 0, st>>>(kp, g, nu, thacc, tcs ? uf : nullptr);
     // charge-field adjoint nu: real-space pairs, reciprocal, intramolecular; vdW; Uelec d/da_cc
@@ -851,7 +872,7 @@ int pimd_pot_backward(pimd_ctx *ctx, const double *Ebar, double *dRRt, double *d
         cudaMemsetAsync(kp.dR, 0, sizeof(double) * sv, st);
         E.kp.fx_mode = 0;
         E.kp.dipf = uf;
-        launch_adj_dforce_tc(E);
+        launch_adj_dforce_tc(E, false);
         E.kp = keep;
         const dim3 gq((unsigned)((kp.S - kp.N + 127) / 128), (unsigned)P);
         k_adj_cross_fold<<<gq, 128, 0, st>>>(kp, kp.N, grad, phin);
@@ -864,13 +885,10 @@ int pimd_pot_backward(pimd_ctx *ctx, const double *Ebar, double *dRRt, double *d
         launch_adj_pairs_m(E, pf.v, ebar, nu, grad, phin, thacc);
     else
         k_adj_pairs<<<gp, 128, 0, st>>>(kp, pf, ebar, nu, grad, phin, thacc);
-    if (!kp.contraction) {
-        k_adj_nasa<<<dim3((unsigned)((4 * kp.N + 127) / 128), (unsigned)P), 128, 0, st>>>(kp, ebar, E.d_nasa4, thacc);
-        ++E.nlaunch;
-    }
     k_adj_mol<0><<<gm, 128, 0, st>>>(kp, ebar, E.d_phiq, nu, grad, phin, dR, thacc);
     k_adj_mol<1><<<gm, 128, 0, st>>>(kp, ebar, E.d_phiq, nu, grad, phin, dR, thacc);
     E.nlaunch += 5 + 8 * (long long)kmax;
+    if (ov && !kp.contraction) cudaStreamWaitEvent(st, E.loop_join, 0);
     // d Uvdw_lrc / dC at fixed cutoff (potential.f90:152-154)
     std::vector<double> th(PIMD_NTHETA);
     cudaMemcpyAsync(th.data(), thacc, sizeof(double) * PIMD_NTHETA, cudaMemcpyDeviceToHost, st);

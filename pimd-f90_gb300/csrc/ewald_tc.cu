@@ -77,8 +77,9 @@ constexpr long long TC_WAIT = 1LL << 28;  // cycles before a wait gives up (~0.1
 enum { TC_OP_Q = 0, TC_OP_MU = 1, TC_OP_DIP = 2 };
 // field passes (values as in ewald.cu): charge field and potential, dipole field + SOR update,
 // and the two halves of the force pass ewald_std_qd: TF_QG the charge force and potential from
-// the dipole structure factor, TF_DG the dipole force from the total (charge + dipole) one
-enum { TF_Q = 0, TF_D = 1, TF_QG = 2, TF_DG = 3 };
+// the dipole structure factor, TF_DG the dipole force from the total (charge + dipole) one; TF_DE is TF_DG
+// with the field itself, into Fx (the reverse sweep)
+enum { TF_Q = 0, TF_D = 1, TF_QG = 2, TF_DG = 3, TF_DE = 4 };
 
 // A run group: slots [p0, p0 + nr), MMA columns, the |kz| rows j0 .. j0 + jm - 1 of its Z
 // operand (6 jm <= 128: |kz| above 20 goes to band groups, j0 = 21, of the same runs), k-vectors
@@ -883,7 +884,7 @@ struct TpSmem {
 template <int MODE>
 __global__ void __launch_bounds__(TP_NT, 1)
     k_field_p(const __grid_constant__ CUtensorMap mapxy, const __grid_constant__ CUtensorMap mapz, KP kp, TpArgs a) {
-    constexpr bool DG = MODE == TF_DG;
+    constexpr bool DG = MODE == TF_DG || MODE == TF_DE;
     constexpr int NC = DG ? 12 : 8, EP = (DG ? TP_RPD : TP_RP) / 4;  // pairs a warp at most
     const int t = blockIdx.x, b = blockIdx.y;
     if (MODE == TF_D) pdl_launch_dependents();
@@ -978,7 +979,7 @@ __global__ void __launch_bounds__(TP_NT, 1)
     umma::fence_before_sync();
     bool bad = __syncthreads_or((int)err) != 0;
     umma::fence_after_sync();
-    constexpr int NA = DG ? 6 : 4;
+    constexpr int NA = MODE == TF_DE ? 9 : DG ? 6 : 4;
     float acc[NA];
 #pragma unroll
     for (int i = 0; i < NA; i++) acc[i] = 0.f;
@@ -1064,6 +1065,11 @@ __global__ void __launch_bounds__(TP_NT, 1)
                     acc[3] = fmaf(kx, fmaf(ex.x, u1r, -ex.y * u1i), acc[3]);
                     acc[4] = fmaf(ky, fmaf(ex.x, v1r, -ex.y * v1i), acc[4]);
                     acc[5] += fmaf(ex.x, u2r, -ex.y * u2i);
+                    if constexpr (MODE == TF_DE) {
+                        acc[6] = fmaf(kx, fmaf(ex.x, u0i, ex.y * u0r), acc[6]);
+                        acc[7] = fmaf(ky, fmaf(ex.x, v0i, ex.y * v0r), acc[7]);
+                        acc[8] += fmaf(ex.x, u1i, ex.y * u1r);
+                    }
                 } else {
                     acc[0] = fmaf(kx, fmaf(ex.x, u0i, ex.y * u0r), acc[0]);
                     acc[1] = fmaf(ky, fmaf(ex.x, v0i, ex.y * v0r), acc[1]);
@@ -1109,7 +1115,23 @@ __global__ void __launch_bounds__(TP_NT, 1)
             for (int i = 0; i < 4; i++) e[i] += red[(rq * TF_SITES + tid) * 4 + i];
     }
     if (bad && tid == 0) atomicOr(kp.err, 8u);
-    field_out<MODE, TP_NT>(kp, b, t, s_own, own && !bad, bad, e, din, iter);
+    if constexpr (MODE == TF_DE) {
+        __syncthreads();
+        if (warp < TF_NT / 32) {
+#pragma unroll
+            for (int i = 0; i < 3; i++) red[(part * TF_SITES + sl) * 4 + i] = acc[6 + i] * (1.f / TP_WS);
+        }
+        __syncthreads();
+        if (own && !bad) {
+            float f[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+            for (int rq = 0; rq < 4; rq++)
+#pragma unroll
+                for (int i = 0; i < 3; i++) f[i] += red[(rq * TF_SITES + tid) * 4 + i];
+            kp.Fx[(size_t)b * kp.S + s_own] = make_double4_32a((double)f[0], (double)f[1], (double)f[2], 0.0);
+        }
+    }
+    field_out<DG ? (int)TF_DG : MODE, TP_NT>(kp, b, t, s_own, own && !bad, bad, e, din, iter);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1228,8 +1250,8 @@ static void tp_setup(Engine &E, PFN_cuTensorMapEncodeTiled_v12000 enc, const std
     KP &kp = E.kp;
     int optin = 0;
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, E.device);
-    const void *fk[4] = {(const void *)k_field_p<TF_Q>, (const void *)k_field_p<TF_D>, (const void *)k_field_p<TF_QG>,
-                         (const void *)k_field_p<TF_DG>};
+    const void *fk[5] = {(const void *)k_field_p<TF_Q>, (const void *)k_field_p<TF_D>, (const void *)k_field_p<TF_QG>,
+                         (const void *)k_field_p<TF_DG>, (const void *)k_field_p<TF_DE>};
     size_t fstat = 0;
     for (const void *f : fk) {
         cudaFuncAttributes fa;
@@ -1488,7 +1510,7 @@ bool field_pdl_ok(const Engine &E) {
 template <int MODE>
 static void launch_field_p(Engine &E, int s0, int s1) {
     const KP &kp = E.kp;
-    constexpr bool DG = MODE == TF_DG;
+    constexpr bool DG = MODE == TF_DG || MODE == TF_DE;
     const Engine::TpSet &T = E.tp[DG ? 1 : 0];
     TpArgs a;
     a.pair = T.pair;
@@ -1545,29 +1567,26 @@ static void launch_field_p(Engine &E, int s0, int s1) {
 // [s0, s1) (k_field_f<F_Q> + k_field_finish<F_Q>); TF_QG, TF_DG: the halves of the force pass
 // (launch_field_qd_tc). 1 when launched, else 0.
 int launch_field_tc(Engine &E, int mode, int s0, int s1) {
-    if (!E.tc_ready || !E.tf_ready || !E.ff_tc || s1 <= s0 || (mode == TF_DG && !E.tf_qd_ready)) return 0;
+    if (!E.tc_ready || !E.tf_ready || !E.ff_tc || s1 <= s0 || (mode >= TF_DG && !E.tf_qd_ready)) return 0;
     if (mode == TF_D)
         launch_field_p<TF_D>(E, s0, s1);
     else if (mode == TF_Q)
         launch_field_p<TF_Q>(E, s0, s1);
     else if (mode == TF_QG)
         launch_field_p<TF_QG>(E, s0, s1);
-    else
+    else if (mode == TF_DG)
         launch_field_p<TF_DG>(E, s0, s1);
+    else
+        launch_field_p<TF_DE>(E, s0, s1);
     return 1;
 }
 
-// The differentiation form's reverse sweep on the mixed engine: the reciprocal field at the
-// dipole sites from the charge weight slot (TF_Q: into kp.Fx with fx_mode 1), and the dipole
-// force of kp.dipf from the two weight slots (TF_DG: into kp.dR, or kp.Fx with fx_mode 2), at
-// [fd, ld). 1 when launched, else 0.
-int launch_adj_field_tc(Engine &E) {
+// The differentiation form's reverse sweep on the mixed engine: the dipole force of kp.dipf from the two weight
+// slots (TF_DG: into kp.dR, or kp.Fx with fx_mode 2) at [fd, ld); with field, also the field of those weights
+// into kp.Fx (TF_DE; a pass of its own took 13 us a sweep at 512 x 32). 1 when launched, else 0.
+int launch_adj_dforce_tc(Engine &E, bool field) {
     if (!E.tf_qd_ready || E.kp.ld <= E.kp.fd) return 0;
-    return launch_field_tc(E, TF_Q, E.kp.fd, E.kp.ld);
-}
-int launch_adj_dforce_tc(Engine &E) {
-    if (!E.tf_qd_ready || E.kp.ld <= E.kp.fd) return 0;
-    return launch_field_tc(E, TF_DG, E.kp.fd, E.kp.ld);
+    return launch_field_tc(E, field ? TF_DE : TF_DG, E.kp.fd, E.kp.ld);
 }
 // the charge half of the force pass (TF_QG: -q E and phi of the dipole slot's weights) at the
 // charged sites from N on (TTM3-F: H1, H2, M), into kp.Fx with fx_mode 2
