@@ -318,7 +318,7 @@ __global__ void __maxnreg__(64) k_sfac_tc(const __grid_constant__ CUtensorMap tm
             umma::mbar_init(&tempty[i], TC_NB);
         }
         for (int i = 0; i < nab; i++) {
-            umma::mbar_init(&afull[i], TC_NB);
+            umma::mbar_init(&afull[i], xm == 2 ? TC_NB / 2 : TC_NB);
             umma::mbar_init(&aempty[i], 1);
             umma::mbar_init(&xfull[i], 1);
         }
@@ -367,9 +367,12 @@ __global__ void __maxnreg__(64) k_sfac_tc(const __grid_constant__ CUtensorMap tm
         }
         // Z items: one row (c, j, cos|sin) x 8 sites each, on the whole warps after the X items
         // (or as many of the last as TC_ZMAX items per thread need); row decoded once here
+        // (X cached: the halves of the builders take the two MMA steps of a stage, one Z item a thread -- at most
+        // 252 -- so that a step's chain of loads, splits and fences runs beside the next one's)
         const int nzi = 2 * NCZ * jm * 2;
-        const int zwarps = xm == 2 ? TC_NB : max((nzi + 32 * TC_ZMAX - 1) / (32 * TC_ZMAX), TC_NB - (2 * nr + 31) / 32);
-        const int zthreads = 32 * zwarps, zbase = 32 * TC_NB - zthreads;
+        const int half = xm == 2 ? warp / (TC_NB / 2) : 0;
+        const int zwarps = xm == 2 ? TC_NB / 2 : max((nzi + 32 * TC_ZMAX - 1) / (32 * TC_ZMAX), TC_NB - (2 * nr + 31) / 32);
+        const int zthreads = 32 * zwarps, zbase = xm == 2 ? half * zthreads : 32 * TC_NB - zthreads;
         int zn = 0, zoff[TC_ZMAX], zmo[TC_ZMAX], zer[TC_ZMAX], zcs[TC_ZMAX], zq[TC_ZMAX];
 #pragma unroll
         for (int u = 0; u < TC_ZMAX; u++) {
@@ -389,13 +392,13 @@ __global__ void __maxnreg__(64) k_sfac_tc(const __grid_constant__ CUtensorMap tm
             err |= (uint32_t)umma::mbar_wait(&mfull[tb], (uint32_t)((ts / TC_NST) & 1), TC_WAIT);
             const unsigned char *tab = sm + tb * L.stage;
             const float *muz = reinterpret_cast<const float *>(tab + L.muz);
-            for (int ks = 0; ks < TC_SS / TC_KS && !err; ks++) {
+            for (int ks = half; ks < (xm == 2 ? half + 1 : TC_SS / TC_KS) && !err; ks++) {
                 const int sub = ts * (TC_SS / TC_KS) + ks, ab = sub % nab, use = sub / nab;
                 if (use > 0) err |= (uint32_t)umma::mbar_wait(&aempty[ab], (uint32_t)((use - 1) & 1), TC_WAIT);
                 unsigned char *Bf = sm + L.buf + ab * L.bufstride;
                 const int so = ks * TC_KS;
                 uint4 *xb = xm ? xc + (size_t)sub * (a.xblock / 16) : nullptr;  // this block in the cache
-                if (xm == 2 && bt == 0) {
+                if (xm == 2 && bt == zbase) {
                     mbar_expect_tx(&xfull[ab], 2u * (uint32_t)xbytes);
                     bulk_load_stream(Bf + L.xoff, xb, (uint32_t)xbytes, &xfull[ab], a.xkeep);
                     bulk_load_stream(Bf + L.xoff + xlo, xb + xbytes / 16, (uint32_t)xbytes, &xfull[ab], a.xkeep);
@@ -570,19 +573,17 @@ __global__ void __maxnreg__(64) k_sfac_tc(const __grid_constant__ CUtensorMap tm
             if (warp < 16) {
                 const int lq = warp & 3, part = warp >> 2;  // 4 lane quarters x 4 column quarters
                 const int col = ch * 2 * TC_CH + 32 * part;
-                float v[8];
+                float v[32];
                 float *row = stg + (32 * lq + lane) * TC_LD + 32 * part;
-    #pragma unroll
-                for (int hh = 0; hh < 4; hh++) {
-                    if (nsub > 0) {
-                        umma::tmem_ld8(tm + ((uint32_t)(32 * lq) << 16) + (uint32_t)(col + 8 * hh), v);
-                    } else {
-    #pragma unroll
-                        for (int j = 0; j < 8; j++) v[j] = 0.f;
-                    }
-                    *reinterpret_cast<float4 *>(row + 8 * hh) = make_float4(v[0], v[1], v[2], v[3]);
-                    *reinterpret_cast<float4 *>(row + 8 * hh + 4) = make_float4(v[4], v[5], v[6], v[7]);
+                const uint32_t t0 = tm + ((uint32_t)(32 * lq) << 16) + (uint32_t)col;
+                if (nsub > 0) {
+                    umma::tmem_ld16x2(t0, t0 + 16, v);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 32; j++) v[j] = 0.f;
                 }
+#pragma unroll
+                for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4 *>(row + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
             }
             __syncthreads();
             for (int i = tid; i < TC_CH * jm; i += TC_NT) {
@@ -593,7 +594,7 @@ __global__ void __maxnreg__(64) k_sfac_tc(const __grid_constant__ CUtensorMap tm
                 const bool minus = j > 0 && -j >= sl.z && -j < sl.z + sl.w;
                 if (!plus && !minus) continue;
                 float2 gp[NCZ], gm[NCZ];
-    #pragma unroll
+#pragma unroll
                 for (int c = 0; c < NCZ; c++) {
                     const int rc = (c * jm + jj) * 2;
                     // (x, y) = (Re exy, Im exy) against mu_c c_j (row rc) and mu_c s_j (row rc + 1)
@@ -617,7 +618,7 @@ __global__ void __maxnreg__(64) k_sfac_tc(const __grid_constant__ CUtensorMap tm
                     }
                 } else {
                     // charges: S itself; dipole components: the three G_c
-    #pragma unroll
+#pragma unroll
                     for (int c = 0; c < NPT; c++) {
                         if (c < c0 || c >= c0 + npt) continue;
                         if (plus) pt[npt * (sl.y + j - sl.z) + c - c0] = make_float2(zs * gp[c].x, zs * gp[c].y);
