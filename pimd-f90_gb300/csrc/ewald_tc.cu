@@ -1347,47 +1347,6 @@ void tc_init(Engine &E) {
     std::vector<float2> runkf(kp.nrun);
     for (int r = 0; r < kp.nrun; r++)
         runkf[r] = make_float2((float)E.h_kvec[3 * E.h_runs[r].kbeg], (float)E.h_kvec[3 * E.h_runs[r].kbeg + 1]);
-    int ncolmax = 16, nklmax = 0, nvalid = 0;
-    // groups of one band hold equally many runs: the bead's CTAs of all groups run side by side, and a last
-    // group of one run (897 runs in groups of 224) would take a CTA's time for it
-    for (int p0 = 0; p0 < nslot;) {
-        const int j0 = src[p0].y, jmg = std::min(TC_JB, jr[src[p0].x] - j0);
-        int left = 0;
-        while (p0 + left < nslot && src[p0 + left].y == j0) left++;
-        // (a pair stays in one group)
-        const int ng = (left + TC_MAXRUN - 2) / (TC_MAXRUN - 1);
-        int nr = (left + ng - 1) / ng;
-        if (nr < left && paired(src[p0 + nr - 1].x, src[p0 + nr].x)) nr++;
-        TcGroup g{p0, nr, 0, jmg, 0, (int)kloc.size(), j0, 0, (int)vp.size()};
-        g.ncol = ((2 * g.nr + 15) / 16) * 16;
-        for (int p = p0; p < p0 + g.nr; p++) {
-            const int r = src[p].x;
-            const KRun &run = E.h_runs[r];
-            slots[p] = make_int4(run.kx + 256 * (run.ky + 128), g.nkl, run.kzlo, run.nkz);
-            skv[p] = runkf[r];
-            for (int j = 0; j < run.nkz; j++) {
-                const int akz = std::abs(run.kzlo + j);
-                const bool mine = akz >= j0 && akz < j0 + g.jm;
-                nvalid += mine;
-                kloc.push_back(TcKW{mine ? run.kbeg + j : -1, (float)(FOURPI * E.h_Ak[run.kbeg + j] / kp.volume)});
-            }
-            g.nkl += run.nkz;
-            const int4 at = place.empty() ? make_int4(0, 0, 0, 0) : place[r];
-            const int q = p - p0, ip = run.ky < 0 ? 0xffff : q, im = run.ky < 0 ? q : 0xffff;
-            if (q > 0 && paired(src[p - 1].x, r) && run.ky != 0) {  // the pair's second run
-                int4 &v = vp.back();
-                v.x = run.ky < 0 ? (v.x & 0xffff) | im << 16 : ip | (v.x & ~0xffff);
-            } else {
-                vp.push_back(make_int4(ip | im << 16, at.x, at.y, at.z));
-            }
-        }
-        g.np = (int)vp.size() - g.vp0;
-        groups.push_back(g);
-        ncolmax = std::max(ncolmax, g.ncol);
-        nklmax = std::max(nklmax, g.nkl);
-        p0 += nr;
-    }
-    if (nvalid != kp.nk) return;  // every k-vector in exactly one group
     // dynamic shared memory available: the opt-in limit minus the kernel's static part
     int optin = 0;
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, E.device);
@@ -1399,13 +1358,61 @@ void tc_init(Engine &E) {
         return;
     }
     const int dmax = optin - (int)std::max(fa.sharedSizeBytes, std::max(fq.sharedSizeBytes, fd.sharedSizeBytes));
-    // operand buffers: three when they fit, else two
-    int nabuf = TC_NABUF_MAX;
-    while (nabuf > 2 && TcSmem(kp.ntab, ncolmax, nabuf).total > dmax) nabuf--;
+    // groups of at most 256 runs, or of fewer until the operand buffers (four to two) and the epilogue's staging
+    // tile and partial S, which reuse the table and operand regions, fit
+    int ncolmax = 0, nklmax = 0, nvalid = 0, nabuf = 0;
+    bool fits = false;
+    for (int maxrun = TC_MAXRUN; maxrun >= 32 && !fits; maxrun -= 32) {
+        groups.clear();
+        kloc.clear();
+        vp.clear();
+        ncolmax = 16, nklmax = nvalid = 0;
+        // groups of one band hold equally many runs: the bead's CTAs of all groups run side by side, and a last
+        // group of one run (897 runs in groups of 224) would take a CTA's time for it
+        for (int p0 = 0; p0 < nslot;) {
+            const int j0 = src[p0].y, jmg = std::min(TC_JB, jr[src[p0].x] - j0);
+            int left = 0;
+            while (p0 + left < nslot && src[p0 + left].y == j0) left++;
+            // (a pair stays in one group)
+            const int ng = (left + maxrun - 2) / (maxrun - 1);
+            int nr = (left + ng - 1) / ng;
+            if (nr < left && paired(src[p0 + nr - 1].x, src[p0 + nr].x)) nr++;
+            TcGroup g{p0, nr, 0, jmg, 0, (int)kloc.size(), j0, 0, (int)vp.size()};
+            g.ncol = ((2 * g.nr + 15) / 16) * 16;
+            for (int p = p0; p < p0 + g.nr; p++) {
+                const int r = src[p].x;
+                const KRun &run = E.h_runs[r];
+                slots[p] = make_int4(run.kx + 256 * (run.ky + 128), g.nkl, run.kzlo, run.nkz);
+                skv[p] = runkf[r];
+                for (int j = 0; j < run.nkz; j++) {
+                    const int akz = std::abs(run.kzlo + j);
+                    const bool mine = akz >= j0 && akz < j0 + g.jm;
+                    nvalid += mine;
+                    kloc.push_back(TcKW{mine ? run.kbeg + j : -1, (float)(FOURPI * E.h_Ak[run.kbeg + j] / kp.volume)});
+                }
+                g.nkl += run.nkz;
+                const int4 at = place.empty() ? make_int4(0, 0, 0, 0) : place[r];
+                const int q = p - p0, ip = run.ky < 0 ? 0xffff : q, im = run.ky < 0 ? q : 0xffff;
+                if (q > 0 && paired(src[p - 1].x, r) && run.ky != 0) {  // the pair's second run
+                    int4 &v = vp.back();
+                    v.x = run.ky < 0 ? (v.x & 0xffff) | im << 16 : ip | (v.x & ~0xffff);
+                } else {
+                    vp.push_back(make_int4(ip | im << 16, at.x, at.y, at.z));
+                }
+            }
+            g.np = (int)vp.size() - g.vp0;
+            groups.push_back(g);
+            ncolmax = std::max(ncolmax, g.ncol);
+            nklmax = std::max(nklmax, g.nkl);
+            p0 += nr;
+        }
+        nabuf = TC_NABUF_MAX;
+        while (nabuf > 2 && TcSmem(kp.ntab, ncolmax, nabuf).total > dmax) nabuf--;
+        const int total = TcSmem(kp.ntab, ncolmax, nabuf).total;
+        fits = total <= dmax && 128 * TC_LD * 4 + 8 * nklmax <= total - 1024;
+    }
+    if (!fits || nvalid != kp.nk) return;  // (every k-vector in exactly one group)
     const TcSmem L(kp.ntab, ncolmax, nabuf);
-    if (L.total > dmax) return;
-    // the epilogue's staging tile and partial S reuse the table and operand regions
-    if (128 * TC_LD * 4 + 8 * nklmax > L.total - 1024) return;
     if (cudaFuncSetAttribute(k_sfac_tc<TC_OP_MU>, cudaFuncAttributeMaxDynamicSharedMemorySize, dmax) != cudaSuccess ||
         cudaFuncSetAttribute(k_sfac_tc<TC_OP_Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, dmax) != cudaSuccess ||
         cudaFuncSetAttribute(k_sfac_tc<TC_OP_DIP>, cudaFuncAttributeMaxDynamicSharedMemorySize, dmax) != cudaSuccess) {
