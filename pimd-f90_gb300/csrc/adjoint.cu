@@ -501,11 +501,11 @@ __global__ void __launch_bounds__(128) k_adj_nasa(KP kp, const double *ebar, con
             f2[j] = f2[j - 1] * x2;
         }
         double sum = 0.0;
-        for (int g = 0; g < c_ngrp[0]; g++) {
-            const int I = c_pg[g][0], J = c_pg[g][1], s0 = c_pg[g][2], n = c_pg[g][3];
+        for (int g = 0; g < c_nasa.ngrp[0]; g++) {
+            const int I = c_nasa.pg[g][0], J = c_nasa.pg[g][1], s0 = c_nasa.pg[g][2], n = c_nasa.pg[g][3];
             double pk = 0.0;
             for (int k = 0; k < n; k++) {
-                const int j = c_ps[s0 + k];
+                const int j = c_nasa.ps[s0 + k];
                 pk = fma(pk, x3, j < 0 ? 0.0 : __ldg(coef + 4 * j + x));
             }
             sum += (f1[I] * f2[J] + f1[J] * f2[I]) * pk;

@@ -9,22 +9,21 @@
 namespace pimd {
 
 // Per translation unit (each .cu that includes this header has its own copy in its own device
-// module): nasa_upload_constants() fills this unit's copy.
-static __constant__ double c_c5z[245];
-static __constant__ double c_coefD[84];
-static __constant__ float c_c5zf[245];  // FP32 copies for the mixed engine's polynomial sums
-static __constant__ float c_coefDf[84];
-static __constant__ unsigned char c_idx[245][3];
-static __constant__ unsigned char c_idxD[84][3];
-// The sums of pot_nasa (terms 1..244) and dms_nasa (terms 1..83) regrouped by the powers (i, j)
-// of x1, x2: per group, slots k = n .. 1 (descending, for Horner in x3) hold the term with
-// power k of f3, or -1 where the table has none. Group: i, j, first slot, slots.
+// module): nasa_upload_constants() fills this unit's copy, in one copy (eleven took 130 us of a
+// context's creation).
 constexpr int NASA_PG = 32, NASA_PS = 256, NASA_DG = 32, NASA_DS = 128;
-static __constant__ unsigned char c_pg[NASA_PG][4];
-static __constant__ short c_ps[NASA_PS];
-static __constant__ unsigned char c_dg[NASA_DG][4];
-static __constant__ short c_ds[NASA_DS];
-static __constant__ int c_ngrp[2];  // groups of the PES and of the DMS
+struct NasaConst {
+    double c5z[245], coefD[84];
+    float c5zf[245], coefDf[84];  // FP32 copies for the mixed engine's polynomial sums
+    // The sums of pot_nasa (terms 1..244) and dms_nasa (terms 1..83) regrouped by the powers (i, j)
+    // of x1, x2: per group, slots k = n .. 1 (descending, for Horner in x3) hold the term with
+    // power k of f3, or -1 where the table has none. Group: i, j, first slot, slots.
+    unsigned char pg[NASA_PG][4], dg[NASA_DG][4];
+    short ps[NASA_PS], ds[NASA_DS];
+    int ngrp[2];  // groups of the PES and of the DMS
+    unsigned char idx[245][3], idxD[84][3];
+};
+static __constant__ NasaConst c_nasa;
 
 // group terms j0 .. j1 - 1 of an (i, j, k) table by (i, j); returns the group count (-1: too many)
 static inline int nasa_group(const int *I, const int *J, const int *K, int j0, int j1, unsigned char (*grp)[4], short *slot,
@@ -54,42 +53,27 @@ static inline int nasa_group(const int *I, const int *J, const int *K, int j0, i
 
 // c5z = f5z C5ZA + fbasis CBASIS + fcore CCORE + frest CREST (nasa_mod.f90) and the index tables
 static inline void nasa_upload_constants() {
-    double c5z[245];
-    for (int j = 0; j < 245; j++)
-        c5z[j] = PIMD_NASA_F5Z * PIMD_NASA_C5ZA[j] + PIMD_NASA_FBASIS * PIMD_NASA_CBASIS[j] +
-                 PIMD_NASA_FCORE * PIMD_NASA_CCORE[j] + PIMD_NASA_FREST * PIMD_NASA_CREST[j];
-    unsigned char idx[245][3], idxD[84][3];
+    NasaConst h{};
     for (int j = 0; j < 245; j++) {
-        idx[j][0] = (unsigned char)PIMD_NASA_IDX1[j];
-        idx[j][1] = (unsigned char)PIMD_NASA_IDX2[j];
-        idx[j][2] = (unsigned char)PIMD_NASA_IDX3[j];
+        h.c5z[j] = PIMD_NASA_F5Z * PIMD_NASA_C5ZA[j] + PIMD_NASA_FBASIS * PIMD_NASA_CBASIS[j] +
+                   PIMD_NASA_FCORE * PIMD_NASA_CCORE[j] + PIMD_NASA_FREST * PIMD_NASA_CREST[j];
+        h.c5zf[j] = (float)h.c5z[j];
+        h.idx[j][0] = (unsigned char)PIMD_NASA_IDX1[j];
+        h.idx[j][1] = (unsigned char)PIMD_NASA_IDX2[j];
+        h.idx[j][2] = (unsigned char)PIMD_NASA_IDX3[j];
     }
     for (int j = 0; j < 84; j++) {
-        idxD[j][0] = (unsigned char)PIMD_NASA_IDXD1[j];
-        idxD[j][1] = (unsigned char)PIMD_NASA_IDXD2[j];
-        idxD[j][2] = (unsigned char)PIMD_NASA_IDXD3[j];
+        h.coefD[j] = PIMD_NASA_COEFD[j];
+        h.coefDf[j] = (float)PIMD_NASA_COEFD[j];
+        h.idxD[j][0] = (unsigned char)PIMD_NASA_IDXD1[j];
+        h.idxD[j][1] = (unsigned char)PIMD_NASA_IDXD2[j];
+        h.idxD[j][2] = (unsigned char)PIMD_NASA_IDXD3[j];
     }
-    cudaMemcpyToSymbol(c_c5z, c5z, sizeof(c5z));
-    cudaMemcpyToSymbol(c_coefD, PIMD_NASA_COEFD, sizeof(double) * 84);
-    float c5zf[245], coefDf[84];
-    for (int j = 0; j < 245; j++) c5zf[j] = (float)c5z[j];
-    for (int j = 0; j < 84; j++) coefDf[j] = (float)PIMD_NASA_COEFD[j];
-    cudaMemcpyToSymbol(c_c5zf, c5zf, sizeof(c5zf));
-    cudaMemcpyToSymbol(c_coefDf, coefDf, sizeof(coefDf));
-    cudaMemcpyToSymbol(c_idx, idx, sizeof(idx));
-    cudaMemcpyToSymbol(c_idxD, idxD, sizeof(idxD));
-    unsigned char pg[NASA_PG][4] = {}, dg[NASA_DG][4] = {};
-    short ps[NASA_PS], ds[NASA_DS];
-    for (int i = 0; i < NASA_PS; i++) ps[i] = -1;
-    for (int i = 0; i < NASA_DS; i++) ds[i] = -1;
-    int ng[2];
-    ng[0] = nasa_group(PIMD_NASA_IDX1, PIMD_NASA_IDX2, PIMD_NASA_IDX3, 1, 245, pg, ps, NASA_PG, NASA_PS);
-    ng[1] = nasa_group(PIMD_NASA_IDXD1, PIMD_NASA_IDXD2, PIMD_NASA_IDXD3, 1, 84, dg, ds, NASA_DG, NASA_DS);
-    cudaMemcpyToSymbol(c_pg, pg, sizeof(pg));
-    cudaMemcpyToSymbol(c_ps, ps, sizeof(ps));
-    cudaMemcpyToSymbol(c_dg, dg, sizeof(dg));
-    cudaMemcpyToSymbol(c_ds, ds, sizeof(ds));
-    cudaMemcpyToSymbol(c_ngrp, ng, sizeof(ng));
+    for (short &x : h.ps) x = -1;
+    for (short &x : h.ds) x = -1;
+    h.ngrp[0] = nasa_group(PIMD_NASA_IDX1, PIMD_NASA_IDX2, PIMD_NASA_IDX3, 1, 245, h.pg, h.ps, NASA_PG, NASA_PS);
+    h.ngrp[1] = nasa_group(PIMD_NASA_IDXD1, PIMD_NASA_IDXD2, PIMD_NASA_IDXD3, 1, 84, h.dg, h.ds, NASA_DG, NASA_DS);
+    cudaMemcpyToSymbol(c_nasa, &h, sizeof(h));
 }
 
 // Sum over the L lanes of a molecule (consecutive lanes of a warp; all of them call)
@@ -127,16 +111,16 @@ PIMD_D void nasa_pot_sums(double x1d, double x2d, double x3d, const double *c5zg
     nasa_powers(x1, f1, g1);
     nasa_powers(x2, f2, g2);
     S sum0 = 0, sum1 = 0, sum2 = 0, sum3 = 0;
-    for (int g = l; g < c_ngrp[0]; g += L) {
-        const int inI = c_pg[g][0], inJ = c_pg[g][1], s0 = c_pg[g][2], n = c_pg[g][3];
+    for (int g = l; g < c_nasa.ngrp[0]; g += L) {
+        const int inI = c_nasa.pg[g][0], inJ = c_nasa.pg[g][1], s0 = c_nasa.pg[g][2], n = c_nasa.pg[g][3];
         S pk = S(0), dpk = S(0);
         for (int t = 0; t < n; t++) {
-            const int j = c_ps[s0 + t];
+            const int j = c_nasa.ps[s0 + t];
             S c;
             if (sizeof(S) == sizeof(float))
-                c = j < 0 ? S(0) : (S)c_c5zf[j];
+                c = j < 0 ? S(0) : (S)c_nasa.c5zf[j];
             else
-                c = j < 0 ? S(0) : (S)(c5zg ? c5zg[j] : c_c5z[j]);
+                c = j < 0 ? S(0) : (S)(c5zg ? c5zg[j] : c_nasa.c5z[j]);
             dpk = dpk * x3 + pk;
             pk = pk * x3 + c;
         }
@@ -218,7 +202,7 @@ PIMD_D void nasa_pot(const double r1[3][3], const double box[3], const double bo
         nasa_pot_sums<float, L>(x1, x2, x3, nullptr, sum0, sum1, sum2, sum3, l);
     else
         nasa_pot_sums<double, L>(x1, x2, x3, c5zg, sum0, sum1, sum2, sum3, l);
-    const double Vc = 2.0 * (c5zg ? c5zg[0] : c_c5z[0]) + efac * sum0;
+    const double Vc = 2.0 * (c5zg ? c5zg[0] : c_nasa.c5z[0]) + efac * sum0;
     *e1 = ((Va + Vb + Vc) + 0.44739574026257) * 0.00285914375100642899;
     const double dVcdr1 = (-2.0 * b1 * efac * (dROH1 - reoh) * sum0 + (efac * sum1) * ireoh) * i1;
     const double dVcdr2 = (-2.0 * b1 * efac * (dROH2 - reoh) * sum0 + (efac * sum2) * ireoh) * i2;
@@ -277,8 +261,8 @@ PIMD_D void nasa_dms_finish(const double ROH1[3], const double ROH2[3], double d
     dp2dr1 = dp2dr1 * efac + P2 * defacdr1 + dpc0dr1;
     dp2dr2 = dp2dr2 * efac + P2 * defacdr2 + dpc0dr2;
     dp2dcabc = dp2dcabc * efac + dpc0dcabc;
-    P1 = c_coefD[0] + P1 * efac + PC0 * B2A;
-    P2 = c_coefD[0] + P2 * efac + PC0 * B2A;
+    P1 = c_nasa.coefD[0] + P1 * efac + PC0 * B2A;
+    P2 = c_nasa.coefD[0] + P2 * efac + PC0 * B2A;
     // nasa.f90:218: bfac = 1.d0/0.529177249 divides by a single-precision literal
     const double bfac = 1.0 / (double)0.529177249f;
     q3[0] = -(P1 + P2);
@@ -335,16 +319,16 @@ PIMD_D void nasa_dms_sums(double x1d, double x2d, double x3d, double (&out)[8], 
     nasa_powers(x1, f1, g1);
     nasa_powers(x2, f2, g2);
     S P1 = 0, P2 = 0, dp1dr1 = 0, dp1dr2 = 0, dp1dcabc = 0, dp2dr1 = 0, dp2dr2 = 0, dp2dcabc = 0;
-    for (int g = l; g < c_ngrp[1]; g += L) {
-        const int inI = c_dg[g][0], inJ = c_dg[g][1], s0 = c_dg[g][2], n = c_dg[g][3];
+    for (int g = l; g < c_nasa.ngrp[1]; g += L) {
+        const int inI = c_nasa.dg[g][0], inJ = c_nasa.dg[g][1], s0 = c_nasa.dg[g][2], n = c_nasa.dg[g][3];
         S qk = S(0), dqk = S(0);
         for (int t = 0; t < n; t++) {
-            const int j = c_ds[s0 + t];
+            const int j = c_nasa.ds[s0 + t];
             S c;
             if (sizeof(S) == sizeof(float))
-                c = j < 0 ? S(0) : (S)c_coefDf[j];
+                c = j < 0 ? S(0) : (S)c_nasa.coefDf[j];
             else
-                c = j < 0 ? S(0) : (S)c_coefD[j];
+                c = j < 0 ? S(0) : (S)c_nasa.coefD[j];
             dqk = dqk * x3 + qk;
             qk = qk * x3 + c;
         }

@@ -15,7 +15,7 @@ namespace pimd {
 
 void pot_init_constants(Engine &E) {
     pair_math_init(E);
-    nasa_upload_constants();
+    if (E.kp.model < 4) nasa_upload_constants();
 }
 
 // ---------------------------------------------------------------------------------------
