@@ -1339,6 +1339,13 @@ void tc_init(Engine &E) {
         if (src.size() == n0) break;
     }
     const int nslot = (int)src.size();
+    E.tc_ng224 = 0;
+    for (int p0 = 0; p0 < nslot;) {
+        int n = 0;
+        while (p0 + n < nslot && src[p0 + n].y == src[p0].y) n++;
+        E.tc_ng224 += (n + 223) / 224;
+        p0 += n;
+    }
     std::vector<int4> slots(nslot);
     std::vector<float2> skv(nslot);
     std::vector<TcGroup> groups;
@@ -1361,8 +1368,7 @@ void tc_init(Engine &E) {
     // groups of at most 256 runs, or of fewer until the operand buffers (four to two) and the epilogue's staging
     // tile and partial S, which reuse the table and operand regions, fit
     int ncolmax = 0, nklmax = 0, nvalid = 0, nabuf = 0;
-    bool fits = false;
-    for (int maxrun = TC_MAXRUN; maxrun >= 32 && !fits; maxrun -= 32) {
+    auto build = [&](int maxrun) {  // false: does not fit
         groups.clear();
         kloc.clear();
         vp.clear();
@@ -1409,9 +1415,12 @@ void tc_init(Engine &E) {
         nabuf = TC_NABUF_MAX;
         while (nabuf > 2 && TcSmem(kp.ntab, ncolmax, nabuf).total > dmax) nabuf--;
         const int total = TcSmem(kp.ntab, ncolmax, nabuf).total;
-        fits = total <= dmax && 128 * TC_LD * 4 + 8 * nklmax <= total - 1024;
-    }
-    if (!fits || nvalid != kp.nk) return;  // (every k-vector in exactly one group)
+        return total <= dmax && 128 * TC_LD * 4 + 8 * nklmax <= total - 1024;
+    };
+    int maxrun = TC_MAXRUN;
+    while (maxrun >= 32 && !build(maxrun)) maxrun -= 32;
+    if (maxrun < 32) return;
+    if (nvalid != kp.nk) return;  // every k-vector in exactly one group
     const TcSmem L(kp.ntab, ncolmax, nabuf);
     if (cudaFuncSetAttribute(k_sfac_tc<TC_OP_MU>, cudaFuncAttributeMaxDynamicSharedMemorySize, dmax) != cudaSuccess ||
         cudaFuncSetAttribute(k_sfac_tc<TC_OP_Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, dmax) != cudaSuccess ||
@@ -1485,24 +1494,8 @@ void tc_init(Engine &E) {
     E.tc_ntg = (int)groups.size();
     E.tc_ncolmax = ncolmax;
     E.tc_nabuf = nabuf;
-    // clusters of n CTAs the device holds at once
-    int nsm = 0;
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, E.device);
-    for (int n = 1; n <= TC_CLMAX; n++) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(n, E.tc_ntg, kp.P);
-        cfg.blockDim = dim3(TC_NT);
-        cfg.dynamicSmemBytes = L.total;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = n;
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        int c = 0;
-        if (cudaOccupancyMaxActiveClusters(&c, k_sfac_tc<TC_OP_MU>, &cfg) != cudaSuccess) cudaGetLastError();
-        E.tc_ncl[n] = c > 0 ? c : std::max(1, nsm / n);
-    }
+    cudaDeviceGetAttribute(&E.tc_nsm, cudaDevAttrMultiProcessorCount, E.device);
+    if (E.tc_nsm <= 0) E.tc_nsm = 152;
     E.tc_ready = true;
     E.tf_ready = E.tp[0].V != nullptr;
     E.tf_qd_ready = E.tf_ready && E.tp[1].V != nullptr;
@@ -1643,18 +1636,13 @@ int launch_sfac_tc(Engine &E, int op, int s0, int nsites, int skipconv) {
     // the iterations' structure factor follows the previous iteration's field pass on the stream
     // (or the charge passes, which need no overlap): its CTAs are scheduled as that grid drains
     a.pdl = (op == TC_OP_MU && skipconv && E.tc_pdl && E.tf_ready && E.ff_tc) ? 1 : 0;
-    // one CTA per SM (shared memory). Site groups (= cluster size) with the fewest waves x stages a CTA; a
-    // CTA's set-up and epilogue take about as long as 6 stages (512 x 32: 4 stages a CTA in 19 us, 4096 x 32:
-    // 128 in 225 us). One group whenever a wave was full took two waves of 152 and 40 CTAs at 4096 x 32
+    // one CTA per SM (shared memory); site groups (= cluster size) so that one wave fills the GPU with groups of
+    // 224 runs. Their number sets how many sites an accumulator adds up, which at 4096 sites shows in the dipoles:
+    // four groups instead of one took 298 us an iteration instead of 420, with dipoles 4e-5 (rms) away
     const int nst = (a.s_hi - a.sbase + TC_SS - 1) / TC_SS;
-    const long per = (long)E.tc_ntg * kp.P;
-    int ng = 1, spg = nst;
-    long best = -1;
-    for (int n = 1; n <= std::min(nst, TC_CLMAX); n++) {
-        const int sp = (nst + n - 1) / n, used = (nst + sp - 1) / sp;
-        const long cost = (per + E.tc_ncl[used] - 1) / E.tc_ncl[used] * (sp + 6);
-        if (best < 0 || cost < best) best = cost, ng = used, spg = sp;
-    }
+    int ng = std::max(1, std::min((int)std::max(1L, E.tc_nsm / ((long)E.tc_ng224 * kp.P)), std::min(nst, TC_CLMAX)));
+    const int spg = (nst + ng - 1) / ng;
+    ng = (nst + spg - 1) / spg;
     a.tsg = spg * TC_SS;
     const TcSmem L(kp.ntab, a.ncolmax, a.nabuf);
     cudaLaunchConfig_t cfg = {};
