@@ -1638,7 +1638,7 @@ int launch_sfac_tc(Engine &E, int op, int s0, int nsites, int skipconv) {
     a.pdl = (op == TC_OP_MU && skipconv && E.tc_pdl && E.tf_ready && E.ff_tc) ? 1 : 0;
     // one CTA per SM (shared memory); site groups (= cluster size) so that one wave fills the GPU with groups of
     // 224 runs. Their number sets how many sites an accumulator adds up, which at 4096 sites shows in the dipoles:
-    // four groups instead of one took 298 us an iteration instead of 420, with dipoles 4e-5 (rms) away
+    // four groups instead of one took 298 us an iteration instead of 398, with dipoles 4e-5 (rms) away
     const int nst = (a.s_hi - a.sbase + TC_SS - 1) / TC_SS;
     int ng = std::max(1, std::min((int)std::max(1L, E.tc_nsm / ((long)E.tc_ng224 * kp.P)), std::min(nst, TC_CLMAX)));
     const int spg = (nst + ng - 1) / ng;
