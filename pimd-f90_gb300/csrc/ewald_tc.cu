@@ -110,7 +110,9 @@ struct TcArgs {
     uint4 *xcache;        // X operand blocks of the dipole sites (null: no cache), see k_sfac_tc
     int xsub, xblock;     // 16-site blocks per bead and run group, bytes per block
     int xkeep;            // load the cached X blocks with the L2 evict-last policy
-    int pdl;              // launched as a programmatic dependent of the previous iteration's field pass
+    int pdl;              // 1: launched as a programmatic dependent of the previous iteration's field pass; 2: of
+                          // the band groups' launch, beside which it runs
+    int tg0, ntg;         // the launch's first run group, all of them
     int npt;              // dipole-component partials held at a time: 3, or 1
     const int4 *vp;       // per pair: group slots of its +ky | -ky << 16 runs (0xffff: none), where its rows of
                           // the field pass's V begin and how far the lo rows are from there (16-byte words), |kz| rows
@@ -256,12 +258,15 @@ __global__ void __maxnreg__(64) k_sfac_tc(const __grid_constant__ CUtensorMap tm
     // Z components: q (charges) or mu_x, mu_y, mu_z; partial sums per k: S, or the three G_c
     constexpr int NCZ = (OP == TC_OP_Q) ? 1 : 3;
     constexpr int NPT = (OP == TC_OP_DIP) ? 3 : 1;
-    const int grp = blockIdx.x, tg = blockIdx.y, b = blockIdx.z;
+    const int grp = blockIdx.x, tg = a.tg0 + blockIdx.y, b = blockIdx.z;
     // a programmatic launch starts under the previous field pass: the convergence flags, the
     // dipoles and the weights are that grid's output
-    if (a.pdl) pdl_wait();
+    if (a.pdl == 1) pdl_wait();
     // the whole cluster (same bead) leaves together
-    if (a.skipconv && bead_converged(kp, b)) return;
+    if (a.skipconv && bead_converged(kp, b)) {
+        if (a.pdl == 2) pdl_wait();
+        return;
+    }
     const TcGroup G = a.grp[tg];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const TcSmem L(kp.ntab, a.ncolmax, a.nabuf);
@@ -289,7 +294,7 @@ __global__ void __maxnreg__(64) k_sfac_tc(const __grid_constant__ CUtensorMap tm
     // layout; the cache is zeroed once, so the rows past 2 nr stay zero.
     const int xm = (OP == TC_OP_MU && a.xcache) ? (kp.dstep[1] == 0 ? 1 : 2) : 0;
     const int xbytes = ((2 * nr + 7) / 8) * 256;
-    uint4 *xc = xm ? a.xcache + ((size_t)(b * gridDim.y + tg) * a.xsub + (g0 - a.sbase) / TC_KS) * (a.xblock / 16)
+    uint4 *xc = xm ? a.xcache + ((size_t)(b * a.ntg + tg) * a.xsub + (g0 - a.sbase) / TC_KS) * (a.xblock / 16)
                    : nullptr;
 
     if (tid < nr) {
@@ -700,6 +705,7 @@ __global__ void __maxnreg__(64) k_sfac_tc(const __grid_constant__ CUtensorMap tm
         cluster_sync();  // remote reads done before any CTA of the cluster leaves (or writes the next component)
     }
     if (bad && tid == 0) atomicOr(kp.err, 8u);
+    if (a.pdl == 2) pdl_wait();  // this grid's end is the band groups' end too
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1492,6 +1498,7 @@ void tc_init(Engine &E) {
         }
     }
     E.tc_ntg = (int)groups.size();
+    E.tc_nband = (int)std::count_if(groups.begin(), groups.end(), [](const TcGroup &g) { return g.j0 > 0; });
     E.tc_ncolmax = ncolmax;
     E.tc_nabuf = nabuf;
     cudaDeviceGetAttribute(&E.tc_nsm, cudaDevAttrMultiProcessorCount, E.device);
@@ -1638,18 +1645,12 @@ int launch_sfac_tc(Engine &E, int op, int s0, int nsites, int skipconv) {
     a.pdl = (op == TC_OP_MU && skipconv && E.tc_pdl && E.tf_ready && E.ff_tc) ? 1 : 0;
     // one CTA per SM (shared memory); site groups (= cluster size) so that one wave fills the GPU with groups of
     // 224 runs. Their number sets how many sites an accumulator adds up, which at 4096 sites shows in the dipoles:
-    // four groups instead of one took 298 us an iteration instead of 398, with dipoles 4e-5 (rms) away
+    // four groups instead of one moved them by 4e-5 (rms)
     const int nst = (a.s_hi - a.sbase + TC_SS - 1) / TC_SS;
     int ng = std::max(1, std::min((int)std::max(1L, E.tc_nsm / ((long)E.tc_ng224 * kp.P)), std::min(nst, TC_CLMAX)));
     const int spg = (nst + ng - 1) / ng;
     ng = (nst + spg - 1) / spg;
-    a.tsg = spg * TC_SS;
-    const TcSmem L(kp.ntab, a.ncolmax, a.nabuf);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ng, E.tc_ntg, kp.P);
-    cfg.blockDim = dim3(TC_NT);
-    cfg.dynamicSmemBytes = L.total;
-    cfg.stream = E.stream;
+    a.ntg = E.tc_ntg;
     // the highest stream priority: the mixed engine's real-space dipole field runs beside this
     // kernel on a second stream and must not hold the SMs its clusters wait for
     static int prio_cache[64] = {0}, prio_set[64] = {0};
@@ -1658,53 +1659,78 @@ int launch_sfac_tc(Engine &E, int op, int s0, int nsites, int skipconv) {
         if (cudaDeviceGetStreamPriorityRange(&least, &greatest) == cudaSuccess) prio_cache[E.device & 63] = greatest;
         prio_set[E.device & 63] = 1;
     }
-    cudaLaunchAttribute at[4];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = ng;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributePriority;
-    at[1].val.priority = prio_cache[E.device & 63];
-    int na = 2;
-    if (a.pdl) {
-        at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[na].val.programmaticStreamSerializationAllowed = 1;
-        na++;
-    }
-    // the caller's programmatic event: recorded once every CTA has passed its set-up
-    // (griddepcontrol.launch_dependents) or left
-    const bool pev = E.sfac_pev_req && op == TC_OP_MU && E.loop_pev;
-    if (pev) {
-        at[na].id = cudaLaunchAttributeProgrammaticEvent;
-        at[na].val.programmaticEvent.event = E.loop_pev;
-        at[na].val.programmaticEvent.flags = 0;
-        at[na].val.programmaticEvent.triggerAtBlockStart = 0;
-        na++;
-    }
-    cfg.attrs = at;
-    cfg.numAttrs = na;
+    const TcSmem L(kp.ntab, a.ncolmax, a.nabuf);
     const CUtensorMap *map = reinterpret_cast<const CUtensorMap *>(E.tc_map);
-    cudaError_t e = cudaErrorInvalidValue;
-    if (op == TC_OP_MU)
-        e = cudaLaunchKernelEx(&cfg, k_sfac_tc<TC_OP_MU>, *map, kp, a);
-    else if (op == TC_OP_Q)
-        e = cudaLaunchKernelEx(&cfg, k_sfac_tc<TC_OP_Q>, *map, kp, a);
-    else
-        e = cudaLaunchKernelEx(&cfg, k_sfac_tc<TC_OP_DIP>, *map, kp, a);
-    if (e == cudaSuccess && pev) E.sfac_pev_armed = true;
-    if (e != cudaSuccess && na > 2) {  // an attribute refused: a plain cluster launch
-        cudaGetLastError();
-        a.pdl = 0;
-        cfg.numAttrs = 2;
-        e = cudaLaunchKernelEx(&cfg, k_sfac_tc<TC_OP_MU>, *map, kp, a);
+    // run groups [tg0, tg1) with clusters of n site groups of sp stages; pdl as in TcArgs
+    auto launch = [&](int tg0, int tg1, int n, int sp, int pdl, bool pev) {
+        a.tg0 = tg0;
+        a.tsg = sp * TC_SS;
+        a.pdl = pdl;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(n, tg1 - tg0, kp.P);
+        cfg.blockDim = dim3(TC_NT);
+        cfg.dynamicSmemBytes = L.total;
+        cfg.stream = E.stream;
+        cudaLaunchAttribute at[4];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = n;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        at[1].id = cudaLaunchAttributePriority;
+        at[1].val.priority = prio_cache[E.device & 63];
+        int na = 2;
+        if (pdl) {
+            at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at[na].val.programmaticStreamSerializationAllowed = 1;
+            na++;
+        }
+        // the caller's programmatic event: recorded once every CTA has passed its set-up
+        // (griddepcontrol.launch_dependents) or left
+        if (pev) {
+            at[na].id = cudaLaunchAttributeProgrammaticEvent;
+            at[na].val.programmaticEvent.event = E.loop_pev;
+            at[na].val.programmaticEvent.flags = 0;
+            at[na].val.programmaticEvent.triggerAtBlockStart = 0;
+            na++;
+        }
+        cfg.attrs = at;
+        cfg.numAttrs = na;
+        auto run = [&] {
+            return op == TC_OP_MU ? cudaLaunchKernelEx(&cfg, k_sfac_tc<TC_OP_MU>, *map, kp, a)
+                   : op == TC_OP_Q ? cudaLaunchKernelEx(&cfg, k_sfac_tc<TC_OP_Q>, *map, kp, a)
+                                   : cudaLaunchKernelEx(&cfg, k_sfac_tc<TC_OP_DIP>, *map, kp, a);
+        };
+        cudaError_t e = run();
+        if (e == cudaSuccess && pev) E.sfac_pev_armed = true;
+        if (e != cudaSuccess && na > 2) {  // an attribute refused: a plain cluster launch
+            cudaGetLastError();
+            a.pdl = 0;
+            cfg.numAttrs = 2;
+            e = run();
+        }
+        if (e == cudaSuccess) ++E.nlaunch;
+        return e;
+    };
+    // Boxes whose CTAs are more than one wave: the band groups (a quarter of the Z rows or less, but a CTA's whole
+    // time) go first, in clusters of four site groups, and the others start beside them, so that the last wave is
+    // not one of a few whole CTAs (4096 x 32: 160 on 152 SMs, 398 us an iteration; 275 so). Their k-vectors have |kz| > 20 and weights of 1e-6
+    // of the largest, so that their shorter sums leave the dipoles as they are.
+    const int main_groups = E.tc_ntg - E.tc_nband;
+    const bool split = E.tc_nband > 0 && main_groups > 0 && E.tc_pdl && (long)E.tc_ntg * kp.P > E.tc_nsm;
+    const bool pev = E.sfac_pev_req && op == TC_OP_MU && E.loop_pev;
+    const int first = a.pdl;
+    cudaError_t e = cudaSuccess;
+    if (split) {
+        const int nb4 = std::min(4, nst), sp4 = (nst + nb4 - 1) / nb4;
+        e = launch(main_groups, E.tc_ntg, (nst + sp4 - 1) / sp4, sp4, first, false);
     }
+    if (e == cudaSuccess) e = launch(0, split ? main_groups : E.tc_ntg, ng, spg, split ? 2 : first, pev);
     if (e != cudaSuccess) {
         cudaGetLastError();
         E.sf_tc = false;  // e.g. no room for the cluster: the FP32-pipe kernel from now on
         return 0;
     }
     if (op != TC_OP_DIP && a.V) E.tp_vslot = op == TC_OP_MU ? 1 : 0;
-    ++E.nlaunch;
     return 1;
 }
 

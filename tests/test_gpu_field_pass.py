@@ -1,7 +1,7 @@
 """The mixed engine's tensor-core structure factor and field passes (ewald_tc.cu) at the edges of their tiles:
-k shells of one K block to five (|kz| 3 to 39, the last with fewer run pairs a chunk and a second band of |kz|
-rows), run pairs around a chunk's 32 (and 20) and run groups around 256, boxes whose directions reach different
-|k|, sites around the tiles of 128, and beads in one site group or several.
+k shells of one K block to five (|kz| 3 to 39, the last with fewer run pairs a chunk; bands of |kz| rows, launched
+apart where the blocks are more than one wave), run pairs around a chunk's 32 (and 20) and run groups around 256,
+boxes whose directions reach different |k|, sites around the tiles of 128, and beads in one site group or several.
 
 Against the FP64 engine within the mixed engine's error budget: 1e-5 rms and 1e-4 of the largest. The operands
 carry 2^-22, their sums of up to 16 000 products of random sign in FP32 about 1e-6 of the field."""
@@ -33,7 +33,8 @@ def case(pkg, model, nw, P, nmax, f):
     ("ttm3f_512x32", 129, 5, 18, (1.0, 1.0, 1.0)), ("ttm3f_512x32", 40, 2, 24, (1.0, 1.0, 1.0)),
     ("ttm3f_512x32", 64, 1, 39, (1.0, 1.0, 1.0)), ("ttm3f_512x32", 300, 3, 13, (1.0, 1.0, 1.0)),
     ("ttm3f_512x32", 50, 2, 0, (1.0, 1.4, 2.0)), ("ttm3f_512x32", 50, 2, 0, (2.4, 1.0, 1.2)),
-    ("ttm21f_128x32", 44, 3, 17, (1.0, 1.0, 1.2)),
+    ("ttm21f_128x32", 44, 3, 17, (1.0, 1.0, 1.2)), ("ttm3f_512x32", 130, 40, 24, (1.0, 1.0, 1.0)),
+    ("ttm3f_512x32", 34, 64, 22, (1.0, 1.1, 1.0)),
 ])
 def test_mixed_passes_match_fp64(pkg, engine_lib, model, nw, P, nmax, f):
     p, RRt, RRc = case(pkg, model, nw, P, nmax, f)
