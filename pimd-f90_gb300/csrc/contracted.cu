@@ -343,14 +343,14 @@ int pimd_contracted_step(pimd_ctx *ctx, const pimd_md_params *mp, double *RRt, d
     if (!ctx->cen) return PIMD_ERR_STATE;
     cudaSetDevice(E.device);
     const size_t n = (size_t)E.kp.P * E.kp.natoms * 3, nc = (size_t)E.kp.natoms * 3, nd = (size_t)E.kp.P * E.kp.N * 3;
-    if (!E.d_con) {  // kept with the context: allocating and freeing it took 0.1 ms a step
-        if (cudaMalloc((void **)&E.d_con, sizeof(double) * (6 * n + nc + 2 * nd + PIMD_MD_NOUT)) != cudaSuccess) {
-            E.d_con = nullptr;
+    if (!E.d_conmd) {  // kept with the context: allocating and freeing it took 0.1 ms a step
+        if (cudaMalloc((void **)&E.d_conmd, sizeof(double) * (6 * n + nc + 2 * nd + PIMD_MD_NOUT)) != cudaSuccess) {
+            E.d_conmd = nullptr;
             return PIMD_ERR_NOMEM;
         }
-        E.allocs.push_back(E.d_con);
+        E.allocs.push_back(E.d_conmd);
     }
-    double *d = E.d_con;
+    double *d = E.d_conmd;
     double *dR = d, *dP = dR + n, *dG = dP + n, *dF = dG + n, *dx1 = dF + n, *dx2 = dx1 + n, *dC = dx2 + n,
            *dI = dC + nc, *dE = dI + nd, *dO = dE + nd;
     HostCopies hc(E);

@@ -348,7 +348,7 @@ struct Engine {
     cudaEvent_t ev_check[2] = {nullptr, nullptr};  // the last two iterations the eager loop may look at
     double *d_out = nullptr;  // small device staging for per-bead scalar outputs
     double *d_md = nullptr;   // device MD state for the host-array step (pimd_md_step)
-    double *d_con = nullptr;  // the same for the contracted step (pimd_contracted_step)
+    double *d_conmd = nullptr;  // the same for the contracted step (pimd_contracted_step)
     std::vector<void *> allocs;
     std::string last_error;
     long long nlaunch = 0;  // kernels launched by this context

@@ -28,7 +28,7 @@
 //     stage to the builders;
 //   * 16 builder warps: per 16 sites build X (exy of every run, one item per thread) and Z
 //     (mu_c ez, on the threads without an X item) in the canonical no-swizzle K-major layout,
-//     split into FP16 hi + lo, into one of three buffers;
+//     split into FP16 hi + lo, into one of up to four buffers (X cached: 8 warps a step, in turn);
 //   * MMA warp: one thread issues the MMAs into TMEM and commits to the buffer's mbarrier, which
 //     releases the buffer to the builders.
 // Only mbarriers connect the roles, so building, copying and MMAs overlap. The epilogue reads
@@ -640,7 +640,7 @@ __global__ void __maxnreg__(64) k_sfac_tc(const __grid_constant__ CUtensorMap tm
             umma::tmem_dealloc(tm, 512);
             umma::tmem_relinquish();
         }
-            // cluster: add the partials of all site groups over this CTA's slice (groups in order, in FP32: FP64
+        // cluster: add the partials of all site groups over this CTA's slice (groups in order, in FP32: FP64
         // arithmetic is slow on this part, and the partials carry only the split operands' ~2^-21 anyway)
         cluster_sync();
         const uint32_t pbase = umma::smem_u32(pt);
