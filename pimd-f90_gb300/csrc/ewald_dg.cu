@@ -855,7 +855,8 @@ int dg_init(Engine &E) {
     a.slotk = d_slotk;
     a.slotkv = d_slotkv;
     const int lim = DG_SMEM;
-    if ((size_t)DG_FST * a.ksf * DG_VT > 48 * 1024) {  // |kz| > 63: the field's V ring
+    // the field's V ring; beside a kernel's static words 48 KB (|kz| > 55) are more than a launch gets unasked
+    if ((size_t)DG_FST * a.ksf * DG_VT + 1024 > 48 * 1024) {
         cudaFuncSetAttribute(k_dg_field<DGF_E, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
         cudaFuncSetAttribute(k_dg_field<DGF_E, 0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
         cudaFuncSetAttribute(k_dg_field<DGF_DG, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
