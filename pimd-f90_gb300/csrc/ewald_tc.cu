@@ -1253,6 +1253,38 @@ static bool tp_init(Engine &E, int which, const std::vector<int> &jr, int dmax, 
     return true;
 }
 
+// Which boxes take the tensor-core passes. Their operands hold 22 bits and an accumulator cuts off what is below
+// its last place; the FP32-pipe passes round, and add the sums of a tile in FP64. So the tensor-core passes are the
+// faster ones and not the more accurate ones, and they take the boxes where groups of TC_BOXRUN runs (256 of at
+// most 10 |kz|), the epilogue over them, and for the field the tables of 128 sites (128 rows at most), Q and the rows of 8
+// runs, leave room in a CTA's shared memory: cubes of |n| from 4 to 41 (but 30), up to 85 A at a 9 A cutoff.
+// Smaller groups and the tables in two parts would reach further, but there the FP32 passes stay. RMS error of the
+// gradient and the induced dipoles against the FP64 engine, and a force call (tensor cores; FP32): 512 x 2,
+// |n| <= 45: 1.5e-6 1.9e-5 7.5 ms; 3.5e-7 4.7e-6 19.9 ms. 512 x 8, 25 x 25 x 199 A: 4.7e-7 1.3e-5 19.9 ms; 1.6e-7
+// 3.9e-6 38.6 ms. 8 x 1, |n| <= 30: 1.9e-6 1.7e-6 2.1 ms; 1.3e-6 1.7e-6 4.6 ms.
+constexpr int TC_BOXRUN = 224;
+static bool sfac_box(const KP &kp, const std::vector<int2> &src, const std::vector<int> &jr, const std::vector<KRun> &runs, int dmax,
+                     int band) {
+    int ncol = 16, nkl = 0;
+    const int n = (int)src.size();
+    for (int p0 = 0; p0 < n;) {
+        const int most = std::min(band, jr[src[p0].x] - src[p0].y) <= 10 ? TC_MAXRUN : TC_BOXRUN;
+        int nr = 0, k = 0;
+        for (; p0 + nr < n && nr < most && src[p0 + nr].y == src[p0].y; nr++) k += runs[src[p0 + nr].x].nkz;
+        ncol = std::max(ncol, (2 * nr + 15) / 16 * 16);
+        nkl = std::max(nkl, k);
+        p0 += nr;
+    }
+    int nabuf = TC_NABUF_MAX;
+    while (nabuf > 2 && TcSmem(kp.ntab, ncol, nabuf).total > dmax) nabuf--;
+    const int total = TcSmem(kp.ntab, ncol, nabuf).total;
+    return total <= dmax && 128 * TC_LD * 4 + 8 * nkl <= total - 1024;
+}
+static bool field_box(const KP &kp, int nc) {  // nc: rows of a run pair
+    const int boxb = (kp.ntab * 128 + 1023) / 1024 * 1024, kq = (2 * kp.lmax + 17) / 16 * 16;
+    return kp.ntab <= 128 && 8 * boxb + 4 * TF_SITES * kq + 16 * nc * kq + 1024 <= 220 * 1024;
+}
+
 static void tp_setup(Engine &E, PFN_cuTensorMapEncodeTiled_v12000 enc, const std::vector<int> &jr, std::vector<int4> *place) {
     KP &kp = E.kp;
     int optin = 0;
@@ -1285,7 +1317,7 @@ static void tp_setup(Engine &E, PFN_cuTensorMapEncodeTiled_v12000 enc, const std
                                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return;
     }
-    if (tp_init(E, 0, jr, dmax, place)) tp_init(E, 1, jr, dmax, nullptr);
+    if (field_box(kp, 8) && tp_init(E, 0, jr, dmax, place) && field_box(kp, 12)) tp_init(E, 1, jr, dmax, nullptr);
 }
 
 void tc_init(Engine &E) {
@@ -1329,9 +1361,6 @@ void tc_init(Engine &E) {
         const KRun &a = E.h_runs[x], &c = E.h_runs[y];
         return a.kx == c.kx && a.ky == -c.ky;
     };
-    // the field passes' tables, and where their V has the rows of each run's pair (its offset, to the lo rows, |kz| rows)
-    std::vector<int4> place;
-    tp_setup(E, enc, jr, &place);
     // slots: every run once with its |kz| rows below TC_JB, then the runs reaching beyond once
     // per further band of TC_JB rows (j0 = TC_JB, 2 TC_JB, ...), each band in groups of <= 256
     // slots; a slot's k-vectors outside its group's rows are local entries with k = -1
@@ -1345,6 +1374,21 @@ void tc_init(Engine &E) {
         if (src.size() == n0) break;
     }
     const int nslot = (int)src.size();
+    // dynamic shared memory available: the opt-in limit minus the kernel's static part
+    int optin = 0;
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, E.device);
+    cudaFuncAttributes fa, fq, fd;
+    if (cudaFuncGetAttributes(&fa, k_sfac_tc<TC_OP_MU>) != cudaSuccess ||
+        cudaFuncGetAttributes(&fq, k_sfac_tc<TC_OP_Q>) != cudaSuccess ||
+        cudaFuncGetAttributes(&fd, k_sfac_tc<TC_OP_DIP>) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    const int dmax = optin - (int)std::max(fa.sharedSizeBytes, std::max(fq.sharedSizeBytes, fd.sharedSizeBytes));
+    if (!sfac_box(kp, src, jr, E.h_runs, dmax, TC_JB)) return;
+    // the field passes' tables, and where their V has the rows of each run's pair (its offset, to the lo rows, |kz| rows)
+    std::vector<int4> place;
+    tp_setup(E, enc, jr, &place);
     E.tc_ng224 = 0;
     for (int p0 = 0; p0 < nslot;) {
         int n = 0;
@@ -1360,17 +1404,6 @@ void tc_init(Engine &E) {
     std::vector<float2> runkf(kp.nrun);
     for (int r = 0; r < kp.nrun; r++)
         runkf[r] = make_float2((float)E.h_kvec[3 * E.h_runs[r].kbeg], (float)E.h_kvec[3 * E.h_runs[r].kbeg + 1]);
-    // dynamic shared memory available: the opt-in limit minus the kernel's static part
-    int optin = 0;
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, E.device);
-    cudaFuncAttributes fa, fq, fd;
-    if (cudaFuncGetAttributes(&fa, k_sfac_tc<TC_OP_MU>) != cudaSuccess ||
-        cudaFuncGetAttributes(&fq, k_sfac_tc<TC_OP_Q>) != cudaSuccess ||
-        cudaFuncGetAttributes(&fd, k_sfac_tc<TC_OP_DIP>) != cudaSuccess) {
-        cudaGetLastError();
-        return;
-    }
-    const int dmax = optin - (int)std::max(fa.sharedSizeBytes, std::max(fq.sharedSizeBytes, fd.sharedSizeBytes));
     // groups of at most 256 runs, or of fewer until the operand buffers (four to two) and the epilogue's staging
     // tile and partial S, which reuse the table and operand regions, fit
     int ncolmax = 0, nklmax = 0, nvalid = 0, nabuf = 0;

@@ -1,0 +1,48 @@
+"""Which boxes the mixed engine's tensor-core Ewald passes take (ewald_tc.cu): large k shells and long boxes keep
+the FP32-pipe passes, whose sums round where the tensor cores' cut off.
+
+RMS errors against the FP64 engine. The bounds are twice the FP32 passes' own errors in these boxes (3.5e-7 and 4.7e-6
+for the gradient and the induced dipoles of 512 molecules with |n| <= 45, 1.6e-7 and 3.9e-6 in the long box); the
+tensor-core passes are at 1.5e-6 and 1.9e-5, 4.7e-7 and 1.3e-5 there."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def rms(a, b):
+    return np.sqrt(((a - b) ** 2).mean() / (b ** 2).mean())
+
+
+def params(pkg, nw, P, f, nmax=0):
+    c = pkg.waterbox.make_config("ttm3f_512x32", nw=nw, P=P, seed=5 + nw)
+    L = c["params"]["box"][0]
+    d = c["RRc"][0::3].repeat(3, axis=0) * (np.array(f) - 1.0)  # molecules moved apart, not stretched
+    rc = min(9.0, 0.48 * L)
+    p = dict(c["params"], box=tuple(L * x for x in f), rc=rc, rc1=0.8 * rc, polar_maxiter=60, polar_eps=1e-9)
+    p.update(dict(alpha=2.6 / rc, nmax=nmax) if nmax else dict(alpha=0.0, eps_ewald=1e-7))
+    return p, c["RRt"] + d[None], c["RRc"] + d
+
+
+@pytest.mark.parametrize("nw,P,f,nmax,force,dip", [(512, 2, (1, 1, 1), 45, 7.0e-7, 9.4e-6), (512, 8, (1, 1, 8), 0, 3.2e-7, 7.8e-6)])
+def test_large_shells_keep_fp32_accuracy(pkg, engine_lib, nw, P, f, nmax, force, dip):
+    p, RRt, RRc = params(pkg, nw, P, f, nmax)
+    out = []
+    for prec in (0, 1):
+        eng = pkg.ForceEngine(p, precision=prec)
+        out.append(eng.full_bead_forces(RRt, RRc))
+        if prec:
+            t = eng.tuning()
+            assert t["sf_tc"] == t["ff_tc"] == t["qd_tc"] == 0
+        eng.close()
+    assert rms(out[1]["dRRt"], out[0]["dRRt"]) < force
+    assert rms(out[1]["dip_momEt"], out[0]["dip_momEt"]) < dip
+
+
+@pytest.mark.parametrize("nmax,on", [(3, 0), (4, 1), (29, 1), (30, 0), (31, 1), (41, 1), (42, 0), (60, 0)])
+def test_rule_of_the_boxes(pkg, engine_lib, nmax, on):
+    p = params(pkg, 8, 1, (1, 1, 1), nmax)[0]
+    eng = pkg.ForceEngine(p, precision=1)
+    t = eng.tuning()
+    assert t["sf_tc"] == t["ff_tc"] == on
+    eng.close()
