@@ -301,7 +301,7 @@ struct Engine {
     // tensor-core (tcgen05, 3xTF32) dipole structure factor of the mixed engine (ewald_tc.cu)
     bool sf_tc = true;        // use it when tc_ready
     bool tc_ready = false;    // run groups built and the table tensor map encoded
-    int tc_npt = 3;           // dipole-component partials a k-vector held at a time
+    bool tc_dip_ok = false;   // the dipole-component sums (three partials per k-vector) take them too
     int tc_nsm = 152, tc_ng224 = 1, tc_nband = 0;
     int tc_ntg = 0, tc_ncolmax = 0, tc_nabuf = 0;
     const int4 *d_tcslot = nullptr;   // per run slot: run, local k offset, kzlo, nkz

@@ -113,7 +113,6 @@ struct TcArgs {
     int pdl;              // 1: launched as a programmatic dependent of the previous iteration's field pass; 2: of
                           // the band groups' launch, beside which it runs
     int tg0, ntg;         // the launch's first run group, all of them
-    int npt;              // dipole-component partials held at a time: 3, or 1
     const int4 *vp;       // per pair: group slots of its +ky | -ky << 16 runs (0xffff: none), where its rows of
                           // the field pass's V begin and how far the lo rows are from there (16-byte words), |kz| rows
     uint4 *V;             // [P][vstride] that operand (null: none)
@@ -570,140 +569,135 @@ __global__ void __maxnreg__(64) k_sfac_tc(const __grid_constant__ CUtensorMap tm
     if (OP != TC_OP_DIP && i0 + tid < i1) fetch(i0 + tid, first);
     // epilogue: TMEM -> shared, 64 runs (128 columns) at a time -> partial S of every k of the group
     float *stg = reinterpret_cast<float *>(sm);                       // [128][TC_LD]
-    float2 *pt = reinterpret_cast<float2 *>(sm + 128 * TC_LD * 4);    // [nkl][npt]
-    // (dipole components: one at a time where the three partials of a group's k-vectors do not fit)
-    const int npt = (OP == TC_OP_DIP) ? a.npt : 1;
-    for (int c0 = 0; c0 < NPT; c0 += npt) {
-        for (int ch = 0; ch * TC_CH < nr && !bad; ch++) {
-            if (warp < 16) {
-                const int lq = warp & 3, part = warp >> 2;  // 4 lane quarters x 4 column quarters
-                const int col = ch * 2 * TC_CH + 32 * part;
-                float v[32];
-                float *row = stg + (32 * lq + lane) * TC_LD + 32 * part;
-                const uint32_t t0 = tm + ((uint32_t)(32 * lq) << 16) + (uint32_t)col;
-                if (nsub > 0) {
-                    umma::tmem_ld16x2(t0, t0 + 16, v);
-                } else {
+    float2 *pt = reinterpret_cast<float2 *>(sm + 128 * TC_LD * 4);    // [nkl][NPT]
+    for (int ch = 0; ch * TC_CH < nr && !bad; ch++) {
+        if (warp < 16) {
+            const int lq = warp & 3, part = warp >> 2;  // 4 lane quarters x 4 column quarters
+            const int col = ch * 2 * TC_CH + 32 * part;
+            float v[32];
+            float *row = stg + (32 * lq + lane) * TC_LD + 32 * part;
+            const uint32_t t0 = tm + ((uint32_t)(32 * lq) << 16) + (uint32_t)col;
+            if (nsub > 0) {
+                umma::tmem_ld16x2(t0, t0 + 16, v);
+            } else {
 #pragma unroll
-                    for (int j = 0; j < 32; j++) v[j] = 0.f;
-                }
-#pragma unroll
-                for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4 *>(row + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                for (int j = 0; j < 32; j++) v[j] = 0.f;
             }
-            __syncthreads();
-            for (int i = tid; i < TC_CH * jm; i += TC_NT) {
-                const int q = i % TC_CH, jj = i / TC_CH, p = ch * TC_CH + q, j = G.j0 + jj;  // row jj: |kz| = j
-                if (p >= nr) continue;
-                const int4 sl = sslot[p];  // run, local offset, kzlo, nkz
-                const bool plus = j >= sl.z && j < sl.z + sl.w;
-                const bool minus = j > 0 && -j >= sl.z && -j < sl.z + sl.w;
-                if (!plus && !minus) continue;
-                float2 gp[NCZ], gm[NCZ];
 #pragma unroll
-                for (int c = 0; c < NCZ; c++) {
-                    const int rc = (c * jm + jj) * 2;
-                    // (x, y) = (Re exy, Im exy) against mu_c c_j (row rc) and mu_c s_j (row rc + 1)
-                    const float2 dc = *reinterpret_cast<const float2 *>(stg + rc * TC_LD + 2 * q);
-                    const float2 ds = *reinterpret_cast<const float2 *>(stg + (rc + 1) * TC_LD + 2 * q);
-                    gp[c] = make_float2(dc.x - ds.y, ds.x + dc.y);
-                    gm[c] = make_float2(dc.x + ds.y, dc.y - ds.x);
-                }
-                const float zs = 1.f / TC_ZS;
-                if (OP == TC_OP_MU) {
-                    const float2 kv = make_float2(sskv[p].x * zs, sskv[p].y * zs);
-                    if (plus) {
-                        const float kz = skz[kp.lmax + j] * zs;
-                        pt[sl.y + j - sl.z] = make_float2(fmaf(kz, gp[NCZ - 1].x, fmaf(kv.y, gp[1 % NCZ].x, kv.x * gp[0].x)),
-                                                          fmaf(kz, gp[NCZ - 1].y, fmaf(kv.y, gp[1 % NCZ].y, kv.x * gp[0].y)));
-                    }
-                    if (minus) {
-                        const float kz = skz[kp.lmax - j] * zs;
-                        pt[sl.y - j - sl.z] = make_float2(fmaf(kz, gm[NCZ - 1].x, fmaf(kv.y, gm[1 % NCZ].x, kv.x * gm[0].x)),
-                                                          fmaf(kz, gm[NCZ - 1].y, fmaf(kv.y, gm[1 % NCZ].y, kv.x * gm[0].y)));
-                    }
-                } else {
-                    // charges: S itself; dipole components: the three G_c
-#pragma unroll
-                    for (int c = 0; c < NPT; c++) {
-                        if (c < c0 || c >= c0 + npt) continue;
-                        if (plus) pt[npt * (sl.y + j - sl.z) + c - c0] = make_float2(zs * gp[c].x, zs * gp[c].y);
-                        if (minus) pt[npt * (sl.y - j - sl.z) + c - c0] = make_float2(zs * gm[c].x, zs * gm[c].y);
-                    }
-                }
-            }
-            __syncthreads();
+            for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4 *>(row + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
         }
-        umma::fence_before_sync();
         __syncthreads();
-        if (warp == 0 && c0 + npt >= NPT) {
-            umma::fence_after_sync();
-            umma::tmem_dealloc(tm, 512);
-            umma::tmem_relinquish();
-        }
-        // cluster: add the partials of all site groups over this CTA's slice (groups in order, in FP32: FP64
-        // arithmetic is slow on this part, and the partials carry only the split operands' ~2^-21 anyway)
-        cluster_sync();
-        const uint32_t pbase = umma::smem_u32(pt);
-        auto total = [&](int i) {
-            float2 v[TC_CLMAX];
+        for (int i = tid; i < TC_CH * jm; i += TC_NT) {
+            const int q = i % TC_CH, jj = i / TC_CH, p = ch * TC_CH + q, j = G.j0 + jj;  // row jj: |kz| = j
+            if (p >= nr) continue;
+            const int4 sl = sslot[p];  // run, local offset, kzlo, nkz
+            const bool plus = j >= sl.z && j < sl.z + sl.w;
+            const bool minus = j > 0 && -j >= sl.z && -j < sl.z + sl.w;
+            if (!plus && !minus) continue;
+            float2 gp[NCZ], gm[NCZ];
 #pragma unroll
-            for (int c = 0; c < TC_CLMAX; c++)
-                if (c < cn) v[c] = ld_cluster_f2(pbase + 8u * (uint32_t)i, (uint32_t)c);
-            float sx = 0.f, sy = 0.f;
-#pragma unroll
-            for (int c = 0; c < TC_CLMAX; c++)
-                if (c < cn) {
-                    sx += v[c].x;
-                    sy += v[c].y;
+            for (int c = 0; c < NCZ; c++) {
+                const int rc = (c * jm + jj) * 2;
+                // (x, y) = (Re exy, Im exy) against mu_c c_j (row rc) and mu_c s_j (row rc + 1)
+                const float2 dc = *reinterpret_cast<const float2 *>(stg + rc * TC_LD + 2 * q);
+                const float2 ds = *reinterpret_cast<const float2 *>(stg + (rc + 1) * TC_LD + 2 * q);
+                gp[c] = make_float2(dc.x - ds.y, ds.x + dc.y);
+                gm[c] = make_float2(dc.x + ds.y, dc.y - ds.x);
+            }
+            const float zs = 1.f / TC_ZS;
+            if (OP == TC_OP_MU) {
+                const float2 kv = make_float2(sskv[p].x * zs, sskv[p].y * zs);
+                if (plus) {
+                    const float kz = skz[kp.lmax + j] * zs;
+                    pt[sl.y + j - sl.z] = make_float2(fmaf(kz, gp[NCZ - 1].x, fmaf(kv.y, gp[1 % NCZ].x, kv.x * gp[0].x)),
+                                                      fmaf(kz, gp[NCZ - 1].y, fmaf(kv.y, gp[1 % NCZ].y, kv.x * gp[0].y)));
                 }
-            return make_float2(sx, sy);
-        };
-        if (OP == TC_OP_DIP && !bad) {
-            for (int i = i0 + tid; i < i1; i += TC_NT) {
-                const TcKW kw = a.kw[G.kgoff + i];
-                if (kw.k < 0) continue;  // a k-vector of the run that another (band) group sums
-                for (int e = 0; e < npt; e++) {
-                    const float2 t = total(npt * i + e);
-                    kp.Sdip[((size_t)b * kp.nk + kw.k) * 3 + c0 + e] = make_double2((double)t.x, (double)t.y);
+                if (minus) {
+                    const float kz = skz[kp.lmax - j] * zs;
+                    pt[sl.y - j - sl.z] = make_float2(fmaf(kz, gm[NCZ - 1].x, fmaf(kv.y, gm[1 % NCZ].x, kv.x * gm[0].x)),
+                                                      fmaf(kz, gm[NCZ - 1].y, fmaf(kv.y, gm[1 % NCZ].y, kv.x * gm[0].y)));
+                }
+            } else {
+                // charges: S itself; dipole components: the three G_c
+#pragma unroll
+                for (int c = 0; c < NPT; c++) {
+                    if (plus) pt[NPT * (sl.y + j - sl.z) + c] = make_float2(zs * gp[c].x, zs * gp[c].y);
+                    if (minus) pt[NPT * (sl.y - j - sl.z) + c] = make_float2(zs * gm[c].x, zs * gm[c].y);
                 }
             }
         }
-        // charges and dipoles: Sq = S or Sm = (-Im, Re), the reference's rQm, iQm (ewald.f90:106-107), the FP32
-        // weights 4 pi Ak / V conj(S), and a pair's rows of the field pass's V (k_field_v's job, which took a
-        // launch of 5 us an iteration at 512 x 32)
-        for (int it = i0 + tid; OP != TC_OP_DIP && it < i1 && !bad; it += TC_NT) {
-            Item x = first;
-            if (it != i0 + tid) fetch(it, x);
-            const int j = G.j0 + it % jm;
-            float2 w[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                w[u] = make_float2(0.f, 0.f);
-                const TcKW kw = x.kw[u];
-                if (kw.k < 0) continue;
-                const float2 t = total(local_k(x.vp, j, u));
-                if (OP == TC_OP_MU) {
-                    kp.Sm[(size_t)b * kp.nk + kw.k] = make_double2(-(double)t.y, (double)t.x);
-                    w[u] = make_float2(-kw.w * t.y, -kw.w * t.x);
-                } else {
-                    kp.Sq[(size_t)b * kp.nk + kw.k] = make_double2((double)t.x, (double)t.y);
-                    w[u] = make_float2(kw.w * t.x, -kw.w * t.y);
-                }
-                kp.Wf[((size_t)b * 2 + (OP == TC_OP_MU ? 1 : 0)) * kp.nk + kw.k] = w[u];
-            }
-            if (!a.V || j >= x.vp.w) continue;
-            uint32_t *hi = reinterpret_cast<uint32_t *>(a.V + (size_t)b * a.vstride + x.vp.y) + (j >> 2) * 32 + (j & 3);
-            uint32_t *lo = hi + 4 * x.vp.z;
-            v_rows(w, skz[kp.lmax + j], [&](int r, float c, float sn) {
-                const __half2 h = __floats2half2_rn(c, sn);
-                const float2 hf = __half22float2(h);
-                const __half2 l = __floats2half2_rn(c - hf.x, sn - hf.y);
-                hi[4 * r] = *reinterpret_cast<const uint32_t *>(&h);
-                lo[4 * r] = *reinterpret_cast<const uint32_t *>(&l);
-            });
-        }
-        cluster_sync();  // remote reads done before any CTA of the cluster leaves (or writes the next component)
+        __syncthreads();
     }
+    umma::fence_before_sync();
+    __syncthreads();
+    if (warp == 0) {
+        umma::fence_after_sync();
+        umma::tmem_dealloc(tm, 512);
+        umma::tmem_relinquish();
+    }
+    // cluster: add the partials of all site groups over this CTA's slice (groups in order, in FP32: FP64
+    // arithmetic is slow on this part, and the partials carry only the split operands' ~2^-21 anyway)
+    cluster_sync();
+    const uint32_t pbase = umma::smem_u32(pt);
+    auto total = [&](int i) {
+        float2 v[TC_CLMAX];
+#pragma unroll
+        for (int c = 0; c < TC_CLMAX; c++)
+            if (c < cn) v[c] = ld_cluster_f2(pbase + 8u * (uint32_t)i, (uint32_t)c);
+        float sx = 0.f, sy = 0.f;
+#pragma unroll
+        for (int c = 0; c < TC_CLMAX; c++)
+            if (c < cn) {
+                sx += v[c].x;
+                sy += v[c].y;
+            }
+        return make_float2(sx, sy);
+    };
+    if (OP == TC_OP_DIP && !bad) {
+        for (int i = i0 + tid; i < i1; i += TC_NT) {
+            const TcKW kw = a.kw[G.kgoff + i];
+            if (kw.k < 0) continue;  // a k-vector of the run that another (band) group sums
+            for (int e = 0; e < NPT; e++) {
+                const float2 t = total(NPT * i + e);
+                kp.Sdip[((size_t)b * kp.nk + kw.k) * 3 + e] = make_double2((double)t.x, (double)t.y);
+            }
+        }
+    }
+    // charges and dipoles: Sq = S or Sm = (-Im, Re), the reference's rQm, iQm (ewald.f90:106-107), the FP32
+    // weights 4 pi Ak / V conj(S), and a pair's rows of the field pass's V (k_field_v's job, which took a
+    // launch of 5 us an iteration at 512 x 32)
+    for (int it = i0 + tid; OP != TC_OP_DIP && it < i1 && !bad; it += TC_NT) {
+        Item x = first;
+        if (it != i0 + tid) fetch(it, x);
+        const int j = G.j0 + it % jm;
+        float2 w[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            w[u] = make_float2(0.f, 0.f);
+            const TcKW kw = x.kw[u];
+            if (kw.k < 0) continue;
+            const float2 t = total(local_k(x.vp, j, u));
+            if (OP == TC_OP_MU) {
+                kp.Sm[(size_t)b * kp.nk + kw.k] = make_double2(-(double)t.y, (double)t.x);
+                w[u] = make_float2(-kw.w * t.y, -kw.w * t.x);
+            } else {
+                kp.Sq[(size_t)b * kp.nk + kw.k] = make_double2((double)t.x, (double)t.y);
+                w[u] = make_float2(kw.w * t.x, -kw.w * t.y);
+            }
+            kp.Wf[((size_t)b * 2 + (OP == TC_OP_MU ? 1 : 0)) * kp.nk + kw.k] = w[u];
+        }
+        if (!a.V || j >= x.vp.w) continue;
+        uint32_t *hi = reinterpret_cast<uint32_t *>(a.V + (size_t)b * a.vstride + x.vp.y) + (j >> 2) * 32 + (j & 3);
+        uint32_t *lo = hi + 4 * x.vp.z;
+        v_rows(w, skz[kp.lmax + j], [&](int r, float c, float sn) {
+            const __half2 h = __floats2half2_rn(c, sn);
+            const float2 hf = __half22float2(h);
+            const __half2 l = __floats2half2_rn(c - hf.x, sn - hf.y);
+            hi[4 * r] = *reinterpret_cast<const uint32_t *>(&h);
+            lo[4 * r] = *reinterpret_cast<const uint32_t *>(&l);
+        });
+    }
+    cluster_sync();  // remote reads done before any CTA of the cluster leaves
     if (bad && tid == 0) atomicOr(kp.err, 8u);
     if (a.pdl == 2) pdl_wait();  // this grid's end is the band groups' end too
 }
@@ -1264,7 +1258,7 @@ static bool tp_init(Engine &E, int which, const std::vector<int> &jr, int dmax, 
 // 3.9e-6 38.6 ms. 8 x 1, |n| <= 30: 1.9e-6 1.7e-6 2.1 ms; 1.3e-6 1.7e-6 4.6 ms.
 constexpr int TC_BOXRUN = 224;
 static bool sfac_box(const KP &kp, const std::vector<int2> &src, const std::vector<int> &jr, const std::vector<KRun> &runs, int dmax,
-                     int band) {
+                     int band, int parts) {  // parts: partial sums a k-vector
     int ncol = 16, nkl = 0;
     const int n = (int)src.size();
     for (int p0 = 0; p0 < n;) {
@@ -1278,7 +1272,7 @@ static bool sfac_box(const KP &kp, const std::vector<int2> &src, const std::vect
     int nabuf = TC_NABUF_MAX;
     while (nabuf > 2 && TcSmem(kp.ntab, ncol, nabuf).total > dmax) nabuf--;
     const int total = TcSmem(kp.ntab, ncol, nabuf).total;
-    return total <= dmax && 128 * TC_LD * 4 + 8 * nkl <= total - 1024;
+    return total <= dmax && 128 * TC_LD * 4 + 8 * parts * nkl <= total - 1024;
 }
 static bool field_box(const KP &kp, int nc) {  // nc: rows of a run pair
     const int boxb = (kp.ntab * 128 + 1023) / 1024 * 1024, kq = (2 * kp.lmax + 17) / 16 * 16;
@@ -1385,7 +1379,12 @@ void tc_init(Engine &E) {
         return;
     }
     const int dmax = optin - (int)std::max(fa.sharedSizeBytes, std::max(fq.sharedSizeBytes, fd.sharedSizeBytes));
-    if (!sfac_box(kp, src, jr, E.h_runs, dmax, TC_JB)) return;
+    if (!sfac_box(kp, src, jr, E.h_runs, dmax, TC_JB, 1)) return;
+    // the dipole-component sums of the virial (three partials a k-vector) likewise, cubes of |n| from 5 to 15. One
+    // component after the other would fit the larger ones and take 481 us instead of 2945 at 4096 x 32, but its
+    // sums over all sites of a bead are off by 2.5e-6 (rms, 700 sites) where the FP32 pass is within 4e-7, and the
+    // virial of 4096 x 32 by 6.02e-6 instead of 5.95e-6
+    E.tc_dip_ok = sfac_box(kp, src, jr, E.h_runs, dmax, TC_JB, 3);
     // the field passes' tables, and where their V has the rows of each run's pair (its offset, to the lo rows, |kz| rows)
     std::vector<int4> place;
     tp_setup(E, enc, jr, &place);
@@ -1454,7 +1453,7 @@ void tc_init(Engine &E) {
         nabuf = TC_NABUF_MAX;
         while (nabuf > 2 && TcSmem(kp.ntab, ncolmax, nabuf).total > dmax) nabuf--;
         const int total = TcSmem(kp.ntab, ncolmax, nabuf).total;
-        return total <= dmax && 128 * TC_LD * 4 + 8 * nklmax <= total - 1024;
+        return total <= dmax && 128 * TC_LD * 4 + 8 * (E.tc_dip_ok ? 3 : 1) * nklmax <= total - 1024;
     };
     int maxrun = TC_MAXRUN;
     while (maxrun >= 32 && !build(maxrun)) maxrun -= 32;
@@ -1467,8 +1466,6 @@ void tc_init(Engine &E) {
         cudaGetLastError();
         return;
     }
-    // the component sums keep three partials per k-vector, or one at a time
-    E.tc_npt = 128 * TC_LD * 4 + 3 * 8 * nklmax <= L.total - 1024 ? 3 : 1;
     int4 *d_slots = nullptr;
     float2 *d_skv = nullptr;
     TcGroup *d_groups = nullptr;
@@ -1649,7 +1646,7 @@ int launch_field_qd_tc(Engine &E, int s0, int s1) {
 // Returns 1 when the launch wrote the structure factor of `op` (Sq and the charge weights, Sm
 // and the dipole weights, or Sdip; no k_sreduce needed), else 0.
 int launch_sfac_tc(Engine &E, int op, int s0, int nsites, int skipconv) {
-    if (!E.tc_ready || !E.sf_tc || nsites <= 0) return 0;
+    if (!E.tc_ready || !E.sf_tc || nsites <= 0 || (op == TC_OP_DIP && !E.tc_dip_ok)) return 0;
     const KP &kp = E.kp;
     TcArgs a;
     a.slot = E.d_tcslot;
@@ -1669,7 +1666,6 @@ int launch_sfac_tc(Engine &E, int op, int s0, int nsites, int skipconv) {
     a.xsub = E.tc_xsub;
     a.xblock = E.tc_xblock;
     a.xkeep = E.l2_keep ? 1 : 0;
-    a.npt = E.tc_npt;
     a.vp = E.d_tcvp;
     a.V = reinterpret_cast<uint4 *>(E.tp[0].V);
     a.vstride = E.tp[0].vstride;

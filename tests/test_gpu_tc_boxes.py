@@ -46,3 +46,30 @@ def test_rule_of_the_boxes(pkg, engine_lib, nmax, on):
     t = eng.tuning()
     assert t["sf_tc"] == t["ff_tc"] == on
     eng.close()
+
+
+@pytest.mark.parametrize("nw,P,nmax", [(700, 32, 17), (300, 40, 20)])
+def test_virial_sums_of_large_shells(pkg, engine_lib, nw, P, nmax):
+    """The dipole-component sums sum_s mu_c e^{ik.r} of the reciprocal virial, one site group a bead, where three partials a
+    k-vector do not fit the tensor-core pass: against 64 bits, from the FP32 dipoles that the pass takes. An entry of
+    the FP32 tables and each of a term's three products is good to 2^-24 and a tile's 32 terms add in FP32, the tiles in
+    FP64: about 3 x 2^-24 of the sum, rms; 4e-7 allowed (an accumulator that cuts off has 1e-6 and more)."""
+    import torch
+
+    import ctx_probe
+
+    p, RRt, RRc = params(pkg, nw, P, (1, 1, 1), nmax)
+    eng = pkg.ForceEngine(p, precision=1)
+    eng.full_bead_forces(RRt, RRc)
+    assert eng.tuning()["sf_tc"] == 1
+    S = nw * 4
+    pos = ctx_probe.array(pkg, eng, "pos").reshape(P, S, 4)[:, 3 * nw:, :3]
+    mu = ctx_probe.array(pkg, eng, "dipf", np.float32).reshape(P, S, 4)[:, 3 * nw:, :3].astype(np.float64)
+    got = ctx_probe.array(pkg, eng, "Sdip").reshape(P, -1, 3, 2)
+    k = torch.from_numpy(ctx_probe.array(pkg, eng, "kinfo").reshape(-1, 4)[:, :3].copy()).cuda()
+    eng.close()
+    for b in (0, P - 1):
+        ph = k @ torch.from_numpy(pos[b].copy()).cuda().T
+        m = torch.from_numpy(mu[b]).cuda()
+        ref = torch.stack([torch.cos(ph) @ m, torch.sin(ph) @ m], -1).cpu().numpy()
+        assert rms(got[b], ref) < 4e-7
