@@ -318,7 +318,8 @@ __global__ void __launch_bounds__(128) k_dm_real(KP kp, DmArgs a) {
 }
 
 // The same on the mixed engine, from the full lists (a warp a molecule's row): the smeared tensor as the
-// iterations' gather forms it (k_dd_real_m with OTF)
+// iterations' gather forms it (k_dd_real_m with OTF). TTM2.1-F's intramolecular tensors stay out of D: their field is
+// taken in FP64 (k_dm_solve), as the gather takes it.
 template <int MODEL>
 __global__ void __launch_bounds__(128) k_dm_real_m(KP kp, DmArgs a) {
     using T = TT<MODEL>;
@@ -374,15 +375,6 @@ __global__ void __launch_bounds__(128) k_dm_real_m(KP kp, DmArgs a) {
                 add((isp - 1) * N + i, (jsp - 1) * N + j, R, t1, 3.f * t2);
             }
     }
-    if (lane < 3) {
-        const double *Tt = kp.Tself + ((size_t)b * N + i) * 18 + 6 * lane;
-        const int s = (lane == 2 ? N : 0) + i, t = (lane == 0 ? N : 2 * N) + i;
-#pragma unroll
-        for (int c = 0; c < 6; c++) {
-            M[((size_t)s * 6 + c) * a.ndp + t] += (float)Tt[c];
-            M[((size_t)t * 6 + c) * a.ndp + s] += (float)Tt[c];
-        }
-    }
 }
 
 // ---- the iterations ------------------------------------------------------------------------------
@@ -423,6 +415,9 @@ PIMD_D long long dm_warp_sum4(long long (&x)[4]) {
 // lo lo: below 2^-52 of the row's largest term, where FP64 sums have 2^-53 of each partial sum, and
 // 20 cycles a product instead of 64. Bound by latency: 3.9 us an iteration of 128 sites in a cluster
 // of 16 CTAs (6.0 with FP64 products).
+// On the mixed engine TTM2.1-F's intramolecular field, the largest of a site's fields, is added by the updating
+// threads from the FP64 tensors and dipoles (six products a component, the dipoles kept a second time in FP64: the
+// same time at 60 x 8, 409 us a call).
 constexpr int DM_MAXROWS = 42;  // of a CTA: their components are four warps' lanes
 template <typename R>
 __global__ void __launch_bounds__(DM_NT) k_dm_solve(KP kp, DmArgs a, int rows) {
@@ -437,13 +432,18 @@ __global__ void __launch_bounds__(DM_NT) k_dm_solve(KP kp, DmArgs a, int rows) {
     int *top = reinterpret_cast<int *>(sums + 128);    // [2][32] their largest dipole component's high word
     int *rexp = top + 64;                              // [44] the rows' scales
     double *ef = reinterpret_cast<double *>(rexp + 44);  // [3 rows + 1] field
-    R *mu = reinterpret_cast<R *>(ef + 3 * rows + (rows & 1));  // [2][3][ndp]
+    const bool intra = !D && kp.model == 2;
+    double *md = ef + 3 * rows + (rows & 1);            // [2][3][ndp] intra: the dipoles in FP64
+    R *mu = reinterpret_cast<R *>(md + (intra ? 6 * ndp : 0));  // [2][3][ndp]
     W *mf = reinterpret_cast<W *>(mu + 6 * ndp);       // [3][ndp] FP64 engine: the dipoles in fixed point
     W *Ms = mf + (D ? 3 * ndp : 0);                    // [rows][6][ndp]
     const R *M = reinterpret_cast<const R *>(a.M) + ((size_t)b * nd + s0) * 6 * ndp;
     const double *dip = kp.dip + 3 * ((size_t)b * kp.S + kp.fd);
     int mt = 0;  // largest dipole component of the bead (high word)
-    for (int i = threadIdx.x; i < 3 * nd; i += DM_NT) mu[(i % 3) * ndp + i / 3] = (R)dip[i];
+    for (int i = threadIdx.x; i < 3 * nd; i += DM_NT) {
+        mu[(i % 3) * ndp + i / 3] = (R)dip[i];
+        if (intra) md[(i % 3) * ndp + i / 3] = dip[i];
+    }
     if constexpr (D) {
         for (int i = lane; i < 3 * nd; i += 32) mt = max(mt, dg_hi(dip[i]));
         mt = __reduce_max_sync(0xffffffffu, mt);
@@ -469,6 +469,20 @@ __global__ void __launch_bounds__(DM_NT) k_dm_solve(KP kp, DmArgs a, int rows) {
         mine = dip[3 * (s0 + ur) + uc];
         eq = reinterpret_cast<const double *>(kp.F + (size_t)b * kp.S + s)[uc];
         pol = kp.polar_sor * kp.polar[s / kp.N + 1];
+    }
+    // intra: the rows of the tensors to the molecule's other two sites (pairs O H1, O H2, H1 H2 of Tself)
+    double tr[2][3] = {{0, 0, 0}, {0, 0, 0}};
+    int other[2] = {0, 0};
+    if (intra && upd) {
+        const int k = (s0 + ur) / kp.N, w = s0 + ur - k * kp.N;
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int j = i + (i >= k);
+            const double *T = kp.Tself + ((size_t)b * kp.N + w) * 18 + 6 * (k + j - 1);
+            other[i] = j * kp.N + w;
+#pragma unroll
+            for (int c = 0; c < 3; c++) tr[i][c] = T[c == uc ? c : c + uc + 2];  // xx yy zz xy xz yz
+        }
     }
     umma::cluster_barrier();  // every CTA has started; this CTA's shared memory is filled
     int it = 0, em = D ? dg_exp(mt) : 0;
@@ -528,7 +542,13 @@ __global__ void __launch_bounds__(DM_NT) k_dm_solve(KP kp, DmArgs a, int rows) {
             double av[2] = {0.0, 0.0};
             int m = 0;
             if (upd) {
-                const double efd = ef[threadIdx.x] + eq + kp.factor * mine;
+                double f = ef[threadIdx.x];
+                if (intra) {
+                    const double *m = md + ((it - 1) & 1) * 3 * ndp;
+#pragma unroll
+                    for (int i = 0; i < 2; i++) f += tr[i][0] * m[other[i]] + tr[i][1] * m[ndp + other[i]] + tr[i][2] * m[2 * ndp + other[i]];
+                }
+                const double efd = f + eq + kp.factor * mine;
                 const double mn = (1.0 - kp.polar_sor) * mine + pol * efd;
                 const double d = it == 1 ? mn : mn - mine;
                 av[0] = d * d;
@@ -537,7 +557,10 @@ __global__ void __launch_bounds__(DM_NT) k_dm_solve(KP kp, DmArgs a, int rows) {
                 mine = mn;
                 m = dg_hi(mn);
                 const R v = (R)mn;
-                for (uint32_t k = 0; k < C; k++) dm_put(nxt + uc * ndp + s0 + ur, k, v);
+                for (uint32_t k = 0; k < C; k++) {
+                    dm_put(nxt + uc * ndp + s0 + ur, k, v);
+                    if (intra) dm_put(md + (it & 1) * 3 * ndp + uc * ndp + s0 + ur, k, mn);
+                }
             }
             int at;
             const double v = warp_sums<2>(av, at);  // lanes 0 and 16
@@ -592,9 +615,9 @@ __global__ void __launch_bounds__(DM_NT) k_dm_solve(KP kp, DmArgs a, int rows) {
 }
 
 // ---- host ----------------------------------------------------------------------------------------
-static size_t solve_smem(const DmArgs &a, int rows, size_t rs) {
-    const size_t row = (size_t)a.ndp * rs;
-    return 128 * 8 + (64 + 44) * 4 + 8 * (size_t)(3 * rows + (rows & 1)) + row * (6 + (rs == 8 ? 3 : 0) + 6 * (size_t)rows);
+static size_t solve_smem(const DmArgs &a, int rows, size_t rs, int model) {
+    const size_t row = (size_t)a.ndp * rs, intra = rs == 4 && model == 2 ? 48 * (size_t)a.ndp : 0;
+    return 128 * 8 + (64 + 44) * 4 + 8 * (size_t)(3 * rows + (rows & 1)) + intra + row * (6 + (rs == 8 ? 3 : 0) + 6 * (size_t)rows);
 }
 
 template <typename R, int NQ>
@@ -655,7 +678,7 @@ void launch_dm_solve(Engine &E) {
     cudaLaunchConfig_t c = {};
     c.gridDim = dim3(C * kp.P);
     c.blockDim = dim3(DM_NT);
-    c.dynamicSmemBytes = solve_smem(a, rows, mixed ? 4 : 8);
+    c.dynamicSmemBytes = solve_smem(a, rows, mixed ? 4 : 8, kp.model);
     c.stream = E.stream;
     cudaLaunchAttribute at = {};
     at.id = cudaLaunchAttributeClusterDimension;
@@ -694,7 +717,7 @@ int dm_init(Engine &E) {
     a.ndp = (a.nd + 3) & ~3;
     const size_t rs = mixed ? 4 : 8;
     const size_t lim = (size_t)226 * 1024;  // (beside the static words)
-    if ((a.nd + 7) / 8 > DM_MAXROWS || solve_smem(a, (a.nd + 7) / 8, rs) > lim) return 0;
+    if ((a.nd + 7) / 8 > DM_MAXROWS || solve_smem(a, (a.nd + 7) / 8, rs, kp.model) > lim) return 0;
     for (int c = 0; c < 3; c++) a.gk[c] = TWOPI * kp.boxi[c];
     a.nqmax = (kp.lmax + 4) / 4;
     const int JM = 4 * a.nqmax;
@@ -820,7 +843,7 @@ int dm_init(Engine &E) {
         cudaLaunchConfig_t c = {};
         c.gridDim = dim3(16);
         c.blockDim = dim3(DM_NT);
-        c.dynamicSmemBytes = solve_smem(a, (a.nd + 15) / 16, rs);
+        c.dynamicSmemBytes = solve_smem(a, (a.nd + 15) / 16, rs, kp.model);
         cudaLaunchAttribute at = {};
         at.id = cudaLaunchAttributeClusterDimension;
         at.val.clusterDim.x = 16;
