@@ -35,6 +35,11 @@ PIMD_D double dg_double(long long t, int e) {
     const unsigned long long r = ((unsigned long long)(E - 1) << 52) + (u >> 11) + ((u >> 10) & 1ULL);
     return __longlong_as_double((long long)(neg ? r | 0x8000000000000000ULL : r));
 }
+// (t + lo 2^-w) 2^e rounded to nearest, |t| <= 2^62, |lo| < 2^(w + 1): to 62 bits first where those do not hold it
+PIMD_D double dg_double(long long t, int lo, int w, int e) {
+    const int m = min(w, max(0, __clzll(t < 0 ? -t : t) - 2)), r = w - m;
+    return dg_double(t * (1LL << m) + ((lo + ((1 << r) >> 1)) >> r), e - m);
+}
 
 // ---- products of fixed-point numbers -----------------------------------------------------------
 // A number in [-1, 1] as 2^62 x = hi 2^32 + lo with both halves signed, so that a product needs no

@@ -17,9 +17,11 @@
 // 6 digits of 9 bits for the field (2^-53 of the largest weight of the run). Products of digits
 // and their sums stay below 2^24, so the FP32 accumulators are exact: |digit| <= 2^(b-1), and one
 // accumulator takes at most 7 products x 128 sites x 2^14, resp. 6 x 32 x 2^16. The digit products
-// of equal weight are added in one accumulator, the accumulators are joined in 64-bit integers
-// (exact), and the sum is rounded to FP64 once. Left out are the products below the last digit
-// (weight 2^-56, resp. 2^-54): the result is nearer to the exact sum than FP64 additions in any
+// of equal weight are added in one accumulator and the accumulators are joined in integers. For the
+// structure factor that is exact for any number of sites (64 bits and a word for what they shift
+// out above 128 sites), and the sum is rounded to FP64 once; a T of the field is cut to 2^-56 of the
+// run's largest weight (2^-53 with more than 32 harmonics). Left out are the products below the last
+// digit (weight 2^-56, resp. 2^-54): the result is nearer to the exact sum than FP64 additions in any
 // order, and it does not depend on the order of the sums.
 //
 // Measured (GB300, TTM3-F 512 x 32, |n| <= 12; FP64 passes -> this): structure factor of an iteration
@@ -394,13 +396,16 @@ __global__ void __launch_bounds__(32 * DG_SW) k_dg_sfac(KP kp, DgArgs a, int nks
         if (threadIdx.x == 0)
             for (int k = 0; k < min(DG_ST - 1, nks); k++) load(k, it + k);
         const int mt = m0 + wp;
+        // the sums so far in units of 2^(ze - 54 + ksum), and what is below (unsigned, units of 2^(ze - 62))
         long long t[2][4];
+        unsigned low[2][4];
         float d[2][DG_SN][4];
 #pragma unroll
         for (int n = 0; n < 2; n++)
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 t[n][i] = 0;
+                low[n][i] = 0;
 #pragma unroll
                 for (int s = 0; s < DG_SN; s++) d[n][s][i] = 0.f;
             }
@@ -439,10 +444,14 @@ __global__ void __launch_bounds__(32 * DG_SW) k_dg_sfac(KP kp, DgArgs a, int nks
                 for (int n = 0; n < 2; n++)
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
-                        // sum_d D_d 2^(40 - 8 d): z x = t 2^(ze - 54)
+                        // sum_d D_d 2^(48 - 8 d) of z x 2^(62 - ze), exactly: the upper part to t, the rest to low
                         const long long hi = (dg_i64(d[n][0][i]) << 16) + (dg_i64(d[n][1][i]) << 8) + dg_i64(d[n][2][i]);
                         const long long lo = (dg_i64(d[n][3][i]) << 16) + (dg_i64(d[n][4][i]) << 8) + dg_i64(d[n][5][i]);
-                        t[n][i] += ((hi << 24) + lo + (dg_i64(d[n][6][i]) >> 8)) >> ksum;
+                        const int d6 = __float2int_rn(d[n][6][i]);
+                        const long long v = (hi << 24) + lo + (d6 >> 8);
+                        low[n][i] += (((unsigned)v & ((1u << ksum) - 1u)) << 8) + ((unsigned)d6 & 255u);
+                        t[n][i] += (v >> ksum) + (low[n][i] >> (8 + ksum));
+                        low[n][i] &= (1u << (8 + ksum)) - 1u;
 #pragma unroll
                         for (int s = 0; s < DG_SN; s++) d[n][s][i] = 0.f;
                     }
@@ -453,12 +462,13 @@ __global__ void __launch_bounds__(32 * DG_SW) k_dg_sfac(KP kp, DgArgs a, int nks
         // e^{ik.r} = exy (cos +- i sin): S(+j) = (cc - ss) + i (sc' + cs'), S(-j) with the signs of sin turned
         const int item = 8 * mt + g;
         if (item < nitem) {
-            const int e = ze - 54 + ksum;
+            const int e = ze - 54 + ksum, wd = 8 + ksum;
 #pragma unroll
             for (int n = 0; n < 2; n++) {
                 double2 *o = sb + ((size_t)(4 * n + q) * nitem + item) * 2;
-                o[0] = make_double2(dg_double(t[n][0] - t[n][3], e), dg_double(t[n][1] + t[n][2], e));
-                o[1] = make_double2(dg_double(t[n][0] + t[n][3], e), dg_double(t[n][1] - t[n][2], e));
+                const int l[4] = {(int)low[n][0], (int)low[n][1], (int)low[n][2], (int)low[n][3]};
+                o[0] = make_double2(dg_double(t[n][0] - t[n][3], l[0] - l[3], wd, e), dg_double(t[n][1] + t[n][2], l[1] + l[2], wd, e));
+                o[1] = make_double2(dg_double(t[n][0] + t[n][3], l[0] + l[3], wd, e), dg_double(t[n][1] - t[n][2], l[1] - l[2], wd, e));
             }
         }
     }
