@@ -409,11 +409,13 @@ PIMD_D long long dm_warp_sum4(long long (&x)[4]) {
 // dipoles (a thread a component) and puts them and its sums into every CTA's shared memory; one
 // cluster barrier an iteration (two sets of dipoles and sums in turn). The CTAs add the same sums
 // in the same order, so they stop together.
-// On the FP64 engine the products are in fixed point: the row's entries at 2^52 of its largest, the
-// dipoles at 2^54 of the bead's largest (known with the sums), exact 64-bit sums of up to 2^9.5 terms
-// (2^(20 + 22 + 9.5) of the high halves, 2^(22 + 31 + 9.5) of the mixed ones) and the high half of
-// lo lo: below 2^-52 of the row's largest term, where FP64 sums have 2^-53 of each partial sum, and
-// 20 cycles a product instead of 64. Bound by latency: 3.9 us an iteration of 128 sites in a cluster
+// On the FP64 engine the products are in fixed point: the row's entries at 2^58 of its largest, the
+// dipoles at 2^58 of the bead's largest (known with the sums), exact 64-bit sums of the high halves'
+// products (2^(26 + 26) each, 552 at most) and of the mixed ones with the high half of lo lo (2^(26 + 31)
+// each, 36 a lane), joined once a row: 2^-59 of the row's largest entry or of the largest dipole in a
+// term, below the rounding of FP64 sums (rms error of an iteration's dipoles at 128 sites 7e-17 of them;
+// 1.4e-16 with FP64 sums, 2.9e-16 with 2^52 and 2^54 and each lane's sum rounded, which is 0.2 us
+// shorter), and 20 cycles a product instead of 64. Bound by latency: 4.1 us an iteration of 128 sites in a cluster
 // of 16 CTAs (6.0 with FP64 products).
 // On the mixed engine TTM2.1-F's intramolecular field, the largest of a site's fields, is added by the updating
 // threads from the FP64 tensors and dipoles (six products a component, the dipoles kept a second time in FP64: the
@@ -455,7 +457,7 @@ __global__ void __launch_bounds__(DM_NT) k_dm_solve(KP kp, DmArgs a, int rows) {
             if (lane == 0) rexp[r] = e;
             for (int c = 0; c < 6; c++)
                 for (int t = lane; t < nd; t += 32)
-                    Ms[((size_t)r * 6 + c) * ndp + t] = e == DG_BAD ? make_int2(0, 0) : dg_split(dg_fix(M[((size_t)r * 6 + c) * ndp + t], 52 - e));
+                    Ms[((size_t)r * 6 + c) * ndp + t] = e == DG_BAD ? make_int2(0, 0) : dg_split(dg_fix(M[((size_t)r * 6 + c) * ndp + t], 58 - e));
         }
     } else {
         for (int i = threadIdx.x; i < nr * 6 * ndp / 4; i += DM_NT) reinterpret_cast<uint4 *>(Ms)[i] = reinterpret_cast<const uint4 *>(M)[i];
@@ -492,7 +494,7 @@ __global__ void __launch_bounds__(DM_NT) k_dm_solve(KP kp, DmArgs a, int rows) {
         R *nxt = mu + (size_t)(it & 1) * 3 * ndp;
         if constexpr (D) {
             for (int i = threadIdx.x; i < 3 * ndp; i += DM_NT)
-                mf[i] = i % ndp < nd && em != DG_BAD ? dg_split(dg_fix(cur[i], 54 - em)) : make_int2(0, 0);
+                mf[i] = i % ndp < nd && em != DG_BAD ? dg_split(dg_fix(cur[i], 58 - em)) : make_int2(0, 0);
             __syncthreads();
         }
         for (int r = wp; r < nr; r += DM_NT / 32) {
@@ -514,13 +516,14 @@ __global__ void __launch_bounds__(DM_NT) k_dm_solve(KP kp, DmArgs a, int rows) {
                     dm_mac_lo(e[2], yz, y);
                     dm_mac_lo(e[2], zz, z);
                 }
-                long long v[4] = {0, 0, 0, 0};
+                long long h[4] = {e[0].h, e[1].h, e[2].h, 0}, m8[4] = {0, 0, 0, 0};
 #pragma unroll
-                for (int c = 0; c < 3; c++) v[c] = (e[c].h << 10) + ((e[c].m + (1LL << 21)) >> 22);  // 2^(52 + 54 - 54)
-                const long long sum = dm_warp_sum4(v);
+                for (int c = 0; c < 3; c++) m8[c] = (e[c].m + 128) >> 8;
+                const long long H = dm_warp_sum4(h), L = dm_warp_sum4(m8);  // 2^-52 and 2^-76 of 2^(er + em)
                 const int er = rexp[r], c = lane >> 3;
                 if ((lane & 7) == 0 && c < 3)
-                    ef[3 * r + c] = er == DG_BAD || em == DG_BAD ? __longlong_as_double(0x7ff8000000000000LL) : dg_double(sum, er + em - 52);
+                    ef[3 * r + c] = er == DG_BAD || em == DG_BAD ? __longlong_as_double(0x7ff8000000000000LL)
+                                                                 : dg_double(H + (L >> 24), (int)(L & 0xffffff), 24, er + em - 52);
             } else {
                 float e[3] = {0.f, 0.f, 0.f};
                 for (int t = lane; t < nd; t += 32) {
