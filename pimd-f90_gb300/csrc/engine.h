@@ -222,16 +222,20 @@ inline void kp_float_tables(KP &kp) {
     }
 }
 
-// acc[ACC_CONV] != 0.0 (bead b's dipoles converged) tested on the bits, without an FP64 compare
+// acc[ACC_CONV] != 0.0 (bead b's dipoles converged) tested on the bits, without an FP64 compare, and the dipole
+// iterations done. Both are read from L2: the iterations' kernels are launched as programmatic dependents, and one that
+// reads them before its griddepcontrol.wait, or without one, must not meet an older line in its SM's cache (the
+// writer, the last field pass, has ended by then).
 PIMD_D bool bead_converged(const KP &kp, int b) {
-    const unsigned long long u = reinterpret_cast<const unsigned long long *>(kp.acc)[(size_t)b * NACC + ACC_CONV];
+    const unsigned long long u = __ldcg(reinterpret_cast<const unsigned long long *>(kp.acc) + (size_t)b * NACC + ACC_CONV);
     return (u & 0x7fffffffffffffffULL) != 0ULL;
 }
+PIMD_D int dd_done(const KP &kp) { return __ldcg(kp.dstep + 1); }
 
 // The FP32 dipoles an iteration reads and the buffer its SOR update writes: the same buffer
 // unless the real-space field runs asynchronously (then iteration d + 1 reads buffer d & 1).
-PIMD_D const float4 *dipf_cur(const KP &kp) { return (kp.dd_async && (kp.dstep[1] & 1)) ? kp.dipf_alt : kp.dipf; }
-PIMD_D float4 *dipf_next(const KP &kp) { return (kp.dd_async && !(kp.dstep[1] & 1)) ? kp.dipf_alt : kp.dipf; }
+PIMD_D const float4 *dipf_cur(const KP &kp) { return (kp.dd_async && (dd_done(kp) & 1)) ? kp.dipf_alt : kp.dipf; }
+PIMD_D float4 *dipf_next(const KP &kp) { return (kp.dd_async && !(dd_done(kp) & 1)) ? kp.dipf_alt : kp.dipf; }
 // the FP32 dipole of dipole site s of bead b into the molecule record (TTM3-F: s = fd + i)
 PIMD_D void mrec_dipole(const KP &kp, int b, int s, float4 m) {
     if (kp.mrec && s >= kp.fd && s < kp.ld) kp.mrec[2 * ((size_t)b * kp.N + (s - kp.fd)) + 1] = m;

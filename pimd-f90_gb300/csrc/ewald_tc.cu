@@ -261,7 +261,11 @@ __global__ void __maxnreg__(64) k_sfac_tc(const __grid_constant__ CUtensorMap tm
     // a programmatic launch starts under the previous field pass: the convergence flags, the
     // dipoles and the weights are that grid's output
     if (a.pdl == 1) pdl_wait();
-    // the whole cluster (same bead) leaves together
+    // Beside the band groups' launch (pdl 2) the previous field pass is the launch before the one that this grid
+    // depends on: it has ended, since every CTA of the band groups waited for it before it let this grid start, but
+    // nothing has made its writes visible to this grid's cached loads. What it wrote and this kernel reads (the
+    // convergence flag, the iteration count, the dipoles by bulk copies) is read from L2. The whole cluster (same
+    // bead) leaves together.
     if (a.skipconv && bead_converged(kp, b)) {
         if (a.pdl == 2) pdl_wait();
         return;
@@ -291,7 +295,7 @@ __global__ void __maxnreg__(64) k_sfac_tc(const __grid_constant__ CUtensorMap tm
     // builds and stores it (xm 1), later ones load it by bulk copies (xm 2) and build only Z.
     // A block holds the X rows [0, 2 nr) rounded to 8-row groups, hi then lo, in the operand
     // layout; the cache is zeroed once, so the rows past 2 nr stay zero.
-    const int xm = (OP == TC_OP_MU && a.xcache) ? (kp.dstep[1] == 0 ? 1 : 2) : 0;
+    const int xm = (OP == TC_OP_MU && a.xcache) ? (dd_done(kp) == 0 ? 1 : 2) : 0;
     const int xbytes = ((2 * nr + 7) / 8) * 256;
     uint4 *xc = xm ? a.xcache + ((size_t)(b * a.ntg + tg) * a.xsub + (g0 - a.sbase) / TC_KS) * (a.xblock / 16)
                    : nullptr;
@@ -304,6 +308,7 @@ __global__ void __maxnreg__(64) k_sfac_tc(const __grid_constant__ CUtensorMap tm
     if (warp == 0) umma::tmem_alloc(&tslot, 512);
     // table stage ts of this group: TMA boxes of the tables and a bulk copy of the dipoles
     const uint32_t box_tx = (uint32_t)(kp.ntab * 128);
+    const float4 *const wsrc = (OP == TC_OP_Q) ? kp.posf : dipf_cur(kp);  // (offset, q) or (mu, 0)
     auto issue_stage = [&](int ts) {
         const int sfirst = g0 + ts * TC_SS, tb = ts % TC_NST;
         unsigned char *dst = sm + tb * L.stage;
@@ -312,7 +317,6 @@ __global__ void __maxnreg__(64) k_sfac_tc(const __grid_constant__ CUtensorMap tm
         mbar_expect_tx(&tfull[tb], 2 * box_tx + mub);
         tma_load_2d(dst, &tmap, 2 * sfirst, b * kp.ntab, &tfull[tb]);
         tma_load_2d(dst + L.boxb, &tmap, 2 * sfirst + 32, b * kp.ntab, &tfull[tb]);
-        const float4 *wsrc = (OP == TC_OP_Q) ? kp.posf : dipf_cur(kp);  // (offset, q) or (mu, 0)
         bulk_load(dst + L.mu, wsrc + (size_t)b * kp.S + sfirst, mub, &tfull[tb]);
     };
     if (tid == 0) {
@@ -936,7 +940,7 @@ __global__ void __launch_bounds__(TP_NT, 1)
         }
     }
     if (warp == 0) umma::tmem_alloc(&tslot, 512);
-    const int iter = kp.dstep[1] + 1;
+    const int iter = dd_done(kp) + 1;
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
