@@ -317,12 +317,12 @@ int pimd_autotune(pimd_ctx *ctx, const double *RRt, const double *RRc);
  * register-row field kernels, max k-slices, one-launch neighbour lists] and, when n >= 6,
  * [wave-quantised split counts], when n >= 7 [tensor-core (tcgen05) dipole structure factor
  * in use], when n >= 8 [tensor-core dipole field pass in use], when n >= 9 [real-space dipole
- * field on a second stream beside the structure factor (mixed engine)], when n >= 10 [the
- * dipole iterations' structure factor reuses its position-only operand from the first
- * iteration], when n >= 11 [the iterations' field pass is a programmatic dependent launch of
+ * field on a second stream beside the structure factor], when n >= 10 [the dipole iterations'
+ * structure factor reuses its position-only operand from the first iteration], when n >= 11 [the iterations' field pass is a programmatic dependent launch of
  * the structure factor (its set-up overlaps that grid's end)], when n >= 12 [dipole iterations
  * per body of the CUDA graph's conditional loop, 1-4], when n >= 13 [the reciprocal charge and
- * force passes on a second stream beside the pair kernels (mixed engine)], when n >= 14
+ * force passes on a second stream beside the pair kernels, and the backward's real-space part
+ * beside its reciprocal passes], when n >= 14
  * [real-space dipole tensors formed inside each iteration rather than cached per list entry
  * (mixed engine)], when n >= 15 [tensor-core force pass in use (follows the field-pass knob;
  * reported only)], when n >= 16 [the iterations' cached operands loaded evict-last in L2], when

@@ -1360,11 +1360,11 @@ int pimd_get_tuning(pimd_ctx *ctx, int *k, int n) {
     if (n >= 6) k[5] = E.wave_shapes;
     if (n >= 7) k[6] = E.sf_tc && E.tc_ready;
     if (n >= 8) k[7] = E.ff_tc && E.tf_ready;
-    if (n >= 9) k[8] = E.dd_overlap && E.loop_aux != nullptr && E.precision == PIMD_MIXED;
+    if (n >= 9) k[8] = E.dd_overlap && E.loop_aux != nullptr;
     if (n >= 10) k[9] = E.tc_xcache && E.d_tcx != nullptr && E.sf_tc && E.tc_ready;
     if (n >= 11) k[10] = E.tc_pdl && E.ff_tc && E.tf_ready && E.sf_tc && E.tc_ready;
     if (n >= 12) k[11] = E.loop_unroll;
-    if (n >= 13) k[12] = E.ewald_overlap && E.aux_stream != nullptr && E.kp.Fx != nullptr;
+    if (n >= 13) k[12] = E.ewald_overlap && E.aux_stream != nullptr && (E.precision != PIMD_MIXED || E.kp.Fx != nullptr);
     if (n >= 14) k[13] = E.dd_otf && E.precision == PIMD_MIXED;
     if (n >= 15) k[14] = E.ff_tc && E.tf_ready && E.tf_qd_ready;
     if (n >= 16) k[15] = E.l2_keep && E.precision == PIMD_MIXED;
