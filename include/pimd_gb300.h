@@ -118,6 +118,13 @@ int pimd_timers_get(pimd_ctx *ctx, int i, char *name, int namelen, double *ms, l
  * `every` iterations (0 = run exactly polar_maxiter iterations with converged beads
  * skipped on the device, which needs no host synchronisation). Default 1. */
 int pimd_set_dipole_check(pimd_ctx *ctx, int every);
+/* The induced-dipole iterations of small boxes run by the matrix of the dipole field, formed once a
+ * force call, instead of a structure factor and a field pass each: chosen by the box's size at
+ * creation, on unless switched off here (a captured MD-step graph is captured again; no effect
+ * where the box has no matrix). *in_use: 1 when the force calls of this context take it; the
+ * forward of the differentiation form never does. No counterpart in the reference. */
+int pimd_set_dipole_matrix(pimd_ctx *ctx, int enable);
+int pimd_get_dipole_matrix(pimd_ctx *ctx, int *in_use);
 
 /* ---------------------------------------------------------------------------------------
  * Ring-polymer normal modes (NormalModes.f90) and PILE thermostat (Langevin.f90).
@@ -315,25 +322,27 @@ int pimd_pot_backward(pimd_ctx *ctx, const double *Ebar, double *dRRt, double *d
 int pimd_autotune(pimd_ctx *ctx, const double *RRt, const double *RRc);
 /* The chosen shapes: [tiled structure factors, site groups (0 = sized from the SM count),
  * register-row field kernels, max k-slices, one-launch neighbour lists] and, when n >= 6,
- * [wave-quantised split counts], when n >= 7 [tensor-core (tcgen05) dipole structure factor
- * in use], when n >= 8 [tensor-core dipole field pass in use], when n >= 9 [real-space dipole
+ * [wave-quantised split counts], when n >= 7 [tensor-core (tcgen05) dipole structure factor in
+ * use], when n >= 8 [tensor-core dipole field pass in use], when n >= 9 [real-space dipole
  * field on a second stream beside the structure factor], when n >= 10 [the dipole iterations'
- * structure factor reuses its position-only operand from the first iteration], when n >= 11 [the iterations' field pass is a programmatic dependent launch of
- * the structure factor (its set-up overlaps that grid's end)], when n >= 12 [dipole iterations
- * per body of the CUDA graph's conditional loop, 1-4], when n >= 13 [the reciprocal charge and
- * force passes on a second stream beside the pair kernels, and the backward's real-space part
- * beside its reciprocal passes], when n >= 14
- * [real-space dipole tensors formed inside each iteration rather than cached per list entry
- * (mixed engine)], when n >= 15 [tensor-core force pass in use (follows the field-pass knob;
- * reported only)], when n >= 16 [the iterations' cached operands loaded evict-last in L2], when
- * n >= 17 [the real-space dipole field beside the field pass too, each unit of 128 dipole
- * sites updated by whichever of the two finishes it last (mixed engine, TTM3-F)], when n >= 18
- * [at the start of each graph-loop body the real-space dipole field waits until every CTA of
- * the structure factor is resident (a programmatic event), mixed engine], when n >= 19 [the
- * iterations' field pass may start as the real-space dipole field drains (a programmatic
- * event; it waits for that grid before reading its output), mixed engine], when n >= 20 [the
- * neighbour lists built from the input positions on the second stream beside the monomer
- * kernel, mixed engine]; n >= 5. */
+ * structure factor reuses its position-only operand from the first iteration], when n >= 11
+ * [the iterations' field pass is a programmatic dependent launch of the structure factor (its
+ * set-up overlaps that grid's end)], when n >= 12 [dipole iterations per body of the CUDA
+ * graph's conditional loop, 1-4], when n >= 13 [the reciprocal charge and force passes on a
+ * second stream beside the pair kernels, and the backward's real-space part beside its
+ * reciprocal passes], when n >= 14 [real-space dipole tensors formed inside each iteration
+ * rather than cached per list entry (mixed engine)], when n >= 15 [tensor-core force pass in
+ * use (follows the field-pass knob; reported only)], when n >= 16 [the iterations' cached
+ * operands loaded evict-last in L2], when n >= 17 [the real-space dipole field beside the
+ * field pass too, each unit of 128 dipole sites updated by whichever of the two finishes it
+ * last (mixed engine, TTM3-F)], when n >= 18 [at the start of each graph-loop body the real-
+ * space dipole field waits until every CTA of the structure factor is resident (a programmatic
+ * event), mixed engine], when n >= 19 [the iterations' field pass may start as the real-space
+ * dipole field drains (a programmatic event; it waits for that grid before reading its
+ * output), mixed engine], when n >= 20 [the neighbour lists built from the input positions on
+ * the second stream beside the monomer kernel, mixed engine]; n >= 5. In a box whose dipole
+ * iterations run by the matrix (pimd_get_dipole_matrix) the entries of the iterations' passes
+ * (9, 10, 12, 14, 16-19) act on the forward of the differentiation form only. */
 int pimd_get_tuning(pimd_ctx *ctx, int *knobs, int n);
 /* Sets the shapes in the order pimd_get_tuning reports them (n >= 5; entry 15, the tensor-core
  * force pass, is a report only), e.g. to reuse an earlier autotune result without timing

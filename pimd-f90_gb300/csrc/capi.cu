@@ -595,7 +595,7 @@ static bool force_overlap(const Engine &E) {
 
 // small boxes iterate with the matrix of the dipole field; a taped forward keeps the passes, whose
 // structure factors the backward reads
-static bool dipole_matrix(const Engine &E) { return E.dm.M && !E.tape_on; }
+static bool dipole_matrix(const Engine &E) { return E.dm.M && E.dm_on && !E.tape_on; }
 
 static bool overlap64(const Engine &E) { return E.precision != PIMD_MIXED && E.ewald_overlap && E.aux_stream; }
 
@@ -1032,6 +1032,19 @@ int pimd_set_dipole_check(pimd_ctx *ctx, int every) {
     return PIMD_OK;
 }
 
+int pimd_set_dipole_matrix(pimd_ctx *ctx, int enable) {
+    if (!ctx) return PIMD_ERR_ARG;
+    ctx->E.dm_on = enable != 0;
+    ctx->E.gkey.clear();  // a captured MD-step graph holds the old launches: capture again
+    return PIMD_OK;
+}
+
+int pimd_get_dipole_matrix(pimd_ctx *ctx, int *in_use) {
+    if (!ctx || !in_use) return PIMD_ERR_ARG;
+    *in_use = ctx->E.dm.M && ctx->E.dm_on;
+    return PIMD_OK;
+}
+
 int pimd_full_bead_forces_device(pimd_ctx *ctx, const double *RRt, const double *RRc, double *Upott, double *dRRt,
                                  double *virialt, double *virialct, double *dip_momIt, double *dip_momEt, double *chg,
                                  int t) {
@@ -1293,12 +1306,13 @@ int pimd_autotune(pimd_ctx *ctx, const double *RRt, const double *RRc) {
         knobs.push_back({&sf_tiled, {1, 0}});
         knobs.push_back({&E.sf_groups, {0, 4, 8, 16, 32}});
         knobs.push_back({&ff_regs, {1, 0}});
-        if (E.loop_aux) knobs.push_back({&dd_overlap, {1, 0}});
-        if (dd_async_ok(E)) knobs.push_back({&dda, {1, 0}});
-        if (E.d_tcx) knobs.push_back({&xcache, {1, 0}});
+        const bool passes = !dipole_matrix(E);  // (knobs of the iterations' passes)
+        if (E.loop_aux && passes) knobs.push_back({&dd_overlap, {1, 0}});
+        if (dd_async_ok(E) && passes) knobs.push_back({&dda, {1, 0}});
+        if (E.d_tcx && passes) knobs.push_back({&xcache, {1, 0}});
         if (E.tf_ready) knobs.push_back({&pdl, {1, 0}});
         if (E.kp.Fx) knobs.push_back({&ewo, {1, 0}});
-        knobs.push_back({&otf, {1, 0}});
+        if (passes) knobs.push_back({&otf, {1, 0}});
     }
     knobs.push_back({&wave, {1, 0}});
     knobs.push_back({&E.max_slices, {16, 8, 4, 2}});

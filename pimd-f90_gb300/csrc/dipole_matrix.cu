@@ -701,7 +701,8 @@ void launch_dm_solve(Engine &E) {
 // 32 x 1 978 -> 453 us, 128 x 8 1599 -> 820, 128 x 64 4570 -> 3325, TTM2.1-F 60 x 16 (180 dipole sites)
 // 2075 -> 1617: wherever its rows fit the shared memory of 8 CTAs (up to 184 sites). Mixed: 32 x 8
 // 3474 -> 272 us, 128 x 32 1120 -> 400, 216 x 32 1024 -> 803, 270 x 8 1055 -> 487, 270 x 32 1209 -> 1129,
-// but 270 x 64 1833 -> 1954: beyond 216 sites only up to 40 beads of 270 (the rows fit up to 276).
+// but 270 x 64 1833 -> 1954: beyond 216 sites only up to 40 beads of 270 (the rows fit up to 272, TTM2.1-F
+// 264). A k shell's tables are to fit 100 KB beside the phases, two blocks a SM: cubes up to |n| = 15, FP64 14.
 static bool dm_wanted(const Engine &E) {
     const KP &kp = E.kp;
     if (kp.model >= 4 || std::max(kp.hmax, std::max(kp.kmax, kp.lmax)) >= DM_JMAX) return false;

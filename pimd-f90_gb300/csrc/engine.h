@@ -337,6 +337,7 @@ struct Engine {
     alignas(64) unsigned char tc_map[128];  // CUtensorMap of the FP32 tables tabf
     DgArgs dg;                 // FP64 engine: digit operands of the reciprocal sums
     DmArgs dm{};               // small boxes: the dipole field as a matrix
+    bool dm_on = true;         // (pimd_set_dipole_matrix)
     bool dg_xall = false;      // the X buffer holds the dipole sites of every bead
     bool dg_xdip = false;      // ... and does so for this force call's positions
     int dg_chain = 0;          // small system's iteration: 1 the first of a loop (body), 2 after another

@@ -65,6 +65,8 @@ SIGNATURES = {
     "pimd_get_virial": [_V, ctypes.c_int, _D],
     "pimd_get_dipole_info": [_V, ctypes.c_int, _I, _D],
     "pimd_set_dipole_check": [_V, ctypes.c_int],
+    "pimd_set_dipole_matrix": [_V, ctypes.c_int],
+    "pimd_get_dipole_matrix": [_V, _I],
     "pimd_get_neighbors": [_V, ctypes.c_int, _I, ctypes.c_int, _I],
     "pimd_nm_init": [_V, ctypes.c_int, ctypes.c_double, ctypes.c_double, ctypes.c_double, _D, _D, _D, _D, _D, _D,
                      _D],
@@ -243,6 +245,16 @@ class ForceEngine:
 
     def set_dipole_check(self, every):
         self._check(load().pimd_set_dipole_check(self.h, int(every)), "set_dipole_check")
+
+    def set_dipole_matrix(self, enable):
+        """Small boxes: the dipole iterations by the matrix of the dipole field (the default) or by passes."""
+        self._check(load().pimd_set_dipole_matrix(self.h, int(bool(enable))), "set_dipole_matrix")
+
+    def dipole_matrix(self):
+        """Whether this context's force calls iterate with the matrix of the dipole field."""
+        n = ctypes.c_int()
+        self._check(load().pimd_get_dipole_matrix(self.h, ctypes.byref(n)), "get_dipole_matrix")
+        return bool(n.value)
 
     def energies(self, bead=0):
         U = np.zeros(4)
