@@ -397,7 +397,7 @@ static int create(Engine &E, const pimd_params *p, int nrep, const int *brep) {
     pot_init_constants(E);
     ewald_init(E);
     if (E.precision != PIMD_MIXED && dg_init(E)) return fail(E, PIMD_ERR_NOMEM, "cudaMalloc");
-    if (dm_init(E)) return fail(E, PIMD_ERR_NOMEM, "cudaMalloc");
+    dm_init(E);
     if ((rc = cuda_check(E, overlap_init(E), "streams"))) return rc;
     if (E.precision == PIMD_MIXED && (rc = cuda_check(E, mixed_init(E), "mixed tables"))) return rc;
     neighbors_init(E);

@@ -711,17 +711,17 @@ static bool dm_wanted(const Engine &E) {
     return nd * nd * kp.P * 6 * (mixed ? 4 : 8) <= 2147483648.0;  // (its memory: at most 2 GB)
 }
 
-int dm_init(Engine &E) {
+void dm_init(Engine &E) {
     KP &kp = E.kp;
     DmArgs &a = E.dm;
     a = DmArgs{};
     const bool mixed = E.precision == PIMD_PREC_MIXED;
-    if (!dm_wanted(E)) return 0;
+    if (!dm_wanted(E)) return;
     a.nd = kp.ld - kp.fd;
     a.ndp = (a.nd + 3) & ~3;
     const size_t rs = mixed ? 4 : 8;
     const size_t lim = (size_t)226 * 1024;  // (beside the static words)
-    if ((a.nd + 7) / 8 > DM_MAXROWS || solve_smem(a, (a.nd + 7) / 8, rs, kp.model) > lim) return 0;
+    if ((a.nd + 7) / 8 > DM_MAXROWS || solve_smem(a, (a.nd + 7) / 8, rs, kp.model) > lim) return;
     for (int c = 0; c < 3; c++) a.gk[c] = TWOPI * kp.boxi[c];
     a.nqmax = (kp.lmax + 4) / 4;
     const int JM = 4 * a.nqmax;
@@ -737,7 +737,7 @@ int dm_init(Engine &E) {
             kx.push_back(make_int4(r.kx, nrun, 0, 0));
             load.push_back(6);
         }
-        if (r.ky != kx.back().z) return 0;
+        if (r.ky != kx.back().z) return;
         kx.back().z++;
         w.resize((size_t)(nrun + 1) * JM, 0.0);
         int top = 0;
@@ -828,10 +828,13 @@ int dm_init(Engine &E) {
     a.phase = (int)(32 * ((mixed ? sizeof(DmTypes<float>::Y) : sizeof(DmTypes<double>::Y)) * (kp.kmax + 1) + 2 * rs * (kp.hmax + 1) +
                           std::max(JM * 2 * (size_t)(mixed ? 4 : 8), DM_NP * 6 * rs)));
     const size_t bsm = a.phase + img.size();
-    if (bsm > (size_t)100 * 1024) return 0;
+    if (bsm > (size_t)100 * 1024) return;
     const size_t head = (img.size() + 255) & ~(size_t)255;
     char *base = nullptr;
-    if (cudaMalloc((void **)&base, head + (size_t)kp.P * a.nd * 6 * a.ndp * rs) != cudaSuccess) return 1;
+    if (cudaMalloc((void **)&base, head + (size_t)kp.P * a.nd * 6 * a.ndp * rs) != cudaSuccess) {
+        cudaGetLastError();  // (no room: the passes)
+        return;
+    }
     E.allocs.push_back(base);
     cudaMemcpy(base, img.data(), img.size(), cudaMemcpyHostToDevice);
     a.tables = reinterpret_cast<const int4 *>(base);
@@ -858,7 +861,6 @@ int dm_init(Engine &E) {
         if (cudaOccupancyMaxActiveClusters(&n, k_dm_solve<double>, &c) == cudaSuccess) a.c16 = n;
         cudaGetLastError();
     }
-    return 0;
 }
 
 }  // namespace pimd

@@ -577,7 +577,7 @@ int launch_dg_field(Engine &E, int mode, int s0, int s1, int part);
 int launch_dg_dforce(Engine &E, const double2 *A, const double2 *B, const double2 *A2, const double *dip2);
 // launchers (spc.cu): q-SPC/Fw and SPC/F
 // dipole_matrix.cu
-int dm_init(Engine &E);                    // 1: out of memory
+void dm_init(Engine &E);
 void launch_dm_build(Engine &E);           // after the site tables
 void launch_dm_solve(Engine &E);           // all dipole iterations
 void launch_sites_spc(Engine &E);

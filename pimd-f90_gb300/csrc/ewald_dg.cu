@@ -819,7 +819,8 @@ int dg_init(Engine &E) {
     const size_t fit_d = std::min(P * kd, ((size_t)8 << 30) / per_step), fit_q = std::min(P * kq, ((size_t)1 << 30) / per_step);
     a.xsteps = (int)std::max(std::max(kq, kd), std::max(fit_d, fit_q));
     E.dg_xall = (size_t)a.xsteps >= P * kd;
-    // one allocation, cut on 256-byte boundaries (the first walk measures, the second places)
+    // One allocation, cut on 256-byte boundaries (a first walk measures, a second places). Where the device has
+    // no room for it, without the kept exy values and then with X of one bead at a time (formed in parts).
     const size_t zt = std::max((size_t)ceil_div(a.jn, 8) * kq, (size_t)ceil_div(3 * a.jn, 8) * kd);
     char *base = nullptr;
     size_t used = 0;
@@ -830,7 +831,8 @@ int dg_init(Engine &E) {
     int4 *d_slot;
     int *d_slotk;
     double2 *d_slotkv;
-    for (int pass = 0; pass < 2; pass++) {
+    bool keep = nd && E.dg_xall;
+    auto place = [&] {
         used = 0;
         cut(d_slot, sizeof(int4) * a.nslot);
         cut(d_slotk, sizeof(int) * a.nslot);
@@ -846,14 +848,24 @@ int dg_init(Engine &E) {
         cut(a.V, P * a.nv8 * a.ksf * (size_t)DG_VT);
         // (two sets where the differentiation form may run)
         if (nd) cut(a.Vd, (kp.model == 3 ? 2 : 1) * P * a.nvd8 * a.ksf * (size_t)DG_VT);
-        if (nd && E.dg_xall) cut(a.exyc, P * a.nslot * (size_t)nd * sizeof(int4));
+        if (keep) cut(a.exyc, P * a.nslot * (size_t)nd * sizeof(int4));
         cut(a.tab, P * (size_t)kp.ntab * kp.S * sizeof(int4));
-        if (pass == 0) {
-            if (cudaMalloc((void **)&base, used) != cudaSuccess) return 1;
-            E.allocs.push_back(base);
+    };
+    place();
+    for (int less = 0; cudaMalloc((void **)&base, used) != cudaSuccess; less++) {
+        cudaGetLastError();
+        base = nullptr;
+        if (less == 2) return 1;
+        keep = false;
+        if (less == 1) {
+            a.xsteps = (int)std::max(kq, kd);
+            E.dg_xall = (size_t)a.xsteps >= P * kd;
         }
+        place();
     }
-    if (!nd || !E.dg_xall) a.exyc = nullptr;
+    E.allocs.push_back(base);
+    place();
+    if (!keep) a.exyc = nullptr;
     // the host tables and the zeroed words after them in one copy
     const size_t head = reinterpret_cast<char *>(a.vexp) - base;
     std::vector<char> img(head, 0);
