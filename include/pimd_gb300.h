@@ -26,7 +26,7 @@ enum {
     PIMD_ERR_ARG = 1,               /* invalid argument / unsupported combination         */
     PIMD_ERR_CUDA = 2,              /* CUDA runtime error (see pimd_last_error)           */
     PIMD_ERR_NEIGHBOR_OVERFLOW = 3, /* more O-O pairs than the neighbour-list capacity     */
-    PIMD_ERR_GAMMQ = 4,             /* Thole Q(2/3,x) iteration did not converge          */
+    PIMD_ERR_GAMMQ = 4,             /* Thole Q(2/3,x) of an x that is not a number         */
     PIMD_ERR_NOMEM = 5,             /* device allocation failed                            */
     PIMD_ERR_STATE = 6              /* call order violated (e.g. no normal modes set up)   */
 };

@@ -74,41 +74,6 @@ PIMD_D float erfc_as<float>(float X) {
     return TP * __expf(-(X * X));
 }
 
-// math.f90:188-285: Q(2/3, x) by the Numerical-Recipes series / Lentz continued fraction,
-// EPS = 3e-7, gln = ln Gamma(2/3). Failure to converge sets bit 2 of *err.
-template <typename R>
-PIMD_D R gammq2_3(R x, unsigned *err) {
-    const R a = R(2.0 / 3.0), gln = R(0.303150275147547), EPS = R(3.e-7);
-    if (x < a + R(1)) {
-        if (x <= R(0)) return R(1);
-        R ap = a, ssum = R(1) / a, del = ssum;
-        for (int n = 1; n <= 800; n++) {
-            ap = ap + R(1);
-            del = del * x / ap;
-            ssum = ssum + del;
-            if (fabs(del) < fabs(ssum) * EPS) return R(1) - ssum * exp(-x + a * log(x) - gln);
-        }
-        *err |= 4u;
-        return R(1);
-    }
-    const R FPMIN = R(1.e-30);
-    R b = x + R(1) - a, c = R(1) / FPMIN, d = R(1) / b, h = d;
-    for (int i = 1; i <= 100; i++) {
-        R an = -R(i) * (R(i) - a);
-        b = b + R(2);
-        d = an * d + b;
-        if (fabs(d) < FPMIN) d = FPMIN;
-        c = b + an / c;
-        if (fabs(c) < FPMIN) c = FPMIN;
-        d = R(1) / d;
-        R del = d * c;
-        h = h * del;
-        if (fabs(del - R(1)) < EPS) return exp(-x + a * log(x) - gln) * h;
-    }
-    *err |= 4u;
-    return R(0);
-}
-
 // Ewald constants shared by the smear kernels (potential.f90:196-198)
 struct EwC {
     double aewald, a2, cts1, cts2, cts3;
@@ -116,30 +81,6 @@ struct EwC {
 struct EwCf {
     float aewald, a2, cts1, cts2, cts3;
 };
-
-// smear.f90:2-34 PBCsmear01: screened + Thole-smeared charge-charge tensors ts0, ts1.
-// ra = a_pol12^(1/3) is passed precomputed (a function of the site kinds only).
-template <typename R, typename EC>
-PIMD_D void smear01(R drsq, R a_pol12, R ra, const EC &e, R *ts0, R *ts1, unsigned *err) {
-    const R g23 = R(1.3541179394264);
-    R dd = sqrt(drsq);
-    R dri = R(1) / dd;
-    R drsqi = dri * dri;
-    R expon = exp(-(R(e.a2) * drsq));
-    R er = erfc_as<R>(R(e.aewald) * dd);
-    R t0 = er * dri;
-    R t1 = (t0 + R(e.cts1) * expon) * drsqi;
-    if (drsq < R(25)) {
-        R rA3 = dd * drsq * a_pol12;
-        R exp1 = exp(-rA3);
-        R ch1 = -dri * drsqi;
-        R sr1 = (R(1) - exp1) * dri * drsqi;
-        t1 = t1 + ch1 + sr1;
-        t0 = t0 - exp1 * dri + ra * g23 * gammq2_3<R>(rA3, err);
-    }
-    *ts0 = t0;
-    *ts1 = t1;
-}
 
 // dd = r, dri = 1/r from r^2, and exp: FP64 as the reference (sqrt, divide, exp); FP32 (the mixed
 // engine) by the hardware reciprocal square root and exp2 (a few ulp, below the FP32 noise of

@@ -12,16 +12,6 @@ struct TT {
     static constexpr int FDI = MODEL == 2 ? 1 : 4;
     static constexpr int LDI = MODEL == 2 ? 3 : 4;
     PIMD_HD static constexpr bool dip(int k) { return k >= FDI && k <= LDI; }
-    PIMD_HD static constexpr bool chg(int k) { return k != 1; }
-    // charge-phase site pairs that change an output (O carries no charge; its field is
-    // only needed when O carries a dipole, TTM2.1-F)
-    PIMD_HD static constexpr bool qq_active(int i, int j) {
-        return !(i == 1 && j == 1) && (MODEL == 2 || (i != 1 && j != 1));
-    }
-    // force-phase site pairs with a dipole-dipole or charge-dipole term
-    PIMD_HD static constexpr bool f_active(int i, int j) {
-        return (dip(i) && dip(j)) || (dip(i) && chg(j)) || (chg(i) && dip(j));
-    }
 };
 
 PIMD_D double3 ld3(const double *p) { return make_double3(p[0], p[1], p[2]); }

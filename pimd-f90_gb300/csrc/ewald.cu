@@ -23,37 +23,15 @@
 
 namespace pimd {
 
-template <typename R>
-struct C2;
-template <>
-struct C2<double> {
-    using T = double2;
-    PIMD_D static T make(double x, double y) { return make_double2(x, y); }
-};
-template <>
-struct C2<float> {
-    using T = float2;
-    PIMD_D static T make(float x, float y) { return make_float2(x, y); }
-};
-
-template <typename V>
-PIMD_D V cmul(V a, V b) {
-    V r;
+PIMD_D float2 cmul(float2 a, float2 b) {
+    float2 r;
     r.x = a.x * b.x - a.y * b.y;
     r.y = a.y * b.x + a.x * b.y;
     return r;
 }
-template <typename V>
-PIMD_D V cconj(V a) {
+PIMD_D float2 cconj(float2 a) {
     a.y = -a.y;
     return a;
-}
-
-template <typename R>
-PIMD_D typename C2<R>::T *tab_base(const KP &kp);
-template <>
-PIMD_D float2 *tab_base<float>(const KP &kp) {
-    return kp.tabf;
 }
 
 // ewald.f90:403-437 ssincos, cos/sin(2 pi n x / L) for n = 0..nmax, without the recurrence: the site's coordinate as a
@@ -85,10 +63,7 @@ __global__ void __launch_bounds__(128) k_ewald_tables_m(KP kp) {
 
 // k-vector components of the phase sums from the precomputed FP32 tables (no double-to-float
 // conversion inside the kernels)
-template <typename R>
-struct KV;
-template <>
-struct KV<float> {
+struct KV {
     PIMD_D static void run_xy(const KP &kp, int r, float &x, float &y) {
         const float2 v = kp.runkf[r];
         x = v.x;
@@ -101,27 +76,21 @@ enum { OP_Q = 0, OP_MU = 1, OP_DIP = 2 };
 constexpr int SP_NT = 256;  // threads (k-vectors) per structure-factor block
 constexpr int SP_TS = 64;   // sites per shared-memory tile
 
-template <typename R>
-PIMD_D typename C2<R>::T tab_x(const KP &kp, int b, int n, int s) {
-    return tab_base<R>(kp)[((size_t)b * kp.ntab + n) * kp.S + s];
-}
-template <typename R>
-PIMD_D typename C2<R>::T tab_y(const KP &kp, int b, int n, int s) {
-    const typename C2<R>::T v = tab_base<R>(kp)[((size_t)b * kp.ntab + kp.hmax + 1 + (n < 0 ? -n : n)) * kp.S + s];
+PIMD_D float2 tab_x(const KP &kp, int b, int n, int s) { return kp.tabf[((size_t)b * kp.ntab + n) * kp.S + s]; }
+PIMD_D float2 tab_y(const KP &kp, int b, int n, int s) {
+    const float2 v = kp.tabf[((size_t)b * kp.ntab + kp.hmax + 1 + (n < 0 ? -n : n)) * kp.S + s];
     return n < 0 ? cconj(v) : v;
 }
-template <typename R>
-PIMD_D typename C2<R>::T tab_z(const KP &kp, int b, int n, int s) {
-    return tab_base<R>(kp)[((size_t)b * kp.ntab + kp.hmax + 1 + kp.kmax + 1 + n) * kp.S + s];
+PIMD_D float2 tab_z(const KP &kp, int b, int n, int s) {
+    return kp.tabf[((size_t)b * kp.ntab + kp.hmax + 1 + kp.kmax + 1 + n) * kp.S + s];
 }
 
 // Per-tile partial structure factors.
 //   OP_Q : sum_s q_s e_s                        (ewald.f90:41-42)
 //   OP_MU: sum_s (k.mu_s) e_s                   (ewald.f90:99-108)
 //   OP_DIP: sum_s mu_{s,c} e_s, c = x, y, z     (ewald.f90:208-213)
-template <int OP, typename R>
+template <int OP>
 __global__ void __launch_bounds__(SP_NT) k_spass(KP kp, int s0, int nsites, int tsg, int ngroups, int skipconv) {
-    using V = typename C2<R>::T;
     constexpr int NC = (OP == OP_DIP) ? 3 : 1;
     const int b = blockIdx.z;
     if (skipconv && kp.acc[(size_t)b * NACC + ACC_CONV] != 0.0) return;
@@ -130,23 +99,23 @@ __global__ void __launch_bounds__(SP_NT) k_spass(KP kp, int s0, int nsites, int 
     const int nr = ch.r1 - ch.r0;
     const int LZ = 2 * kp.lmax + 1;
     extern __shared__ double smem[];
-    V *ez = reinterpret_cast<V *>(smem);               // [TS][LZ]
-    V *exy = ez + SP_TS * LZ;                          // [TS][nr]
-    R *aa = reinterpret_cast<R *>(exy + SP_TS * nr);   // [TS][nr] (OP_MU)
-    R *wt = aa + SP_TS * nr;                           // [TS][4]
+    float2 *ez = reinterpret_cast<float2 *>(smem);               // [TS][LZ]
+    float2 *exy = ez + SP_TS * LZ;                          // [TS][nr]
+    float *aa = reinterpret_cast<float *>(exy + SP_TS * nr);   // [TS][nr] (OP_MU)
+    float *wt = aa + SP_TS * nr;                           // [TS][4]
     const int k = ch.k0 + threadIdx.x;
     const bool valid = k < ch.k1;
     int rk = 0, kz = 0;
-    R kzv = R(0);
+    float kzv = 0.f;
     if (valid) {
         const int2 ki = kp.kidx[k];
         rk = ki.x - ch.r0;
         kz = ki.y;
-        kzv = KV<R>::z(kp, k);
+        kzv = KV::z(kp, k);
     }
-    V acc[NC];
+    float2 acc[NC];
 #pragma unroll
-    for (int c = 0; c < NC; c++) acc[c] = C2<R>::make(R(0), R(0));
+    for (int c = 0; c < NC; c++) acc[c] = make_float2(0.f, 0.f);
     const int gbeg = s0 + grp * tsg, gend = min(s0 + nsites, gbeg + tsg);
     for (int sb = gbeg; sb < gend; sb += SP_TS) {
         const int nloc = min(SP_TS, gend - sb);
@@ -154,16 +123,16 @@ __global__ void __launch_bounds__(SP_NT) k_spass(KP kp, int s0, int nsites, int 
         if (threadIdx.x < nloc) {
             const size_t gs = (size_t)b * kp.S + sb + threadIdx.x;
             if (OP == OP_Q) {
-                wt[4 * threadIdx.x] = R(kp.pos[gs].w);
+                wt[4 * threadIdx.x] = (float)kp.pos[gs].w;
             } else {
-                wt[4 * threadIdx.x + 0] = R(kp.dip[3 * gs + 0]);
-                wt[4 * threadIdx.x + 1] = R(kp.dip[3 * gs + 1]);
-                wt[4 * threadIdx.x + 2] = R(kp.dip[3 * gs + 2]);
+                wt[4 * threadIdx.x + 0] = (float)kp.dip[3 * gs + 0];
+                wt[4 * threadIdx.x + 1] = (float)kp.dip[3 * gs + 1];
+                wt[4 * threadIdx.x + 2] = (float)kp.dip[3 * gs + 2];
             }
         }
         for (int idx = threadIdx.x; idx < nloc * (kp.lmax + 1); idx += SP_NT) {
             const int site = idx % nloc, n = idx / nloc;
-            const V v = tab_z<R>(kp, b, n, sb + site);
+            const float2 v = tab_z(kp, b, n, sb + site);
             ez[site * LZ + kp.lmax + n] = v;
             ez[site * LZ + kp.lmax - n] = cconj(v);
         }
@@ -171,29 +140,29 @@ __global__ void __launch_bounds__(SP_NT) k_spass(KP kp, int s0, int nsites, int 
         for (int idx = threadIdx.x; idx < nloc * nr; idx += SP_NT) {
             const int site = idx % nloc, r = idx / nloc;
             const KRun run = kp.runs[ch.r0 + r];
-            const V ex = tab_x<R>(kp, b, run.kx, sb + site);
-            const V ey = tab_y<R>(kp, b, run.ky, sb + site);
+            const float2 ex = tab_x(kp, b, run.kx, sb + site);
+            const float2 ey = tab_y(kp, b, run.ky, sb + site);
             // ewald.f90:30-31: coskxky = cx cy - sx sy, sinkxky = sx cy + cx sy
-            exy[site * nr + r] = C2<R>::make(ex.x * ey.x - ex.y * ey.y, ex.y * ey.x + ex.x * ey.y);
+            exy[site * nr + r] = make_float2(ex.x * ey.x - ex.y * ey.y, ex.y * ey.x + ex.x * ey.y);
             if (OP == OP_MU) {
-                R kx, ky;
-                KV<R>::run_xy(kp, ch.r0 + r, kx, ky);
+                float kx, ky;
+                KV::run_xy(kp, ch.r0 + r, kx, ky);
                 aa[site * nr + r] = kx * wt[4 * site] + ky * wt[4 * site + 1];
             }
         }
         __syncthreads();
         if (valid) {
             for (int site = 0; site < nloc; site++) {
-                const V a = exy[site * nr + rk];
-                const V z = ez[site * LZ + kp.lmax + kz];
+                const float2 a = exy[site * nr + rk];
+                const float2 z = ez[site * LZ + kp.lmax + kz];
                 // ewald.f90:37-39: coskr = cxy cz - sxy sz, sinkr = sxy cz + cxy sz
-                const V e = C2<R>::make(a.x * z.x - a.y * z.y, a.y * z.x + a.x * z.y);
+                const float2 e = make_float2(a.x * z.x - a.y * z.y, a.y * z.x + a.x * z.y);
                 if (OP == OP_Q) {
-                    const R q = wt[4 * site];
+                    const float q = wt[4 * site];
                     acc[0].x += q * e.x;
                     acc[0].y += q * e.y;
                 } else if (OP == OP_MU) {
-                    const R t = aa[site * nr + rk] + kzv * wt[4 * site + 2];
+                    const float t = aa[site * nr + rk] + kzv * wt[4 * site + 2];
                     acc[0].x += t * e.x;
                     acc[0].y += t * e.y;
                 } else {
@@ -207,7 +176,7 @@ __global__ void __launch_bounds__(SP_NT) k_spass(KP kp, int s0, int nsites, int 
         }
     }
     if (valid) {
-        V *out = reinterpret_cast<V *>(kp.Spart) + (((size_t)b * ngroups + grp) * kp.nk + k) * NC;
+        float2 *out = reinterpret_cast<float2 *>(kp.Spart) + (((size_t)b * ngroups + grp) * kp.nk + k) * NC;
 #pragma unroll
         for (int c = 0; c < NC; c++) out[c] = acc[c];
     }
@@ -289,7 +258,7 @@ __global__ void __launch_bounds__(SF_MAXT) k_sfac_f(KP kp, int s0, int nsites, i
             const int site = idx / KZP, kz = zb + (idx - site * KZP) - L;
             float2 v = make_float2(0.f, 0.f);
             if (site < nloc && kz <= L) {
-                v = tab_z<float>(kp, b, kz < 0 ? -kz : kz, sb + site);
+                v = tab_z(kp, b, kz < 0 ? -kz : kz, sb + site);
                 if (kz < 0) v = cconj(v);
             }
             ez[idx] = v;
@@ -303,8 +272,8 @@ __global__ void __launch_bounds__(SF_MAXT) k_sfac_f(KP kp, int s0, int nsites, i
             for (int m = 0; m < M; m++) a[m] = make_float2(0.f, 0.f);
             if (site < nloc && r < nr) {
                 const int2 xy = rxy[r];
-                const float2 ex = tab_x<float>(kp, b, xy.x, sb + site);
-                const float2 ey = tab_y<float>(kp, b, xy.y, sb + site);
+                const float2 ex = tab_x(kp, b, xy.x, sb + site);
+                const float2 ey = tab_y(kp, b, xy.y, sb + site);
                 // ewald.f90:30-31: coskxky = cx cy - sx sy, sinkxky = sx cy + cx sy
                 const float2 exy = make_float2(ex.x * ey.x - ex.y * ey.y, ex.y * ey.x + ex.x * ey.y);
                 const float4 w = wt[site];
@@ -376,9 +345,8 @@ __global__ void __launch_bounds__(SF_MAXT) k_sfac_f(KP kp, int s0, int nsites, i
 
 // Sum the tile partials in FP64 in a fixed order. OP_MU stores (rQm, iQm) = (-Im, Re) of
 // sum (k.mu) e (ewald.f90:106-107).
-template <int OP, typename R>
+template <int OP>
 __global__ void __launch_bounds__(256) k_sreduce(KP kp, int ngroups, int skipconv) {
-    using V = typename C2<R>::T;
     constexpr int NC = (OP == OP_DIP) ? 3 : 1;
     const int k = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
     if (k >= kp.nk) return;
@@ -386,9 +354,9 @@ __global__ void __launch_bounds__(256) k_sreduce(KP kp, int ngroups, int skipcon
     double2 s[NC];
 #pragma unroll
     for (int c = 0; c < NC; c++) s[c] = make_double2(0.0, 0.0);
-    const V *part = reinterpret_cast<const V *>(kp.Spart);
+    const float2 *part = reinterpret_cast<const float2 *>(kp.Spart);
     for (int g = 0; g < ngroups; g++) {
-        const V *p = part + (((size_t)b * ngroups + g) * kp.nk + k) * NC;
+        const float2 *p = part + (((size_t)b * ngroups + g) * kp.nk + k) * NC;
 #pragma unroll
         for (int c = 0; c < NC; c++) {
             s[c].x += (double)p[c].x;
@@ -397,7 +365,7 @@ __global__ void __launch_bounds__(256) k_sreduce(KP kp, int ngroups, int skipcon
     }
     if (OP == OP_Q) kp.Sq[(size_t)b * kp.nk + k] = s[0];
     if (OP == OP_MU) kp.Sm[(size_t)b * kp.nk + k] = make_double2(-s[0].y, s[0].x);
-    if (sizeof(R) == 4 && OP != OP_DIP) {
+    if (OP != OP_DIP) {
         // FP32 field weights 4 pi Ak / V conj(S) of the mixed engine's field passes
         const double w = kp.kinfo[k].w;
         const double2 a = (OP == OP_Q) ? s[0] : make_double2(-s[0].y, s[0].x);
@@ -421,22 +389,21 @@ constexpr int KCH = 256;  // k-vectors staged per chunk (== SP_NT)
 // The k-list is split over gridDim.z slices (whole chunks each); every block writes its
 // slice's FP64 partial (E or G, phi) per site to Fpart[slice][bead][site], and
 // k_field_finish adds the slices in a fixed order and applies the epilogue.
-template <int MODE, int NT, typename R>
+template <int MODE, int NT>
 __global__ void __launch_bounds__(NT) k_field(KP kp, int s0, int s1) {
-    using V = typename C2<R>::T;
     const int b = blockIdx.y, slice = blockIdx.z, nslice = gridDim.z;
     if (MODE == F_D && kp.acc[(size_t)b * NACC + ACC_CONV] != 0.0) return;
     const int s = s0 + blockIdx.x * NT + threadIdx.x;
     const bool valid = s < s1;
     const int LZ = 2 * kp.lmax + 1;
     extern __shared__ double smem[];
-    V *ez = reinterpret_cast<V *>(smem);  // [LZ][NT]
-    V *W1 = ez + LZ * NT;                 // [KCH]
-    V *W2 = W1 + KCH;                     // [KCH] (QD)
-    R *kzs = reinterpret_cast<R *>(W2 + KCH);  // [KCH]
+    float2 *ez = reinterpret_cast<float2 *>(smem);  // [LZ][NT]
+    float2 *W1 = ez + LZ * NT;                 // [KCH]
+    float2 *W2 = W1 + KCH;                     // [KCH] (QD)
+    float *kzs = reinterpret_cast<float *>(W2 + KCH);  // [KCH]
     const size_t gs = (size_t)b * kp.S + (valid ? s : s0);
     for (int n = 0; n <= kp.lmax; n++) {
-        const V v = valid ? tab_z<R>(kp, b, n, s) : C2<R>::make(R(0), R(0));
+        const float2 v = valid ? tab_z(kp, b, n, s) : make_float2(0.f, 0.f);
         ez[(kp.lmax + n) * NT + threadIdx.x] = v;
         ez[(kp.lmax - n) * NT + threadIdx.x] = cconj(v);
     }
@@ -451,54 +418,42 @@ __global__ void __launch_bounds__(NT) k_field(KP kp, int s0, int s1) {
             mu[2] = kp.dip[3 * gs + 2];
         }
     }
-    const R qr = R(q), mur[3] = {R(mu[0]), R(mu[1]), R(mu[2])};
+    const float qr = (float)q, mur[3] = {(float)mu[0], (float)mu[1], (float)mu[2]};
     double E[3] = {0, 0, 0}, phi = 0.0, G[3] = {0, 0, 0};
-    const double2 *S1 = (MODE == F_Q) ? kp.Sq : kp.Sm;
     const int c0 = (int)((long)slice * kp.nchunk / nslice), c1 = (int)((long)(slice + 1) * kp.nchunk / nslice);
     for (int chn = c0; chn < c1; chn++) {
         const KChunk ch = kp.chunks[chn];
         __syncthreads();
         for (int i = threadIdx.x; i < ch.k1 - ch.k0; i += NT) {
             const int k = ch.k0 + i;
-            if constexpr (sizeof(R) == 4) {
-                const float2 wq = kp.Wf[((size_t)b * 2) * kp.nk + k], wm = kp.Wf[((size_t)b * 2 + 1) * kp.nk + k];
-                W1[i] = (MODE == F_Q) ? wq : wm;
-                if (MODE == F_QD) W2[i] = make_float2(wq.x + wm.x, wq.y + wm.y);
-                kzs[i] = kp.kzf[k];
-            } else {
-                const double4_32a ki = kp.kinfo[k];
-                const double2 a = S1[(size_t)b * kp.nk + k];
-                W1[i] = C2<R>::make(R(ki.w * a.x), R(-ki.w * a.y));  // 4 pi Ak / V conj(S)
-                if (MODE == F_QD) {
-                    const double2 c = kp.Sq[(size_t)b * kp.nk + k];
-                    W2[i] = C2<R>::make(R(ki.w * (c.x + a.x)), R(-ki.w * (c.y + a.y)));
-                }
-                kzs[i] = R(ki.z);
-            }
+            const float2 wq = kp.Wf[((size_t)b * 2) * kp.nk + k], wm = kp.Wf[((size_t)b * 2 + 1) * kp.nk + k];
+            W1[i] = (MODE == F_Q) ? wq : wm;
+            if (MODE == F_QD) W2[i] = make_float2(wq.x + wm.x, wq.y + wm.y);
+            kzs[i] = kp.kzf[k];
         }
         __syncthreads();
         if (!valid) continue;
-        // per-chunk partial sums in R, added to the FP64 totals once per chunk
-        R cE[3] = {R(0), R(0), R(0)}, cphi = R(0), cG[3] = {R(0), R(0), R(0)};
+        // per-chunk partial sums in FP32, added to the FP64 totals once per chunk
+        float cE[3] = {0.f, 0.f, 0.f}, cphi = 0.f, cG[3] = {0.f, 0.f, 0.f};
         for (int r = ch.r0; r < ch.r1; r++) {
             const KRun run = kp.runs[r];
-            R kvx, kvy;
-            KV<R>::run_xy(kp, r, kvx, kvy);
-            const V ex = tab_x<R>(kp, b, run.kx, s);
-            const V ey = tab_y<R>(kp, b, run.ky, s);
-            const V exy = C2<R>::make(ex.x * ey.x - ex.y * ey.y, ex.y * ey.x + ex.x * ey.y);
-            V U0 = C2<R>::make(R(0), R(0)), U1 = U0, V0 = U0, V1 = U0, V2 = U0;
+            float kvx, kvy;
+            KV::run_xy(kp, r, kvx, kvy);
+            const float2 ex = tab_x(kp, b, run.kx, s);
+            const float2 ey = tab_y(kp, b, run.ky, s);
+            const float2 exy = make_float2(ex.x * ey.x - ex.y * ey.y, ex.y * ey.x + ex.x * ey.y);
+            float2 U0 = make_float2(0.f, 0.f), U1 = U0, V0 = U0, V1 = U0, V2 = U0;
             const int i0 = run.kbeg - ch.k0;
             for (int j = 0; j < run.nkz; j++) {
-                const V z = ez[(kp.lmax + run.kzlo + j) * NT + threadIdx.x];
-                const R kz = kzs[i0 + j];
-                const V t = cmul(z, W1[i0 + j]);
+                const float2 z = ez[(kp.lmax + run.kzlo + j) * NT + threadIdx.x];
+                const float kz = kzs[i0 + j];
+                const float2 t = cmul(z, W1[i0 + j]);
                 U0.x += t.x;
                 U0.y += t.y;
                 U1.x += kz * t.x;
                 U1.y += kz * t.y;
                 if (MODE == F_QD && isdip) {
-                    const V u = cmul(z, W2[i0 + j]);
+                    const float2 u = cmul(z, W2[i0 + j]);
                     V0.x += u.x;
                     V0.y += u.y;
                     V1.x += kz * u.x;
@@ -507,17 +462,17 @@ __global__ void __launch_bounds__(NT) k_field(KP kp, int s0, int s1) {
                     V2.y += kz * kz * u.y;
                 }
             }
-            const V z0 = cmul(exy, U0), z1 = cmul(exy, U1);
+            const float2 z0 = cmul(exy, U0), z1 = cmul(exy, U1);
             if (MODE == F_QD) {
                 cphi += z0.x;
                 cG[0] -= qr * z0.y * kvx;
                 cG[1] -= qr * z0.y * kvy;
                 cG[2] -= qr * z1.y;
                 if (isdip) {
-                    const R R0 = exy.x * V0.x - exy.y * V0.y;
-                    const R R1 = exy.x * V1.x - exy.y * V1.y;
-                    const R R2 = exy.x * V2.x - exy.y * V2.y;
-                    const R a = kvx * mur[0] + kvy * mur[1];
+                    const float R0 = exy.x * V0.x - exy.y * V0.y;
+                    const float R1 = exy.x * V1.x - exy.y * V1.y;
+                    const float R2 = exy.x * V2.x - exy.y * V2.y;
+                    const float a = kvx * mur[0] + kvy * mur[1];
                     cG[0] -= kvx * (a * R0 + mur[2] * R1);
                     cG[1] -= kvy * (a * R0 + mur[2] * R1);
                     cG[2] -= a * R1 + mur[2] * R2;
@@ -605,7 +560,7 @@ __global__ void __launch_bounds__(FF_NT) k_field_f(KP kp, int s0, int s1) {
         const int kz = j - LM;
         float2 v = make_float2(0.f, 0.f);
         if (valid && kz >= -L && kz <= L) {
-            v = tab_z<float>(kp, b, kz < 0 ? -kz : kz, s);
+            v = tab_z(kp, b, kz < 0 ? -kz : kz, s);
             if (kz < 0) v = cconj(v);
         }
         ez[j] = v;
@@ -655,8 +610,8 @@ __global__ void __launch_bounds__(FF_NT) k_field_f(KP kp, int s0, int s1) {
         for (int rl = 0; rl < nr; rl++) {
             const int4 ri = rinfo[rl];
             const float2 kv = rkv[rl];
-            const float2 ex = tab_x<float>(kp, b, ri.x, s);
-            const float2 ey = tab_y<float>(kp, b, ri.y, s);
+            const float2 ex = tab_x(kp, b, ri.x, s);
+            const float2 ey = tab_y(kp, b, ri.y, s);
             const float2 exy = make_float2(ex.x * ey.x - ex.y * ey.y, ex.y * ey.x + ex.x * ey.y);
             FAcc a;
             a.U0 = a.U1 = a.V0 = a.V1 = a.V2 = make_float2(0.f, 0.f);
@@ -877,19 +832,19 @@ static int spass_groups(const Engine &E, int nsites) {
     return g;
 }
 
-template <int OP, typename R>
+template <int OP>
 static void run_spass_t(Engine &E, int s0, int nsites, int skipconv) {
     const int ng = spass_groups(E, nsites);
     const int ntile = (nsites + SP_TS - 1) / SP_TS;
     const int tsg = ((ntile + ng - 1) / ng) * SP_TS;
     const int ngr = (nsites + tsg - 1) / tsg;
     const int LZ = 2 * E.kp.lmax + 1;
-    const size_t smem = ((size_t)SP_TS * LZ * 2 + (size_t)SP_TS * E.max_runs_chunk * 3 + (size_t)SP_TS * 4) * sizeof(R);
+    const size_t smem = ((size_t)SP_TS * LZ * 2 + (size_t)SP_TS * E.max_runs_chunk * 3 + (size_t)SP_TS * 4) * sizeof(float);
     dim3 g(E.nchunk, ngr, E.kp.P);
-    k_spass<OP, R><<<g, SP_NT, smem, E.stream>>>(E.kp, s0, nsites, tsg, ngr, skipconv);
+    k_spass<OP><<<g, SP_NT, smem, E.stream>>>(E.kp, s0, nsites, tsg, ngr, skipconv);
     ++E.nlaunch;
     dim3 g2((E.kp.nk + 255) / 256, E.kp.P);
-    k_sreduce<OP, R><<<g2, 256, 0, E.stream>>>(E.kp, ngr, skipconv);
+    k_sreduce<OP><<<g2, 256, 0, E.stream>>>(E.kp, ngr, skipconv);
     if (OP != OP_DIP) E.tp_vslot = -1;
     ++E.nlaunch;
 }
@@ -919,7 +874,7 @@ static void run_sfac_f(Engine &E, int s0, int nsites, int skipconv) {
     k_sfac_f<OP><<<g, SF_RT * E.sf_nkg_max, smem, E.stream>>>(E.kp, s0, nsites, tsg, ngr, skipconv);
     ++E.nlaunch;
     dim3 g2((kp.nk + 255) / 256, kp.P);
-    k_sreduce<OP, float><<<g2, 256, 0, E.stream>>>(E.kp, ngr, skipconv);
+    k_sreduce<OP><<<g2, 256, 0, E.stream>>>(E.kp, ngr, skipconv);
     if (OP != OP_DIP) E.tp_vslot = -1;
     ++E.nlaunch;
 }
@@ -932,7 +887,7 @@ static void run_spass(Engine &E, int s0, int nsites, int skipconv) {
         if (E.sf_tiled && E.sf_nkg_max * SF_RT <= SF_MAXT)
             run_sfac_f<OP>(E, s0, nsites, skipconv);
         else
-            run_spass_t<OP, float>(E, s0, nsites, skipconv);
+            run_spass_t<OP>(E, s0, nsites, skipconv);
     } else {
         launch_dg_sfac(E, OP, s0, nsites, skipconv);
     }
@@ -971,17 +926,17 @@ static int wave_split(const Engine &E, K kernel, int threads, size_t smem, long 
     return best;
 }
 
-template <int MODE, int NT, typename R>
+template <int MODE, int NT>
 static void launch_field_nt(Engine &E, int s0, int s1) {
     const int LZ = 2 * E.kp.lmax + 1;
-    const size_t smem = ((size_t)LZ * NT * 2 + (size_t)KCH * 5) * sizeof(R);
+    const size_t smem = ((size_t)LZ * NT * 2 + (size_t)KCH * 5) * sizeof(float);
     // k-slices: enough blocks for ~8 (FP32) / ~4 (FP64) resident blocks per SM
     const int sblocks = (s1 - s0 + NT - 1) / NT;
-    const long want = (sizeof(R) == 4 ? 8L : 4L) * 152;
+    const long want = 8L * 152;
     int ns = (int)((want + (long)sblocks * E.kp.P - 1) / ((long)sblocks * E.kp.P));
     ns = std::max(1, std::min(ns, std::min(E.nchunk, E.max_slices)));
     dim3 g(sblocks, E.kp.P, ns);
-    k_field<MODE, NT, R><<<g, NT, smem, E.stream>>>(E.kp, s0, s1);
+    k_field<MODE, NT><<<g, NT, smem, E.stream>>>(E.kp, s0, s1);
     dim3 g2((s1 - s0 + 127) / 128, E.kp.P);
     k_field_finish<MODE, 128><<<g2, 128, 0, E.stream>>>(E.kp, s0, s1, ns);
     E.nlaunch += 2;
@@ -1047,9 +1002,9 @@ static void run_field(Engine &E, int s0, int s1) {
     }
     if (E.precision == PIMD_PREC_MIXED) {
         if ((size_t)LZ * 128 * 8 <= 64 * 1024)
-            launch_field_nt<MODE, 128, float>(E, s0, s1);
+            launch_field_nt<MODE, 128>(E, s0, s1);
         else
-            launch_field_nt<MODE, 64, float>(E, s0, s1);
+            launch_field_nt<MODE, 64>(E, s0, s1);
     } else {
         const int ns = launch_dg_field(E, MODE, s0, s1, 0);
         if (MODE == F_D) return;  // (the update is part of the pass)
@@ -1065,18 +1020,17 @@ static void run_field(Engine &E, int s0, int s1) {
 }
 
 // dynamic shared-memory limits of the Ewald kernels, set once per context on its device
-template <typename R>
 static void ewald_attrs() {
     const int lim = 200 * 1024;
-    cudaFuncSetAttribute(k_spass<OP_Q, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    cudaFuncSetAttribute(k_spass<OP_MU, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    cudaFuncSetAttribute(k_spass<OP_DIP, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    cudaFuncSetAttribute(k_field<F_Q, 128, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    cudaFuncSetAttribute(k_field<F_D, 128, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    cudaFuncSetAttribute(k_field<F_QD, 128, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    cudaFuncSetAttribute(k_field<F_Q, 64, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    cudaFuncSetAttribute(k_field<F_D, 64, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    cudaFuncSetAttribute(k_field<F_QD, 64, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+    cudaFuncSetAttribute(k_spass<OP_Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+    cudaFuncSetAttribute(k_spass<OP_MU>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+    cudaFuncSetAttribute(k_spass<OP_DIP>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+    cudaFuncSetAttribute(k_field<F_Q, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+    cudaFuncSetAttribute(k_field<F_D, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+    cudaFuncSetAttribute(k_field<F_QD, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+    cudaFuncSetAttribute(k_field<F_Q, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+    cudaFuncSetAttribute(k_field<F_D, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+    cudaFuncSetAttribute(k_field<F_QD, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
 }
 // Tiles of the register-tiled structure factor: runs sorted by kz extent (longest first), 32 per
 // tile; each tile records the first ez slot of its kz window and the number of kz groups.
@@ -1118,7 +1072,7 @@ static int sfac_tiles(Engine &E) {
 void ewald_init(Engine &E) {
     if (sfac_tiles(E) != 0) E.sf_tiled = false;  // allocation failed: untiled kernel
     tc_init(E);
-    ewald_attrs<float>();
+    ewald_attrs();
     // k_field_f stages [1 or 2][64 runs][LZM] complex weights: 50 KB for LZM = 49 in QD mode
 #define PIMD_FF_ATTR(MODE, LZM) cudaFuncSetAttribute(k_field_f<MODE, LZM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
     PIMD_FF_ATTR(F_Q, 17) PIMD_FF_ATTR(F_D, 17) PIMD_FF_ATTR(F_QD, 17)
@@ -1161,10 +1115,10 @@ void adj_structure_factor(Engine &E, const double *dipbuf, const float4 *dipf32,
             if (E.sf_tiled && E.sf_nkg_max * SF_RT <= SF_MAXT)
                 run_sfac_f<OP_MU>(E, E.kp.fd, E.kp.ld - E.kp.fd, 1);
             else
-                run_spass_t<OP_MU, float>(E, E.kp.fd, E.kp.ld - E.kp.fd, 1);
+                run_spass_t<OP_MU>(E, E.kp.fd, E.kp.ld - E.kp.fd, 1);
         }
     } else if (E.precision == PIMD_PREC_MIXED) {
-        run_spass_t<OP_MU, float>(E, E.kp.fd, E.kp.ld - E.kp.fd, 1);
+        run_spass_t<OP_MU>(E, E.kp.fd, E.kp.ld - E.kp.fd, 1);
     } else {
         launch_dg_sfac(E, OP_MU, E.kp.fd, E.kp.ld - E.kp.fd, 1);
     }
@@ -1189,17 +1143,17 @@ __global__ void __launch_bounds__(128) k_adj_fsum(KP kp, int s0, int s1, int nsl
     o[2] += E[2];
 }
 
-template <int NT, typename R>
+template <int NT>
 static void adj_field_t(Engine &E, double *Dr) {
     const int s0 = E.kp.fd, s1 = E.kp.ld;
     const int LZ = 2 * E.kp.lmax + 1;
-    const size_t smem = ((size_t)LZ * NT * 2 + (size_t)KCH * 5) * sizeof(R);
+    const size_t smem = ((size_t)LZ * NT * 2 + (size_t)KCH * 5) * sizeof(float);
     const int sblocks = (s1 - s0 + NT - 1) / NT;
-    const long want = (sizeof(R) == 4 ? 8L : 4L) * 152;
+    const long want = 8L * 152;
     int ns = (int)((want + (long)sblocks * E.kp.P - 1) / ((long)sblocks * E.kp.P));
     ns = std::max(1, std::min(ns, std::min(E.nchunk, E.max_slices)));
     dim3 g(sblocks, E.kp.P, ns);
-    k_field<F_D, NT, R><<<g, NT, smem, E.stream>>>(E.kp, s0, s1);
+    k_field<F_D, NT><<<g, NT, smem, E.stream>>>(E.kp, s0, s1);
     dim3 g2((s1 - s0 + 127) / 128, E.kp.P);
     k_adj_fsum<<<g2, 128, 0, E.stream>>>(E.kp, s0, s1, ns, Dr);
     E.nlaunch += 2;
@@ -1238,9 +1192,9 @@ void adj_dipole_field(Engine &E, double2 *Sm_u, double *bacc, double *Dr) {
             adj_field_f<49>(E, Dr);
     } else if (E.precision == PIMD_PREC_MIXED) {
         if ((size_t)LZ * 128 * 8 <= 64 * 1024)
-            adj_field_t<128, float>(E, Dr);
+            adj_field_t<128>(E, Dr);
         else
-            adj_field_t<64, float>(E, Dr);
+            adj_field_t<64>(E, Dr);
     } else {
         const int s0 = E.kp.fd, s1 = E.kp.ld, ns = launch_dg_field(E, F_D, s0, s1, 1);
         k_adj_fsum<<<dim3((s1 - s0 + 127) / 128, E.kp.P), 128, 0, E.stream>>>(E.kp, s0, s1, ns, Dr);
@@ -1271,28 +1225,26 @@ template <int MODE>
 __global__ void __launch_bounds__(128) k_adj_rec(KP kp, int s0, int s1, const double *a, const double *bvec,
                                                  const double2 *SA, const double2 *SB, const double *ebw,
                                                  double *grad, double *phi) {
-    using R = float;
-    using V = float2;
-    __shared__ R sk[KCH][4];            // kx, ky, kz, c_k
-    __shared__ R s1x[KCH][2], s2x[KCH][2];  // BIL: conj(raw S_u), conj(raw S_v); CROSS: raw S_q, conj(raw S_nu)
+    __shared__ float sk[KCH][4];            // kx, ky, kz, c_k
+    __shared__ float s1x[KCH][2], s2x[KCH][2];  // BIL: conj(raw S_u), conj(raw S_v); CROSS: raw S_q, conj(raw S_nu)
     const int b = blockIdx.y, s = s0 + blockIdx.x * blockDim.x + threadIdx.x;
     if (ebw[b] == 0.0) return;  // the whole block: bead inactive
     const bool valid = s < s1;
     const size_t gs = (size_t)b * kp.S + (valid ? s : s0);
-    const R q = valid ? R(kp.pos[gs].w) : R(0);
+    const float q = valid ? (float)kp.pos[gs].w : 0.f;
     const bool isdip = valid && s >= kp.fd && s < kp.ld;
     const bool act = (MODE == ADJ_BIL) ? isdip : valid;
-    R av[3] = {R(0), R(0), R(0)}, bv[3] = {R(0), R(0), R(0)};
+    float av[3] = {0.f, 0.f, 0.f}, bv[3] = {0.f, 0.f, 0.f};
     if (isdip) {
         for (int c = 0; c < 3; c++) {
-            av[c] = R(a[3 * gs + c]);
-            if (MODE == ADJ_BIL) bv[c] = R(bvec[3 * gs + c]);
+            av[c] = (float)a[3 * gs + c];
+            if (MODE == ADJ_BIL) bv[c] = (float)bvec[3 * gs + c];
         }
     }
     // this site's kz table column in shared memory (dynamic, (lmax + 1) x 128), read in
     // the k loop instead of from the global table
     extern __shared__ float2 adj_ez[];
-    for (int n = 0; n <= kp.lmax; n++) adj_ez[n * 128 + threadIdx.x] = valid ? tab_z<float>(kp, b, n, s) : make_float2(0.f, 0.f);
+    for (int n = 0; n <= kp.lmax; n++) adj_ez[n * 128 + threadIdx.x] = valid ? tab_z(kp, b, n, s) : make_float2(0.f, 0.f);
     double G[3] = {0, 0, 0}, ph = 0.0;
     const int slice = blockIdx.z, nslice = gridDim.z;
     const int c0 = (int)((long)slice * kp.nchunk / nslice), c1 = (int)((long)(slice + 1) * kp.nchunk / nslice);
@@ -1302,49 +1254,49 @@ __global__ void __launch_bounds__(128) k_adj_rec(KP kp, int s0, int s1, const do
         for (int i = threadIdx.x; i < ch.k1 - ch.k0; i += blockDim.x) {
             const int k = ch.k0 + i;
             const double4_32a ki = kp.kinfo[k];
-            sk[i][0] = R(ki.x);
-            sk[i][1] = R(ki.y);
-            sk[i][2] = R(ki.z);
-            sk[i][3] = R(ki.w);
+            sk[i][0] = (float)ki.x;
+            sk[i][1] = (float)ki.y;
+            sk[i][2] = (float)ki.z;
+            sk[i][3] = (float)ki.w;
             const double2 x1 = (MODE == ADJ_BIL) ? SA[(size_t)b * kp.nk + k] : kp.Sq[(size_t)b * kp.nk + k];
             const double2 x2 = (MODE == ADJ_BIL) ? SB[(size_t)b * kp.nk + k] : SA[(size_t)b * kp.nk + k];
             // rotated (-Im, Re) forms: conj(raw) = (y, x); the raw charge structure factor as is
-            s1x[i][0] = (MODE == ADJ_BIL) ? R(x1.y) : R(x1.x);
-            s1x[i][1] = (MODE == ADJ_BIL) ? R(x1.x) : R(x1.y);
-            s2x[i][0] = R(x2.y);
-            s2x[i][1] = R(x2.x);
+            s1x[i][0] = (MODE == ADJ_BIL) ? (float)x1.y : (float)x1.x;
+            s1x[i][1] = (MODE == ADJ_BIL) ? (float)x1.x : (float)x1.y;
+            s2x[i][0] = (float)x2.y;
+            s2x[i][1] = (float)x2.x;
         }
         __syncthreads();
         if (!act) continue;
-        // per-chunk partial sums in R, added to the FP64 totals once per chunk (FP64 is a narrow
+        // per-chunk partial sums in FP32, added to the FP64 totals once per chunk (FP64 is a narrow
         // pipe on this part)
-        R Gr[3] = {R(0), R(0), R(0)}, phr = R(0);
+        float Gr[3] = {0.f, 0.f, 0.f}, phr = 0.f;
         for (int r = ch.r0; r < ch.r1; r++) {
             const KRun run = kp.runs[r];
-            const V ex = tab_x<R>(kp, b, run.kx, s);
-            const V ey = tab_y<R>(kp, b, run.ky, s);
-            const V exy = make_float2(ex.x * ey.x - ex.y * ey.y, ex.y * ey.x + ex.x * ey.y);
+            const float2 ex = tab_x(kp, b, run.kx, s);
+            const float2 ey = tab_y(kp, b, run.ky, s);
+            const float2 exy = make_float2(ex.x * ey.x - ex.y * ey.y, ex.y * ey.x + ex.x * ey.y);
             const int i0 = run.kbeg - ch.k0;
             for (int j = 0; j < run.nkz; j++) {
                 const int kz = run.kzlo + j, i = i0 + j;
-                V z = adj_ez[(kz < 0 ? -kz : kz) * 128 + threadIdx.x];
+                float2 z = adj_ez[(kz < 0 ? -kz : kz) * 128 + threadIdx.x];
                 if (kz < 0) z = cconj(z);
-                const V e = make_float2(exy.x * z.x - exy.y * z.y, exy.y * z.x + exy.x * z.y);
-                const R kv[3] = {sk[i][0], sk[i][1], sk[i][2]}, ck = sk[i][3];
+                const float2 e = make_float2(exy.x * z.x - exy.y * z.y, exy.y * z.x + exy.x * z.y);
+                const float kv[3] = {sk[i][0], sk[i][1], sk[i][2]}, ck = sk[i][3];
                 if (MODE == ADJ_BIL) {
-                    const R imu = e.x * s1x[i][1] + e.y * s1x[i][0], imv = e.x * s2x[i][1] + e.y * s2x[i][0];
-                    const R ku = kv[0] * av[0] + kv[1] * av[1] + kv[2] * av[2];
-                    const R kw = kv[0] * bv[0] + kv[1] * bv[1] + kv[2] * bv[2];
-                    const R f = ck * (ku * imv + kw * imu);
+                    const float imu = e.x * s1x[i][1] + e.y * s1x[i][0], imv = e.x * s2x[i][1] + e.y * s2x[i][0];
+                    const float ku = kv[0] * av[0] + kv[1] * av[1] + kv[2] * av[2];
+                    const float kw = kv[0] * bv[0] + kv[1] * bv[1] + kv[2] * bv[2];
+                    const float f = ck * (ku * imv + kw * imu);
                     for (int c = 0; c < 3; c++) Gr[c] += f * kv[c];
                 } else {
                     if (isdip) {
-                        const R re = e.x * s1x[i][0] + e.y * s1x[i][1];  // Re(e conj Sq)
-                        const R kn = kv[0] * av[0] + kv[1] * av[1] + kv[2] * av[2];
+                        const float re = e.x * s1x[i][0] + e.y * s1x[i][1];  // Re(e conj Sq)
+                        const float kn = kv[0] * av[0] + kv[1] * av[1] + kv[2] * av[2];
                         for (int c = 0; c < 3; c++) Gr[c] += ck * kn * re * kv[c];
                     }
-                    if (q != R(0)) {
-                        const R re = e.x * s2x[i][0] - e.y * s2x[i][1], im = e.x * s2x[i][1] + e.y * s2x[i][0];
+                    if (q != 0.f) {
+                        const float re = e.x * s2x[i][0] - e.y * s2x[i][1], im = e.x * s2x[i][1] + e.y * s2x[i][0];
                         for (int c = 0; c < 3; c++) Gr[c] -= q * ck * re * kv[c];
                         phr -= ck * im;
                     }

@@ -111,7 +111,7 @@ PIMD_D float gq_h(const float4 *tab, float u) {
     return c.x + t * (c.y + t * (c.z + t * c.w));
 }
 
-// smear01<float> (smear.f90:2-34) with the tabulated Q(2/3, x)
+// PBCsmear01 (smear.f90:2-34) in FP32 with the tabulated Q(2/3, x)
 PIMD_D void smear01_m(float drsq, float a_pol12, float ra, const EwCf &e, const float4 *gq, float *ts0, float *ts1) {
     float dd, dri;
     rinv<float>(drsq, dd, dri);

@@ -21,7 +21,6 @@ struct NasaConst {
     unsigned char pg[NASA_PG][4], dg[NASA_DG][4];
     short ps[NASA_PS], ds[NASA_DS];
     int ngrp[2];  // groups of the PES and of the DMS
-    unsigned char idx[245][3], idxD[84][3];
 };
 static __constant__ NasaConst c_nasa;
 
@@ -58,16 +57,10 @@ static inline void nasa_upload_constants() {
         h.c5z[j] = PIMD_NASA_F5Z * PIMD_NASA_C5ZA[j] + PIMD_NASA_FBASIS * PIMD_NASA_CBASIS[j] +
                    PIMD_NASA_FCORE * PIMD_NASA_CCORE[j] + PIMD_NASA_FREST * PIMD_NASA_CREST[j];
         h.c5zf[j] = (float)h.c5z[j];
-        h.idx[j][0] = (unsigned char)PIMD_NASA_IDX1[j];
-        h.idx[j][1] = (unsigned char)PIMD_NASA_IDX2[j];
-        h.idx[j][2] = (unsigned char)PIMD_NASA_IDX3[j];
     }
     for (int j = 0; j < 84; j++) {
         h.coefD[j] = PIMD_NASA_COEFD[j];
         h.coefDf[j] = (float)PIMD_NASA_COEFD[j];
-        h.idxD[j][0] = (unsigned char)PIMD_NASA_IDXD1[j];
-        h.idxD[j][1] = (unsigned char)PIMD_NASA_IDXD2[j];
-        h.idxD[j][2] = (unsigned char)PIMD_NASA_IDXD3[j];
     }
     for (short &x : h.ps) x = -1;
     for (short &x : h.ds) x = -1;

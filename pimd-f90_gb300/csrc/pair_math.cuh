@@ -31,8 +31,8 @@ PIMD_D void pair_r(double d2, const EwC &e, PairR &p) {
     p.t1 = (p.t0 + e.cts1 * p.g) * p.drsqi;
 }
 
-// Q(2/3, x) as gammq2_3 leaves it, with the number of terms from the bounds in tb and
-// pre = x^(2/3) exp(-x) / Gamma(2/3). The continued fraction's convergent by the forward recurrence
+// Q(2/3, x) as the reference's gammq2_3 leaves it (math.f90:188-285), with the number of terms from
+// the bounds in tb and pre = x^(2/3) exp(-x) / Gamma(2/3). The continued fraction's convergent by the forward recurrence
 // of its numerators and denominators (no division until the end).
 PIMD_D double thole_q23(double x, double pre, const GqBounds &tb, unsigned *err) {
     const double a = 2.0 / 3.0;
