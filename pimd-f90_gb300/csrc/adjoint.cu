@@ -894,6 +894,7 @@ int pimd_pot_backward(pimd_ctx *ctx, const double *Ebar, double *dRRt, double *d
     cudaMemcpyAsync(th.data(), thacc, sizeof(double) * PIMD_NTHETA, cudaMemcpyDeviceToHost, st);
     if (dRRt) cudaMemcpyAsync(dRRt, dR, sizeof(double) * P * kp.natoms * 3, cudaMemcpyDeviceToHost, st);
     cudaError_t e = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) e = cudaGetLastError();  // (a launch that was refused)
     if (e != cudaSuccess) return adj_fail(E, PIMD_ERR_CUDA, cudaGetErrorString(e));
     double esum = 0;
     for (size_t b = 0; b < P; b++) esum += Ebar[b];

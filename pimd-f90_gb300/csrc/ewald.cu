@@ -1364,7 +1364,7 @@ void adj_rec(Engine &E, int mode, const double *a, const double *bvec, const dou
                                         std::min(E.kp.nchunk, E.max_slices)));
     dim3 g(sblocks, E.kp.P, ns), g2(sblocks, E.kp.P);
     const size_t ezb = sizeof(float2) * 128 * (E.kp.lmax + 1);  // FP32 kz column, <= 128 KB (lmax <= 127)
-    if (ezb > 48 * 1024) {
+    if (ezb + 16 * 1024 > 48 * 1024) {  // (beside the staged k-vectors: 8 KB)
         cudaFuncSetAttribute(k_adj_rec<ADJ_BIL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ezb);
         cudaFuncSetAttribute(k_adj_rec<ADJ_CROSS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ezb);
     }

@@ -73,3 +73,18 @@ def test_virial_sums_of_large_shells(pkg, engine_lib, nw, P, nmax):
         m = torch.from_numpy(mu[b]).cuda()
         ref = torch.stack([torch.cos(ph) @ m, torch.sin(ph) @ m], -1).cpu().numpy()
         assert rms(got[b], ref) < 4e-7
+
+
+@pytest.mark.parametrize("nmax", [38, 42, 47, 48, 64])
+def test_gradients_of_large_shells(pkg, engine_lib, nmax):
+    """The backward of boxes whose k shell leaves the tensor cores, where its kz column passes 48 KB of shared memory with
+    and without the words beside it (|kz| from 40): the mixed gradients' budget, 1e-4 rms of the FP64 engine's."""
+    p, RRt, RRc = params(pkg, 6, 2, (1, 1, 1), nmax)
+    out = []
+    for prec in (0, 1):
+        eng = pkg.ForceEngine(p, precision=prec)
+        eng.pot_forward(RRt, RRc)
+        out.append(eng.pot_backward(np.array([1.0, 0.5])))
+        eng.close()
+    for a, b in zip(out[1], out[0]):
+        assert rms(a, b) < 1e-4
