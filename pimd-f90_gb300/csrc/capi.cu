@@ -200,6 +200,8 @@ static int create(Engine &E, const pimd_params *p, int nrep, const int *brep) {
     int rc = cuda_check(E, cudaSetDevice(p->device), "cudaSetDevice");
     if (rc) return rc;
     E.device = p->device;
+    cudaDeviceGetAttribute(&E.nsm, cudaDevAttrMultiProcessorCount, E.device);
+    if (E.nsm <= 0) E.nsm = 152;
     E.precision = p->precision;
     rc = cuda_check(E, cudaStreamCreateWithFlags(&E.stream, cudaStreamNonBlocking), "stream");
     if (rc) return rc;

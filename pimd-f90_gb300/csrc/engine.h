@@ -302,11 +302,12 @@ struct Engine {
     bool wave_shapes = true;  // k-slices / site groups chosen by wave quantisation (occupancy API)
     bool dd_overlap = true;   // mixed engine: real-space dipole field beside the structure factor
     bool dd_async = false;    // ... and beside the field pass too, the SOR by the last to finish (TTM3-F)
-    // tensor-core (tcgen05, 3xTF32) dipole structure factor of the mixed engine (ewald_tc.cu)
+    int nsm = 152;            // SMs of the device
+    // tensor-core (tcgen05, FP16 hi + lo) structure factors of the mixed engine (ewald_tc.cu)
     bool sf_tc = true;        // use it when tc_ready
     bool tc_ready = false;    // run groups built and the table tensor map encoded
     bool tc_dip_ok = false;   // the dipole-component sums (three partials per k-vector) take them too
-    int tc_nsm = 152, tc_ng224 = 1, tc_nband = 0;
+    int tc_nsplit = 1, tc_nband = 0;
     int tc_ntg = 0, tc_ncolmax = 0, tc_nabuf = 0;
     const int4 *d_tcslot = nullptr;   // per run slot: run, local k offset, kzlo, nkz
     const float2 *d_tcskv = nullptr;  // per run slot: FP32 (k_x, k_y)

@@ -825,7 +825,7 @@ static void launch_qd_virial(Engine &E, bool dip) {
 static int spass_groups(const Engine &E, int nsites) {
     const int ntile = (nsites + SP_TS - 1) / SP_TS;
     const long per = (long)E.nchunk * E.kp.P;
-    int g = (int)((152L * 8 + per - 1) / per);
+    int g = (int)((8L * E.nsm + per - 1) / per);
     if (g < 1) g = 1;
     if (g > ntile) g = ntile;
     if (g > E.sp_cap) g = E.sp_cap;
@@ -866,7 +866,7 @@ static void run_sfac_f(Engine &E, int s0, int nsites, int skipconv) {
     else if (E.wave_shapes)
         ng = wave_split(E, k_sfac_f<OP>, SF_RT * E.sf_nkg_max, smem, per, gmax);
     else
-        ng = (int)((152L * 8 + per - 1) / per);
+        ng = (int)((8L * E.nsm + per - 1) / per);
     ng = std::max(1, std::min(ng, gmax));
     const int tsg = ((ntile + ng - 1) / ng) * SF_TS;
     const int ngr = (nsites + tsg - 1) / tsg;
@@ -897,22 +897,11 @@ static void run_spass(Engine &E, int s0, int nsites, int skipconv) {
 // ceil(B / (SMs R)) waves; when the split count c divides the work (each block does ~1/c of it),
 // the time goes as waves(c) / c. Pick the c in [1, cmax] that minimises it (ties: smallest c,
 // fewest partials to add afterwards). R comes from the occupancy calculator for the kernel.
-static int sm_count(const Engine &E) {
-    static int cached[64] = {0};
-    const int d = E.device & 63;
-    if (!cached[d]) {
-        int n = 0;
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, E.device);
-        cached[d] = n > 0 ? n : 152;
-    }
-    return cached[d];
-}
-
 template <typename K>
 static int wave_split(const Engine &E, K kernel, int threads, size_t smem, long base_blocks, int cmax) {
     int R = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&R, kernel, threads, smem);
-    const long slots = (long)sm_count(E) * std::max(R, 1);
+    const long slots = (long)E.nsm * std::max(R, 1);
     int best = 1;
     double best_t = 1e300;
     for (int c = 1; c <= std::max(1, cmax); c++) {
@@ -932,7 +921,7 @@ static void launch_field_nt(Engine &E, int s0, int s1) {
     const size_t smem = ((size_t)LZ * NT * 2 + (size_t)KCH * 5) * sizeof(float);
     // k-slices: enough blocks for ~8 (FP32) / ~4 (FP64) resident blocks per SM
     const int sblocks = (s1 - s0 + NT - 1) / NT;
-    const long want = 8L * 152;
+    const long want = 8L * E.nsm;
     int ns = (int)((want + (long)sblocks * E.kp.P - 1) / ((long)sblocks * E.kp.P));
     ns = std::max(1, std::min(ns, std::min(E.nchunk, E.max_slices)));
     dim3 g(sblocks, E.kp.P, ns);
@@ -948,7 +937,7 @@ static void launch_field_f(Engine &E, int s0, int s1) {
     const int sblocks = (s1 - s0 + FF_NT - 1) / FF_NT;
     const int cmax = std::min(E.nchunk, E.max_slices);
     const int ns = E.wave_shapes ? wave_split(E, k_field_f<MODE, LZM>, FF_NT, smem, (long)sblocks * E.kp.P, cmax)
-                                 : std::max(1, std::min((int)((8L * 152 + (long)sblocks * E.kp.P - 1) /
+                                 : std::max(1, std::min((int)((8L * E.nsm + (long)sblocks * E.kp.P - 1) /
                                                               ((long)sblocks * E.kp.P)), cmax));
     dim3 g(sblocks, E.kp.P, ns);
     k_field_f<MODE, LZM><<<g, FF_NT, smem, E.stream>>>(E.kp, s0, s1);
@@ -1149,7 +1138,7 @@ static void adj_field_t(Engine &E, double *Dr) {
     const int LZ = 2 * E.kp.lmax + 1;
     const size_t smem = ((size_t)LZ * NT * 2 + (size_t)KCH * 5) * sizeof(float);
     const int sblocks = (s1 - s0 + NT - 1) / NT;
-    const long want = 8L * 152;
+    const long want = 8L * E.nsm;
     int ns = (int)((want + (long)sblocks * E.kp.P - 1) / ((long)sblocks * E.kp.P));
     ns = std::max(1, std::min(ns, std::min(E.nchunk, E.max_slices)));
     dim3 g(sblocks, E.kp.P, ns);
@@ -1165,7 +1154,7 @@ static void adj_field_f(Engine &E, double *Dr) {
     const size_t smem = sizeof(float2) * FF_RUNS * LZM;
     const int sblocks = (s1 - s0 + FF_NT - 1) / FF_NT;
     const int cmax = std::min(E.nchunk, E.max_slices);
-    const int ns = std::max(1, std::min((int)((8L * 152 + (long)sblocks * E.kp.P - 1) / ((long)sblocks * E.kp.P)), cmax));
+    const int ns = std::max(1, std::min((int)((8L * E.nsm + (long)sblocks * E.kp.P - 1) / ((long)sblocks * E.kp.P)), cmax));
     dim3 g(sblocks, E.kp.P, ns);
     k_field_f<F_D, LZM><<<g, FF_NT, smem, E.stream>>>(E.kp, s0, s1);
     dim3 g2((s1 - s0 + 127) / 128, E.kp.P);
@@ -1360,7 +1349,7 @@ void adj_rec(Engine &E, int mode, const double *a, const double *bvec, const dou
         }
         return;
     }
-    const int ns = std::max(1, std::min((int)((8L * 152 + (long)sblocks * E.kp.P - 1) / ((long)sblocks * E.kp.P)),
+    const int ns = std::max(1, std::min((int)((8L * E.nsm + (long)sblocks * E.kp.P - 1) / ((long)sblocks * E.kp.P)),
                                         std::min(E.kp.nchunk, E.max_slices)));
     dim3 g(sblocks, E.kp.P, ns), g2(sblocks, E.kp.P);
     const size_t ezb = sizeof(float2) * 128 * (E.kp.lmax + 1);  // FP32 kz column, <= 128 KB (lmax <= 127)

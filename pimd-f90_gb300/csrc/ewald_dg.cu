@@ -923,7 +923,7 @@ static void sfac(Engine &E, int s0, int nsites, int skipconv) {
     const int nks = ceil_div(nsites, 16), nmt = ceil_div(NC * a.jn, 8);
     // blocks of the Z kernel: enough to fill the chip, few enough that finding the bead's largest
     // weight (each block reads all of them) stays small
-    const int upb = std::max(1, (int)((long)nmt * nks * kp.P / (8L * 608)));
+    const int upb = std::max(1, (int)((long)nmt * nks * kp.P / (8L * 4 * E.nsm)));
     const int nzb = ceil_div(ceil_div(nmt * nks, 8), upb);
     const bool have = OP != OP_Q && E.dg_xdip;
     const int nbmax = have ? kp.P : std::max(1, a.xsteps / nks);
@@ -982,7 +982,7 @@ static int field(Engine &E, int s0, int s1, int sor, const double *dip2 = nullpt
     const int mb = ceil_div(ceil_div(s1, 16) - s0 / 16, 4), tiles = MODE == DGF_DG ? a.nvd8 : a.nv8;
     // slices of the runs, at least four tiles each: the count whose waves of four blocks a SM do
     // the work soonest (512 x 32: 7 slices, 2.9 waves; 3 slices were 1.3 waves)
-    const long base = (long)mb * kp.P, room = 152L * 4;
+    const long base = (long)mb * kp.P, room = 4L * E.nsm;
     int ns = 1;
     double best = 1e300;
     const int most = dip2 ? E.max_slices / 2 : E.max_slices;

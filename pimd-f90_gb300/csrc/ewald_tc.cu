@@ -1392,11 +1392,11 @@ void tc_init(Engine &E) {
     // the field passes' tables, and where their V has the rows of each run's pair (its offset, to the lo rows, |kz| rows)
     std::vector<int4> place;
     tp_setup(E, enc, jr, &place);
-    E.tc_ng224 = 0;
+    E.tc_nsplit = 0;
     for (int p0 = 0; p0 < nslot;) {
         int n = 0;
         while (p0 + n < nslot && src[p0 + n].y == src[p0].y) n++;
-        E.tc_ng224 += (n + 223) / 224;
+        E.tc_nsplit += (n + TC_BOXRUN - 1) / TC_BOXRUN;
         p0 += n;
     }
     std::vector<int4> slots(nslot);
@@ -1535,8 +1535,6 @@ void tc_init(Engine &E) {
     E.tc_nband = (int)std::count_if(groups.begin(), groups.end(), [](const TcGroup &g) { return g.j0 > 0; });
     E.tc_ncolmax = ncolmax;
     E.tc_nabuf = nabuf;
-    cudaDeviceGetAttribute(&E.tc_nsm, cudaDevAttrMultiProcessorCount, E.device);
-    if (E.tc_nsm <= 0) E.tc_nsm = 152;
     E.tc_ready = true;
     E.tf_ready = E.tp[0].V != nullptr;
     E.tf_qd_ready = E.tf_ready && E.tp[1].V != nullptr;
@@ -1676,11 +1674,13 @@ int launch_sfac_tc(Engine &E, int op, int s0, int nsites, int skipconv) {
     // the iterations' structure factor follows the previous iteration's field pass on the stream
     // (or the charge passes, which need no overlap): its CTAs are scheduled as that grid drains
     a.pdl = (op == TC_OP_MU && skipconv && E.tc_pdl && E.tf_ready && E.ff_tc) ? 1 : 0;
-    // one CTA per SM (shared memory); site groups (= cluster size) so that one wave fills the GPU with groups of
-    // 224 runs. Their number sets how many sites an accumulator adds up, which at 4096 sites shows in the dipoles:
-    // four groups instead of one moved them by 4e-5 (rms)
+    // one CTA per SM (shared memory); site groups (= cluster size) so that one wave fills the GPU if the runs were in
+    // groups of TC_BOXRUN. The launch's own groups may be larger; the site groups stay those, since their number sets
+    // how many sites an accumulator, which cuts off, adds up, and with it the result: 4096 x 32 has one group, and its
+    // dipoles are off by 4.4e-5 (rms, against the FP64 engine); in four groups, by the waves of the launch's own run
+    // groups, they move by 4e-5
     const int nst = (a.s_hi - a.sbase + TC_SS - 1) / TC_SS;
-    int ng = std::max(1, std::min((int)std::max(1L, E.tc_nsm / ((long)E.tc_ng224 * kp.P)), std::min(nst, TC_CLMAX)));
+    int ng = std::max(1, std::min((int)std::max(1L, E.nsm / ((long)E.tc_nsplit * kp.P)), std::min(nst, TC_CLMAX)));
     const int spg = (nst + ng - 1) / ng;
     ng = (nst + spg - 1) / spg;
     a.ntg = E.tc_ntg;
@@ -1749,7 +1749,7 @@ int launch_sfac_tc(Engine &E, int op, int s0, int nsites, int skipconv) {
     // not one of a few whole CTAs (4096 x 32: 160 on 152 SMs, 398 us an iteration; 275 so). Their k-vectors have |kz| > 20 and weights of 1e-6
     // of the largest, so that their shorter sums leave the dipoles as they are.
     const int main_groups = E.tc_ntg - E.tc_nband;
-    const bool split = E.tc_nband > 0 && main_groups > 0 && E.tc_pdl && (long)E.tc_ntg * kp.P > E.tc_nsm;
+    const bool split = E.tc_nband > 0 && main_groups > 0 && E.tc_pdl && (long)E.tc_ntg * kp.P > E.nsm;
     const bool pev = E.sfac_pev_req && op == TC_OP_MU && E.loop_pev;
     const int first = a.pdl;
     cudaError_t e = cudaSuccess;

@@ -314,8 +314,8 @@ static void pair_qq(Engine &E) {
     constexpr int NI = MODEL == 2 ? 4 : 3, PW = 32 / NI;
     const long est = std::max(1L, (long)E.pair_est), P = E.kp.P;
     const long full = (est + 4L * PW * NI - 1) / (4L * PW * NI);
-    if (full * P >= 2 * 152) {
-        const long nb = std::max(1L, std::min(full, (152L * 5 + P - 1) / P));
+    if (full * P >= 2 * E.nsm) {
+        const long nb = std::max(1L, std::min(full, (5L * E.nsm + P - 1) / P));
         k_pair_qq<MODEL, NI><<<dim3((unsigned)nb, (unsigned)P), PQ_NT, 0, E.stream>>>(E.kp);
     } else {
         const long nb = std::max(1L, (est + 4L * PW - 1) / (4L * PW));
@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(PQ_NT) k_pair_force(KP kp) {
 void launch_pair_force(Engine &E) {
     const long P = E.kp.P, pw = E.kp.model == 2 ? 2 : 6;
     const long full = std::max((long)(E.kp.N + 19) / 20, (long)(E.pair_est / (4 * pw)) + 1);
-    const dim3 g((unsigned)std::max(1L, std::min(full, (152L * 4 + P - 1) / P)), (unsigned)P);
+    const dim3 g((unsigned)std::max(1L, std::min(full, (4L * E.nsm + P - 1) / P)), (unsigned)P);
     if (E.kp.model == 2)
         k_pair_force<2><<<g, PQ_NT, 0, E.stream>>>(E.kp);
     else
