@@ -414,15 +414,16 @@ PIMD_D long long dm_warp_sum4(long long (&x)[4]) {
 // products (2^(26 + 26) each, 552 at most) and of the mixed ones with the high half of lo lo (2^(26 + 31)
 // each, 36 a lane), joined once a row: 2^-59 of the row's largest entry or of the largest dipole in a
 // term, below the rounding of FP64 sums (rms error of an iteration's dipoles at 128 sites 7e-17 of them;
-// 1.4e-16 with FP64 sums, 2.9e-16 with 2^52 and 2^54 and each lane's sum rounded, which is 0.2 us
-// shorter), and 20 cycles a product instead of 64. Bound by latency: 4.1 us an iteration of 128 sites in a cluster
-// of 16 CTAs (6.0 with FP64 products).
-// On the mixed engine TTM2.1-F's intramolecular field, the largest of a site's fields, is added by the updating
-// threads from the FP64 tensors and dipoles (six products a component, the dipoles kept a second time in FP64: the
-// same time at 60 x 8, 409 us a call).
+// 1.4e-16 with FP64 sums, 2.9e-16 with 2^52 and 2^54 and each lane's sum rounded, 1 % faster where many
+// small beads share the SMs), and 20 cycles a product instead of 64. Four CTAs a SM (64 registers): 48 spill,
+// and 80 leave small boxes of 64 beads in two waves (32 x 64 790 us a call, 715 so). Bound by latency: 3.9 us an
+// iteration of 128 sites in a cluster of 16 CTAs (6.0 with FP64 products).
+// intra: on the mixed engine TTM2.1-F's intramolecular field, the largest of a site's fields, is added by the updating
+// threads from the FP64 tensors and dipoles (six products a component, the dipoles kept a second time in FP64: 60 x 8
+// 409 us a call as with all in FP32, a step of 30 x 2 347 instead of 336).
 constexpr int DM_MAXROWS = 42;  // of a CTA: their components are four warps' lanes
-template <typename R>
-__global__ void __launch_bounds__(DM_NT) k_dm_solve(KP kp, DmArgs a, int rows) {
+template <typename R, bool INTRA>
+__global__ void __launch_bounds__(DM_NT, sizeof(R) == 8 ? 4 : 0) k_dm_solve(KP kp, DmArgs a, int rows) {
     constexpr bool D = sizeof(R) == 8;
     using W = typename std::conditional<D, int2, float>::type;  // an entry of D in shared memory
     extern __shared__ __align__(16) unsigned char dm_sm[];
@@ -434,7 +435,7 @@ __global__ void __launch_bounds__(DM_NT) k_dm_solve(KP kp, DmArgs a, int rows) {
     int *top = reinterpret_cast<int *>(sums + 128);    // [2][32] their largest dipole component's high word
     int *rexp = top + 64;                              // [44] the rows' scales
     double *ef = reinterpret_cast<double *>(rexp + 44);  // [3 rows + 1] field
-    const bool intra = !D && kp.model == 2;
+    const bool intra = INTRA && kp.model == 2;          // (a branch: without it the FP64 chain is hoisted, 3 % slower)
     double *md = ef + 3 * rows + (rows & 1);            // [2][3][ndp] intra: the dipoles in FP64
     R *mu = reinterpret_cast<R *>(md + (intra ? 6 * ndp : 0));  // [2][3][ndp]
     W *mf = reinterpret_cast<W *>(mu + 6 * ndp);       // [3][ndp] FP64 engine: the dipoles in fixed point
@@ -689,10 +690,12 @@ void launch_dm_solve(Engine &E) {
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     c.attrs = &at;
     c.numAttrs = 1;
-    if (mixed)
-        cudaLaunchKernelEx(&c, k_dm_solve<float>, kp, a, rows);
+    if (!mixed)
+        cudaLaunchKernelEx(&c, k_dm_solve<double, false>, kp, a, rows);
+    else if (kp.model == 2)
+        cudaLaunchKernelEx(&c, k_dm_solve<float, true>, kp, a, rows);
     else
-        cudaLaunchKernelEx(&c, k_dm_solve<double>, kp, a, rows);
+        cudaLaunchKernelEx(&c, k_dm_solve<float, false>, kp, a, rows);
     E.nlaunch += 2;
 }
 
@@ -840,13 +843,11 @@ void dm_init(Engine &E) {
     a.tables = reinterpret_cast<const int4 *>(base);
     a.M = base + head;
     build_attr(a, mixed);
-    if (mixed)
-        cudaFuncSetAttribute(k_dm_solve<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim);
-    else
-        cudaFuncSetAttribute(k_dm_solve<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim);
+    const void *solve = !mixed ? (const void *)k_dm_solve<double, false> : kp.model == 2 ? (const void *)k_dm_solve<float, true> : (const void *)k_dm_solve<float, false>;
+    cudaFuncSetAttribute(solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim);
     if (!mixed) {
         // clusters of 16 are beyond the portable size: as many as the device says it holds at once
-        cudaFuncSetAttribute(k_dm_solve<double>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        cudaFuncSetAttribute(solve, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         cudaLaunchConfig_t c = {};
         c.gridDim = dim3(16);
         c.blockDim = dim3(DM_NT);
@@ -858,7 +859,7 @@ void dm_init(Engine &E) {
         c.attrs = &at;
         c.numAttrs = 1;
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, k_dm_solve<double>, &c) == cudaSuccess) a.c16 = n;
+        if (cudaOccupancyMaxActiveClusters(&n, solve, &c) == cudaSuccess) a.c16 = n;
         cudaGetLastError();
     }
 }
